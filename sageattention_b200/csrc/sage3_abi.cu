@@ -102,7 +102,7 @@ sage3::PartsPtr one_part(const void* p) {
     return r;
 }
 
-int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, float* debug, void* stream,
+int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, void* stream,
               const Sage3Carry* carry = nullptr, const int32_t* cu_q = nullptr, const int32_t* cu_k = nullptr) {
     Sage3Workspace w;
     int rc = layout(desc, &w);
@@ -146,11 +146,6 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.status = reinterpret_cast<int*>(base + w.status) + kAttnStatusWord;
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
     a.cu_q = cu_q; a.cu_k = cu_k;
-#ifdef SAGE3_DEV_TRACE
-    a.debug = debug;
-#else
-    (void)debug;
-#endif
     int drv = 0;
     return sage3::launch_attn(a, st, &drv) == cudaSuccess ? SAGE3_OK : SAGE3_E_CUDA;
 }
@@ -323,7 +318,7 @@ SAGE3_API int sage3_fwd_varlen(const Sage3Desc* desc, const int32_t* cu_seqlens_
     if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(cu_seqlens_q, 4) || !aligned(cu_seqlens_k, 4)) return SAGE3_E_ALIGN;
     const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, cu_seqlens_q, cu_seqlens_k);
     if (rc != SAGE3_OK) return rc;
-    return attn_impl(desc, ws, one_part(out), lse, nullptr, stream, nullptr, cu_seqlens_q, cu_seqlens_k);
+    return attn_impl(desc, ws, one_part(out), lse, stream, nullptr, cu_seqlens_q, cu_seqlens_k);
 }
 
 SAGE3_API int sage3_prepass_kmean(const Sage3Desc* desc, const void* q, const void* k, const void* v, const void* km, void* ws,
@@ -346,7 +341,7 @@ SAGE3_API int sage3_prepass_parts(const Sage3Desc* desc, const Sage3Parts* q, co
 
 SAGE3_API int sage3_attn_fwd_carry(const Sage3Desc* desc, void* ws, const Sage3Carry* carry, void* out, float* lse, void* stream) {
     if (!carry) return SAGE3_E_NULL;
-    return attn_impl(desc, ws, one_part(out), lse, nullptr, stream, carry);
+    return attn_impl(desc, ws, one_part(out), lse, stream, carry);
 }
 
 SAGE3_API int sage3_attn_fwd_parts(const Sage3Desc* desc, void* ws, const Sage3Parts* out, float* lse, void* stream) {
@@ -354,7 +349,7 @@ SAGE3_API int sage3_attn_fwd_parts(const Sage3Desc* desc, void* ws, const Sage3P
     sage3::PartsPtr op;
     const int rc = to_parts(out, desc->Nq, &op);
     if (rc != SAGE3_OK) return rc;
-    return attn_impl(desc, ws, op, lse, nullptr, stream);
+    return attn_impl(desc, ws, op, lse, stream);
 }
 
 // ---- memory that other processes of the node can map (for the peer-to-peer form of sequence parallelism) ----------
@@ -390,15 +385,8 @@ SAGE3_API int sage3_shared_free(void* ptr) {
 }
 
 SAGE3_API int sage3_attn_fwd(const Sage3Desc* desc, void* ws, void* out, float* lse, void* stream) {
-    return attn_impl(desc, ws, one_part(out), lse, nullptr, stream);
+    return attn_impl(desc, ws, one_part(out), lse, stream);
 }
-
-#ifdef SAGE3_DEV_TRACE
-// development builds only (not declared in the public header): attention with the instrumentation dump
-SAGE3_API int sage3_attn_fwd_debug(const Sage3Desc* desc, void* ws, void* out, float* debug, void* stream) {
-    return attn_impl(desc, ws, one_part(out), nullptr, debug, stream);
-}
-#endif
 
 SAGE3_API int sage3_fwd(const Sage3Desc* desc, const void* q, const void* k, const void* v, void* ws, void* out, float* lse,
               void* stream) {

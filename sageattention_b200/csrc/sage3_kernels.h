@@ -52,9 +52,6 @@ struct AttnArgs {
     int causal_shift;               // key j visible to query i iff j <= i + causal_shift (Nk - Nq unless the caller offsets it)
     const int* prepass_status;      // the pre-pass's status word (non-zero: the workspace is incomplete, do nothing)
     const int *cu_q, *cu_k;         // packed variable-length sequences, as in PrepassArgs (nullptr: uniform lengths)
-#ifdef SAGE3_DEV_TRACE
-    float* debug;                   // development dump of the first CTA; nullptr in normal use
-#endif
 };
 
 // Encodes a tensor map over a byte tensor [n2][n1][n0] (n0 contiguous) with box [1][b1][b0]; swizzle: 0 none, 1 32 B, 2 64 B,
