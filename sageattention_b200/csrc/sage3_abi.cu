@@ -77,7 +77,8 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 
 // Status words: [0, 32) belong to the pre-pass, [32, 64) to the attention kernel.  Each stage clears its own half only,
 // so a wait the pre-pass gave up on is still there after the attention launch (whose CTAs read it and exit at once).
-constexpr int kStatusWords = 64, kAttnStatusWord = 32;
+// Behind them (the region is 1 024 bytes) lies the attention kernel's work counter, cleared with its half.
+constexpr int kStatusWords = 64, kAttnStatusWord = 32, kUnitCounterWord = 64;
 
 // checks a Sage3Parts argument and converts it; `align`: required alignment of every base pointer
 int to_parts(const Sage3Parts* in, int64_t rows_total, sage3::PartsPtr* out) {
@@ -122,7 +123,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     if (rc != SAGE3_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    if (cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0, (kStatusWords - kAttnStatusWord) * sizeof(int32_t), st) !=
+    if (cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0, (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st) !=
         cudaSuccess)
         return SAGE3_E_CUDA;
     sage3::AttnArgs a;
@@ -144,6 +145,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.carry_o_out = carry ? carry->o_out : nullptr; a.carry_m_out = carry ? carry->m_out : nullptr; a.carry_l_out = carry ? carry->l_out : nullptr;
     a.causal_shift = (carry && carry->use_causal_shift) ? carry->causal_shift : desc->Nk - desc->Nq;
     a.status = reinterpret_cast<int*>(base + w.status) + kAttnStatusWord;
+    a.unit_counter = reinterpret_cast<int*>(base + w.status) + kUnitCounterWord;
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
     a.cu_q = cu_q; a.cu_k = cu_k;
     int drv = 0;

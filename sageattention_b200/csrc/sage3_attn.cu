@@ -1,17 +1,18 @@
 // Block-scaled FP4 attention for sm_100a: TMA-staged E2M1 tiles, tcgen05 NVFP4 MMAs with the S and O
 // accumulators in tensor memory, exp2 online softmax, P re-quantized to NVFP4 before the PV MMA.
 //
-// One CTA per PAIR of 128-row query tiles of one head; every K / V^T stage in shared memory serves both tiles.  The
-// CTA's work is one stream of items (key block, tile), the two tiles in turn.  Six warpgroups (setmaxnreg moves
-// registers to the softmax warpgroups):
-//   warp 0       TMA producer (one lane): both Q tiles once, then K (+ one delta_s row per tile) / V^T / scale atoms per block
+// One CTA per SM; each draws units of work from a counter.  A unit is a PAIR of 128-row query tiles of one head (every K / V^T
+// stage in shared memory serves both tiles), a stream of items (key block, tile), the two tiles in turn; all pipelines run on
+// from unit to unit.  Six warpgroups (setmaxnreg moves registers to the softmax warpgroups):
+//   warp 0       draws and publishes the units; TMA producer: Q tiles, then K (+ one delta_s row per tile) / V^T / scale atoms per block
 //   warps 1, 3   Q K^T MMA issuers, for keys [0, 64) and [64, 128) of every item; warp 1 owns the tensor-memory allocation
 //   warp 2       P V MMA issuer
 //   warps 4-19   four softmax groups of four warps; group g takes the items g, g + 4, ...  A thread owns one row of the block
 //                and walks its 128 keys in two halves of 64 (the scores of a half live in registers).
 //   warps 20-23  O rescale ("correction"), one warp per tensor-memory lane quarter: when a row of the quarter moved
 //                its maximum, the warp multiplies the 32 O rows of its quarter by their factors before the block's
-//                P V MMA is issued; it also keeps the running row sums.  The softmax warps never touch O inside the loop.
+//                P V MMA is issued; it also keeps the running row sums and writes O / l while the softmax groups are
+//                already at work on the next unit.
 // Per half a softmax thread pulls its 64 scores out of tensor memory (the S buffer is free again at once) and runs the
 // exp2 pass microblock by microblock, the maxima of the next microblock found under the exponentials of the current one:
 // with E = P~ / sf = 6 * 2^((S - bm) s), the exp2 values and FP4 codes of a microblock depend on the maximum bm of that
@@ -20,9 +21,12 @@
 // nothing else connects the groups: four independent chains per scheduler, a quarter of an item apart.
 // What bounds it: the exp2 unit (16 results per clock and SM: 1 096 cycles per 128 x 128 block with the exponentials of the
 // scales) and, next to it, the instruction latency of the softmax warps; the tensor pipe needs 580 cycles.  Measured (B = 2,
-// H = 32, N = 16 384): 1 545 cycles per block at D = 128 and 1 525 at D = 64, the exp2 unit 77 % busy.  (With a row shared by two
-// threads and all warps of a tile in step, as this kernel was before: 1 640 and 1 590.)  Halves of 64 keys because a thread's
-// registers hold 64 scores, and because tensor memory has room for three 64-key buffers next to two O tiles at D = 128.
+// H = 32, N = 16 384): 1 525 cycles per block at D = 128 and 1 490 at D = 64, the exp2 unit 77 % busy.  (With a row shared by two
+// threads and all warps of a tile in step, as this kernel was first: 1 640 and 1 590.)  Units in place of one CTA per pair took the
+// drain and refill of the pipeline, 10 us per pair, out: B = 2, H = 32, N = 8 192 causal 960 -> 776 us, B = 4, H = 32, N = 1 024
+// 99 -> 77 us, two key blocks per tile (B = 2, H = 48, 17 550 queries x 226 keys, D = 64) 483 -> 250 us.
+// Halves of 64 keys because a thread's registers hold 64 scores, and because tensor memory has room for three 64-key buffers
+// next to two O tiles at D = 128.
 
 // Arithmetic follows (paths inside the reference project, sageattention3_blackwell/sageattn3/blackwell/...):
 //   mainloop_tma_ws.h:509, 532-551, 865     KV blocks are walked from the last to the first
@@ -48,7 +52,9 @@ constexpr float kLog2Of6 = 2.584962500721156f;
 constexpr float kPScaleLog2 = -11.392317422778762f;   // log2(1 / (448 * 6)), softmax_fused.h:33
 
 struct AttnParams {
-    int Hq, Hkv, Nq, Nk, nqt, nkb, nqm;   // nqt = query tiles per head, nkb = KV blocks per head
+    int BHq, Hq, Hkv, Nq, Nk, nqt, nkb, nqm;   // nqt = query tiles per head, nkb = KV blocks per head
+    int units, whole_units;             // units of work; those from whole_units on are single query tiles instead of pairs
+    int* unit_counter;                  // zero at launch: next unit after the first gridDim.x
     float sm_scale_log2;
     const float* sm_scale_per_head;
     const uint8_t *q_sf, *k_sf, *v_sf;
@@ -68,9 +74,11 @@ struct AttnParams {
     const int *cu_q, *cu_k;             // packed variable-length sequences (VARLEN kernels): entry b owns rows cu[b] .. cu[b + 1]
 };
 
+constexpr int kUnitRing = 4;
+
 template <int D>
 struct Cfg {
-    static constexpr int kStages = (D == 128) ? 5 : 8;        // K and V^T stages, each shared by the two query tiles
+    static constexpr int kStages = (D == 128) ? 4 : 8;        // K and V^T stages, each shared by the two query tiles
     static constexpr int kThreads = 768;                      // 6 warpgroups, see the kernel
     // S buffers of 128 rows x 64 keys: a rotation for the first halves of the items and one for the second halves
     static constexpr int kSBufs0 = 2, kSBufs1 = (D == 128) ? 1 : 2, kSBufs = kSBufs0 + kSBufs1;
@@ -82,12 +90,12 @@ struct Cfg {
     static constexpr int kDeltaBytes = 256;
     static constexpr int kPBytes = 8192;
     // shared-memory map (bytes from a 1024-aligned base)
-    static constexpr int oQ = 0;                              // [tile] 8192
-    static constexpr int oK = oQ + 2 * 8192;
+    static constexpr int oQ = 0;                              // [buffer][tile] 8192
+    static constexpr int oK = oQ + 4 * 8192;
     static constexpr int oV = oK + kStages * kKBytes;
     static constexpr int oP = oV + kStages * kVBytes;            // [slot] 8192
-    static constexpr int oSfQ = oP + 8 * kPBytes;             // [tile] 1024
-    static constexpr int oSfK = oSfQ + 2 * 1024;
+    static constexpr int oSfQ = oP + 8 * kPBytes;             // [buffer][tile] 1024
+    static constexpr int oSfK = oSfQ + 4 * 1024;
     static constexpr int oSfV = oSfK + kStages * 1024;
     static constexpr int oSfP = oSfV + kStages * 1024;        // [slot] 1024
     static constexpr int kDeltaPitch = 512;                   // 256 B of delta_s + 256 B that stay zero
@@ -96,12 +104,14 @@ struct Cfg {
     static constexpr int oStat = oOnes + 4096;                // float2 [slot][128 rows]: running maximum, rescale factor
     static constexpr int oSum = oStat + 8192;                 // float2 [slot][128 rows]: row sums of the two key halves of a block
     static constexpr int oL = oSum + 8192;                    // float2 [tile][128 rows]: running row sums of the two key halves
-    static constexpr int oBar = oL + 2048;
-    static constexpr int kNumBars = 2 + 4 * kStages + kSBufs + 8 + 7 * 8 + 8;
-    static constexpr int oMisc = oBar + kNumBars * 8;
+    static constexpr int oM = oL + 2048;                      // float [tile][128 rows]: running maximum
+    static constexpr int oBar = oM + 1024;
+    static constexpr int kNumBars = 4 + 4 * kStages + kSBufs + 8 + 7 * 8 + 2 * kUnitRing;
+    static constexpr int oUnit = (oBar + kNumBars * 8 + 15) / 16 * 16;      // descriptors of the units being worked on
+    static constexpr int oMisc = oUnit + kUnitRing * 64;
     static constexpr int kSmemBytes = oMisc + 64 + 1024;      // + slack for the manual 1024-byte alignment
-    // tensor-memory columns: the S buffers, one O accumulator per tile, scale factors (K: one copy per issuer)
-    static constexpr uint32_t cS = 0, cO = 64 * kSBufs, cSfQ = cO + 2 * D, cSfK = cSfQ + 16, cSfV = cSfK + 16, cSfP = cSfV + 8;
+    // tensor-memory columns: the S buffers, one O accumulator per tile, scale factors (Q, K: one copy per issuer)
+    static constexpr uint32_t cS = 0, cO = 64 * kSBufs, cSfQ = cO + 2 * D, cSfK = cSfQ + 32, cSfV = cSfK + 16, cSfP = cSfV + 8;
     static_assert(cSfP + 8 <= 512, "tensor memory");
     static constexpr uint64_t kSwzQK = (D == 128) ? kSwz64 : kSwz32;
     static constexpr uint32_t kSboQK = (D == 128) ? 512 : 256;
@@ -121,9 +131,80 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 // Wait executed by a whole converged warp; the verdict is made warp-uniform so that no lane leaves a loop alone.
+template <bool kBackoff = false>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-    const bool ok = mbar_wait(bar, parity, abort_flag, status, code);
+    const bool ok = mbar_wait<kBackoff>(bar, parity, abort_flag, status, code);
     return __all_sync(0xffffffffu, ok);
+}
+
+// One unit of work of a CTA: one or two query tiles of one head, walked over their key blocks.
+struct __align__(16) Unit {
+    // The unit is a stream of (block step jj, tile t) items, s = 0 ... ns - 1; with sd = s + d, t = sd & two and jj = sd >> two: two
+    // tiles alternate (d = 1: under a causal mask tile 1 may start one block before tile 0), a single tile walks alone.
+    int ns, two, d;               // ns < 0: no more units
+    int nbmax;                    // the unit walks key block n = nbmax - 1 ... 0
+    int mt0, nv;                  // first query tile, number of tiles
+    int Nq, Nk, shift;            // lengths of this batch entry; key j is visible to query i iff j <= i + shift
+    int nb[2];                    // key blocks per tile
+    int bhq, hq, bhkv;
+    int64_t out_base;
+};
+
+// Unit number u of the launch; false when it is empty (beyond a short sequence of a packed batch).
+// Order: without a mask pairs of tiles of one head are neighbours (its K and V are shared in L2); under a causal mask the
+// pairs with the most keys of all heads come first, so that the short ones level out the end of the launch.
+template <bool CAUSAL, bool VARLEN>
+__device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
+    const int npair = (p.nqt + 1) >> 1;
+    int pair = u, half = -1;
+    if (u >= p.whole_units) {                      // the last units are single tiles
+        pair = p.whole_units + ((u - p.whole_units) >> 1);
+        half = (u - p.whole_units) & 1;
+    }
+    int pr;
+    if (CAUSAL) {
+        pr = npair - 1 - pair / p.BHq;
+        w.bhq = pair % p.BHq;
+    } else {
+        w.bhq = pair / npair;
+        pr = pair % npair;
+    }
+    w.mt0 = 2 * pr + (half > 0 ? 1 : 0);
+    const int b = w.bhq / p.Hq;
+    w.hq = w.bhq % p.Hq;
+    w.bhkv = b * p.Hkv + w.hq / (p.Hq / p.Hkv);
+    // p.Nq, p.Nk, p.nqt, p.nkb stay the strides of the workspace layouts; with packed variable-length sequences they are the
+    // maxima and the entry's own lengths come from the cu arrays.
+    w.Nq = p.Nq;
+    w.Nk = p.Nk;
+    w.shift = p.causal_shift;
+    w.out_base = b * p.os0;
+    int nqt = p.nqt, nkb = p.nkb;
+    if constexpr (VARLEN) {
+        const int q0 = p.cu_q[b], k0 = p.cu_k[b];
+        w.Nq = min(max(p.cu_q[b + 1] - q0, 0), p.Nq);
+        w.Nk = min(max(p.cu_k[b + 1] - k0, 0), p.Nk);
+        nqt = (w.Nq + kBlock - 1) / kBlock;
+        nkb = (w.Nk + kBlock - 1) / kBlock;
+        w.shift = w.Nk - w.Nq;
+        w.out_base = (int64_t)q0 * p.os2;
+    }
+    w.nv = min(half < 0 ? 2 : 1, nqt - w.mt0);
+    if (w.nv <= 0) return false;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        int nb = nkb;
+        if (CAUSAL) {
+            const int max_key = min(w.Nk - 1, (w.mt0 + t) * kBlock + kBlock - 1 + w.shift);
+            nb = max_key < 0 ? 0 : max_key / kBlock + 1;
+        }
+        w.nb[t] = t < w.nv ? nb : 0;
+    }
+    w.nbmax = max(w.nb[0], w.nb[1]);
+    w.two = w.nv == 2 ? 1 : 0;
+    w.d = w.two ? w.nb[1] - w.nb[0] : 0;
+    w.ns = w.nb[0] + w.nb[1];
+    return true;
 }
 
 template <int D, bool CAUSAL, typename OutT, bool VARLEN>
@@ -141,66 +222,30 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // barriers
     const uint32_t bars = uniform(sbase + C::oBar);
     auto bar = [&](int i) { return bars + 8u * i; };
-    constexpr int bQ = 0, bSQ = 1, bKF = 2, bKE = bKF + S, bVF = bKE + S, bVE = bVF + S, bSF = bVE + S, bSE = bSF + 8, bM = bSE + C::kSBufs,
-                  bPF = bM + 32, bPV = bPF + 8, bOS = bPV + 8, bL = bOS + 8;
+    constexpr int bQF = 0, bQE = 2, bKF = 4, bKE = bKF + S, bVF = bKE + S, bVE = bVF + S, bSF = bVE + S, bSE = bSF + 8, bM = bSE + C::kSBufs,
+                  bPF = bM + 32, bPV = bPF + 8, bOS = bPV + 8, bWF = bOS + 8, bWE = bWF + kUnitRing, bEnd = bWE + kUnitRing;
+    static_assert(bEnd == C::kNumBars, "barriers");
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + C::oMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + C::oMisc + 8);
-
-    // CTA -> (batch*head, pair of query tiles); heavier causal pairs are scheduled first
-    const int npair = (p.nqt + 1) >> 1;
-    const int bhq = blockIdx.x / npair;
-    int pr = blockIdx.x % npair;
-    if (CAUSAL) pr = npair - 1 - pr;
-    const int mt0 = 2 * pr;
-    const int b = bhq / p.Hq, hq = bhq % p.Hq;
-    const int bhkv = b * p.Hkv + hq / (p.Hq / p.Hkv);
-    // Lengths of this batch entry.  p.Nq, p.Nk, p.nqt, p.nkb stay the strides of the workspace layouts; with packed
-    // variable-length sequences they are the maxima and the entry's own lengths come from the cu arrays.
-    int Nq = p.Nq, Nk = p.Nk, nqt = p.nqt, nkb = p.nkb, shift = p.causal_shift;
-    int64_t out_base = b * p.os0;
-    if constexpr (VARLEN) {
-        const int q0 = p.cu_q[b], k0 = p.cu_k[b];
-        Nq = min(max(p.cu_q[b + 1] - q0, 0), p.Nq);
-        Nk = min(max(p.cu_k[b + 1] - k0, 0), p.Nk);
-        nqt = (Nq + kBlock - 1) / kBlock;
-        nkb = (Nk + kBlock - 1) / kBlock;
-        shift = Nk - Nq;
-        out_base = (int64_t)q0 * p.os2;
-    }
-    const int nv = (mt0 + 1 < nqt) ? 2 : (VARLEN && mt0 >= nqt ? 0 : 1);   // query tiles this CTA really has
-    // an earlier CTA of this launch gave up, or the pre-pass did (the workspace is then incomplete)
-    const bool dead_launch = (*reinterpret_cast<volatile int*>(p.status) != 0) || (*reinterpret_cast<const volatile int*>(p.prepass_status) != 0);
-    // KV blocks of tile t: [0, nbt[t]); the CTA walks block n = nbmax - 1 ... 0.  Under a causal mask tile 1 may start one
-    // block earlier than tile 0 (their rows differ by one block), never more.
-    int nbt[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        int nb = nkb;
-        if (CAUSAL) {
-            const int max_key = min(Nk - 1, (mt0 + t) * kBlock + kBlock - 1 + shift);
-            nb = max_key < 0 ? 0 : max_key / kBlock + 1;
-        }
-        nbt[t] = (dead_launch || t >= nv) ? 0 : nb;
-    }
-    const int nbmax = uniform(max(nbt[0], nbt[1]));
-    // The work is one stream of (block step jj, tile t) items, s = 0 ... ns - 1: with two tiles they alternate, sd = s + d,
-    // t = sd & 1, jj = sd >> 1 (d = 1: the stream starts with tile 1 alone); with one tile jj = s.
-    const int two = uniform(nv == 2 ? 1 : 0);
-    const int d = uniform(two ? nbt[1] - nbt[0] : 0);
-    const int ns = uniform(nbt[0] + nbt[1]);
 
     // One barrier per thread: the number of arrivals that completes a phase.
     if (threadIdx.x < C::kNumBars) {
         const int i = threadIdx.x;
         uint32_t count = 1;                                      // copies landed, MMAs complete, one warp's statistics
-        if (i >= bKE && i < bKE + S) count = 2;                  // K stage free: both Q K^T issuers are done with it
+        if (i >= bQE && i < bKF) count = 2;                      // Q buffer free: both Q K^T issuers are done with it
+        if (i >= bKE && i < bKE + S) count = 2;                  // K stage free: likewise
         if (i >= bSE && i < bM) count = 4;                       // S buffer free: the four warps of its group hold the scores
         if (i >= bPF && i < bPV) count = 4;                      // P, its scales and the row sums written
-        if (i >= bOS && i < bL) count = 4;                       // the correction warps are done with O (and have seen P written)
+        if (i >= bOS && i < bWF) count = 4;                               // the correction warps are done with O (and have seen P written)
+        if (i >= bWE) count = C::kThreads / 32 - 1;              // unit descriptor free: every warp but the producer has finished the unit
         mbar_init(bar(i), count);
         mbar_fence_init();
     }
-    if (threadIdx.x == 0) *abort_flag = 0;
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        // an earlier CTA of this launch gave up, or the pre-pass did (the workspace is then incomplete): nothing is done
+        tmem_slot[1] = (*reinterpret_cast<volatile int*>(p.status) != 0) || (*reinterpret_cast<const volatile int*>(p.prepass_status) != 0);
+    }
     // delta_s stages: the 256 bytes behind each row stay zero for the whole kernel; ones tile:
     // [k chunk][row group][8 rows][16 bytes], 1.0 in element 0 of every row of chunk 0
     {
@@ -222,172 +267,277 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = uniform(*tmem_slot);
-
-    const float sl2 = p.sm_scale_per_head ? p.sm_scale_per_head[hq] * 1.4426950408889634f : p.sm_scale_log2;
+    const uint32_t tmem = uniform(tmem_slot[0]);
+    const bool dead = uniform(tmem_slot[1]) != 0;
     const bool carry_in = (p.carry_o_in != nullptr);
-    if (carry_in) {
-        // resume: O continues from the state an earlier call left (its key range came later in the walk)
-        if (warp >= 4 && warp < 4 + 4 * 2) {
-            const int t = (warp >> 2) - 1, r = (warp & 3) * 32 + lane, grow = (mt0 + t) * kBlock + r;
-            const bool live = t < nv && grow < Nq && !dead_launch;
-            const float* src = p.carry_o_in + ((size_t)bhq * p.Nq + grow) * D;
-            for (int cc = 0; cc < D / 16; ++cc) {
-                float o[16];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 v4 = live ? *reinterpret_cast<const float4*>(src + cc * 16 + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    o[4 * i] = v4.x; o[4 * i + 1] = v4.y; o[4 * i + 2] = v4.z; o[4 * i + 3] = v4.w;
-                }
-                tmem_st16(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::cO + t * D + cc * 16, o);
-            }
-            tc_wait_st();
-        }
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-    }
 
     // Register budget: 768 threads start with 80 registers each, and that allocation (61 440) is all the CTA can
-    // ever hold: 128 x kRoleRegs for warpgroup 0 (three single-lane roles) + 128 x kCorrRegs for the correction
-    // warpgroup + 512 x 104 for the softmax warpgroups.  (An increase beyond the launch allocation would wait forever.)
-    constexpr int kRoleRegs = (D == 64) ? 24 : 32, kCorrRegs = 64 - kRoleRegs;
+    // ever hold: 128 x kRoleRegs for warpgroup 0 (the copy and MMA roles) + 128 x kCorrRegs for the correction
+    // warpgroup + 512 x 96 for the softmax warpgroups (32 / 32 / 104 and 24 / 40 / 104 spill in the roles: 1 to 3 % slower).  (An increase beyond the launch allocation would wait forever.)
+    constexpr int kRoleRegs = 48, kCorrRegs = 48;
+    // A CTA runs unit after unit (the grid is one CTA per SM): the producer draws the next unit's number from a counter and
+    // publishes the unit in shared memory, so the loads, scores and exponentials of the next unit fill in while the last one
+    // drains, and uneven units (causal masks, packed batches) level out.
+    const Unit* units = reinterpret_cast<const Unit*>(sgen + C::oUnit);
+    auto next_unit = [&](int i) -> const Unit* {       // nullptr: none, or a wait gave up
+        const int e = i % kUnitRing;
+        if (!warp_wait(bar(bWF + e), (i / kUnitRing) & 1, abort_flag, p.status, kWaitUnit)) return nullptr;
+        return units[e].ns < 0 ? nullptr : &units[e];
+    };
+    auto unit_done = [&](int i) { warp_arrive(bar(bWE + i % kUnitRing), lane); };
+    int base = 0;                 // items of the units before this one: groups, slots and phases count through all units
     if (warp >= 20) {
       reg_dealloc<kCorrRegs>();
-      // ------------------------------------------------------------------ O rescale (correction), one warp per lane quarter
+      // ------------------------------------------------------------------ O rescale (correction) and output, one warp per lane quarter
       // Also keeps the running row sums: l = l alpha + (sum over the block), for each half of the keys.
       const int quarter = warp & 3, row = quarter * 32 + lane;
       const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-      const float2* stat = reinterpret_cast<const float2*>(sgen + C::oStat);
-      const float2* sum = reinterpret_cast<const float2*>(sgen + C::oSum);
-      float2* l_s = reinterpret_cast<float2*>(sgen + C::oL);
-      for (int t = 0; t < 2; ++t) {
-          const int grow = (mt0 + t) * kBlock + row;
-          const bool from = p.carry_l_in != nullptr && t < nv && grow < Nq && !dead_launch;
-          l_s[t * 128 + row] = from ? *reinterpret_cast<const float2*>(p.carry_l_in + 2 * ((size_t)bhq * p.Nq + grow)) : make_float2(0.f, 0.f);
-      }
-      bool ok = true;
-      for (int s = 0; s < ns; ++s) {
-          const int g = s & 7, ph = (s >> 3) & 1;
-          const int t = two ? (s + d) & 1 : 0;
-          const bool first = s <= two;                              // the tile's first block
-          if (!warp_wait(bar(bM + g * 4 + quarter), ph, abort_flag, p.status, kWaitAlpha)) { ok = false; break; }
-          const float alpha = stat[g * 128 + row].y;
-          // the first block has nothing to rescale unless the accumulator was carried in
-          if ((!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
-              // the P V MMA of the tile's previous block must have landed first
-              if (!first) {
-                  const int sp = s - 1 - two;
-                  if (!warp_wait(bar(bPV + (sp & 7)), (sp >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
+      const float2* stat = reinterpret_cast<const float2*>(sgen + C::oStat) + row;
+      const float2* sum = reinterpret_cast<const float2*>(sgen + C::oSum) + row;
+      float2* l_s = reinterpret_cast<float2*>(sgen + C::oL) + row;
+      float* m_s = reinterpret_cast<float*>(sgen + C::oM) + row;
+      const Unit* u;
+      bool ok = !dead;
+      for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
+          const Unit& w = *u;
+          const int ns = w.ns, two = w.two, d = w.d;
+          for (int t = 0; t < w.nv; ++t) {
+              l_s[t * 128] = make_float2(0.f, 0.f);
+              m_s[t * 128] = -INFINITY;
+              const int grow = (w.mt0 + t) * kBlock + row;
+              if (carry_in && grow < w.Nq) {
+                  const size_t crow = (size_t)w.bhq * p.Nq + grow;
+                  l_s[t * 128] = *reinterpret_cast<const float2*>(p.carry_l_in + 2 * crow);
+                  m_s[t * 128] = p.carry_m_in[crow];
+              }
+              if (carry_in) {
+                  // resume: O continues from the state an earlier call left (its key range came later in the walk)
+                  const float* src = p.carry_o_in + ((size_t)w.bhq * p.Nq + min(grow, w.Nq - 1)) * D;
+                  for (int c = 0; c < D; c += 16) {
+                      float o[16];
+#pragma unroll
+                      for (int q = 0; q < 4; ++q) {
+                          const float4 v4 = *reinterpret_cast<const float4*>(src + c + 4 * q);
+                          o[4 * q] = v4.x; o[4 * q + 1] = v4.y; o[4 * q + 2] = v4.z; o[4 * q + 3] = v4.w;
+                      }
+                      tmem_st16(tmem + lane_addr + C::cO + t * D + c, o);
+                  }
+                  tc_wait_st();
+              }
+          }
+          for (int s = 0; s < ns; ++s) {
+              const int sg = base + s, slot = sg & 7, ph = (sg >> 3) & 1;
+              const int t = (s + d) & two;
+              const bool first = s <= two;                            // the tile's first block
+              if (!warp_wait(bar(bM + slot * 4 + quarter), ph, abort_flag, p.status, kWaitAlpha)) { ok = false; break; }
+              const float2 ma = stat[slot * 128];
+              const float alpha = ma.y;
+              // the first block has nothing to rescale unless the accumulator was carried in
+              if ((!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                  // the P V MMA of the tile's previous block must have landed first
+                  if (!first) {
+                      const int sp = sg - 1 - two;
+                      if (!warp_wait(bar(bPV + (sp & 7)), (sp >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
+                  }
+                  tc_fence_after();
+                  const uint64_t a2 = pack2f(alpha, alpha);
+                  const uint32_t o_addr = tmem + lane_addr + C::cO + t * D;
+#pragma unroll
+                  for (int cc = 0; cc < D / 16; ++cc) {
+                      float o0[16];
+                      tmem_ld16(o_addr + cc * 16, o0);
+                      tc_wait_ld();
+#pragma unroll
+                      for (int q = 0; q < 8; ++q)
+                          unpack2f(mul2(pack2f(o0[2 * q], o0[2 * q + 1]), a2), o0[2 * q], o0[2 * q + 1]);
+                      tmem_st16(o_addr + cc * 16, o0);
+                  }
+                  tc_wait_st();
+              }
+              tc_fence_before();
+              // P V issue waits for this warpgroup only, so its arrival also stands for "P is written"
+              if (!warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
+              const float2 rs = sum[slot * 128];
+              warp_arrive(bar(bOS + slot), lane);
+              float2 l = l_s[t * 128];
+              l.x = fmaf(l.x, alpha, rs.x);
+              l.y = fmaf(l.y, alpha, rs.y);
+              l_s[t * 128] = l;
+              m_s[t * 128] = ma.x;
+          }
+          // ---------------------------------------------------------------- O / l of the unit's tiles
+          // (The accumulators belong to the next unit once this warpgroup arrives for its first items.)
+          for (int t = 0; ok && t < w.nv; ++t) {
+              const int grow = (w.mt0 + t) * kBlock + row;
+              const bool live = grow < w.Nq;
+              const bool have = w.nb[t] > 0 || carry_in;
+              if (w.nb[t] > 0) {
+                  const int sl = base + (w.two ? 2 * (w.nbmax - 1) + t - w.d : w.nb[t] - 1);       // the tile's last item
+                  if (!warp_wait(bar(bPV + (sl & 7)), (sl >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
               }
               tc_fence_after();
-              const uint64_t a2 = pack2f(alpha, alpha);
-              const uint32_t o_addr = tmem + lane_addr + C::cO + t * D;
-#pragma unroll
-              for (int cc = 0; cc < D / 16; ++cc) {
-                  float o0[16];
-                  tmem_ld16(o_addr + cc * 16, o0);
-                  tc_wait_ld();
-#pragma unroll
-                  for (int i = 0; i < 8; ++i)
-                      unpack2f(mul2(pack2f(o0[2 * i], o0[2 * i + 1]), a2), o0[2 * i], o0[2 * i + 1]);
-                  tmem_st16(o_addr + cc * 16, o0);
+              const float2 l2 = l_s[t * 128];
+              const float l_tot = l2.x + l2.y;
+              if (live && (p.lse != nullptr || p.carry_o_out != nullptr)) {
+                  const float m_fin = m_s[t * 128];
+                  const size_t crow = (size_t)w.bhq * p.Nq + grow;
+                  if (p.lse != nullptr) {
+                      // ln sum_k exp(scale * q.k): the kernel's row sum is 2688 * sum_k 2^((S_k - m) s) over the smoothed
+                      // scores S (delta_s included); K smoothing took scale * q.km out of every score of the row
+                      const float scale = p.sm_scale_per_head ? p.sm_scale_per_head[w.hq] : p.sm_scale;
+                      const float ms_fin = (m_fin == -INFINITY ? 0.f : m_fin) * (p.sm_scale_per_head ? scale * 1.4426950408889634f : p.sm_scale_log2);
+                      const float v = (ms_fin + __log2f(l_tot) + kPScaleLog2) * 0.6931471805599453f +
+                                      scale * p.qkm[(size_t)w.bhq * p.nqt * kBlock + grow];
+                      p.lse[crow] = (l_tot == 0.f) ? -INFINITY : v;
+                  }
+                  if (p.carry_o_out != nullptr) {
+                      p.carry_m_out[crow] = m_fin > kNoKey ? m_fin : -INFINITY;
+                      *reinterpret_cast<float2*>(p.carry_l_out + 2 * crow) = l2;
+                  }
               }
-              tc_wait_st();
+              const float inv_l = (l_tot == 0.f || l_tot != l_tot) ? 0.f : __frcp_rn(l_tot);
+              // the row's home: one output buffer, or the part that owns this token (another GPU's memory when the
+              // output goes straight back to the token shards of a sequence-parallel group: plain stores)
+              const int opart = (p.out_rows == 0) ? 0 : min(grow / p.out_rows, kMaxParts - 1);
+              OutT* orow = p.out[opart] == nullptr || !live ? nullptr
+                         : static_cast<OutT*>(p.out[opart]) + w.out_base + w.hq * p.os1 + (int64_t)(grow - opart * p.out_rows) * p.os2;
+              for (int c = 0; c < D; c += 16) {
+                  float o[16];
+                  if (have) {
+                      tmem_ld16(tmem + lane_addr + C::cO + t * D + c, o);
+                      tc_wait_ld();
+                  } else {
+#pragma unroll
+                      for (int q = 0; q < 16; ++q) o[q] = 0.f;
+                  }
+                  if (p.carry_o_out != nullptr && live) {
+#pragma unroll
+                      for (int q = 0; q < 4; ++q)
+                          *reinterpret_cast<float4*>(p.carry_o_out + ((size_t)w.bhq * p.Nq + grow) * D + c + 4 * q) =
+                              make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                  }
+                  if (orow != nullptr) {
+#pragma unroll
+                      for (int q = 0; q < 2; ++q) {
+                          uint4 v4;
+                          v4.x = pack2<OutT>(o[8 * q] * inv_l, o[8 * q + 1] * inv_l);
+                          v4.y = pack2<OutT>(o[8 * q + 2] * inv_l, o[8 * q + 3] * inv_l);
+                          v4.z = pack2<OutT>(o[8 * q + 4] * inv_l, o[8 * q + 5] * inv_l);
+                          v4.w = pack2<OutT>(o[8 * q + 6] * inv_l, o[8 * q + 7] * inv_l);
+                          *reinterpret_cast<uint4*>(orow + c + q * 8) = v4;
+                      }
+                  }
+              }
           }
-          tc_fence_before();
-          // P V issue waits for this warpgroup only, so its arrival also stands for "P is written"
-          if (!warp_wait(bar(bPF + g), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
-          const float2 rs = sum[g * 128 + row];
-          warp_arrive(bar(bOS + g), lane);
-          float2 l = l_s[t * 128 + row];
-          l.x = fmaf(l.x, alpha, rs.x);
-          l.y = fmaf(l.y, alpha, rs.y);
-          l_s[t * 128 + row] = l;
-      }
-      if (ok && !dead_launch) {
-          for (int t = 0; t < nv; ++t) {
-              const int grow = (mt0 + t) * kBlock + row;
-              if (p.carry_l_out != nullptr && grow < Nq)
-                  *reinterpret_cast<float2*>(p.carry_l_out + 2 * ((size_t)bhq * p.Nq + grow)) = l_s[t * 128 + row];
-              warp_arrive(bar(bL + t * 4 + quarter), lane);
-          }
+          unit_done(i);
+          base += ns;
       }
       __syncwarp();
     } else if (warp < 4) {
       reg_dealloc<kRoleRegs>();
       if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0 && nbmax > 0) {
-            mbar_expect_tx(bar(bQ), nv * (C::kQBytes + C::kSfQkBytes));
-            const uint16_t* dptr[2];
-            for (int t = 0; t < nv; ++t) {
-                tma_load_3d(sbase + C::oQ + t * 8192, &tm_q, bar(bQ), 0, (mt0 + t) * kBlock, bhq);
-                bulk_load(sbase + C::oSfQ + t * 1024, p.q_sf + ((size_t)bhq * p.nqt + mt0 + t) * C::kSfQkBytes,
-                          C::kSfQkBytes, bar(bQ));
-                const int drow = (p.nqm > 1) ? mt0 + t : 0;
-                dptr[t] = p.delta + ((size_t)bhq * p.nqm + drow) * ((size_t)p.nkb * kBlock);
+        int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
+        int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
+        bool ok = !dead;
+        while (ok) {
+            int next = 0;
+            if (lane == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
+            Unit w;
+            const bool more = u < p.units;
+            if (!more) w.ns = -1;
+            else if (!make_unit<CAUSAL, VARLEN>(p, u, w)) { u = uniform(next); continue; }
+            if (!warp_wait<true>(bar(bWE + k % kUnitRing), ((k / kUnitRing) & 1) ^ 1, abort_flag, p.status, kWaitUnit)) break;
+            if (lane == 0) {
+                *reinterpret_cast<Unit*>(sgen + C::oUnit + (k % kUnitRing) * 64) = w;
+                mbar_arrive(bar(bWF + k % kUnitRing));
             }
-            for (int jj = 0; jj < nbmax; ++jj) {
-                const int n = nbmax - 1 - jj, st = jj % S;
-                if (jj >= S && !mbar_wait<true>(bar(bKE + st), ((jj / S) - 1) & 1, abort_flag, p.status, kWaitKEmpty)) break;
-                mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + nv * C::kDeltaBytes);
-                tma_load_3d(sbase + C::oK + st * C::kKBytes, &tm_k, bar(bKF + st), 0, n * kBlock, bhkv);
-                bulk_load(sbase + C::oSfK + st * 1024, p.k_sf + ((size_t)bhkv * p.nkb + n) * C::kSfQkBytes,
-                          C::kSfQkBytes, bar(bKF + st));
-                for (int t = 0; t < nv; ++t)
-                    bulk_load(sbase + C::oDelta + (st * 2 + t) * C::kDeltaPitch, dptr[t] + (size_t)n * kBlock,
-                              C::kDeltaBytes, bar(bKF + st));
-                if (jj >= S && !mbar_wait<true>(bar(bVE + st), ((jj / S) - 1) & 1, abort_flag, p.status, kWaitVEmpty)) break;
-                mbar_expect_tx(bar(bVF + st), C::kVBytes + C::kSfVBytes);
-                tma_load_3d(sbase + C::oV + st * C::kVBytes, &tm_v, bar(bVF + st), n * 64, 0, bhkv);
-                bulk_load(sbase + C::oSfV + st * 1024, p.v_sf + ((size_t)bhkv * p.nkb + n) * C::kSfVBytes,
-                          C::kSfVBytes, bar(bVF + st));
+            ++k;
+            if (!more) break;
+            if (w.ns == 0) { u = uniform(next); continue; }
+            const int qb = kq & 1;                // Q buffer
+            if (!warp_wait<true>(bar(bQE + qb), ((kq >> 1) & 1) ^ 1, abort_flag, p.status, kWaitKEmpty)) break;
+            ++kq;
+            const uint16_t* dptr0 = p.delta + ((size_t)w.bhq * p.nqm + ((p.nqm > 1) ? w.mt0 : 0)) * ((size_t)p.nkb * kBlock);
+            const size_t dstep = (p.nqm > 1) ? (size_t)p.nkb * kBlock : 0;
+            if (lane == 0) {
+                mbar_expect_tx(bar(bQF + qb), w.nv * (C::kQBytes + C::kSfQkBytes));
+                for (int t = 0; t < w.nv; ++t) {
+                    tma_load_3d(sbase + C::oQ + (qb * 2 + t) * 8192, &tm_q, bar(bQF + qb), 0, (w.mt0 + t) * kBlock, w.bhq);
+                    bulk_load(sbase + C::oSfQ + (qb * 2 + t) * 1024, p.q_sf + ((size_t)w.bhq * p.nqt + w.mt0 + t) * C::kSfQkBytes,
+                              C::kSfQkBytes, bar(bQF + qb));
+                }
             }
+            for (int n = w.nbmax - 1; n >= 0; --n) {
+                if (!warp_wait<true>(bar(bKE + st), st_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
+                if (lane == 0) {
+                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + w.nv * C::kDeltaBytes);
+                    tma_load_3d(sbase + C::oK + st * C::kKBytes, &tm_k, bar(bKF + st), 0, n * kBlock, w.bhkv);
+                    bulk_load(sbase + C::oSfK + st * 1024, p.k_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfQkBytes,
+                              C::kSfQkBytes, bar(bKF + st));
+                    for (int t = 0; t < w.nv; ++t)
+                        bulk_load(sbase + C::oDelta + (st * 2 + t) * C::kDeltaPitch, dptr0 + t * dstep + (size_t)n * kBlock,
+                                  C::kDeltaBytes, bar(bKF + st));
+                }
+                if (!warp_wait<true>(bar(bVE + st), st_parity, abort_flag, p.status, kWaitVEmpty)) { ok = false; break; }
+                if (lane == 0) {
+                    mbar_expect_tx(bar(bVF + st), C::kVBytes + C::kSfVBytes);
+                    tma_load_3d(sbase + C::oV + st * C::kVBytes, &tm_v, bar(bVF + st), n * 64, 0, w.bhkv);
+                    bulk_load(sbase + C::oSfV + st * 1024, p.v_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfVBytes,
+                              C::kSfVBytes, bar(bVF + st));
+                }
+                __syncwarp();
+                if (++st == S) { st = 0; st_parity ^= 1; }
+            }
+            u = uniform(next);
         }
         __syncwarp();
       } else if (warp == 1 || warp == 3) {
         // ------------------------------------------------------------------ Q K^T MMA issuers
-        // The scores of a stream item are formed in two halves of 64 keys; warp 1 issues the first halves, warp 3 the second
+        // The scores of an item are formed in two halves of 64 keys; warp 1 issues the first halves, warp 3 the second
         // ones, each into its own S buffers (issuing one half takes a few hundred cycles next to busy softmax warps: one
         // issuer for both would be the slowest part of the pipeline).  The whole warp walks the loop and one elected lane
         // issues, so loop state and descriptors stay in uniform registers.
         const int h = warp >> 1;
-        if (ns > 0) {
-            constexpr uint32_t idesc_qk = make_idesc_nvfp4(64);
-            constexpr uint32_t idesc_delta = make_idesc_f16_bmn(64, std::is_same<OutT, __nv_bfloat16>::value);
-            // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
-            constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(16, kSwzNone);
-            const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo = sdesc_lo(sbase + C::oQ, 16);
-            const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 128, 16);
-            const uint32_t sfk_lo0 = sdesc_lo(sbase + C::oSfK, 0);
-            const uint32_t sfk_col = tmem + C::cSfK + 8 * h;        // the 128-key atoms; keys 64 .. 127 start two columns in
-            bool ok;
-            if (h == 0) {
-                ok = warp_wait(bar(bQ), 0, abort_flag, p.status, kWaitQFull);
-                if (ok && elect_one()) {
-                    for (int t = 0; t < nv; ++t)
+        constexpr uint32_t idesc_qk = make_idesc_nvfp4(64);
+        constexpr uint32_t idesc_delta = make_idesc_f16_bmn(64, std::is_same<OutT, __nv_bfloat16>::value);
+        // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
+        constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(16, kSwzNone);
+        const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo0 = sdesc_lo(sbase + C::oQ, 16), sfq_lo0 = sdesc_lo(sbase + C::oSfQ, 0);
+        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 128, 16);
+        const uint32_t sfk_lo0 = sdesc_lo(sbase + C::oSfK, 0);
+        // each issuer has its own copies of the scale factors in tensor memory, so that its MMAs and copies stay in one order
+        const uint32_t sfk_col = tmem + C::cSfK + 8 * h;        // the 128-key atoms; keys 64 .. 127 start two columns in
+        const uint32_t sfq_col0 = tmem + C::cSfQ + 16 * h;
+        const int nbuf = h == 0 ? C::kSBufs0 : C::kSBufs1, buf0 = h == 0 ? 0 : C::kSBufs0;
+        int buf = 0, buf_parity = 1;              // next S buffer; parity of its "empty" phase (a fresh barrier passes parity 1)
+        int st = 0, st_parity = 0;                // K stage
+        bool ok = !dead;
+        const Unit* u;
+        for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
+            const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
+            unit_done(i);
+            if (ns == 0) continue;
+            const int qb = k & 1;
+            if (!warp_wait(bar(bQF + qb), (k >> 1) & 1, abort_flag, p.status, kWaitQFull)) break;
+            ++k;
+            tc_fence_after();
+            if (elect_one()) {
+                for (int t = 0; t < nv; ++t)
 #pragma unroll
-                        for (int ks = 0; ks < D / 64; ++ks)
-                            tc_cp_sf(tmem + C::cSfQ + 8 * t + 4 * ks, make_sdesc(sbase + C::oSfQ + t * 1024 + ks * 512, 0, 128, kSwzNone));
-                    tc_commit(bar(bSQ));
-                }
-                __syncwarp();
-            } else {
-                ok = warp_wait(bar(bSQ), 0, abort_flag, p.status, kWaitQFull);
+                    for (int ks = 0; ks < D / 64; ++ks)
+                        tc_cp_sf(sfq_col0 + 8 * t + 4 * ks, sdesc(sfq_lo0 + (qb * 2 + t) * 64 + ks * 32, sdesc_hi(128, kSwzNone)));
             }
-            const int nbuf = h == 0 ? C::kSBufs0 : C::kSBufs1, buf0 = h == 0 ? 0 : C::kSBufs0;
-            int buf = 0, buf_parity = 1;              // next S buffer; parity of its "empty" phase (a fresh barrier passes parity 1)
-            int st = 0, st_parity = 0;                // K stage
-            for (int s = 0; ok && s < ns; ++s) {
-                const int t = two ? (s + d) & 1 : 0;
+            __syncwarp();
+            for (int s = 0; s < ns; ++s) {
+                const int t = (s + d) & two;
                 const bool opens = t == 0 || s == 0, closes = t == two;       // first / last item of its K block
-                if (opens && !warp_wait(bar(bKF + st), st_parity, abort_flag, p.status, kWaitKFull)) break;
-                if (!warp_wait(bar(bSE + buf0 + buf), buf_parity, abort_flag, p.status, kWaitSEmpty)) break;
+                if (opens && !warp_wait(bar(bKF + st), st_parity, abort_flag, p.status, kWaitKFull)) { ok = false; break; }
+                if (!warp_wait(bar(bSE + buf0 + buf), buf_parity, abort_flag, p.status, kWaitSEmpty)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t k_lo = k_lo0 + st * (C::kKBytes / 16), delta_lo = delta_lo0 + (st * 2 + t) * (C::kDeltaPitch / 16);
-                const uint32_t sfk_lo = sfk_lo0 + st * (1024 / 16), qt_lo = q_lo + t * (8192 / 16);
-                const uint32_t s_col = tmem + C::cS + 64 * (buf0 + buf), sfq_col = tmem + C::cSfQ + 8 * t;
+                const uint32_t sfk_lo = sfk_lo0 + st * (1024 / 16), q_lo = q_lo0 + (qb * 2 + t) * (8192 / 16);
+                const uint32_t s_col = tmem + C::cS + 64 * (buf0 + buf), sfq_col = sfq_col0 + 8 * t;
                 if (elect_one()) {
                     if (opens) {
 #pragma unroll
@@ -398,34 +548,40 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     tc_mma_f16(s_col, sdesc(ones_lo, hi_ones), sdesc(delta_lo, hi_delta), idesc_delta, false);
 #pragma unroll
                     for (int ks = 0; ks < D / 64; ++ks)
-                        tc_mma_nvfp4(s_col, sdesc(qt_lo + 2 * ks, hi_qk), sdesc(k_lo + 2 * ks, hi_qk), idesc_qk, sfq_col + 4 * ks,
+                        tc_mma_nvfp4(s_col, sdesc(q_lo + 2 * ks, hi_qk), sdesc(k_lo + 2 * ks, hi_qk), idesc_qk, sfq_col + 4 * ks,
                                      sfk_col + 4 * ks + 2 * h, true);
-                    tc_commit(bar(bSF + 2 * (s & 3) + h));
+                    tc_commit(bar(bSF + 2 * ((base + s) & 3) + h));
                     if (closes) tc_commit(bar(bKE + st));
+                    if (s == ns - 1) tc_commit(bar(bQE + qb));
                 }
                 __syncwarp();
                 if (++buf == nbuf) { buf = 0; buf_parity ^= 1; }
                 if (closes && ++st == S) { st = 0; st_parity ^= 1; }
             }
+            base += ns;
         }
         __syncwarp();
-      } else if (warp == 2) {
+      } else {
         // ------------------------------------------------------------------ PV MMA issuer
-        if (ns > 0) {
-            constexpr uint32_t idesc_pv = make_idesc_nvfp4(D);
-            constexpr uint32_t hi_pv = sdesc_hi(512, kSwz64), hi_sf = sdesc_hi(128, kSwzNone);
-            const uint32_t v_lo0 = sdesc_lo(sbase + C::oV, 16), p_lo0 = sdesc_lo(sbase + C::oP, 16);
-            const uint32_t sfv_lo0 = sdesc_lo(sbase + C::oSfV, 0), sfp_lo0 = sdesc_lo(sbase + C::oSfP, 0);
-            const uint32_t sfp_col = tmem + C::cSfP, sfv_col = tmem + C::cSfV;
-            int st = 0, st_parity = 0;
+        constexpr uint32_t idesc_pv = make_idesc_nvfp4(D);
+        constexpr uint32_t hi_pv = sdesc_hi(512, kSwz64), hi_sf = sdesc_hi(128, kSwzNone);
+        const uint32_t v_lo0 = sdesc_lo(sbase + C::oV, 16), p_lo0 = sdesc_lo(sbase + C::oP, 16);
+        const uint32_t sfv_lo0 = sdesc_lo(sbase + C::oSfV, 0), sfp_lo0 = sdesc_lo(sbase + C::oSfP, 0);
+        const uint32_t sfp_col = tmem + C::cSfP, sfv_col = tmem + C::cSfV;
+        int st = 0, st_parity = 0;
+        bool ok = !dead;
+        const Unit* u;
+        for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
+            const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d);
+            unit_done(i);
             for (int s = 0; s < ns; ++s) {
-                const int g = s & 7, t = two ? (s + d) & 1 : 0;
+                const int slot = (base + s) & 7, t = (s + d) & two;
                 const bool opens = t == 0 || s == 0, closes = t == two;       // first / last item of its V block
-                if (opens && !warp_wait(bar(bVF + st), st_parity, abort_flag, p.status, kWaitVFull)) break;
-                if (!warp_wait(bar(bOS + g), (s >> 3) & 1, abort_flag, p.status, kWaitOScaled)) break;
+                if (opens && !warp_wait(bar(bVF + st), st_parity, abort_flag, p.status, kWaitVFull)) { ok = false; break; }
+                if (!warp_wait(bar(bOS + slot), ((base + s) >> 3) & 1, abort_flag, p.status, kWaitOScaled)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t v_lo = v_lo0 + st * (C::kVBytes / 16), p_lo = p_lo0 + g * (C::kPBytes / 16);
-                const uint32_t sfv_lo = sfv_lo0 + st * (1024 / 16), sfp_lo = sfp_lo0 + g * (1024 / 16), o_col = tmem + C::cO + t * D;
+                const uint32_t v_lo = v_lo0 + st * (C::kVBytes / 16), p_lo = p_lo0 + slot * (C::kPBytes / 16);
+                const uint32_t sfv_lo = sfv_lo0 + st * (1024 / 16), sfp_lo = sfp_lo0 + slot * (1024 / 16), o_col = tmem + C::cO + t * D;
                 if (elect_one()) {
                     if (opens) {
 #pragma unroll
@@ -437,17 +593,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     for (int ks = 0; ks < 2; ++ks)
                         tc_mma_nvfp4(o_col, sdesc(p_lo + 2 * ks, hi_pv), sdesc(v_lo + 2 * ks, hi_pv), idesc_pv, sfp_col + 4 * ks, sfv_col + 4 * ks,
                                      s > two || (ks > 0) || carry_in);
-                    tc_commit(bar(bPV + g));
+                    tc_commit(bar(bPV + slot));
                     if (closes) tc_commit(bar(bVE + st));
                 }
                 __syncwarp();
                 if (closes && ++st == S) { st = 0; st_parity ^= 1; }
             }
+            base += ns;
         }
         __syncwarp();
       }
     } else {
-        reg_alloc<104>();
+        reg_alloc<96>();
         // ------------------------------------------------------------------ softmax groups (4 x 4 warps)
         // Group g (one warpgroup) takes the stream items s = g, g + 4, ...; a thread owns one row (tensor-memory lane) of the
         // block and walks its 128 keys in two halves of 64.  With two tiles a group always serves the same tile.
@@ -455,28 +612,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int quarter = warp & 3;            // tensor-memory lane quarter this warp may touch
         const int r = quarter * 32 + lane;       // row inside the tile
         const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-        const int t = two ? (g + d) & 1 : 0;
-        const int mt = mt0 + t;
-        const int grow = mt * kBlock + r;        // query index
         const int sw = (r >> 1) & 3;
-        const uint64_t sl2x2 = pack2f(sl2, sl2);
         float2* stat = reinterpret_cast<float2*>(sgen + C::oStat) + r;
-        const size_t crow = (size_t)bhq * p.Nq + grow;           // row of the carried state
-        float m_run = -INFINITY;
-        if (carry_in && t < nv && grow < Nq) m_run = p.carry_m_in[crow];
-        bool alive = true;
-        for (int s = g; s < ns; s += 4) {
-            const int n = nbmax - 1 - (two ? (s + d) >> 1 : s);      // key block
-            const bool need_mask = ((n + 1) * kBlock > Nk) || (CAUSAL && (n * kBlock + kBlock - 1 > mt * kBlock + shift));
+        bool alive = !dead;
+        const Unit* u;
+        for (int i = 0; alive && (u = next_unit(i)) != nullptr; ++i) {
+        const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nb1 = uniform(u->nbmax) - 1, row0 = uniform(u->mt0) * kBlock;
+        const int Nk = uniform(u->Nk), shift = CAUSAL ? uniform(u->shift) : 0;
+        const float sl2 = p.sm_scale_per_head ? p.sm_scale_per_head[u->hq] * 1.4426950408889634f : p.sm_scale_log2;
+        const uint64_t sl2x2 = pack2f(sl2, sl2);
+        for (int s = (g - base) & 3; s < ns; s += 4) {
+            const int sg = base + s;
+            const int t = (s + d) & two, n = nb1 - ((s + d) >> two);      // tile, key block
+            const int trow = row0 + t * kBlock;                           // the tile's first query row
+            const bool need_mask = ((n + 1) * kBlock > Nk) || (CAUSAL && (n * kBlock + kBlock - 1 > trow + shift));
             // Slot of the item (P buffer, statistics, barriers): each group alternates between two, so that it need not wait for the
             // P V MMA of its previous item.
-            const int slot = s & 7, slot_prev = (s - 1 - two) & 7;      // ... and of the tile's previous block
+            const int slot = sg & 7, slot_prev = (sg - 1 - two) & 7;      // ... and of the tile's previous block
             uint8_t* prow = sgen + C::oP + slot * C::kPBytes + r * 64;
-            float bm[8], se[8];
+            float bm[8], se[8], m_run;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int buf = h == 0 ? s % C::kSBufs0 : C::kSBufs0 + s % C::kSBufs1;
-                if (!warp_wait(bar(bSF + 2 * g + h), (s >> 2) & 1, abort_flag, p.status, kWaitSFull)) { alive = false; break; }
+                const int buf = h == 0 ? sg % C::kSBufs0 : C::kSBufs0 + sg % C::kSBufs1;
+                if (!warp_wait(bar(bSF + 2 * g + h), (sg >> 2) & 1, abort_flag, p.status, kWaitSFull)) { alive = false; break; }
                 tc_fence_after();
                 float x[64];
                 tmem_ld32(tmem + lane_addr + C::cS + 64 * buf, x);
@@ -486,7 +644,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 warp_arrive(bar(bSE + buf), lane);     // in registers: the buffer may be overwritten
                 if (need_mask) {
                     int lim = Nk - 1;
-                    if (CAUSAL) lim = min(lim, grow + shift);
+                    if (CAUSAL) lim = min(lim, trow + r + shift);
                     const int key0 = n * kBlock + 64 * h;
 #pragma unroll
                     for (int i = 0; i < 64; ++i)
@@ -524,12 +682,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     if (h == 1 && i == 2) {
                         // All maxima of the row are known: running maximum (with the previous block's, from the group that has it)
                         // and O rescale factor, handed to the next block's group and to the correction warps.
+                        float m_old = -INFINITY;
                         if (s > two) {
-                            if (!warp_wait(bar(bM + slot_prev * 4 + quarter), ((s - 1 - two) >> 3) & 1, abort_flag, p.status, kWaitPair)) { alive = false; break; }
-                            m_run = stat[slot_prev * 128].x;
+                            if (!warp_wait(bar(bM + slot_prev * 4 + quarter), ((sg - 1 - two) >> 3) & 1, abort_flag, p.status, kWaitPair)) { alive = false; break; }
+                            m_old = stat[slot_prev * 128].x;
+                        } else if (carry_in && trow + r < u->Nq) {
+                            m_old = p.carry_m_in[(size_t)u->bhq * p.Nq + trow + r];
                         }
-                        const float m_old = m_run;
-                        m_run = fmax3(fmax3(fmaxf(bm[0], bm[1]), bm[2], bm[3]), fmax3(bm[4], bm[5], bm[6]), fmaxf(bm[7], m_run));
+                        m_run = fmax3(fmax3(fmaxf(bm[0], bm[1]), bm[2], bm[3]), fmax3(bm[4], bm[5], bm[6]), fmaxf(bm[7], m_old));
                         const float alpha = ex2_approx((m_old - m_run) * sl2);        // m_old = -inf  ->  0
                         stat[slot * 128] = make_float2(m_run, alpha);
                         warp_arrive(bar(bM + slot * 4 + quarter), lane);
@@ -549,8 +709,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     if (i & 1) {
                         // P codes of 32 keys: one 16-byte chunk of the 64-byte-swizzled K-major row.  The P buffer was last read
                         // by the P V MMA of the group's item before the previous one.
-                        if (h == 0 && i == 1 && s >= 8 &&
-                            !warp_wait(bar(bPV + slot), ((s >> 3) - 1) & 1, abort_flag, p.status, kWaitPEmpty)) { alive = false; break; }
+                        if (h == 0 && i == 1 && sg >= 8 &&
+                            !warp_wait(bar(bPV + slot), ((sg >> 3) - 1) & 1, abort_flag, p.status, kWaitPEmpty)) { alive = false; break; }
                         *reinterpret_cast<uint4*>(prow + (((2 * h + (i >> 1)) ^ sw) << 4)) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
                     }
                 }
@@ -578,64 +738,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             fence_proxy_async_smem();
             warp_arrive(bar(bPF + slot), lane);
         }
-        // ------------------------------------------------------------------ epilogue: O / l
-        // The groups of a tile take equal shares of its columns.
-        if (alive && !dead_launch && nv > 0) {
-            const int nb = nbt[t];
-            const int share = two ? D / 2 : D / 4, c0 = (two ? g >> 1 : g) * share;
-            const int s_last = two ? 2 * (nbmax - 1) + t - d : nb - 1;
-            alive = warp_wait(bar(bL + t * 4 + quarter), 0, abort_flag, p.status, kWaitPair);
-            if (alive && nb > 0) alive = warp_wait(bar(bPV + (s_last & 7)), (s_last >> 3) & 1, abort_flag, p.status, kWaitOReady);
-            tc_fence_after();
-            const float2 l2 = reinterpret_cast<const float2*>(sgen + C::oL)[t * 128 + r];
-            const float l_tot = l2.x + l2.y;
-            if (alive && grow < Nq && (nb > 0 ? g == (s_last & 3) : c0 == 0)) {      // the group that has the final maximum
-                if (p.lse != nullptr) {
-                    // ln sum_k exp(scale * q.k): the kernel's row sum is 2688 * sum_k 2^((S_k - m) s) over the smoothed
-                    // scores S (delta_s included); K smoothing took scale * q.km out of every score of the row
-                    const float ms_fin = m_run * sl2;       // (without keys l is 0, whatever this is)
-                    const float scale = p.sm_scale_per_head ? p.sm_scale_per_head[hq] : p.sm_scale;
-                    const float v = (ms_fin + __log2f(l_tot) + kPScaleLog2) * 0.6931471805599453f +
-                                    scale * p.qkm[(size_t)bhq * p.nqt * kBlock + grow];
-                    p.lse[(size_t)bhq * p.Nq + grow] = (l_tot == 0.f) ? -INFINITY : v;
-                }
-                if (p.carry_o_out != nullptr) p.carry_m_out[crow] = m_run > kNoKey ? m_run : -INFINITY;
-            }
-            if (alive) {
-                const float inv_l = (l_tot == 0.f || l_tot != l_tot) ? 0.f : __frcp_rn(l_tot);
-                const bool want_out = (p.out[0] != nullptr);
-                // the row's home: one output buffer, or the part that owns this token (another GPU's memory when the
-                // output goes straight back to the token shards of a sequence-parallel group: plain stores)
-                const int opart = (p.out_rows == 0) ? 0 : min(grow / p.out_rows, kMaxParts - 1);
-                const int orow_l = grow - opart * p.out_rows;
-                OutT* orow = static_cast<OutT*>(p.out[opart]) + out_base + hq * p.os1 + (int64_t)orow_l * p.os2;
-                for (int c = c0; c < c0 + share; c += 16) {
-                    float o[16];
-                    if (nb > 0 || carry_in) {
-                        tmem_ld16(tmem + lane_addr + C::cO + t * D + c, o);
-                        tc_wait_ld();
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = 0.f;
-                    }
-                    if (p.carry_o_out != nullptr && grow < Nq) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            *reinterpret_cast<float4*>(p.carry_o_out + crow * D + c + 4 * i) = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-                    }
-                    if (want_out && grow < Nq) {
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            uint4 w;
-                            w.x = pack2<OutT>(o[8 * i] * inv_l, o[8 * i + 1] * inv_l);
-                            w.y = pack2<OutT>(o[8 * i + 2] * inv_l, o[8 * i + 3] * inv_l);
-                            w.z = pack2<OutT>(o[8 * i + 4] * inv_l, o[8 * i + 5] * inv_l);
-                            w.w = pack2<OutT>(o[8 * i + 6] * inv_l, o[8 * i + 7] * inv_l);
-                            *reinterpret_cast<uint4*>(orow + c + i * 8) = w;
-                        }
-                    }
-                }
-            }
+        unit_done(i);
+        base += ns;
         }
         __syncwarp();
     }
@@ -695,21 +799,20 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
 
 template <int D, bool CAUSAL, typename OutT, bool VARLEN>
 static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                            const AttnParams& p, cudaStream_t st) {
+                            const AttnParams& p, int grid, cudaStream_t st) {
     auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes);
     if (e != cudaSuccess) return e;
-    const int grid = a.B * a.Hq * ((a.Nq_p / kBlock + 1) / 2);      // one CTA per pair of query tiles
     kern<<<grid, Cfg<D>::kThreads, Cfg<D>::kSmemBytes, st>>>(tq, tk, tv, p);
     return cudaGetLastError();
 }
 
 template <int D, bool CAUSAL, typename OutT>
 static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                            const AttnParams& p, cudaStream_t st) {
+                            const AttnParams& p, int grid, cudaStream_t st) {
     // packed variable-length batches run their own instantiation, so that the uniform kernels carry none of it
-    return a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true>(a, tq, tk, tv, p, st)
-                             : launch_v<D, CAUSAL, OutT, false>(a, tq, tk, tv, p, st);
+    return a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true>(a, tq, tk, tv, p, grid, st)
+                             : launch_v<D, CAUSAL, OutT, false>(a, tq, tk, tv, p, grid, st);
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
@@ -727,7 +830,19 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
         *driver_rc = (int)r;
         return cudaErrorInvalidValue;
     }
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return cudaErrorInvalidDevice;
     AttnParams p;
+    // Units of work: pairs of query tiles; when the last round of pairs fills at most half of the SMs it is dealt out as
+    // single tiles (half the time for the round, twice the SMs).
+    const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), rest = pairs % sms;
+    const bool split = nqt > 1 && 2 * rest <= sms;
+    p.unit_counter = a.unit_counter;
+    p.whole_units = split ? pairs - rest : pairs;
+    p.units = split ? pairs + rest : pairs;
+    const int grid = p.units < sms ? p.units : sms;
+    p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;
     p.nqt = a.Nq_p / kBlock; p.nkb = a.Nk_p / kBlock; p.nqm = a.nqm;
     p.sm_scale_log2 = a.sm_scale * 1.4426950408889634f;
@@ -745,15 +860,15 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.causal_shift = a.causal_shift;
     p.cu_q = a.cu_q; p.cu_k = a.cu_k;
     if (a.is_bf16) {
-        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, p, st)
-                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, p, st);
-        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, p, st)
-                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, p, st);
+        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, p, grid, st)
+                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, p, grid, st);
+        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, p, grid, st)
+                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, p, grid, st);
     }
-    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, p, st)
-                                       : launch_t<128, false, __half>(a, tq, tk, tv, p, st);
-    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, p, st)
-                       : launch_t<64, false, __half>(a, tq, tk, tv, p, st);
+    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, p, grid, st)
+                                       : launch_t<128, false, __half>(a, tq, tk, tv, p, grid, st);
+    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, p, grid, st)
+                       : launch_t<64, false, __half>(a, tq, tk, tv, p, grid, st);
 }
 
 }  // namespace sage3

@@ -46,6 +46,7 @@ struct AttnArgs {
     float* lse;                     // optional fp32 [B][Hq][Nq]; nullptr if not wanted
     const float* qkm;               // fp32 [B][Hq][Nq_p] from the pre-pass
     int* status;                    // the attention kernel's status word
+    int* unit_counter;              // work counter, zeroed before the launch
     // accumulator state carried between calls (all nullptr: none); fp32, unnormalized O [B][Hq][Nq][D], m [B][Hq][Nq], l [B][Hq][Nq][2]
     const float *carry_o_in, *carry_m_in, *carry_l_in;
     float *carry_o_out, *carry_m_out, *carry_l_out;
