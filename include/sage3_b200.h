@@ -75,7 +75,7 @@ typedef struct Sage3Desc {
  *   status   int32[64]                        device-written status words (0 = fine): [0, 32) pre-pass, [32, 64) attention;
  *                                             each stage clears its own half, so sage3_check_status after sage3_fwd sees both
  *                                             (word 64, in the same 1 024 bytes: the attention kernel's work counter)
- *   kpart    fp32 [B*Hkv][chunks][D]          scratch: partial column sums of K (and of Q when per_block_mean = 0)
+ *   kpart    fp32 [B*Hkv][chunks][D]          scratch: partial column sums of K (followed by those of Q when per_block_mean = 0)
  *   km       dtype[B][Hkv][D]                 mean of K over its Nk tokens
  *   qm       dtype[B][Hq][nqm][D]             Q means; nqm = Nq_p/128, or 1 when per_block_mean = 0
  *   delta    dtype[B][Hq][nqm][Nk_p]          qm . k'^T  (api.py:91)
@@ -86,7 +86,8 @@ typedef struct Sage3Desc {
  *   v_codes  u8   [B][Hkv][D][Nk_p/2]         V transposed, microblocks of 16 consecutive tokens
  *   v_sf     u8   [B][Hkv][Nk_p/128][2][512]  atoms with r = channel, c = (token % 128) / 16
  *   qkm      fp32 [B][Hq][Nq_p]               q . km per query row (the part of q k^T that K smoothing removes;
- *                                             core.py:289-293 `lse_correction`), used by the LSE output
+ *                                             core.py:289-293 `lse_correction`), used by the LSE output (sage3_fwd and
+ *                                             sage3_fwd_varlen write it only when `lse` is asked for)
  */
 typedef struct Sage3Workspace {
     size_t status, kpart, km, qm, delta, q_codes, q_sf, k_codes, k_sf, v_codes, v_sf, qkm;

@@ -3,9 +3,60 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/sage3_b200.h"
 #include "sage3_common.cuh"
 #include "sage3_kernels.h"
+
+namespace sage3 {
+
+constexpr int kMaxDevices = 64;
+
+cudaError_t current_device(int* dev, DeviceInfo* info) {
+    static std::atomic<int> known[kMaxDevices];       // 0: not looked up yet, else SM count * 2 + (compute capability 10.0)
+    cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    int v = *dev < kMaxDevices ? known[*dev].load(std::memory_order_relaxed) : 0;
+    if (v == 0) {
+        int sms = 0, major = 0, minor = 0;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, *dev)) != cudaSuccess ||
+            (e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, *dev)) != cudaSuccess ||
+            (e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, *dev)) != cudaSuccess)
+            return e;
+        v = 2 * sms + (major == 10 && minor == 0 ? 1 : 0);
+        if (*dev < kMaxDevices) known[*dev].store(v, std::memory_order_relaxed);
+    }
+    info->sms = v >> 1;
+    info->ok = (v & 1) != 0;
+    return cudaSuccess;
+}
+
+cudaError_t allow_smem(const void* kernel, int bytes) {
+    struct Entry { const void* kernel; uint64_t devices; };
+    static Entry done[64];                            // one per kernel instantiation (fewer than 32 exist)
+    static std::mutex mutex;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    Entry* slot = nullptr;
+    for (Entry& d : done)
+        if (d.kernel == kernel || d.kernel == nullptr) {
+            slot = &d;
+            break;
+        }
+    if (slot && dev < kMaxDevices && (slot->devices >> dev & 1)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && slot && dev < kMaxDevices) {
+        slot->kernel = kernel;
+        slot->devices |= 1ull << dev;
+    }
+    return e;
+}
+
+}  // namespace sage3
 
 namespace {
 
@@ -42,8 +93,7 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     const size_t nqm = d->per_block_mean ? nqp / 128 : 1;
     const size_t kch_k = ((size_t)d->Nk + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t kch_q = ((size_t)d->Nq + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
-    size_t part = B * Hkv * kch_k;
-    if (!d->per_block_mean && B * Hq * kch_q > part) part = B * Hq * kch_q;
+    const size_t part = B * Hkv * kch_k + (d->per_block_mean ? 0 : B * Hq * kch_q);
     size_t off = 0;
     w->status = off;  off += align_up(64 * sizeof(int32_t));
     w->kpart = off;   off += align_up(part * D * sizeof(float));
@@ -66,11 +116,10 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
 }
 
 int check_arch() {
-    int dev = 0, major = 0, minor = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return SAGE3_E_CUDA;
-    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return SAGE3_E_CUDA;
-    if (cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev) != cudaSuccess) return SAGE3_E_CUDA;
-    return (major == 10 && minor == 0) ? SAGE3_OK : SAGE3_E_ARCH;
+    int dev = 0;
+    sage3::DeviceInfo info;
+    if (sage3::current_device(&dev, &info) != cudaSuccess) return SAGE3_E_CUDA;
+    return info.ok ? SAGE3_OK : SAGE3_E_ARCH;
 }
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -103,7 +152,8 @@ sage3::PartsPtr one_part(const void* p) {
     return r;
 }
 
-int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, void* stream,
+// `cleared`: the pre-pass of the same call has already zeroed the attention half of the status words and the work counter
+int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, void* stream, bool cleared = false,
               const Sage3Carry* carry = nullptr, const int32_t* cu_q = nullptr, const int32_t* cu_k = nullptr) {
     Sage3Workspace w;
     int rc = layout(desc, &w);
@@ -123,7 +173,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     if (rc != SAGE3_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    if (cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0, (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st) !=
+    if (!cleared && cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0, (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st) !=
         cudaSuccess)
         return SAGE3_E_CUDA;
     sage3::AttnArgs a;
@@ -266,7 +316,8 @@ SAGE3_API size_t sage3_workspace_bytes(const Sage3Desc* desc) {
 }
 
 static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const sage3::PartsPtr& k, const sage3::PartsPtr& v,
-                        const void* km_in, void* ws, void* stream, const int32_t* cu_q = nullptr, const int32_t* cu_k = nullptr) {
+                        const void* km_in, void* ws, void* stream, bool want_qkm = true, const int32_t* cu_q = nullptr,
+                        const int32_t* cu_k = nullptr) {
     Sage3Workspace w;
     int rc = layout(desc, &w);
     if (rc != SAGE3_OK) return rc;
@@ -297,7 +348,9 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     a.status = reinterpret_cast<int*>(base + w.status);
     a.cu_q = cu_q; a.cu_k = cu_k;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(base + w.status, 0, kStatusWords * sizeof(int32_t), st) != cudaSuccess) return SAGE3_E_CUDA;
+    a.want_qkm = want_qkm;
+    a.clear = a.status;
+    a.n_clear = kUnitCounterWord + 1;
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
         cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
@@ -318,9 +371,9 @@ SAGE3_API int sage3_fwd_varlen(const Sage3Desc* desc, const int32_t* cu_seqlens_
                                const void* k, const void* v, void* out, float* lse, void* ws, void* stream) {
     if (!desc || !cu_seqlens_q || !cu_seqlens_k || !q || !k || !v || !out) return SAGE3_E_NULL;
     if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(cu_seqlens_q, 4) || !aligned(cu_seqlens_k, 4)) return SAGE3_E_ALIGN;
-    const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, cu_seqlens_q, cu_seqlens_k);
+    const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, lse != nullptr, cu_seqlens_q, cu_seqlens_k);
     if (rc != SAGE3_OK) return rc;
-    return attn_impl(desc, ws, one_part(out), lse, stream, nullptr, cu_seqlens_q, cu_seqlens_k);
+    return attn_impl(desc, ws, one_part(out), lse, stream, true, nullptr, cu_seqlens_q, cu_seqlens_k);
 }
 
 SAGE3_API int sage3_prepass_kmean(const Sage3Desc* desc, const void* q, const void* k, const void* v, const void* km, void* ws,
@@ -343,7 +396,7 @@ SAGE3_API int sage3_prepass_parts(const Sage3Desc* desc, const Sage3Parts* q, co
 
 SAGE3_API int sage3_attn_fwd_carry(const Sage3Desc* desc, void* ws, const Sage3Carry* carry, void* out, float* lse, void* stream) {
     if (!carry) return SAGE3_E_NULL;
-    return attn_impl(desc, ws, one_part(out), lse, stream, carry);
+    return attn_impl(desc, ws, one_part(out), lse, stream, false, carry);
 }
 
 SAGE3_API int sage3_attn_fwd_parts(const Sage3Desc* desc, void* ws, const Sage3Parts* out, float* lse, void* stream) {
@@ -392,9 +445,11 @@ SAGE3_API int sage3_attn_fwd(const Sage3Desc* desc, void* ws, void* out, float* 
 
 SAGE3_API int sage3_fwd(const Sage3Desc* desc, const void* q, const void* k, const void* v, void* ws, void* out, float* lse,
               void* stream) {
-    const int rc = sage3_prepass(desc, q, k, v, ws, stream);
+    if (!q || !k || !v) return SAGE3_E_NULL;
+    if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16)) return SAGE3_E_ALIGN;
+    const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, lse != nullptr);
     if (rc != SAGE3_OK) return rc;
-    return sage3_attn_fwd(desc, ws, out, lse, stream);
+    return attn_impl(desc, ws, one_part(out), lse, stream, true);
 }
 
 SAGE3_API int sage3_selftest_wait_timeout(void* ws, void* stream) {

@@ -243,8 +243,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        // an earlier CTA of this launch gave up, or the pre-pass did (the workspace is then incomplete): nothing is done
-        tmem_slot[1] = (*reinterpret_cast<volatile int*>(p.status) != 0) || (*reinterpret_cast<const volatile int*>(p.prepass_status) != 0);
     }
     // delta_s stages: the 256 bytes behind each row stay zero for the whole kernel; ones tile:
     // [k chunk][row group][8 rows][16 bytes], 1.0 in element 0 of every row of chunk 0
@@ -264,6 +262,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         prefetch_tmap(&tm_k);
         prefetch_tmap(&tm_v);
     }
+    pdl_wait();                       // nothing above reads what the pre-pass writes
+    // an earlier CTA of this launch gave up, or the pre-pass did (the workspace is then incomplete): nothing is done
+    if (threadIdx.x == 0)
+        tmem_slot[1] = (*reinterpret_cast<volatile int*>(p.status) != 0) || (*reinterpret_cast<const volatile int*>(p.prepass_status) != 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -801,10 +803,9 @@ template <int D, bool CAUSAL, typename OutT, bool VARLEN>
 static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const AttnParams& p, int grid, cudaStream_t st) {
     auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), Cfg<D>::kSmemBytes);
     if (e != cudaSuccess) return e;
-    kern<<<grid, Cfg<D>::kThreads, Cfg<D>::kSmemBytes, st>>>(tq, tk, tv, p);
-    return cudaGetLastError();
+    return launch_pdl(kern, dim3(grid), dim3(Cfg<D>::kThreads), Cfg<D>::kSmemBytes, st, tq, tk, tv, p);
 }
 
 template <int D, bool CAUSAL, typename OutT>
@@ -830,9 +831,11 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
         *driver_rc = (int)r;
         return cudaErrorInvalidValue;
     }
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return cudaErrorInvalidDevice;
+    int dev = 0;
+    DeviceInfo info;
+    const cudaError_t e = current_device(&dev, &info);
+    if (e != cudaSuccess) return e;
+    const int sms = info.sms;
     AttnParams p;
     // Units of work: pairs of query tiles; when the last round of pairs fills at most half of the SMs it is dealt out as
     // single tiles (half the time for the round, twice the SMs).

@@ -48,6 +48,10 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     return r;
 }
 
+// programmatic dependent launch: let the next kernel of the stream start its prologue; wait until the ones before are complete
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // per-warpgroup register budget (all four warps of a warpgroup execute the same call)
 template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }

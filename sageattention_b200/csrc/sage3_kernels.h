@@ -29,6 +29,9 @@ struct PrepassArgs {
     uint8_t *q_codes, *q_sf, *k_codes, *k_sf, *v_codes, *v_sf;
     float* qkm;                    // fp32 [B][Hq][Nq_p]: q . km per query row
     int* status;                   // device status words (bounded waits report here)
+    int want_qkm;                  // q . km per query row is wanted (the LSE output needs it)
+    int* clear;                    // words the first kernel zeroes: all status words and the attention kernel's work counter
+    int n_clear;
     // packed variable-length sequences (both nullptr: every batch entry has Nq / Nk tokens): device int32 [B + 1], entry b
     // owns rows cu[b] .. cu[b + 1] of the packed tensor; Nq / Nk are then the maximum lengths, stride 0 is unused
     const int *cu_q, *cu_k;
@@ -54,6 +57,29 @@ struct AttnArgs {
     const int* prepass_status;      // the pre-pass's status word (non-zero: the workspace is incomplete, do nothing)
     const int *cu_q, *cu_k;         // packed variable-length sequences, as in PrepassArgs (nullptr: uniform lengths)
 };
+
+// Device the calling thread has current, its SM count and whether it is compute capability 10.0 (looked up once per device).
+struct DeviceInfo { int sms; bool ok; };
+cudaError_t current_device(int* dev, DeviceInfo* info);
+
+// Dynamic shared memory of a kernel beyond 48 KB (set once per kernel and device).
+cudaError_t allow_smem(const void* kernel, int bytes);
+
+// Launch that may begin (up to its griddepcontrol.wait) while the kernel before it in the stream is still running.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 // Encodes a tensor map over a byte tensor [n2][n1][n0] (n0 contiguous) with box [1][b1][b0]; swizzle: 0 none, 1 32 B, 2 64 B,
 // 3 128 B.  Returns 0, or the driver's error code (-1: the driver entry point could not be resolved).

@@ -167,38 +167,68 @@ __device__ __forceinline__ void quant16_packed(const uint32_t* w, uint32_t& lo, 
 // (deterministic: no atomics, the summation order depends on N only)
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
-__global__ void __launch_bounds__(256) colsum_partial_kernel(const __grid_constant__ Src<T> x, int64_t sb, int64_t sh,
-                                                             int64_t sn, int H, int N,
-                                                             float* __restrict__ part, int chunks) {   // N: by value, narrowed per entry
+__device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, float* __restrict__ part,
+                                             int chunks, int chunk, int bh, float* red) {   // red: shared, [RPP][D + 1]
     constexpr int TPR = D / 8;           // threads per row (8 elements = 16 bytes each)
     constexpr int RPP = 256 / TPR;       // rows per pass
-    const int chunk = blockIdx.x, bh = blockIdx.y;
     const int b = bh / H, h = bh % H;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int c8 = threadIdx.x % TPR, rl = threadIdx.x / TPR;
     const int r0 = chunk * kRowsPerChunk;
     const int r1 = min(N, r0 + kRowsPerChunk);
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int r = r0 + rl; r < r1; r += RPP) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(x.row(bh_off, r, sn) + c8 * 8));
-        const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+    // Eight rows in flight per thread (a load per addition made the two CTAs of a 1 024-token head take 19 us); the additions
+    // keep their order.
+    constexpr int U = 8;
+    for (int r = r0 + rl; r < r1; r += U * RPP) {
+        uint4 a[U];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float2 v = Num<T>::to_f2(w[i]);
-            acc[2 * i] += v.x;
-            acc[2 * i + 1] += v.y;
+        for (int u = 0; u < U; ++u) {
+            a[u] = make_uint4(0, 0, 0, 0);
+            if (r + u * RPP < r1) a[u] = __ldg(reinterpret_cast<const uint4*>(x.row(bh_off, r + u * RPP, sn) + c8 * 8));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t w[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float2 v = Num<T>::to_f2(w[i]);
+                acc[2 * i] += v.x;
+                acc[2 * i + 1] += v.y;
+            }
         }
     }
-    __shared__ float red[RPP][D + 1];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) red[rl][c8 * 8 + i] = acc[i];
+    for (int i = 0; i < 8; ++i) red[rl * (D + 1) + c8 * 8 + i] = acc[i];
     __syncthreads();
     if (threadIdx.x < D) {
         float s = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < RPP; ++i) s += red[i][threadIdx.x];
+#pragma unroll
+        for (int i = 0; i < RPP; ++i) s += red[i * (D + 1) + threadIdx.x];
         part[((int64_t)bh * chunks + chunk) * D + threadIdx.x] = s;
     }
+}
+
+// One sum of a column's partial sums, in the order of the chunks.
+__device__ __forceinline__ float sum_chunks(const float* __restrict__ part, int chunks, int D) {
+    float s = 0.f;
+    int c = 0;
+    for (; c + 8 <= chunks; c += 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = part[(int64_t)(c + i) * D];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += v[i];
+    }
+    for (; c < chunks; ++c) s += part[(int64_t)c * D];
+    return s;
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
+                                                             float* __restrict__ part, int chunks) {
+    __shared__ float red[(2048 / D) * (D + 1)];
+    colsum_chunk<T, D>(x, sb, sh, sn, H, N, part, chunks, blockIdx.x, blockIdx.y, red);
 }
 
 template <typename T, int D>
@@ -212,8 +242,7 @@ __global__ void colmean_finalize_kernel(const float* __restrict__ part, int chun
         if (pad_to_block) n = (n + kBlock - 1) / kBlock * kBlock;
         inv_count = n > 0 ? 1.0f / (float)n : 0.f;
     }
-    float s = 0.f;
-    for (int c = 0; c < chunks; ++c) s += part[((int64_t)bh * chunks + c) * D + d];
+    const float s = sum_chunks(part + (int64_t)bh * chunks * D + d, chunks, D);
     mean[(int64_t)bh * D + d] = Num<T>::from_f(s * inv_count);
 }
 
@@ -223,20 +252,20 @@ __global__ void colmean_finalize_kernel(const float* __restrict__ part, int chun
 enum { kModeQBlockMean = 0, kModeQGlobalMean = 1 };
 
 template <typename T, int D, int MODE>
-__global__ void __launch_bounds__(256, D == 128 ? 4 : 3) quant_rows_kernel(
-    const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
+__device__ __forceinline__ void quant_q_tile(
+    const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
     const T* __restrict__ mean_in,     // one mean per head: qm [B*H][D]; unused for block mean
     T* __restrict__ qm_out,            // block mean: [B*H][Np/128][D]
     uint8_t* __restrict__ codes,       // [B*H][Np][D/2]
     uint8_t* __restrict__ sfs,         // [B*H][Np/128][D/64][512]
     const T* __restrict__ km,          // K means [B*Hkv][D]
     int group,                         // query heads per kv head
-    float* __restrict__ qkm) {         // [B*H][Np]: x . km per row (the score part that K smoothing removes)
+    float* __restrict__ qkm,           // [B*H][Np]: x . km per row (the score part that K smoothing removes); nullptr: not wanted
+    int tile, int bh, uint8_t* smem_raw) {
     constexpr int CH = D / 16;            // microblocks per row
     constexpr int RPP = 256 / CH;         // rows per pass
     constexpr int ITEMS = kBlock / RPP;   // microblocks per thread
 
-    const int tile = blockIdx.x, bh = blockIdx.y;
     const int b = bh / H, h = bh % H;
     const int t = threadIdx.x;
     const int c = t % CH, rl = t / CH;
@@ -244,7 +273,6 @@ __global__ void __launch_bounds__(256, D == 128 ? 4 : 3) quant_rows_kernel(
     const int row0 = tile * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
 
-    extern __shared__ __align__(16) uint8_t smem_raw[];
     float* s_mean = reinterpret_cast<float*>(smem_raw);                        // [D]
     uint8_t* s_sf = smem_raw + D * 4;                                          // [(D/64) * 512]
     uint8_t* s_more = s_sf + (D / 64) * 512;                                   // block mean only: staged tile, chain sums
@@ -257,7 +285,7 @@ __global__ void __launch_bounds__(256, D == 128 ? 4 : 3) quant_rows_kernel(
     }
 
     // x . km of every row: 16 products per thread, then a sum over the CH neighbouring lanes that share the row
-    {
+    if (qkm != nullptr) {
         const T* kmh = km + ((int64_t)b * (H / group) + h / group) * D + c * 16;
         uint4 k0, k1;
         load16_packed<T>(kmh, true, k0, k1);
@@ -366,7 +394,9 @@ __global__ void __launch_bounds__(256, D == 128 ? 4 : 3) quant_rows_kernel(
 // ------------------------------------------------------------------------------------------------
 // K: smooth + quantize one 128-key tile per CTA, and its delta_s columns on the tensor core:
 // delta_s[qb][key] = sum_d qm[qb][d] * k'[key][d] as 128 x 128 x D tcgen05 MMAs (16-bit operands from shared
-// memory in the 128-byte-swizzled K-major layout, fp32 accumulator in tensor memory), one per 128 query blocks.
+// memory in the 128-byte-swizzled K-major layout, fp32 accumulator in tensor memory), one per 128 query blocks, counted
+// through all query heads of the kv head (their means follow one another): four query heads of one block each took four
+// rounds of copy, MMA and store, 150 us for 4 096 key tiles, and take one now, 68 us.
 // The query-block means arrive through TMA (a tensor map over qm) and the delta_s tiles leave through TMA (a tensor
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
@@ -374,12 +404,15 @@ __global__ void __launch_bounds__(256, D == 128 ? 4 : 3) quant_rows_kernel(
 template <typename T, int D>
 __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
-    const T* __restrict__ km,          // [B*H][D]
+    T* __restrict__ km,                // [B*H][D]
+    const float* __restrict__ part,    // partial column sums to form the mean from ([B*H][chunks][D]), or nullptr: `km` holds it
+    int chunks,
     uint8_t* __restrict__ codes,       // [B*H][Np][D/2]
     uint8_t* __restrict__ sfs,         // [B*H][Np/128][D/64][512]
-    int Hq, int nqm, int* __restrict__ status, const int* __restrict__ cu_q,
-    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*Hq][nqm][2 D], box 128 rows x 128 bytes, 128-byte swizzle
-    const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*Hq][nqm][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
+    int rows,                          // query blocks of all query heads of a kv head
+    int* __restrict__ status,
+    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 rows x 128 bytes, 128-byte swizzle
+    const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*H][rows][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
     constexpr int CH = D / 16;            // microblocks per row
     constexpr int RPP = 256 / CH;         // rows per pass
     constexpr int ITEMS = kBlock / RPP;   // microblocks per thread
@@ -394,8 +427,6 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int row0 = tile * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
-    // query blocks this entry really has (nqm stays the row count of the qm / delta_s layouts)
-    const int nqm_live = (cu_q != nullptr) ? min(nqm, (max(cu_q[b + 1] - cu_q[b], 0) + kBlock - 1) / kBlock) : nqm;
 
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t sbase = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -427,7 +458,25 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
         const int r = row0 + rl + RPP * i;
         load16_packed<T>(x.row(bh_off, r, sn) + c * 16, r < N, raw[i][0], raw[i][1]);
     }
-    if (t < D) s_mean[t] = Num<T>::to_f(km[(int64_t)bh * D + t]);
+    pdl_launch_dependents();
+    pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
+    if (t < D) {
+        if (part != nullptr) {
+            const T m = Num<T>::from_f(sum_chunks(part + (int64_t)bh * chunks * D + t, chunks, D) * (N > 0 ? 1.0f / (float)N : 0.f));
+            if (tile == 0) km[(int64_t)bh * D + t] = m;
+            s_mean[t] = Num<T>::to_f(m);
+        } else {
+            s_mean[t] = Num<T>::to_f(km[(int64_t)bh * D + t]);
+        }
+    }
+    // the first A tile (see below) comes in while K is quantized
+    auto load_a = [&](int m0) {
+        mbar_expect_tx(bar_a, SUB * 16384);
+#pragma unroll
+        for (int sub = 0; sub < SUB; ++sub)
+            tma_load_3d(sbase + oA + sub * 16384, &tm_qm, bar_a, sub * 128, m0, bh);
+    };
+    if (t == 0) load_a(0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -463,76 +512,69 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
         if (t < (D / 64) * 32) reinterpret_cast<uint4*>(dst)[t] = reinterpret_cast<const uint4*>(s_sf)[t];
     }
 
-    // delta_s for every query head of this kv head, 128 query blocks per MMA group
+    // delta_s of all query heads of this kv head, 128 query blocks per MMA group
     constexpr uint32_t idesc = make_idesc_f16_kk(128, kBf16);
-    const int group = Hq / H;
     const int quarter = warp & 3, chalf = warp >> 2;       // tensor-memory lane quarter, column half of the epilogue
     uint32_t iter = 0;
     bool alive = true;
-    for (int g = 0; g < group && alive; ++g) {
-        const int hq = h * group + g;
-        for (int m0 = 0; m0 < nqm_live && alive; m0 += 128, ++iter) {
-            // A tile: 128 query-block means, fetched by the copy engine in the 128-byte swizzle the MMA reads.  Rows beyond
-            // the tensor's nqm arrive as zeros; rows of a shorter sequence of a packed batch only feed accumulator rows
-            // that nobody reads.
-            fence_proxy_async_smem();       // this thread's stores (the k' tile; the previous epilogue's staging) before the engine touches the tiles
+    for (int m0 = 0; m0 < rows && alive; m0 += 128, ++iter) {
+        // A tile: 128 query-block means, fetched by the copy engine in the 128-byte swizzle the MMA reads.  Rows beyond
+        // the tensor arrive as zeros; rows of a shorter sequence of a packed batch only feed accumulator rows
+        // that nobody reads.
+        fence_proxy_async_smem();       // this thread's stores (the k' tile; the previous epilogue's staging) before the engine touches the tiles
+        if (m0 > 0) {
             __syncthreads();
-            if (t == 0) {
-                mbar_expect_tx(bar_a, SUB * 16384);
-#pragma unroll
-                for (int sub = 0; sub < SUB; ++sub)
-                    tma_load_3d(sbase + oA + sub * 16384, &tm_qm, bar_a, sub * 128, m0, b * Hq + hq);
-            }
-            alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);
-            tc_fence_before();
-            alive = __syncthreads_and(alive ? 1 : 0) != 0;
-            if (!alive) break;
-            if (t == 0) {
-                tc_fence_after();
-#pragma unroll
-                for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-                    tc_mma_f16(tmem, make_sdesc(sbase + oA + off, 16, 1024, kSwz128), make_sdesc(sbase + oB + off, 16, 1024, kSwz128),
-                               idesc, ks > 0);
-                }
-                tc_commit(bar);
-            }
-            alive = mbar_wait(bar, iter & 1, abort_flag, status, kWaitDeltaMma);
-            alive = __syncthreads_and(alive ? 1 : 0) != 0;
-            if (!alive) break;
-            tc_fence_after();
-            // epilogue: thread = query block (row) of the accumulator, 64 keys of its row = 128 contiguous bytes of delta_s.
-            // The warp's 32 rows x 128 bytes are staged in shared memory in the 128-byte swizzle (at D = 128 in the A tile,
-            // which is free once the MMAs have completed) and leave as one TMA tile store; the engine clips rows beyond nqm.
-            {
-                const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + chalf * 64;
-                uint8_t* stg = sgen + oStg + warp * 4096;
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    float v[32];
-                    tmem_ld32(acc + cc * 32, v);
-                    tc_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint32_t p4[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
-                        *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
-                            make_uint4(p4[0], p4[1], p4[2], p4[3]);
-                    }
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0 && m0 + quarter * 32 < nqm) {
-                    tma_store_3d(&tm_delta, sbase + oStg + warp * 4096, (row0 + chalf * 64) * 2, m0 + quarter * 32, b * Hq + hq);
-                    bulk_commit_group();
-                    bulk_wait_group_read0();      // the engine has read the staging tile: it may be written again
-                }
-                __syncwarp();
-            }
-            tc_fence_before();
-            __syncthreads();      // the accumulator and the A tile are free again
+            if (t == 0) load_a(m0);
         }
+        alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);
+        tc_fence_before();
+        alive = __syncthreads_and(alive ? 1 : 0) != 0;
+        if (!alive) break;
+        if (t == 0) {
+            tc_fence_after();
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+                const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
+                tc_mma_f16(tmem, make_sdesc(sbase + oA + off, 16, 1024, kSwz128), make_sdesc(sbase + oB + off, 16, 1024, kSwz128),
+                           idesc, ks > 0);
+            }
+            tc_commit(bar);
+        }
+        alive = mbar_wait(bar, iter & 1, abort_flag, status, kWaitDeltaMma);
+        alive = __syncthreads_and(alive ? 1 : 0) != 0;
+        if (!alive) break;
+        tc_fence_after();
+        // epilogue: thread = query block (row) of the accumulator, 64 keys of its row = 128 contiguous bytes of delta_s.
+        // The warp's 32 rows x 128 bytes are staged in shared memory in the 128-byte swizzle (at D = 128 in the A tile,
+        // which is free once the MMAs have completed) and leave as one TMA tile store; the engine clips rows beyond nqm.
+        if (m0 + quarter * 32 < rows) {
+            const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + chalf * 64;
+            uint8_t* stg = sgen + oStg + warp * 4096;
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+                float v[32];
+                tmem_ld32(acc + cc * 32, v);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint32_t p4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
+                    *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
+                        make_uint4(p4[0], p4[1], p4[2], p4[3]);
+                }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_3d(&tm_delta, sbase + oStg + warp * 4096, (row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
+                bulk_commit_group();
+                bulk_wait_group_read0();      // the engine has read the staging tile: it may be written again
+            }
+            __syncwarp();
+        }
+        tc_fence_before();
+        __syncthreads();      // the accumulator and the A tile are free again
     }
     tc_fence_before();
     __syncthreads();
@@ -546,18 +588,15 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
 // V: one tile of 128 tokens x D channels per CTA -> V^T codes (microblocks along tokens) + scale atoms
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
-__global__ void __launch_bounds__(256, 5) quant_vt_kernel(const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn,
-                                                       int H, int N, int Np, uint8_t* __restrict__ codes,
-                                                       uint8_t* __restrict__ sfs) {
+__device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
+                                              uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, int tile, int bh, uint8_t* smem_raw) {
     constexpr int PITCH = D + 2;          // elements; word pitch odd -> column reads are conflict-free
-    const int tile = blockIdx.x, bh = blockIdx.y;
     const int b = bh / H, h = bh % H;
     const int t = threadIdx.x;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int row0 = tile * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
 
-    extern __shared__ __align__(16) uint8_t smem_raw[];
     T* s_v = reinterpret_cast<T*>(smem_raw);                                  // [128][PITCH]
     constexpr int OPITCH = 72;            // bytes per staged output row (64 + 8: 8-byte stores stay conflict-free)
     uint8_t* s_out = smem_raw + ((kBlock * PITCH * 2 + 15) / 16) * 16;          // [D][OPITCH] codes
@@ -612,55 +651,132 @@ __global__ void __launch_bounds__(256, 5) quant_vt_kernel(const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------
+// Everything of the pre-pass that reads raw inputs only, in one launch: partial column sums of K (and of Q, when it is smoothed
+// by one mean per head), V quantization, and Q quantization when it needs no mean of a whole head.  Block b works on the b-th
+// piece of the list; the parts have nothing to wait for from one another, so their tails and launch gaps disappear.
+// With the status words cleared here, the K mean formed by the K kernel where that is cheap, and the K and attention kernels
+// launched early (griddepcontrol), a call is 3 launches instead of 6 and 2 memsets: 1 024 tokens of two heads 51 -> 26 us, a
+// 3 001-token prompt 151 -> 106 us.  HBM-bound at size: 0.47 GB read and 0.16 GB written in 85 us for 17 550 queries of 96 heads.
+// ------------------------------------------------------------------------------------------------
+template <typename T>
+struct StageArgs {
+    Src<T> q, k, v;
+    int64_t qs[3], ks[3], vs[3];
+    int Hq, Hkv, Nq, Nk, Nq_p, Nk_p;
+    int n_colk, n_colq, n_q, n_v;      // pieces of each kind, in this order
+    int chunks_k, chunks_q, tiles_q, tiles_k;
+    int q_block_mean;
+    float *part_k, *part_q;
+    T *km, *qm;
+    uint8_t *q_codes, *q_sf, *v_codes, *v_sf;
+    float* qkm;                        // nullptr: not wanted
+    int* clear;                        // status words and work counter to zero (nullptr: not in this launch)
+    int n_clear;
+};
+
+template <typename T, int D>
+struct StageCfg {
+    static constexpr int kQ = D * 4 + (D / 64) * 512 + (kBlock + 4 * (32 / (D / 8))) * D * (int)sizeof(T);   // staged tile and chain sums
+    static constexpr int kV = ((kBlock * (D + 2) * (int)sizeof(T) + 15) / 16) * 16 + D * 72 + 1024;
+    static constexpr int kCol = (2048 / D) * (D + 1) * 4;
+    static constexpr int kSmem = kQ > kV ? (kQ > kCol ? kQ : kCol) : (kV > kCol ? kV : kCol);
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(256, 4) prepass_stage_kernel(const __grid_constant__ StageArgs<T> a) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    pdl_launch_dependents();
+    int i = blockIdx.x;
+    if (a.clear != nullptr && i == 0 && threadIdx.x < a.n_clear) a.clear[threadIdx.x] = 0;
+    if (i < a.n_colk) {
+        colsum_chunk<T, D>(a.k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk, a.part_k, a.chunks_k, i % a.chunks_k, i / a.chunks_k,
+                           reinterpret_cast<float*>(smem_raw));
+        return;
+    }
+    i -= a.n_colk;
+    if (i < a.n_colq) {
+        colsum_chunk<T, D>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.part_q, a.chunks_q, i % a.chunks_q, i / a.chunks_q,
+                           reinterpret_cast<float*>(smem_raw));
+        return;
+    }
+    i -= a.n_colq;
+    if (i < a.n_q) {
+        if (a.q_block_mean)
+            quant_q_tile<T, D, kModeQBlockMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, nullptr, a.qm, a.q_codes, a.q_sf, a.km,
+                                                a.Hq / a.Hkv, a.qkm, i % a.tiles_q, i / a.tiles_q, smem_raw);
+        else
+            quant_q_tile<T, D, kModeQGlobalMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, a.qm, nullptr, a.q_codes, a.q_sf, a.km,
+                                                 a.Hq / a.Hkv, a.qkm, i % a.tiles_q, i / a.tiles_q, smem_raw);
+        return;
+    }
+    i -= a.n_q;
+    quant_vt_tile<T, D>(a.v, a.vs[0], a.vs[1], a.vs[2], a.Hkv, a.Nk, a.Nk_p, a.v_codes, a.v_sf, i % a.tiles_k, i / a.tiles_k, smem_raw);
+}
+
+// ------------------------------------------------------------------------------------------------
 // host-side launch
 // ------------------------------------------------------------------------------------------------
+// Up to this many chunks (16 384 keys) every CTA of the K kernel forms the K mean itself from the partial sums (an 8 KB read
+// from L2 at 8 192 keys); beyond, one small kernel does.
+constexpr int kInlineMeanChunks = 32;
+
 template <typename T, int D>
 static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
-    const Src<T> q = make_src<T>(a.q, a.cu_q), k = make_src<T>(a.k, a.cu_k), v = make_src<T>(a.v, a.cu_k);
     T* km = static_cast<T*>(a.km);
     T* qm = static_cast<T*>(a.qm);
     T* delta = static_cast<T*>(a.delta);
     const int BHq = a.B * a.Hq, BHkv = a.B * a.Hkv;
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(prepass_stage_kernel<T, D>), StageCfg<T, D>::kSmem);
+    if (e != cudaSuccess) return e;
 
-    // K mean over its Nk tokens (unless the caller supplied it, e.g. the mean over all shards of a longer sequence)
-    if (!a.km_given) {
-        colsum_partial_kernel<T, D><<<dim3(a.kchunks_k, BHkv), 256, 0, st>>>(k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk,
-                                                                             a.kpart, a.kchunks_k);
-        colmean_finalize_kernel<T, D><<<BHkv, D, 0, st>>>(a.kpart, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0);
+    StageArgs<T> s = {};
+    s.q = make_src<T>(a.q, a.cu_q);
+    s.k = make_src<T>(a.k, a.cu_k);
+    s.v = make_src<T>(a.v, a.cu_k);
+    for (int i = 0; i < 3; ++i) {
+        s.qs[i] = a.qs[i];
+        s.ks[i] = a.ks[i];
+        s.vs[i] = a.vs[i];
     }
-
-    const size_t smem_q = D * 4 + (D / 64) * 512;
-    if (a.per_block_mean) {
-        // + the staged tile [128][D] and the chain sums [4 * 32 / (D / 8)][D] of the block mean
-        const size_t smem_qb = smem_q + (kBlock + 4 * (32 / (D / 8))) * D * sizeof(T);
-        quant_rows_kernel<T, D, kModeQBlockMean><<<dim3(a.Nq_p / kBlock, BHq), 256, smem_qb, st>>>(
-            q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, nullptr, qm, a.q_codes, a.q_sf, km, a.Hq / a.Hkv, a.qkm);
-    } else {
-        // one mean per head over the padded rows (api.py:88-90); kpart is free again: the K finalize has
-        // consumed it and stream order serializes the two uses
-        colsum_partial_kernel<T, D><<<dim3(a.kchunks_q, BHq), 256, 0, st>>>(q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq,
-                                                                            a.kpart, a.kchunks_q);
-        colmean_finalize_kernel<T, D><<<BHq, D, 0, st>>>(a.kpart, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1);
-        quant_rows_kernel<T, D, kModeQGlobalMean><<<dim3(a.Nq_p / kBlock, BHq), 256, smem_q, st>>>(
-            q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, qm, nullptr, a.q_codes, a.q_sf, km, a.Hq / a.Hkv, a.qkm);
+    s.Hq = a.Hq; s.Hkv = a.Hkv; s.Nq = a.Nq; s.Nk = a.Nk; s.Nq_p = a.Nq_p; s.Nk_p = a.Nk_p;
+    s.chunks_k = a.kchunks_k; s.chunks_q = a.kchunks_q; s.tiles_q = a.Nq_p / kBlock; s.tiles_k = a.Nk_p / kBlock;
+    s.q_block_mean = a.per_block_mean;
+    s.part_k = a.kpart; s.part_q = a.kpart + (size_t)BHkv * a.kchunks_k * D;
+    s.km = km; s.qm = qm;
+    s.q_codes = a.q_codes; s.q_sf = a.q_sf; s.v_codes = a.v_codes; s.v_sf = a.v_sf;
+    s.clear = a.clear; s.n_clear = a.n_clear;
+    // Q waits for the means when it is smoothed by one mean per head (api.py:88-90) or when q . km is wanted
+    const bool q_late = !a.per_block_mean || a.want_qkm;
+    const bool km_here = !a.km_given;
+    const bool km_inline = km_here && !q_late && a.kchunks_k <= kInlineMeanChunks;
+    s.n_colk = km_here ? a.kchunks_k * BHkv : 0;
+    s.n_colq = a.per_block_mean ? 0 : a.kchunks_q * BHq;
+    s.n_q = q_late ? 0 : s.tiles_q * BHq;
+    s.n_v = s.tiles_k * BHkv;
+    prepass_stage_kernel<T, D><<<s.n_colk + s.n_colq + s.n_q + s.n_v, 256, StageCfg<T, D>::kSmem, st>>>(s);
+    if (km_here && !km_inline)
+        colmean_finalize_kernel<T, D><<<BHkv, D, 0, st>>>(s.part_k, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0);
+    if (!a.per_block_mean)
+        colmean_finalize_kernel<T, D><<<BHq, D, 0, st>>>(s.part_q, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1);
+    if (q_late) {
+        s.n_colk = s.n_colq = s.n_v = 0;
+        s.n_q = s.tiles_q * BHq;
+        s.qkm = a.want_qkm ? a.qkm : nullptr;
+        s.clear = nullptr;
+        prepass_stage_kernel<T, D><<<s.n_q, 256, StageCfg<T, D>::kSmem, st>>>(s);
     }
     const size_t smem_k = 2 * (D / 64) * 16384 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + 32768 : 0);
-    cudaError_t e = cudaFuncSetAttribute(quant_k_delta_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k);
+    e = allow_smem(reinterpret_cast<const void*>(quant_k_delta_kernel<T, D>), (int)smem_k);
     if (e != cudaSuccess) return e;
-    // tensor maps for the K kernel: the Q means [B*Hq][nqm][D] and delta_s [B*Hq][nqm][Nk_p] as byte tensors
+    // tensor maps for the K kernel: the Q means and delta_s of a kv head's query heads follow one another, so both are byte
+    // tensors [B*Hkv][group * nqm][...] and one MMA takes the blocks of several heads
+    const uint64_t rows = (uint64_t)(a.Hq / a.Hkv) * a.nqm;
     alignas(64) CUtensorMap tm_qm, tm_delta;
-    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, (uint64_t)a.nqm, (uint64_t)a.B * a.Hq, 128, 128, 3) != 0 ||
-        encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, (uint64_t)a.nqm, (uint64_t)a.B * a.Hq, 128, 32, 3) != 0)
+    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, 128, 3) != 0 ||
+        encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    quant_k_delta_kernel<T, D><<<dim3(a.Nk_p / kBlock, BHkv), 256, smem_k, st>>>(
-        k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk, a.Nk_p, km, a.k_codes, a.k_sf, a.Hq, a.nqm, a.status, a.cu_q, tm_qm, tm_delta);
-
-    const size_t smem_v = ((kBlock * (D + 2) * sizeof(T) + 15) / 16) * 16 + D * 72 + 1024;
-    e = cudaFuncSetAttribute(quant_vt_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_v);
-    if (e != cudaSuccess) return e;
-    quant_vt_kernel<T, D><<<dim3(a.Nk_p / kBlock, BHkv), 256, smem_v, st>>>(v, a.vs[0], a.vs[1], a.vs[2], a.Hkv, a.Nk,
-                                                                           a.Nk_p, a.v_codes, a.v_sf);
-    return cudaGetLastError();
+    return launch_pdl(quant_k_delta_kernel<T, D>, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk,
+                      a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status, tm_qm, tm_delta);
 }
 
 cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t st) {
