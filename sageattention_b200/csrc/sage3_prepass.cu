@@ -19,6 +19,23 @@
 
 namespace sage3 {
 
+// Division of block indices by a run-time constant: q = (mulhi(n, m) + n) >> s for 0 <= n < 2^31 (Granlund and Montgomery 1994);
+// a plain integer division costs every thread of a block some 25 instructions.
+struct FastDiv {
+    uint32_t d, m, s;
+    FastDiv() = default;
+    explicit FastDiv(int div) : d((uint32_t)div), s(0) {
+        while ((1ull << s) < d) ++s;
+        m = (uint32_t)((((1ull << s) - d) << 32) / d + 1);
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s); }
+    __device__ __forceinline__ int divmod(int n, int& rem) const {
+        const int q = div(n);
+        rem = n - q * (int)d;
+        return q;
+    }
+};
+
 template <typename T> struct Num;
 template <> struct Num<__nv_bfloat16> {
     using T2 = __nv_bfloat162;
@@ -89,6 +106,19 @@ struct Src {
         }
         return b * sb + h * sh;
     }
+    // Visits rows r0, r0 + step, ... (n of them): f(i, pointer to the row).  One buffer: the pointer is stepped.
+    template <int n, typename F>
+    __device__ __forceinline__ void rows_each(int64_t bh_off, int r0, int step, int64_t sn, F f) const {
+        if (rows == 0) {
+            const T* p = part[0] + bh_off + (int64_t)r0 * sn;
+            const int64_t d = (int64_t)step * sn;
+#pragma unroll
+            for (int i = 0; i < n; ++i, p += d) f(i, p);
+        } else {
+#pragma unroll
+            for (int i = 0; i < n; ++i) f(i, row(bh_off, r0 + i * step, sn));
+        }
+    }
     __device__ __forceinline__ const T* row(int64_t bh_off, int r, int64_t sn) const {
         if (rows == 0) return part[0] + bh_off + (int64_t)r * sn;
         const int pi = min(r / rows, kMaxParts - 1);
@@ -126,20 +156,7 @@ __device__ __forceinline__ void unpack16(const uint4& a, const uint4& b, float* 
     }
 }
 
-// One NVFP4 microblock: 16 fp32 values (already on the input type's grid) and their maximum magnitude -> 8 bytes of
-// codes + scale byte.
-__device__ __forceinline__ void quant16_amax(const float* x, float amax, uint32_t& lo, uint32_t& hi, uint32_t& sf_byte) {
-    sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xffu;
-    const float sf = e4m3_to_float(sf_byte);
-    const float inv = (sf == 0.f) ? 0.f : __frcp_rn(sf);
-    float y[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) y[i] = __fmul_rn(x[i], inv);
-    lo = cvt_e2m1x8(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]);
-    hi = cvt_e2m1x8(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]);
-}
-
-// The same from eight packed words of the input type (16 values): the maximum magnitude is found on the packed pairs
+// One NVFP4 microblock, eight packed words of the input type (16 values) -> 8 bytes of codes + scale byte: the maximum magnitude is found on the packed pairs
 // (exact, as fp4_quantization_4d.cu:186-196 does), the scaling runs in fp32.
 template <typename T>
 __device__ __forceinline__ void quant16_packed(const uint32_t* w, uint32_t& lo, uint32_t& hi, uint32_t& sf_byte) {
@@ -167,11 +184,12 @@ __device__ __forceinline__ void quant16_packed(const uint32_t* w, uint32_t& lo, 
 // (deterministic: no atomics, the summation order depends on N only)
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
-__device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, float* __restrict__ part,
+__device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, float* __restrict__ part,
                                              int chunks, int chunk, int bh, float* red) {   // red: shared, [RPP][D + 1]
     constexpr int TPR = D / 8;           // threads per row (8 elements = 16 bytes each)
     constexpr int RPP = 256 / TPR;       // rows per pass
-    const int b = bh / H, h = bh % H;
+    int h;
+    const int b = H.divmod(bh, h);
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int c8 = threadIdx.x % TPR, rl = threadIdx.x / TPR;
     const int r0 = chunk * kRowsPerChunk;
@@ -179,14 +197,13 @@ __device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     // Eight rows in flight per thread (a load per addition made the two CTAs of a 1 024-token head take 19 us); the additions
     // keep their order.
-    constexpr int U = 8;
+    constexpr int U = D == 64 ? 4 : 8;
     for (int r = r0 + rl; r < r1; r += U * RPP) {
         uint4 a[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
+        x.template rows_each<U>(bh_off, r, RPP, sn, [&](int u, const T* p) {
             a[u] = make_uint4(0, 0, 0, 0);
-            if (r + u * RPP < r1) a[u] = __ldg(reinterpret_cast<const uint4*>(x.row(bh_off, r + u * RPP, sn) + c8 * 8));
-        }
+            if (r + u * RPP < r1) a[u] = __ldg(reinterpret_cast<const uint4*>(p + c8 * 8));
+        });
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t w[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
@@ -225,7 +242,7 @@ __device__ __forceinline__ float sum_chunks(const float* __restrict__ part, int 
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(256) colsum_partial_kernel(const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N,
                                                              float* __restrict__ part, int chunks) {
     __shared__ float red[(2048 / D) * (D + 1)];
     colsum_chunk<T, D>(x, sb, sh, sn, H, N, part, chunks, blockIdx.x, blockIdx.y, red);
@@ -253,7 +270,7 @@ enum { kModeQBlockMean = 0, kModeQGlobalMean = 1 };
 
 template <typename T, int D, int MODE>
 __device__ __forceinline__ void quant_q_tile(
-    const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
+    const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     const T* __restrict__ mean_in,     // one mean per head: qm [B*H][D]; unused for block mean
     T* __restrict__ qm_out,            // block mean: [B*H][Np/128][D]
     uint8_t* __restrict__ codes,       // [B*H][Np][D/2]
@@ -266,7 +283,8 @@ __device__ __forceinline__ void quant_q_tile(
     constexpr int RPP = 256 / CH;         // rows per pass
     constexpr int ITEMS = kBlock / RPP;   // microblocks per thread
 
-    const int b = bh / H, h = bh % H;
+    int h;
+    const int b = H.divmod(bh, h);
     const int t = threadIdx.x;
     const int c = t % CH, rl = t / CH;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
@@ -278,15 +296,13 @@ __device__ __forceinline__ void quant_q_tile(
     uint8_t* s_more = s_sf + (D / 64) * 512;                                   // block mean only: staged tile, chain sums
 
     uint4 raw[ITEMS][2];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int r = row0 + rl + RPP * i;
-        load16_packed<T>(x.row(bh_off, r, sn) + c * 16, r < N, raw[i][0], raw[i][1]);
-    }
+    x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
+        load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
+    });
 
     // x . km of every row: 16 products per thread, then a sum over the CH neighbouring lanes that share the row
     if (qkm != nullptr) {
-        const T* kmh = km + ((int64_t)b * (H / group) + h / group) * D + c * 16;
+        const T* kmh = km + ((int64_t)b * ((int)H.d / group) + h / group) * D + c * 16;
         uint4 k0, k1;
         load16_packed<T>(kmh, true, k0, k1);
         float kf[16];
@@ -403,7 +419,7 @@ __device__ __forceinline__ void quant_q_tile(
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
 __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
-    const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
+    const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     T* __restrict__ km,                // [B*H][D]
     const float* __restrict__ part,    // partial column sums to form the mean from ([B*H][chunks][D]), or nullptr: `km` holds it
     int chunks,
@@ -421,7 +437,8 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     constexpr bool kBf16 = sizeof(T) == 2 && Num<T>::kIsBf16;
 
     const int tile = blockIdx.x, bh = blockIdx.y;
-    const int b = bh / H, h = bh % H;
+    int h;
+    const int b = H.divmod(bh, h);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int c = t % CH, rl = t / CH;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
@@ -453,11 +470,9 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
         tmem_relinquish();
     }
     uint4 raw[ITEMS][2];
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const int r = row0 + rl + RPP * i;
-        load16_packed<T>(x.row(bh_off, r, sn) + c * 16, r < N, raw[i][0], raw[i][1]);
-    }
+    x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
+        load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
+    });
     pdl_launch_dependents();
     pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
     if (t < D) {
@@ -588,10 +603,11 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
 // V: one tile of 128 tokens x D channels per CTA -> V^T codes (microblocks along tokens) + scale atoms
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
-__device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int H, int N, int Np,
+__device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
                                               uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, int tile, int bh, uint8_t* smem_raw) {
     constexpr int PITCH = D + 2;          // elements; word pitch odd -> column reads are conflict-free
-    const int b = bh / H, h = bh % H;
+    int h;
+    const int b = H.divmod(bh, h);
     const int t = threadIdx.x;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int row0 = tile * kBlock;
@@ -606,36 +622,51 @@ __device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64
     if (t < 64) reinterpret_cast<uint4*>(s_sf)[t] = make_uint4(0, 0, 0, 0);
     // coalesced load: 16 bytes per thread per pass
     constexpr int TPR = D / 8, RPP = 256 / TPR;
-    for (int r = t / TPR; r < kBlock; r += RPP) {
-        const int c8 = t % TPR;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (row0 + r < N) val = __ldg(reinterpret_cast<const uint4*>(x.row(bh_off, row0 + r, sn) + c8 * 8));
-        uint32_t* dst = reinterpret_cast<uint32_t*>(s_v + r * PITCH + c8 * 8);   // 4-byte aligned (PITCH even)
-        dst[0] = val.x; dst[1] = val.y; dst[2] = val.z; dst[3] = val.w;
+    {
+        const int c8 = t % TPR, rl = t / TPR;
+        uint4 val[kBlock / RPP];
+        x.template rows_each<kBlock / RPP>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
+            val[i] = make_uint4(0, 0, 0, 0);
+            if (row0 + rl + i * RPP < N) val[i] = __ldg(reinterpret_cast<const uint4*>(p + c8 * 8));
+        });
+#pragma unroll
+        for (int i = 0; i < kBlock / RPP; ++i) {
+            uint32_t* dst = reinterpret_cast<uint32_t*>(s_v + (rl + i * RPP) * PITCH + c8 * 8);   // 4-byte aligned (PITCH even)
+            dst[0] = val[i].x; dst[1] = val[i].y; dst[2] = val[i].z; dst[3] = val[i].w;
+        }
     }
     __syncthreads();
     // two microblocks per item: (channels 2*dp and 2*dp + 1, token group mb); channel pair fastest across
     // threads, so every shared-memory read is one conflict-free 32-bit word holding both channels
     for (int item = t; item < (D / 2) * 8; item += 256) {
         const int dp = item % (D / 2), mb = item / (D / 2);
-        float y0[16], y1[16];
+        uint32_t w[16];             // 16 tokens of both channels
         uint32_t m2 = 0u;           // running maximum magnitude of both channels, packed
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const uint32_t w = *reinterpret_cast<const uint32_t*>(s_v + (mb * 16 + i) * PITCH + 2 * dp);
-            m2 = Num<T>::absmax2(m2, w);
-            const float2 v2 = Num<T>::to_f2(w);
-            y0[i] = v2.x;
-            y1[i] = v2.y;
+            w[i] = *reinterpret_cast<const uint32_t*>(s_v + (mb * 16 + i) * PITCH + 2 * dp);
+            m2 = Num<T>::absmax2(m2, w[i]);
         }
         const float2 amax2 = Num<T>::to_f2(m2);
-        uint32_t lo, hi, sfb;
-        quant16_amax(y0, amax2.x, lo, hi, sfb);
-        *reinterpret_cast<uint2*>(s_out + (2 * dp) * OPITCH + mb * 8) = make_uint2(lo, hi);
-        s_sf[sf_atom_offset(2 * dp, mb)] = static_cast<uint8_t>(sfb);
-        quant16_amax(y1, amax2.y, lo, hi, sfb);
-        *reinterpret_cast<uint2*>(s_out + (2 * dp + 1) * OPITCH + mb * 8) = make_uint2(lo, hi);
-        s_sf[sf_atom_offset(2 * dp + 1, mb)] = static_cast<uint8_t>(sfb);
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+            const uint32_t sfb = cvt_e4m3x2(__fdiv_rn(ch == 0 ? amax2.x : amax2.y, 6.0f), 0.f) & 0xffu;
+            const float sf = e4m3_to_float(sfb);
+            const float inv = (sf == 0.f) ? 0.f : __frcp_rn(sf);
+            uint32_t code[2];
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                float y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 v2 = Num<T>::to_f2(w[8 * g + i]);
+                    y[i] = __fmul_rn(ch == 0 ? v2.x : v2.y, inv);
+                }
+                code[g] = cvt_e2m1x8(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]);
+            }
+            *reinterpret_cast<uint2*>(s_out + (2 * dp + ch) * OPITCH + mb * 8) = make_uint2(code[0], code[1]);
+            s_sf[sf_atom_offset(2 * dp + ch, mb)] = static_cast<uint8_t>(sfb);
+        }
     }
     __syncthreads();
     // coalesced stores: D rows of 64 bytes
@@ -662,9 +693,9 @@ template <typename T>
 struct StageArgs {
     Src<T> q, k, v;
     int64_t qs[3], ks[3], vs[3];
-    int Hq, Hkv, Nq, Nk, Nq_p, Nk_p;
+    FastDiv Hq, Hkv, chunks_k, chunks_q, tiles_q, tiles_k;
+    int group, Nq, Nk, Nq_p, Nk_p;
     int n_colk, n_colq, n_q, n_v;      // pieces of each kind, in this order
-    int chunks_k, chunks_q, tiles_q, tiles_k;
     int q_block_mean;
     float *part_k, *part_q;
     T *km, *qm;
@@ -682,35 +713,40 @@ struct StageCfg {
     static constexpr int kSmem = kQ > kV ? (kQ > kCol ? kQ : kCol) : (kV > kCol ? kV : kCol);
 };
 
+// Six resident blocks at D = 64 (40 registers, column sums four rows deep): 17 550 queries of 96 heads 71 -> 58 us against four.  At
+// D = 128 four: five spill (131 -> 149 us for 8 x 8 x 8 192 keys with their K kernel).
 template <typename T, int D>
-__global__ void __launch_bounds__(256, 4) prepass_stage_kernel(const __grid_constant__ StageArgs<T> a) {
+__global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(const __grid_constant__ StageArgs<T> a) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     pdl_launch_dependents();
     int i = blockIdx.x;
     if (a.clear != nullptr && i == 0 && threadIdx.x < a.n_clear) a.clear[threadIdx.x] = 0;
+    int tile, bh;
     if (i < a.n_colk) {
-        colsum_chunk<T, D>(a.k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk, a.part_k, a.chunks_k, i % a.chunks_k, i / a.chunks_k,
-                           reinterpret_cast<float*>(smem_raw));
+        bh = a.chunks_k.divmod(i, tile);
+        colsum_chunk<T, D>(a.k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk, a.part_k, a.chunks_k.d, tile, bh, reinterpret_cast<float*>(smem_raw));
         return;
     }
     i -= a.n_colk;
     if (i < a.n_colq) {
-        colsum_chunk<T, D>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.part_q, a.chunks_q, i % a.chunks_q, i / a.chunks_q,
-                           reinterpret_cast<float*>(smem_raw));
+        bh = a.chunks_q.divmod(i, tile);
+        colsum_chunk<T, D>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.part_q, a.chunks_q.d, tile, bh, reinterpret_cast<float*>(smem_raw));
         return;
     }
     i -= a.n_colq;
     if (i < a.n_q) {
+        bh = a.tiles_q.divmod(i, tile);
         if (a.q_block_mean)
             quant_q_tile<T, D, kModeQBlockMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, nullptr, a.qm, a.q_codes, a.q_sf, a.km,
-                                                a.Hq / a.Hkv, a.qkm, i % a.tiles_q, i / a.tiles_q, smem_raw);
+                                                a.group, a.qkm, tile, bh, smem_raw);
         else
             quant_q_tile<T, D, kModeQGlobalMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, a.qm, nullptr, a.q_codes, a.q_sf, a.km,
-                                                 a.Hq / a.Hkv, a.qkm, i % a.tiles_q, i / a.tiles_q, smem_raw);
+                                                 a.group, a.qkm, tile, bh, smem_raw);
         return;
     }
     i -= a.n_q;
-    quant_vt_tile<T, D>(a.v, a.vs[0], a.vs[1], a.vs[2], a.Hkv, a.Nk, a.Nk_p, a.v_codes, a.v_sf, i % a.tiles_k, i / a.tiles_k, smem_raw);
+    bh = a.tiles_k.divmod(i, tile);
+    quant_vt_tile<T, D>(a.v, a.vs[0], a.vs[1], a.vs[2], a.Hkv, a.Nk, a.Nk_p, a.v_codes, a.v_sf, tile, bh, smem_raw);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -738,8 +774,10 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         s.ks[i] = a.ks[i];
         s.vs[i] = a.vs[i];
     }
-    s.Hq = a.Hq; s.Hkv = a.Hkv; s.Nq = a.Nq; s.Nk = a.Nk; s.Nq_p = a.Nq_p; s.Nk_p = a.Nk_p;
-    s.chunks_k = a.kchunks_k; s.chunks_q = a.kchunks_q; s.tiles_q = a.Nq_p / kBlock; s.tiles_k = a.Nk_p / kBlock;
+    const int tiles_q = a.Nq_p / kBlock, tiles_k = a.Nk_p / kBlock;
+    s.Hq = FastDiv(a.Hq); s.Hkv = FastDiv(a.Hkv);
+    s.chunks_k = FastDiv(a.kchunks_k); s.chunks_q = FastDiv(a.kchunks_q); s.tiles_q = FastDiv(tiles_q); s.tiles_k = FastDiv(tiles_k);
+    s.group = a.Hq / a.Hkv; s.Nq = a.Nq; s.Nk = a.Nk; s.Nq_p = a.Nq_p; s.Nk_p = a.Nk_p;
     s.q_block_mean = a.per_block_mean;
     s.part_k = a.kpart; s.part_q = a.kpart + (size_t)BHkv * a.kchunks_k * D;
     s.km = km; s.qm = qm;
@@ -751,8 +789,8 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     const bool km_inline = km_here && !q_late && a.kchunks_k <= kInlineMeanChunks;
     s.n_colk = km_here ? a.kchunks_k * BHkv : 0;
     s.n_colq = a.per_block_mean ? 0 : a.kchunks_q * BHq;
-    s.n_q = q_late ? 0 : s.tiles_q * BHq;
-    s.n_v = s.tiles_k * BHkv;
+    s.n_q = q_late ? 0 : tiles_q * BHq;
+    s.n_v = tiles_k * BHkv;
     prepass_stage_kernel<T, D><<<s.n_colk + s.n_colq + s.n_q + s.n_v, 256, StageCfg<T, D>::kSmem, st>>>(s);
     if (km_here && !km_inline)
         colmean_finalize_kernel<T, D><<<BHkv, D, 0, st>>>(s.part_k, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0);
@@ -760,7 +798,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         colmean_finalize_kernel<T, D><<<BHq, D, 0, st>>>(s.part_q, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1);
     if (q_late) {
         s.n_colk = s.n_colq = s.n_v = 0;
-        s.n_q = s.tiles_q * BHq;
+        s.n_q = tiles_q * BHq;
         s.qkm = a.want_qkm ? a.qkm : nullptr;
         s.clear = nullptr;
         prepass_stage_kernel<T, D><<<s.n_q, 256, StageCfg<T, D>::kSmem, st>>>(s);
@@ -775,7 +813,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, 128, 3) != 0 ||
         encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    return launch_pdl(quant_k_delta_kernel<T, D>, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], a.Hkv, a.Nk,
+    return launch_pdl(quant_k_delta_kernel<T, D>, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
                       a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status, tm_qm, tm_delta);
 }
 
@@ -823,7 +861,7 @@ cudaError_t launch_kmean_t(const Sage3Desc* d, const void* k, void* km, float* s
     sage3::PartsPtr one = {};
     one.base[0] = const_cast<void*>(k);
     sage3::colsum_partial_kernel<T, D><<<dim3(chunks, BH), 256, 0, st>>>(
-        sage3::make_src<T>(one), d->k_stride[0], d->k_stride[1], d->k_stride[2], d->Hkv, d->Nk, scratch, chunks);
+        sage3::make_src<T>(one), d->k_stride[0], d->k_stride[1], d->k_stride[2], sage3::FastDiv(d->Hkv), d->Nk, scratch, chunks);
     sage3::colmean_finalize_kernel<T, D><<<BH, D, 0, st>>>(scratch, chunks, 1.0f / (float)d->Nk, static_cast<T*>(km), nullptr, d->Hkv, 0);
     return cudaGetLastError();
 }
