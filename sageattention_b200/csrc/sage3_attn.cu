@@ -54,6 +54,7 @@ constexpr float kPScaleLog2 = -11.392317422778762f;   // log2(1 / (448 * 6)), so
 struct AttnParams {
     int BHq, Hq, Hkv, Nq, Nk, nqt, nkb, nqm;   // nqt = query tiles per head, nkb = KV blocks per head
     int units, whole_units;             // units of work; those from whole_units on are single query tiles instead of pairs
+    int pack_heads, pack_tiles;         // PACK kernels: query heads per tile, tiles per kv head
     int* unit_counter;                  // zero at launch: next unit after the first gridDim.x
     float sm_scale_log2;
     const float* sm_scale_per_head;
@@ -76,9 +77,12 @@ struct AttnParams {
 
 constexpr int kUnitRing = 4;
 
-template <int D>
+// PACK: few query rows and several query heads per kv head.  The rows of all these heads share one 128-row tile (row = head * Nq +
+// token), so the keys are walked once instead of once per head: 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv
+// heads 122 -> 64 us.
+template <int D, bool PACK>
 struct Cfg {
-    static constexpr int kStages = (D == 128) ? 4 : 8;        // K and V^T stages, each shared by the two query tiles
+    static constexpr int kStages = (D == 128) ? 4 : (PACK ? 6 : 8);        // K and V^T stages, each shared by the two query tiles
     static constexpr int kThreads = 768;                      // 6 warpgroups, see the kernel
     // S buffers of 128 rows x 64 keys: a rotation for the first halves of the items and one for the second halves
     static constexpr int kSBufs0 = 2, kSBufs1 = (D == 128) ? 1 : 2, kSBufs = kSBufs0 + kSBufs1;
@@ -98,9 +102,10 @@ struct Cfg {
     static constexpr int oSfK = oSfQ + 4 * 1024;
     static constexpr int oSfV = oSfK + kStages * 1024;
     static constexpr int oSfP = oSfV + kStages * 1024;        // [slot] 1024
-    static constexpr int kDeltaPitch = 512;                   // 256 B of delta_s + 256 B that stay zero
-    static constexpr int oDelta = oSfP + 8 * 1024;            // [stage][tile] kDeltaPitch
-    static constexpr int oOnes = oDelta + kStages * 2 * kDeltaPitch;   // 128 x 16 tile: column 0 = 1.0, rest 0
+    // delta_s per stage: one row per tile, 256 B + 256 B that stay zero; PACK: [16 chunks of 8 keys][8 heads] 16 B + 128 B that stay zero
+    static constexpr int kDeltaPitch = 512, kDeltaStage = PACK ? 16 * 128 + 128 : 2 * kDeltaPitch;
+    static constexpr int oDelta = oSfP + 8 * 1024;            // [stage] kDeltaStage
+    static constexpr int oOnes = oDelta + kStages * kDeltaStage;   // 128 x 16 tile: 1.0 in column 0 (PACK: in the column of the row's head), rest 0
     static constexpr int oStat = oOnes + 4096;                // float2 [slot][128 rows]: running maximum, rescale factor
     static constexpr int oSum = oStat + 8192;                 // float2 [slot][128 rows]: row sums of the two key halves of a block
     static constexpr int oL = oSum + 8192;                    // float2 [tile][128 rows]: running row sums of the two key halves
@@ -145,7 +150,7 @@ struct __align__(16) Unit {
     int nbmax;                    // the unit walks key block n = nbmax - 1 ... 0
     int mt0, nv;                  // first query tile, number of tiles
     int Nq, Nk, shift;            // lengths of this batch entry; key j is visible to query i iff j <= i + shift
-    int nb[2];                    // key blocks per tile
+    int nb[2];                    // key blocks per tile (PACK: nb[1] = query heads in the tile, bhq, hq = the first of them)
     int bhq, hq, bhkv;
     int64_t out_base;
 };
@@ -153,8 +158,25 @@ struct __align__(16) Unit {
 // Unit number u of the launch; false when it is empty (beyond a short sequence of a packed batch).
 // Order: without a mask pairs of tiles of one head are neighbours (its K and V are shared in L2); under a causal mask the
 // pairs with the most keys of all heads come first, so that the short ones level out the end of the launch.
-template <bool CAUSAL, bool VARLEN>
+template <bool CAUSAL, bool VARLEN, bool PACK>
 __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
+    if constexpr (PACK) {
+        w.bhkv = u / p.pack_tiles;
+        const int h0 = (u % p.pack_tiles) * p.pack_heads, group = p.Hq / p.Hkv, b = w.bhkv / p.Hkv;
+        w.hq = (w.bhkv % p.Hkv) * group + h0;
+        w.bhq = b * p.Hq + w.hq;
+        w.mt0 = 0;
+        w.nv = 1;
+        w.Nq = p.Nq;
+        w.Nk = p.Nk;
+        w.shift = p.causal_shift;
+        w.out_base = b * p.os0;
+        const int max_key = CAUSAL ? min(w.Nk - 1, w.Nq - 1 + w.shift) : w.Nk - 1;
+        w.nb[0] = w.nbmax = w.ns = max_key < 0 ? 0 : max_key / kBlock + 1;
+        w.nb[1] = min(p.pack_heads, group - h0);
+        w.two = w.d = 0;
+        return true;
+    }
     const int npair = (p.nqt + 1) >> 1;
     int pair = u, half = -1;
     if (u >= p.whole_units) {                      // the last units are single tiles
@@ -207,11 +229,11 @@ __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
     return true;
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN>
-__global__ void __launch_bounds__(Cfg<D>::kThreads, 1)
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, bool PACK>
+__global__ void __launch_bounds__(Cfg<D, PACK>::kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ AttnParams p) {
-    using C = Cfg<D>;
+                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ AttnParams p) {
+    using C = Cfg<D, PACK>;
     constexpr int S = C::kStages;
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t sbase = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -244,13 +266,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (threadIdx.x == 0) {
         *abort_flag = 0;
     }
-    // delta_s stages: the 256 bytes behind each row stay zero for the whole kernel; ones tile:
-    // [k chunk][row group][8 rows][16 bytes], 1.0 in element 0 of every row of chunk 0
+    // delta_s stages: the bytes behind the rows stay zero for the whole kernel; ones tile:
+    // [k chunk][row group][8 rows][16 bytes], 1.0 in element 0 of every row of chunk 0 (PACK: in the element of the row's head);
+    // PACK: rows beyond the packed ones stay zero, codes and scales
     {
         uint4* z = reinterpret_cast<uint4*>(sgen + C::oDelta);
-        constexpr int nd = S * 2 * C::kDeltaPitch / 16;
+        constexpr int nd = S * C::kDeltaStage / 16;
         const uint32_t one = std::is_same<OutT, __nv_bfloat16>::value ? 0x3F80u : 0x3C00u;
-        for (int i = threadIdx.x; i < nd + 4096 / 16; i += C::kThreads) z[i] = make_uint4(i >= nd && i < nd + 128 ? one : 0u, 0, 0, 0);
+        for (int i = threadIdx.x; i < nd + 4096 / 16; i += C::kThreads) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (i >= nd && i < nd + 128) {
+                const int g = PACK ? (i - nd) / p.Nq : 0;
+                const uint32_t w = one << (16 * (g & 1));
+                if (!PACK || g < p.pack_heads) v = make_uint4(g >> 1 == 0 ? w : 0, g >> 1 == 1 ? w : 0, g >> 1 == 2 ? w : 0, g >> 1 == 3 ? w : 0);
+            }
+            z[i] = v;
+        }
+        if constexpr (PACK) {
+            for (int i = threadIdx.x; i < 4 * 8192 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oQ)[i] = make_uint4(0, 0, 0, 0);
+            for (int i = threadIdx.x; i < 4 * 1024 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oSfQ)[i] = make_uint4(0, 0, 0, 0);
+        }
         fence_proxy_async_smem();
     }
     if (warp == 1) {
@@ -293,6 +328,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // ------------------------------------------------------------------ O rescale (correction) and output, one warp per lane quarter
       // Also keeps the running row sums: l = l alpha + (sum over the block), for each half of the keys.
       const int quarter = warp & 3, row = quarter * 32 + lane;
+      const int prow_head = PACK ? row / p.Nq : 0, prow_tok = PACK ? row - prow_head * p.Nq : 0;      // packed row -> head, token
       const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
       const float2* stat = reinterpret_cast<const float2*>(sgen + C::oStat) + row;
       const float2* sum = reinterpret_cast<const float2*>(sgen + C::oSum) + row;
@@ -370,8 +406,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           // ---------------------------------------------------------------- O / l of the unit's tiles
           // (The accumulators belong to the next unit once this warpgroup arrives for its first items.)
           for (int t = 0; ok && t < w.nv; ++t) {
-              const int grow = (w.mt0 + t) * kBlock + row;
-              const bool live = grow < w.Nq;
+              const int grow = PACK ? prow_tok : (w.mt0 + t) * kBlock + row;
+              const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq;
+              const int bhq = w.bhq + prow_head, hq = w.hq + prow_head;
               const bool have = w.nb[t] > 0 || carry_in;
               if (w.nb[t] > 0) {
                   const int sl = base + (w.two ? 2 * (w.nbmax - 1) + t - w.d : w.nb[t] - 1);       // the tile's last item
@@ -382,14 +419,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const float l_tot = l2.x + l2.y;
               if (live && (p.lse != nullptr || p.carry_o_out != nullptr)) {
                   const float m_fin = m_s[t * 128];
-                  const size_t crow = (size_t)w.bhq * p.Nq + grow;
+                  const size_t crow = (size_t)bhq * p.Nq + grow;
                   if (p.lse != nullptr) {
                       // ln sum_k exp(scale * q.k): the kernel's row sum is 2688 * sum_k 2^((S_k - m) s) over the smoothed
                       // scores S (delta_s included); K smoothing took scale * q.km out of every score of the row
-                      const float scale = p.sm_scale_per_head ? p.sm_scale_per_head[w.hq] : p.sm_scale;
+                      const float scale = p.sm_scale_per_head ? p.sm_scale_per_head[hq] : p.sm_scale;
                       const float ms_fin = (m_fin == -INFINITY ? 0.f : m_fin) * (p.sm_scale_per_head ? scale * 1.4426950408889634f : p.sm_scale_log2);
                       const float v = (ms_fin + __log2f(l_tot) + kPScaleLog2) * 0.6931471805599453f +
-                                      scale * p.qkm[(size_t)w.bhq * p.nqt * kBlock + grow];
+                                      scale * p.qkm[(size_t)bhq * p.nqt * kBlock + grow];
                       p.lse[crow] = (l_tot == 0.f) ? -INFINITY : v;
                   }
                   if (p.carry_o_out != nullptr) {
@@ -402,7 +439,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               // output goes straight back to the token shards of a sequence-parallel group: plain stores)
               const int opart = (p.out_rows == 0) ? 0 : min(grow / p.out_rows, kMaxParts - 1);
               OutT* orow = p.out[opart] == nullptr || !live ? nullptr
-                         : static_cast<OutT*>(p.out[opart]) + w.out_base + w.hq * p.os1 + (int64_t)(grow - opart * p.out_rows) * p.os2;
+                         : static_cast<OutT*>(p.out[opart]) + w.out_base + hq * p.os1 + (int64_t)(grow - opart * p.out_rows) * p.os2;
               for (int c = 0; c < D; c += 16) {
                   float o[16];
                   if (have) {
@@ -415,7 +452,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   if (p.carry_o_out != nullptr && live) {
 #pragma unroll
                       for (int q = 0; q < 4; ++q)
-                          *reinterpret_cast<float4*>(p.carry_o_out + ((size_t)w.bhq * p.Nq + grow) * D + c + 4 * q) =
+                          *reinterpret_cast<float4*>(p.carry_o_out + ((size_t)bhq * p.Nq + grow) * D + c + 4 * q) =
                               make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                   }
                   if (orow != nullptr) {
@@ -448,7 +485,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             Unit w;
             const bool more = u < p.units;
             if (!more) w.ns = -1;
-            else if (!make_unit<CAUSAL, VARLEN>(p, u, w)) { u = uniform(next); continue; }
+            else if (!make_unit<CAUSAL, VARLEN, PACK>(p, u, w)) { u = uniform(next); continue; }
             if (!warp_wait<true>(bar(bWE + k % kUnitRing), ((k / kUnitRing) & 1) ^ 1, abort_flag, p.status, kWaitUnit)) break;
             if (lane == 0) {
                 *reinterpret_cast<Unit*>(sgen + C::oUnit + (k % kUnitRing) * 64) = w;
@@ -462,7 +499,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             ++kq;
             const uint16_t* dptr0 = p.delta + ((size_t)w.bhq * p.nqm + ((p.nqm > 1) ? w.mt0 : 0)) * ((size_t)p.nkb * kBlock);
             const size_t dstep = (p.nqm > 1) ? (size_t)p.nkb * kBlock : 0;
-            if (lane == 0) {
+            if constexpr (PACK) {
+                // one box holds the rows of all heads; the scales move one word (four scales of a row) at a time into the packed row's place
+                const int live = w.nb[1] * p.Nq;
+                for (int r = lane; r < live; r += 32) {
+                    const int g = r / p.Nq, i = r - g * p.Nq;
+#pragma unroll
+                    for (int a = 0; a < D / 64; ++a)
+                        *reinterpret_cast<uint32_t*>(sgen + C::oSfQ + qb * 2048 + sf_atom_offset(r, 4 * a)) =
+                            *reinterpret_cast<const uint32_t*>(p.q_sf + (size_t)(w.bhq + g) * C::kSfQkBytes + sf_atom_offset(i, 4 * a));
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_expect_tx(bar(bQF + qb), p.pack_heads * p.Nq * (D / 2));
+                    tma_load_3d(sbase + C::oQ + qb * 2 * 8192, &tm_q, bar(bQF + qb), 0, 0, w.bhq);
+                }
+            } else if (lane == 0) {
                 mbar_expect_tx(bar(bQF + qb), w.nv * (C::kQBytes + C::kSfQkBytes));
                 for (int t = 0; t < w.nv; ++t) {
                     tma_load_3d(sbase + C::oQ + (qb * 2 + t) * 8192, &tm_q, bar(bQF + qb), 0, (w.mt0 + t) * kBlock, w.bhq);
@@ -473,11 +526,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int n = w.nbmax - 1; n >= 0; --n) {
                 if (!warp_wait<true>(bar(bKE + st), st_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
                 if (lane == 0) {
-                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + w.nv * C::kDeltaBytes);
+                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (PACK ? 8 : w.nv) * C::kDeltaBytes);
                     tma_load_3d(sbase + C::oK + st * C::kKBytes, &tm_k, bar(bKF + st), 0, n * kBlock, w.bhkv);
                     bulk_load(sbase + C::oSfK + st * 1024, p.k_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfQkBytes,
                               C::kSfQkBytes, bar(bKF + st));
-                    for (int t = 0; t < w.nv; ++t)
+                    // PACK: [16 chunks of 8 keys][8 heads], the canonical core matrices of an MN-major operand (heads beyond the packed ones
+                    // bring data that meets zeros).  One tensor copy: 64 copies of 16 bytes took 2.9 us per key block.
+                    if constexpr (PACK) tma_load_3d(sbase + C::oDelta + st * C::kDeltaStage, &tm_d, bar(bKF + st), 0, w.bhq, n * (kBlock / 8));
+                    for (int t = 0; !PACK && t < w.nv; ++t)
                         bulk_load(sbase + C::oDelta + (st * 2 + t) * C::kDeltaPitch, dptr0 + t * dstep + (size_t)n * kBlock,
                                   C::kDeltaBytes, bar(bKF + st));
                 }
@@ -504,9 +560,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         constexpr uint32_t idesc_qk = make_idesc_nvfp4(64);
         constexpr uint32_t idesc_delta = make_idesc_f16_bmn(64, std::is_same<OutT, __nv_bfloat16>::value);
         // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
-        constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(16, kSwzNone);
+        constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(PACK ? 128 : 16, kSwzNone);
         const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo0 = sdesc_lo(sbase + C::oQ, 16), sfq_lo0 = sdesc_lo(sbase + C::oSfQ, 0);
-        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 128, 16);
+        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_lo0 = sdesc_lo(sbase + C::oDelta + h * (PACK ? 1024 : 128), PACK ? 128 : 16);
         const uint32_t sfk_lo0 = sdesc_lo(sbase + C::oSfK, 0);
         // each issuer has its own copies of the scale factors in tensor memory, so that its MMAs and copies stay in one order
         const uint32_t sfk_col = tmem + C::cSfK + 8 * h;        // the 128-key atoms; keys 64 .. 127 start two columns in
@@ -537,7 +593,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 if (opens && !warp_wait(bar(bKF + st), st_parity, abort_flag, p.status, kWaitKFull)) { ok = false; break; }
                 if (!warp_wait(bar(bSE + buf0 + buf), buf_parity, abort_flag, p.status, kWaitSEmpty)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t k_lo = k_lo0 + st * (C::kKBytes / 16), delta_lo = delta_lo0 + (st * 2 + t) * (C::kDeltaPitch / 16);
+                const uint32_t k_lo = k_lo0 + st * (C::kKBytes / 16), delta_lo = delta_lo0 + st * (C::kDeltaStage / 16) + t * (C::kDeltaPitch / 16);
                 const uint32_t sfk_lo = sfk_lo0 + st * (1024 / 16), q_lo = q_lo0 + (qb * 2 + t) * (8192 / 16);
                 const uint32_t s_col = tmem + C::cS + 64 * (buf0 + buf), sfq_col = sfq_col0 + 8 * t;
                 if (elect_one()) {
@@ -546,7 +602,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         for (int ks = 0; ks < D / 64; ++ks) tc_cp_sf(sfk_col + 4 * ks, sdesc(sfk_lo + ks * 32, sdesc_hi(128, kSwzNone)));
                     }
                     // S <- 1 (x) delta_s: A = [128 x 16] with ones in column 0 (K-major), B = 64 elements of the delta_s row read as an
-                    // MN-major [16 x 64] operand whose rows 1..15 alias finite data and meet zeros in A
+                    // MN-major [16 x 64] operand whose rows 1..15 alias finite data and meet zeros in A (PACK: rows 0..7 are the heads')
                     tc_mma_f16(s_col, sdesc(ones_lo, hi_ones), sdesc(delta_lo, hi_delta), idesc_delta, false);
 #pragma unroll
                     for (int ks = 0; ks < D / 64; ++ks)
@@ -614,6 +670,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int quarter = warp & 3;            // tensor-memory lane quarter this warp may touch
         const int r = quarter * 32 + lane;       // row inside the tile
         const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+        const int prow_head = PACK ? r / p.Nq : 0, tok = PACK ? r - prow_head * p.Nq : r;      // packed row -> head, token
         const int sw = (r >> 1) & 3;
         float2* stat = reinterpret_cast<float2*>(sgen + C::oStat) + r;
         bool alive = !dead;
@@ -621,7 +678,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int i = 0; alive && (u = next_unit(i)) != nullptr; ++i) {
         const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nb1 = uniform(u->nbmax) - 1, row0 = uniform(u->mt0) * kBlock;
         const int Nk = uniform(u->Nk), shift = CAUSAL ? uniform(u->shift) : 0;
-        const float sl2 = p.sm_scale_per_head ? p.sm_scale_per_head[u->hq] * 1.4426950408889634f : p.sm_scale_log2;
+        const float sl2 = p.sm_scale_per_head ? p.sm_scale_per_head[u->hq + (PACK ? min(prow_head, u->nb[1] - 1) : 0)] * 1.4426950408889634f : p.sm_scale_log2;
         const uint64_t sl2x2 = pack2f(sl2, sl2);
         for (int s = (g - base) & 3; s < ns; s += 4) {
             const int sg = base + s;
@@ -646,7 +703,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 warp_arrive(bar(bSE + buf), lane);     // in registers: the buffer may be overwritten
                 if (need_mask) {
                     int lim = Nk - 1;
-                    if (CAUSAL) lim = min(lim, trow + r + shift);
+                    if (CAUSAL) lim = min(lim, trow + tok + shift);
                     const int key0 = n * kBlock + 64 * h;
 #pragma unroll
                     for (int i = 0; i < 64; ++i)
@@ -780,12 +837,12 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-// byte tensor [n2][n1][n0] (n0 contiguous), box [1][b1][b0]
+// byte tensor [n2][n1][n0] (n0 contiguous), box [b2][b1][b0]
 static CUresult make_map(EncodeTiledFn fn, CUtensorMap* m, const void* base, uint64_t n0, uint64_t n1, uint64_t n2,
-                         uint32_t b0, uint32_t b1, CUtensorMapSwizzle swz) {
+                         uint32_t b0, uint32_t b1, CUtensorMapSwizzle swz, uint32_t b2 = 1) {
     cuuint64_t dims[3] = {n0, n1, n2};
     cuuint64_t strides[2] = {n0, n0 * n1};
-    cuuint32_t box[3] = {b0, b1, 1};
+    cuuint32_t box[3] = {b0, b1, b2};
     cuuint32_t estr[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -799,34 +856,52 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
     return (int)make_map(fn, static_cast<CUtensorMap*>(map64), base, n0, n1, n2, b0, b1, swz);
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN>
-static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, bool PACK>
+static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int grid, cudaStream_t st) {
-    auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN>;
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), Cfg<D>::kSmemBytes);
+    auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK>;
+    using C = Cfg<D, PACK>;
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), C::kSmemBytes);
     if (e != cudaSuccess) return e;
-    return launch_pdl(kern, dim3(grid), dim3(Cfg<D>::kThreads), Cfg<D>::kSmemBytes, st, tq, tk, tv, p);
+    return launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, p);
 }
 
 template <int D, bool CAUSAL, typename OutT>
-static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int grid, cudaStream_t st) {
     // packed variable-length batches run their own instantiation, so that the uniform kernels carry none of it
-    return a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true>(a, tq, tk, tv, p, grid, st)
-                             : launch_v<D, CAUSAL, OutT, false>(a, tq, tk, tv, p, grid, st);
+    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, false>(a, tq, tk, tv, td, p, grid, st)
+           : p.pack_heads > 1 ? launch_v<D, CAUSAL, OutT, false, true>(a, tq, tk, tv, td, p, grid, st)
+                              : launch_v<D, CAUSAL, OutT, false, false>(a, tq, tk, tv, td, p, grid, st);
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     *driver_rc = 0;
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) return cudaErrorNotSupported;
-    CUtensorMap tq, tk, tv;
+    CUtensorMap tq, tk, tv, td;
     const uint32_t rowb = a.D / 2;
     const CUtensorMapSwizzle swz_qk = (a.D == 128) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-    CUresult r = make_map(fn, &tq, a.q_codes, rowb, a.Nq_p, (uint64_t)a.B * a.Hq, rowb, kBlock, swz_qk);
+    // Few query rows and several heads per kv head (token generation): as many heads as fit share a tile.  Two heads at least,
+    // eight at most (the operand that adds delta_s has eight rows), and no carried state.
+    const int group = a.Hq / a.Hkv;
+    int pack = 1;
+    if (a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr && a.Nq <= kBlock / 2) {
+        pack = kBlock / a.Nq < group ? kBlock / a.Nq : group;
+        if (pack > 8) pack = 8;
+    }
+    CUresult r = make_map(fn, &tq, a.q_codes, rowb, a.Nq_p, (uint64_t)a.B * a.Hq, rowb, pack > 1 ? a.Nq : kBlock, swz_qk, pack);
     if (r == CUDA_SUCCESS) r = make_map(fn, &tk, a.k_codes, rowb, a.Nk_p, (uint64_t)a.B * a.Hkv, rowb, kBlock, swz_qk);
     if (r == CUDA_SUCCESS)
         r = make_map(fn, &tv, a.v_codes, a.Nk_p / 2, a.D, (uint64_t)a.B * a.Hkv, 64, a.D, CU_TENSOR_MAP_SWIZZLE_64B);
+    td = tv;                            // (only the PACK kernels use it)
+    if (r == CUDA_SUCCESS && pack > 1) {
+        // delta_s as [Nk_p / 8][B * Hq][8 keys]: eight keys of eight heads are one core matrix
+        const cuuint64_t dims[3] = {16, (cuuint64_t)a.B * a.Hq, (cuuint64_t)a.Nk_p / 8}, strides[2] = {(cuuint64_t)a.Nk_p * 2, 16};
+        const cuuint32_t box[3] = {16, 8, kBlock / 8}, estr[3] = {1, 1, 1};
+        r = fn(&td, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(a.delta), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     if (r != CUDA_SUCCESS) {
         *driver_rc = (int)r;
         return cudaErrorInvalidValue;
@@ -843,7 +918,9 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     const bool split = nqt > 1 && 2 * rest <= sms;
     p.unit_counter = a.unit_counter;
     p.whole_units = split ? pairs - rest : pairs;
-    p.units = split ? pairs + rest : pairs;
+    p.pack_heads = pack;
+    p.pack_tiles = (group + pack - 1) / pack;
+    p.units = pack > 1 ? a.B * a.Hkv * p.pack_tiles : split ? pairs + rest : pairs;
     const int grid = p.units < sms ? p.units : sms;
     p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;
@@ -863,15 +940,15 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.causal_shift = a.causal_shift;
     p.cu_q = a.cu_q; p.cu_k = a.cu_k;
     if (a.is_bf16) {
-        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, p, grid, st)
-                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, p, grid, st);
-        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, p, grid, st)
-                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, p, grid, st);
+        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st)
+                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st);
+        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st)
+                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st);
     }
-    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, p, grid, st)
-                                       : launch_t<128, false, __half>(a, tq, tk, tv, p, grid, st);
-    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, p, grid, st)
-                       : launch_t<64, false, __half>(a, tq, tk, tv, p, grid, st);
+    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, td, p, grid, st)
+                                       : launch_t<128, false, __half>(a, tq, tk, tv, td, p, grid, st);
+    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, td, p, grid, st)
+                       : launch_t<64, false, __half>(a, tq, tk, tv, td, p, grid, st);
 }
 
 }  // namespace sage3
