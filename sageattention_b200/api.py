@@ -220,65 +220,50 @@ def sageattn3(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, tensor_layout: 
         if return_lse:
             return torch.ops.sageattention_b200.fwd_lse(q, k, v, tensor_layout, bool(is_causal), scale_f, scale_t, bool(per_block_mean))
         return torch.ops.sageattention_b200.fwd(q, k, v, tensor_layout, bool(is_causal), scale_f, scale_t, bool(per_block_mean))
-    # Repeated calls with one signature (the common case: every layer of a model) reuse the validated descriptor: what is
-    # left per call is two allocations and one call into the library.
-    plan_key = None
-    if workspace is None and not isinstance(sm_scale, torch.Tensor) and q.is_cuda:
-        plan_key = (q.device.index, q.dtype, k.dtype, v.dtype, tuple(q.shape), tuple(k.shape), tuple(v.shape), q.stride(), k.stride(),
-                    v.stride(), tensor_layout, bool(is_causal), sm_scale, bool(per_block_mean))
-        plan = _PLANS.get(plan_key)
-        if plan is not None:
-            desc, total_bytes, lse_shape = plan
-            dev = q.device
-            out = torch.empty(q.shape, dtype=q.dtype, device=dev)
-            lse = torch.empty(lse_shape, dtype=torch.float32, device=dev) if return_lse else None
-            buf = _shared_buffer(dev, total_bytes + 256)
-            ws_ptr = buf.data_ptr()
-            ws_ptr += (-ws_ptr) % 256
-            args = (C.byref(desc), q.data_ptr(), k.data_ptr(), v.data_ptr(), ws_ptr, out.data_ptr(),
-                    None if lse is None else lse.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
-            if torch.cuda.current_device() == dev.index:
-                rc = _cabi.lib().sage3_fwd(*args)
-            else:
-                with torch.cuda.device(dev):
-                    rc = _cabi.lib().sage3_fwd(*args)
-            _cabi.check(rc, "sage3_fwd")
-            return (out, lse) if return_lse else out
+    # The common case goes through the host extension; it answers None where copies, checks or errors are due.
+    if workspace is None and not isinstance(sm_scale, torch.Tensor) and (tensor_layout == "HND" or tensor_layout == "NHD") and \
+            (sm_scale is None or sm_scale > 0):
+        res = _bound_host().fwd(q, k, v, tensor_layout == "NHD", is_causal, 0.0 if sm_scale is None else sm_scale, per_block_mean, return_lse)
+        if res is not None:
+            if type(res) is int:
+                _cabi.check(res, "sage3_fwd")
+            return res
     prob = Sage3Problem(q, k, v, tensor_layout, is_causal, sm_scale, per_block_mean,
                         workspace=CACHED_WORKSPACE if workspace is None else workspace, return_lse=return_lse)
     out = prob.run()
-    if plan_key is not None and prob.q is q and prob.k is k and prob.v is v:      # no copies were needed: the signature is reusable
-        if len(_PLANS) >= 256:
-            _PLANS.clear()
-        hd, nd = (1, 2) if tensor_layout == "HND" else (2, 1)
-        _PLANS[plan_key] = (prob.desc, prob.ws.layout.total_bytes, (q.shape[0], q.shape[hd], q.shape[nd]))
     return (out, prob.lse) if return_lse else out
 
 
 # ------------------------------------------------------------------------------------------------------
 # workspace cache of the functional entry points
 # ------------------------------------------------------------------------------------------------------
-# One workspace per (device, stream), grown on demand and reused by later calls: kernels of successive calls on one
-# stream run in order, so they may share it; calls on different streams get different buffers.  (Allocating 3.4 GB anew
-# on every call of the benchmark shape costs more than the pre-pass.)  Sage3Problem users manage their own.
-_WORKSPACES: dict = {}
-_PLANS: dict = {}            # signature of a sageattn3 call -> (validated descriptor, workspace bytes, LSE shape)
+# (kept in the host extension: one per device and stream, grown on demand.)  Sage3Problem users manage their own.
+_host_module = None
+
+
+def _bound_host():
+    """The host extension, loaded and told where the library's entry points are on first use.  No fallback."""
+    global _host_module
+    if _host_module is None:
+        lib = _cabi.lib()
+        try:
+            from . import _host
+        except ImportError as exc:
+            raise ImportError("sageattention_b200/_host.so is missing or was built for another torch; build it with "
+                              "`python -m sageattention_b200.build`") from exc
+        _host.bind(*(C.cast(f, C.c_void_p).value for f in (lib.sage3_fwd, lib.sage3_fwd_varlen, lib.sage3_workspace_bytes)))
+        _host_module = _host
+    return _host_module
 
 
 def _shared_buffer(device: torch.device, nbytes: int) -> torch.Tensor:
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _WORKSPACES.get(key)
-    if buf is None or buf.numel() < nbytes:
-        _WORKSPACES.pop(key, None)
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = buf
-    return buf
+    return _bound_host().shared_buffer(torch.cuda.current_device() if device.index is None else device.index, nbytes)
 
 
 def release_workspaces() -> None:
-    """Drops the workspaces (and call signatures) that sageattn3 / sageattn / sageattn_varlen keep between calls."""
-    _WORKSPACES.clear()
-    _PLANS.clear()
+    """Drops the workspaces that sageattn3 / sageattn / sageattn_varlen keep between calls."""
+    if _host_module is not None:
+        _host_module.release()
 
 
 # ------------------------------------------------------------------------------------------------------
@@ -344,6 +329,15 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
     sized for `number of sequences x maximum lengths`.  `smooth_k` is accepted for compatibility; a scalar `sm_scale`
     only.  With `return_lse=True` the result is `(out, lse)`, lse fp32 [number of sequences, Hq, max_seqlen_q]: row i of
     sequence b at [b, :, i], -inf beyond a sequence's length (natural log, as `sageattn3(..., return_lse=True)`)."""
+    if max_seqlen_q is not None and max_seqlen_k is not None and isinstance(cu_seqlens_q, torch.Tensor) and isinstance(cu_seqlens_k, torch.Tensor) \
+            and (sm_scale is None or (not isinstance(sm_scale, torch.Tensor) and sm_scale > 0)) and not torch.compiler.is_compiling():
+        # the common case: device cu_seqlens and the maxima given (None: copies, conversions or errors are due)
+        res = _bound_host().fwd_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), is_causal,
+                                       0.0 if sm_scale is None else sm_scale, per_block_mean, return_lse)
+        if res is not None:
+            if type(res) is int:
+                _cabi.check(res, "sage3_fwd_varlen")
+            return res
     if q.dim() != 3 or k.dim() != 3 or v.dim() != 3:
         raise ValueError("q, k, v must be packed as [tokens, heads, head_dim]")
     for name, t in (("q", q), ("k", k), ("v", v)):

@@ -1,4 +1,4 @@
-"""Builds libsage3_b200.so (sm_100a only) next to this file with nvcc.
+"""Builds libsage3_b200.so (sm_100a only, nvcc) and the host extension _host.so (g++, against the installed torch) next to this file.
 
 Usage:  python -m sageattention_b200.build [--force]
 The library is plain CUDA C++ behind a C ABI (include/sage3_b200.h); it links the CUDA runtime
@@ -15,6 +15,8 @@ import sys
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libsage3_b200.so"
+HOST_LIB = PKG / "_host.so"
+HOST_SOURCE = "sage3_host.cpp"
 SOURCES = ["sage3_abi.cu", "sage3_prepass.cu", "sage3_attn.cu"]
 HEADERS = ["sage3_common.cuh", "sage3_kernels.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,7 +31,27 @@ def _stale() -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _build_host(force: bool) -> None:
+    """The CPython extension behind the functional entry points (argument checks, output and workspace tensors)."""
+    deps = [CSRC / HOST_SOURCE, PKG.parent / "include" / "sage3_b200.h", pathlib.Path(__file__)]
+    if not force and HOST_LIB.exists() and all(d.stat().st_mtime <= HOST_LIB.stat().st_mtime for d in deps):
+        return
+    import sysconfig
+
+    import torch
+    root = pathlib.Path(torch.__file__).resolve().parent
+    cuda = pathlib.Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in inc], str(CSRC / HOST_SOURCE),
+           "-o", str(HOST_LIB), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on {HOST_SOURCE}:\n{r.stdout}")
+
+
 def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
+    _build_host(force)
     if not force and not _stale():
         return LIB
     nvcc = os.environ.get("NVCC", "nvcc")
