@@ -61,6 +61,7 @@ struct AttnParams {
     const uint8_t *q_sf, *k_sf, *v_sf;
     const uint16_t* delta;              // 16-bit elements [B*Hq][nqm][nkb*128]
     void* out[kMaxParts];               // output buffers; out_rows == 0: one buffer
+    int out_wide;                       // rows of the output start on 32-byte boundaries: 256-bit stores
     int out_rows;                       // query rows per output part (rows of one (batch, head) go to part row / out_rows)
     int64_t os0, os1, os2;
     float* lse;                         // optional fp32 [B*Hq][Nq]
@@ -84,8 +85,9 @@ template <int D, bool PACK>
 struct Cfg {
     static constexpr int kStages = (D == 128) ? 4 : (PACK ? 6 : 8);        // K and V^T stages, each shared by the two query tiles
     static constexpr int kThreads = 768;                      // 6 warpgroups, see the kernel
-    // S buffers of 128 rows x 64 keys: a rotation for the first halves of the items and one for the second halves
-    static constexpr int kSBufs0 = 2, kSBufs1 = (D == 128) ? 1 : 2, kSBufs = kSBufs0 + kSBufs1;
+    // S buffers of 128 rows x 64 keys: a rotation for the first halves of the items and one for the second halves (D = 64 has room for
+    // a second one of the latter: 1 % slower)
+    static constexpr int kSBufs0 = 2, kSBufs1 = 1, kSBufs = kSBufs0 + kSBufs1;
     static constexpr int kQBytes = 128 * D / 2;               // per query tile
     static constexpr int kSfQkBytes = (D / 64) * 512;
     static constexpr int kKBytes = 128 * D / 2;
@@ -132,12 +134,20 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// 32 bytes to a 32-byte aligned address in one store: a whole sector per lane, since the rows of the output are far apart.  (Two
+// 16-byte stores: 2 to 4 % of the attention time at two to four key blocks per tile.)
+__device__ __forceinline__ void store_32b(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+
 // A value that is the same in all lanes, marked as such for the compiler (uniform registers feed the tcgen05 instructions).
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 // Wait executed by a whole converged warp; the verdict is made warp-uniform so that no lane leaves a loop alone.
 template <bool kBackoff = false>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;       // (0.5 to 1.5 % over going through the loop's first look)
     const bool ok = mbar_wait<kBackoff>(bar, parity, abort_flag, status, code);
     return __all_sync(0xffffffffu, ok);
 }
@@ -298,14 +308,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         prefetch_tmap(&tm_v);
     }
     pdl_wait();                       // nothing above reads what the pre-pass writes
-    // an earlier CTA of this launch gave up, or the pre-pass did (the workspace is then incomplete): nothing is done
-    if (threadIdx.x == 0)
-        tmem_slot[1] = (*reinterpret_cast<volatile int*>(p.status) != 0) || (*reinterpret_cast<const volatile int*>(p.prepass_status) != 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = uniform(tmem_slot[0]);
-    const bool dead = uniform(tmem_slot[1]) != 0;
+    const uint32_t tmem = uniform(*tmem_slot);
     const bool carry_in = (p.carry_o_in != nullptr);
 
     // Register budget: 768 threads start with 80 registers each, and that allocation (61 440) is all the CTA can
@@ -334,8 +340,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const float2* sum = reinterpret_cast<const float2*>(sgen + C::oSum) + row;
       float2* l_s = reinterpret_cast<float2*>(sgen + C::oL) + row;
       float* m_s = reinterpret_cast<float*>(sgen + C::oM) + row;
+      // The pre-pass gave up (the workspace is then incomplete): the units are walked, but nothing is written.  (Read here, needed at
+      // the first epilogue: off the path to the first scores.)
+      const int broken = *reinterpret_cast<const volatile int*>(p.prepass_status);
       const Unit* u;
-      bool ok = !dead;
+      bool ok = true;
       for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
           const Unit& w = *u;
           const int ns = w.ns, two = w.two, d = w.d;
@@ -405,7 +414,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
           // ---------------------------------------------------------------- O / l of the unit's tiles
           // (The accumulators belong to the next unit once this warpgroup arrives for its first items.)
-          for (int t = 0; ok && t < w.nv; ++t) {
+          for (int t = 0; ok && broken == 0 && t < w.nv; ++t) {
               const int grow = PACK ? prow_tok : (w.mt0 + t) * kBlock + row;
               const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq;
               const int bhq = w.bhq + prow_head, hq = w.hq + prow_head;
@@ -456,14 +465,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                               make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                   }
                   if (orow != nullptr) {
+                      uint32_t v[8];
 #pragma unroll
-                      for (int q = 0; q < 2; ++q) {
-                          uint4 v4;
-                          v4.x = pack2<OutT>(o[8 * q] * inv_l, o[8 * q + 1] * inv_l);
-                          v4.y = pack2<OutT>(o[8 * q + 2] * inv_l, o[8 * q + 3] * inv_l);
-                          v4.z = pack2<OutT>(o[8 * q + 4] * inv_l, o[8 * q + 5] * inv_l);
-                          v4.w = pack2<OutT>(o[8 * q + 6] * inv_l, o[8 * q + 7] * inv_l);
-                          *reinterpret_cast<uint4*>(orow + c + q * 8) = v4;
+                      for (int q = 0; q < 8; ++q) v[q] = pack2<OutT>(o[2 * q] * inv_l, o[2 * q + 1] * inv_l);
+                      if (p.out_wide) {
+                          store_32b(orow + c, v);
+                      } else {
+                          *reinterpret_cast<uint4*>(orow + c) = make_uint4(v[0], v[1], v[2], v[3]);
+                          *reinterpret_cast<uint4*>(orow + c + 8) = make_uint4(v[4], v[5], v[6], v[7]);
                       }
                   }
               }
@@ -478,7 +487,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
         int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
-        bool ok = !dead;
+        bool ok = true;
         while (ok) {
             int next = 0;
             if (lane == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
@@ -570,7 +579,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int nbuf = h == 0 ? C::kSBufs0 : C::kSBufs1, buf0 = h == 0 ? 0 : C::kSBufs0;
         int buf = 0, buf_parity = 1;              // next S buffer; parity of its "empty" phase (a fresh barrier passes parity 1)
         int st = 0, st_parity = 0;                // K stage
-        bool ok = !dead;
+        bool ok = true;
         const Unit* u;
         for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
@@ -627,7 +636,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t sfv_lo0 = sdesc_lo(sbase + C::oSfV, 0), sfp_lo0 = sdesc_lo(sbase + C::oSfP, 0);
         const uint32_t sfp_col = tmem + C::cSfP, sfv_col = tmem + C::cSfV;
         int st = 0, st_parity = 0;
-        bool ok = !dead;
+        bool ok = true;
         const Unit* u;
         for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d);
@@ -673,7 +682,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int prow_head = PACK ? r / p.Nq : 0, tok = PACK ? r - prow_head * p.Nq : r;      // packed row -> head, token
         const int sw = (r >> 1) & 3;
         float2* stat = reinterpret_cast<float2*>(sgen + C::oStat) + r;
-        bool alive = !dead;
+        bool alive = true;
         const Unit* u;
         for (int i = 0; alive && (u = next_unit(i)) != nullptr; ++i) {
         const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nb1 = uniform(u->nbmax) - 1, row0 = uniform(u->mt0) * kBlock;
@@ -931,6 +940,8 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.delta = static_cast<const uint16_t*>(a.delta);
     for (int i = 0; i < kMaxParts; ++i) p.out[i] = a.out.base[i];
     p.out_rows = a.out.rows;
+    p.out_wide = a.os[0] % 16 == 0 && a.os[1] % 16 == 0 && a.os[2] % 16 == 0;
+    for (int i = 0; i < kMaxParts; ++i) p.out_wide &= reinterpret_cast<uintptr_t>(a.out.base[i]) % 32 == 0;
     p.lse = a.lse; p.qkm = a.qkm; p.sm_scale = a.sm_scale;
     p.os0 = a.os[0]; p.os1 = a.os[1]; p.os2 = a.os[2];
     p.status = a.status;

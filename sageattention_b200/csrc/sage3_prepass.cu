@@ -229,15 +229,13 @@ __device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_
 // One sum of a column's partial sums, in the order of the chunks.
 __device__ __forceinline__ float sum_chunks(const float* __restrict__ part, int chunks, int D) {
     float s = 0.f;
-    int c = 0;
-    for (; c + 8 <= chunks; c += 8) {
+    for (int c = 0; c < chunks; c += 8) {
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = part[(int64_t)(c + i) * D];
+        for (int i = 0; i < 8; ++i) v[i] = c + i < chunks ? part[(int64_t)(c + i) * D] : 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s += v[i];
+        for (int i = 0; i < 8; ++i) s += v[i];       // (+ 0 beyond the last chunk: no change)
     }
-    for (; c < chunks; ++c) s += part[(int64_t)c * D];
     return s;
 }
 
