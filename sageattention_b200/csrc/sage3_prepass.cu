@@ -266,6 +266,14 @@ __global__ void colmean_finalize_kernel(const float* __restrict__ part, int chun
 // ------------------------------------------------------------------------------------------------
 enum { kModeQBlockMean = 0, kModeQGlobalMean = 1 };
 
+// Partial column sums for the blocks that form the means they need themselves (nullptr: the means are in memory).
+struct MeanParts {
+    const float *k, *q;                // [B*Hkv][chunks_k][D], [B*H][chunks_q][D]
+    int chunks_k, chunks_q, Nk;
+    const int* cu_k;
+    bool wait;                         // the sums come from the launch before this one (programmatic dependent launch)
+};
+
 template <typename T, int D, int MODE>
 __device__ __forceinline__ void quant_q_tile(
     const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
@@ -276,6 +284,7 @@ __device__ __forceinline__ void quant_q_tile(
     const T* __restrict__ km,          // K means [B*Hkv][D]
     int group,                         // query heads per kv head
     float* __restrict__ qkm,           // [B*H][Np]: x . km per row (the score part that K smoothing removes); nullptr: not wanted
+    const MeanParts& mp,
     int tile, int bh, uint8_t* smem_raw) {
     constexpr int CH = D / 16;            // microblocks per row
     constexpr int RPP = 256 / CH;         // rows per pass
@@ -298,13 +307,26 @@ __device__ __forceinline__ void quant_q_tile(
         load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
     });
 
+    if (mp.wait) pdl_wait();               // the rows above are inputs; the means are not
     // x . km of every row: 16 products per thread, then a sum over the CH neighbouring lanes that share the row
     if (qkm != nullptr) {
-        const T* kmh = km + ((int64_t)b * ((int)H.d / group) + h / group) * D + c * 16;
-        uint4 k0, k1;
-        load16_packed<T>(kmh, true, k0, k1);
+        const int bhk = b * ((int)H.d / group) + h / group;
         float kf[16];
-        unpack16<T>(k0, k1, kf);
+        if (mp.k != nullptr) {
+            if (t < D) {
+                const int nk = mp.cu_k != nullptr ? min(max(mp.cu_k[b + 1] - mp.cu_k[b], 0), mp.Nk) : mp.Nk;
+                const float m = sum_chunks(mp.k + (int64_t)bhk * mp.chunks_k * D + t, mp.chunks_k, D) * (nk > 0 ? 1.0f / (float)nk : 0.f);
+                s_mean[t] = Num<T>::to_f(Num<T>::from_f(m));
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) kf[j] = s_mean[c * 16 + j];
+            __syncthreads();               // s_mean takes the Q mean next
+        } else {
+            uint4 k0, k1;
+            load16_packed<T>(km + (int64_t)bhk * D + c * 16, true, k0, k1);
+            unpack16<T>(k0, k1, kf);
+        }
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             float f[16];
@@ -375,7 +397,16 @@ __device__ __forceinline__ void quant_q_tile(
             qm_out[((int64_t)bh * (Np / kBlock) + tile) * D + t] = m;
         }
     } else {
-        if (t < D) s_mean[t] = Num<T>::to_f(mean_in[(int64_t)bh * D + t]);
+        if (t < D) {
+            if (mp.q != nullptr) {         // mean over the rows padded to whole blocks (api.py:88-90)
+                const int np = (N + kBlock - 1) / kBlock * kBlock;
+                const T m = Num<T>::from_f(sum_chunks(mp.q + (int64_t)bh * mp.chunks_q * D + t, mp.chunks_q, D) * (np > 0 ? 1.0f / (float)np : 0.f));
+                if (tile == 0) qm_out[(int64_t)bh * D + t] = m;
+                s_mean[t] = Num<T>::to_f(m);
+            } else {
+                s_mean[t] = Num<T>::to_f(mean_in[(int64_t)bh * D + t]);
+            }
+        }
     }
     __syncthreads();
 
@@ -699,6 +730,7 @@ struct StageArgs {
     T *km, *qm;
     uint8_t *q_codes, *q_sf, *v_codes, *v_sf;
     float* qkm;                        // nullptr: not wanted
+    MeanParts means;
     int* clear;                        // status words and work counter to zero (nullptr: not in this launch)
     int n_clear;
 };
@@ -736,10 +768,10 @@ __global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(con
         bh = a.tiles_q.divmod(i, tile);
         if (a.q_block_mean)
             quant_q_tile<T, D, kModeQBlockMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, nullptr, a.qm, a.q_codes, a.q_sf, a.km,
-                                                a.group, a.qkm, tile, bh, smem_raw);
+                                                a.group, a.qkm, a.means, tile, bh, smem_raw);
         else
-            quant_q_tile<T, D, kModeQGlobalMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, a.qm, nullptr, a.q_codes, a.q_sf, a.km,
-                                                 a.group, a.qkm, tile, bh, smem_raw);
+            quant_q_tile<T, D, kModeQGlobalMean>(a.q, a.qs[0], a.qs[1], a.qs[2], a.Hq, a.Nq, a.Nq_p, a.qm, a.qm, a.q_codes, a.q_sf, a.km,
+                                                 a.group, a.qkm, a.means, tile, bh, smem_raw);
         return;
     }
     i -= a.n_q;
@@ -750,8 +782,8 @@ __global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(con
 // ------------------------------------------------------------------------------------------------
 // host-side launch
 // ------------------------------------------------------------------------------------------------
-// Up to this many chunks (16 384 keys) every CTA of the K kernel forms the K mean itself from the partial sums (an 8 KB read
-// from L2 at 8 192 keys); beyond, one small kernel does.
+// Up to this many chunks (16 384 rows) the blocks that need a mean form it themselves from the partial sums (an 8 KB read from L2 at
+// 8 192 keys); beyond, one small kernel does.
 constexpr int kInlineMeanChunks = 32;
 
 template <typename T, int D>
@@ -784,7 +816,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     // Q waits for the means when it is smoothed by one mean per head (api.py:88-90) or when q . km is wanted
     const bool q_late = !a.per_block_mean || a.want_qkm;
     const bool km_here = !a.km_given;
-    const bool km_inline = km_here && !q_late && a.kchunks_k <= kInlineMeanChunks;
+    const bool km_inline = km_here && a.kchunks_k <= kInlineMeanChunks, qm_inline = !a.per_block_mean && a.kchunks_q <= kInlineMeanChunks;
     s.n_colk = km_here ? a.kchunks_k * BHkv : 0;
     s.n_colq = a.per_block_mean ? 0 : a.kchunks_q * BHq;
     s.n_q = q_late ? 0 : tiles_q * BHq;
@@ -792,14 +824,21 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     prepass_stage_kernel<T, D><<<s.n_colk + s.n_colq + s.n_q + s.n_v, 256, StageCfg<T, D>::kSmem, st>>>(s);
     if (km_here && !km_inline)
         colmean_finalize_kernel<T, D><<<BHkv, D, 0, st>>>(s.part_k, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0);
-    if (!a.per_block_mean)
+    if (!a.per_block_mean && !qm_inline)
         colmean_finalize_kernel<T, D><<<BHq, D, 0, st>>>(s.part_q, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1);
     if (q_late) {
         s.n_colk = s.n_colq = s.n_v = 0;
         s.n_q = tiles_q * BHq;
         s.qkm = a.want_qkm ? a.qkm : nullptr;
         s.clear = nullptr;
-        prepass_stage_kernel<T, D><<<s.n_q, 256, StageCfg<T, D>::kSmem, st>>>(s);
+        s.means.k = km_inline ? s.part_k : nullptr;
+        s.means.q = qm_inline ? s.part_q : nullptr;
+        s.means.chunks_k = a.kchunks_k;
+        s.means.chunks_q = a.kchunks_q;
+        s.means.Nk = a.Nk;
+        s.means.cu_k = a.cu_k;
+        s.means.wait = true;
+        if ((e = launch_pdl(prepass_stage_kernel<T, D>, dim3(s.n_q), dim3(256), (size_t)StageCfg<T, D>::kSmem, st, s)) != cudaSuccess) return e;
     }
     const size_t smem_k = 2 * (D / 64) * 16384 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + 32768 : 0);
     e = allow_smem(reinterpret_cast<const void*>(quant_k_delta_kernel<T, D>), (int)smem_k);
