@@ -1,0 +1,105 @@
+"""The sizes at which the launch path changes: work units of the attention kernel (pairs and single query tiles around
+multiples of the SM count), query heads packed into one tile, means formed inside the kernels or by a launch of their own,
+output rows on 16- and on 32-byte boundaries, and the host extension against the Python path.  Every head is computed from
+its own q, k, v alone, in one order of operations, so the results of different paths must agree bit for bit; against the
+oracle the gate is the one of the whole path (cosine >= 0.999, relative L1 <= 1 %)."""
+import pytest
+import torch
+
+from oracle import sage3_oracle as O
+from sageattention_b200 import Sage3Problem, sageattn3
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(device, B, Hq, Hkv, Nq, Nk, D, seed, dtype=torch.bfloat16):
+    q, k, v = O.make_inputs(B, Hq, Hkv, Nq, Nk, D, seed=seed, dtype=dtype, k_offset_std=1.0)
+    return q.to(device), k.to(device), v.to(device)
+
+
+@pytest.mark.parametrize("D,causal", [(128, False), (64, True)])
+@pytest.mark.parametrize("extra", [-1, 0, 1, 74, 76])
+def test_units_around_the_sm_count(cuda_device, D, causal, extra):
+    """Three query tiles per head (a pair and a single one); two units per head, 2 x heads around one round of all SMs: one
+    round less a unit, full, and a second round that is dealt out as single tiles (up to half of the SMs) or not."""
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    H = (sms + extra + 1) // 2
+    q, k, v = _inputs(cuda_device, 1, H, H, 300, 260, D, seed=700 + extra)
+    out = sageattn3(q, k, v, is_causal=causal)
+    for h in sorted({0, 1, H // 2, H - 2, H - 1}):
+        one = sageattn3(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], is_causal=causal)
+        assert torch.equal(out[:, h:h + 1], one), f"head {h} of {H}"
+
+
+@pytest.mark.parametrize("Nq,Hq,Hkv,Nk,D,causal", [(1, 8, 2, 700, 128, True), (1, 32, 2, 129, 64, False), (9, 14, 2, 128, 128, True),
+                                                   (16, 8, 1, 1000, 64, True), (64, 4, 2, 300, 128, True), (65, 4, 2, 300, 128, True),
+                                                   (3, 12, 4, 2, 64, True)])
+def test_heads_sharing_a_tile(cuda_device, Nq, Hq, Hkv, Nk, D, causal):
+    """One to sixteen query heads per kv head, up to eight of them in one tile, at the row counts where a tile is just
+    full: the same bits as with the keys and values repeated per query head (no sharing), and the oracle's result."""
+    q, k, v = _inputs(cuda_device, 2, Hq, Hkv, Nq, Nk, D, seed=800 + Nq + Hq)
+    scale = torch.rand(Hq, generator=torch.Generator().manual_seed(1)) * 0.1 + 0.05
+    out, lse = sageattn3(q, k, v, is_causal=causal, sm_scale=scale, return_lse=True)
+    g = Hq // Hkv
+    rep, rep_lse = sageattn3(q, k.repeat_interleave(g, 1), v.repeat_interleave(g, 1), is_causal=causal, sm_scale=scale, return_lse=True)
+    assert torch.equal(out, rep) and torch.equal(lse, rep_lse)
+    ref = O.sageattn3_oracle(q.cpu(), k.cpu(), v.cpu(), is_causal=causal, sm_scale=scale)
+    assert O.cosine(out.cpu(), ref) >= 0.999 and O.rel_l1(out.cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("Nk", [1, 512, 513, 16384, 16385])
+@pytest.mark.parametrize("block_mean", [True, False])
+def test_means_inside_and_outside_the_kernels(cuda_device, Nk, block_mean):
+    """The K mean is formed by the kernels that use it up to 16 384 keys and by a launch of its own beyond; Q is quantized before
+    the means are known unless the LSE or one mean per head is wanted.  All of them against the oracle, and against one another."""
+    q, k, v = _inputs(cuda_device, 1, 2, 1, 140, Nk, 64, seed=900 + Nk)
+    out = sageattn3(q, k, v, per_block_mean=block_mean)
+    out2, lse = sageattn3(q, k, v, per_block_mean=block_mean, return_lse=True)
+    assert torch.equal(out, out2)
+    ref, ref_lse = O.sageattn3_oracle(q.cpu(), k.cpu(), v.cpu(), per_block_mean=block_mean, return_lse=True)
+    assert O.cosine(out.cpu(), ref) >= 0.999 and O.rel_l1(out.cpu(), ref) <= 0.01
+    assert (lse.cpu() - ref_lse).abs().max() <= 1e-3       # log2 / exp2 approximations, as in the LSE tests of the whole path
+
+
+@pytest.mark.parametrize("heads,Nq", [(1, 128 * 128), (1, 128 * 128 + 1), (8, 16 * 128), (8, 16 * 128 + 1)])
+def test_query_blocks_of_a_kv_head_around_one_mma(cuda_device, heads, Nq):
+    """delta_s takes 128 query blocks of all heads of a kv head at a time: 128 blocks, and one more per head."""
+    q, k, v = _inputs(cuda_device, 1, heads, 1, Nq, 200, 64, seed=1000 + heads)
+    out = sageattn3(q, k, v)
+    for h in {0, heads - 1}:
+        tail = sageattn3(q[:, h:h + 1, -(Nq % 128 or 128):], k, v)         # the last block alone has the same block mean
+        assert torch.equal(out[:, h:h + 1, -tail.shape[2]:], tail)
+
+
+@pytest.mark.parametrize("pad", [8, 16])
+def test_output_rows_on_16_and_32_byte_boundaries(cuda_device, pad):
+    q, k, v = _inputs(cuda_device, 1, 3, 3, 200, 300, 64, seed=1100)
+    wide = torch.full((1, 3, 200, 64 + pad), 7.0, dtype=q.dtype, device=cuda_device)
+    Sage3Problem(q, k, v, out=wide[..., :64]).run()
+    assert torch.equal(wide[..., :64], sageattn3(q, k, v))
+    assert (wide[..., 64:] == 7.0).all()
+
+
+def test_host_extension_and_python_path_agree(cuda_device):
+    """Plain tensors go through the host extension; a last dimension that is not contiguous, and a scale given as a tensor, through
+    Python.  Two streams have a workspace each."""
+    q, k, v = _inputs(cuda_device, 1, 4, 2, 200, 300, 64, seed=1200)
+    ref = sageattn3(q, k, v, is_causal=True, sm_scale=0.2)
+    qt = q.transpose(2, 3).contiguous().transpose(2, 3)
+    assert torch.equal(sageattn3(qt, k, v, is_causal=True, sm_scale=0.2), ref)
+    assert torch.equal(sageattn3(q, k, v, is_causal=True, sm_scale=torch.full((4,), 0.2)), ref)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(cuda_device) for _ in range(2)]
+    outs = []
+    for _ in range(4):
+        for s in streams:
+            with torch.cuda.stream(s):
+                outs.append(sageattn3(q, k, v, is_causal=True, sm_scale=0.2))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, ref) for o in outs)
+    with pytest.raises(ValueError):
+        sageattn3(q, k, v, sm_scale=-1.0)
+    with pytest.raises(ValueError):
+        sageattn3(q, k, v, tensor_layout="BHND")
+    with pytest.raises(RuntimeError):
+        sageattn3(q.cpu(), k, v)
