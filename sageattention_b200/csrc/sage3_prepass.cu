@@ -8,7 +8,7 @@
 //   api.py:91            delta_s = qm . k'^T, rounded to the input type (tcgen05 16-bit MMA, accumulator in TMEM)
 //   quantization/fp4_quantization_4d.cu:185-225   SF = e4m3(amax / 6), code = e2m1(x * (1 / SF))
 //   quantization/fp4_quantization_4d.cu:300-349   V: microblocks are 16 consecutive tokens of one channel
-// Divisions and reciprocals are IEEE (div.rn / rcp.rn) so the result can be checked bit for bit.
+// Quotients and reciprocals are those of IEEE arithmetic (see micro_scale), so the result can be checked bit for bit.
 #include <mutex>
 
 #include "../../include/sage3_b200.h"
@@ -156,6 +156,19 @@ __device__ __forceinline__ void unpack16(const uint4& a, const uint4& b, float* 
     }
 }
 
+// Scale byte of a microblock with maximum magnitude amax, SF = e4m3(amax / 6), and the factor 1 / SF its values are scaled with
+// (0 when SF is 0).  Both without the division and reciprocal routines (a quarter of the stage kernel's instructions):
+//   amax * RN(1/6) and RN(amax / 6) round to the same E4M3 value for every 16-bit amax.  A quotient on a rounding boundary of E4M3 (a
+//   significand of at most 5 bits) means amax = 6 x boundary, and RN(1/6) = 1/6 (1 + 2^-25.0) is close enough for the product to
+//   round to the boundary itself (half an ulp is more than 2^-24.96 of it); any other quotient is at least 2^-14 away from one.
+//   rcp.approx of the 126 positive E4M3 values is their correctly rounded reciprocal (checked for each of them).
+__device__ __forceinline__ float micro_scale(float amax, uint32_t& sf_byte) {
+    sf_byte = cvt_e4m3x2(__fmul_rn(amax, 1.0f / 6.0f), 0.f) & 0xffu;
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(e4m3_to_float(sf_byte)));
+    return sf_byte == 0u ? 0.f : inv;
+}
+
 // One NVFP4 microblock, eight packed words of the input type (16 values) -> 8 bytes of codes + scale byte: the maximum magnitude is found on the packed pairs
 // (exact, as fp4_quantization_4d.cu:186-196 does), the scaling runs in fp32.
 template <typename T>
@@ -165,15 +178,13 @@ __device__ __forceinline__ void quant16_packed(const uint32_t* w, uint32_t& lo, 
     for (int i = 1; i < 8; ++i) m = Num<T>::absmax2(m, w[i]);
     const float2 mm = Num<T>::to_f2(m);
     const float amax = fmaxf(mm.x, mm.y);
-    sf_byte = cvt_e4m3x2(__fdiv_rn(amax, 6.0f), 0.f) & 0xffu;
-    const float sf = e4m3_to_float(sf_byte);
-    const float inv = (sf == 0.f) ? 0.f : __frcp_rn(sf);
+    const float inv = micro_scale(amax, sf_byte);
+    const uint64_t inv2 = pack2f(inv, inv);
     float y[16];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float2 v = Num<T>::to_f2(w[i]);
-        y[2 * i] = __fmul_rn(v.x, inv);
-        y[2 * i + 1] = __fmul_rn(v.y, inv);
+        unpack2f(mul2(pack2f(v.x, v.y), inv2), y[2 * i], y[2 * i + 1]);
     }
     lo = cvt_e2m1x8(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]);
     hi = cvt_e2m1x8(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]);
@@ -679,9 +690,8 @@ __device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64
         const float2 amax2 = Num<T>::to_f2(m2);
 #pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
-            const uint32_t sfb = cvt_e4m3x2(__fdiv_rn(ch == 0 ? amax2.x : amax2.y, 6.0f), 0.f) & 0xffu;
-            const float sf = e4m3_to_float(sfb);
-            const float inv = (sf == 0.f) ? 0.f : __frcp_rn(sf);
+            uint32_t sfb;
+            const float inv = micro_scale(ch == 0 ? amax2.x : amax2.y, sfb);
             uint32_t code[2];
 #pragma unroll
             for (int g = 0; g < 2; ++g) {

@@ -103,3 +103,25 @@ def test_host_extension_and_python_path_agree(cuda_device):
         sageattn3(q, k, v, tensor_layout="BHND")
     with pytest.raises(RuntimeError):
         sageattn3(q.cpu(), k, v)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_scale_of_every_microblock_maximum(cuda_device, dtype):
+    """The scale byte and the codes come from a product with 1/6 and an approximate reciprocal of the scale; for every finite positive
+    16-bit maximum they have to equal those of the IEEE division and reciprocal.  V is the tensor without smoothing: one maximum
+    per microblock of 16 tokens, the other 15 values anywhere below it."""
+    from tests._util import canon, read_workspace
+    D, groups = 64, 512
+    bits = torch.arange(D * groups, dtype=torch.int32) % 0x7F80 if dtype == torch.bfloat16 else torch.arange(D * groups, dtype=torch.int32) % 0x7C00
+    peak = bits.to(torch.int16).view(dtype).float().reshape(D, groups)
+    g = torch.Generator().manual_seed(5)
+    v = peak[..., None] * (2 * torch.rand(D, groups, 16, generator=g) - 1)
+    v[..., 3] = peak
+    v = v.reshape(D, groups * 16).t().contiguous().to(dtype)[None, None]
+    q, k = torch.randn(1, 1, 128, D, generator=g).to(dtype), torch.randn(1, 1, groups * 16, D, generator=g).to(dtype)
+    prob = Sage3Problem(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device))
+    prob.prepass()
+    torch.cuda.synchronize()
+    ws, ref = read_workspace(prob), O.prepass(q, k, v)
+    assert torch.equal(ws["vt_sf"], ref.vt_sf)
+    assert torch.equal(canon(ws["vt_codes"]), canon(ref.vt_codes))
