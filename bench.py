@@ -75,6 +75,12 @@ def prepass_bytes_of(w) -> float:
     return b
 
 
+def launches_per_step(w, base: int) -> int:
+    """Kernels of one call: `base` (stage, K and attention; one more for q.km, which the stand-alone pre-pass and the LSE need) and
+    one for the K mean beyond 16 384 keys."""
+    return base + (1 if w["Nk"] > 16384 else 0)
+
+
 def measured_peaks():
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -330,7 +336,7 @@ def run_ulysses(args, w, rank, world, local, dev):
             scaling="strong", vs_baseline=None, dtype="fp4 (e2m1 x ue4m3), fp32 accumulate", data="synthetic",
             config=dict(workload=args.workload, l2="inputs larger than L2", head_slices_in_flight=groups,
                         **{k_: v_ for k_, v_ in res.items() if k_ not in ("tops", "ms_per_step", "steps", "scaling")}),
-            clocks=clocks, gpu_launches=((6 + 1) * world if args.ring else 6 * groups + 4) * args.steps)))
+            clocks=clocks, gpu_launches=((launches_per_step(w, 4) + 1) * world if args.ring else launches_per_step(w, 3) * groups + 4) * args.steps)))
     if world > 1:
         dist.destroy_process_group()
 
@@ -522,7 +528,7 @@ def main():
         roofline=dict(bound="tensor", kernel="attn_fwd_kernel", achieved=att_tops, peak=fp4_peak, unit="TFLOP/s", frac=att_tops / fp4_peak,
                       traffic=traffic, traffic_source=traffic_src, peak_source=f"4 x bf16_tflops_sustained of MEASURED_PEAKS.json ({peaks['source']})",
                       frac_of_nominal_fp4=att_tops / NOMINAL_FP4_TFLOPS),
-        clocks=clocks, e2e=e2e, gpu_launches=6 * args.steps, ulysses=ulysses,
+        clocks=clocks, e2e=e2e, gpu_launches=launches_per_step(w, 4) * args.steps, ulysses=ulysses,
     )
     if not args.no_cpu_baseline:
         line["parity"] = parity_of_timed_output(w, *parity_in)
