@@ -457,8 +457,11 @@ __device__ __forceinline__ void quant_q_tile(
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
 // ------------------------------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
+// FEW: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
+// looks at), which makes room for a fourth block per SM:
+// 1 000 queries of 32 heads against 9 192 keys 143.9 -> 141.9 us per call, 4 250 tokens of 48 heads 359.0 -> 356.9 us.
+template <typename T, int D, bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     T* __restrict__ km,                // [B*H][D]
     const float* __restrict__ part,    // partial column sums to form the mean from ([B*H][chunks][D]), or nullptr: `km` holds it
@@ -467,7 +470,7 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     uint8_t* __restrict__ sfs,         // [B*H][Np/128][D/64][512]
     int rows,                          // query blocks of all query heads of a kv head
     int* __restrict__ status,
-    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 rows x 128 bytes, 128-byte swizzle
+    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 (FEW: 64) rows x 128 bytes, 128-byte swizzle
     const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*H][rows][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
     constexpr int CH = D / 16;            // microblocks per row
     constexpr int RPP = 256 / CH;         // rows per pass
@@ -488,9 +491,12 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t sbase = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     uint8_t* sgen = smem_dyn + (sbase - smem_u32(smem_dyn));
-    // [B tile: k' | A tile: qm chunk] as SUB sub-tiles of 128 rows x 128 bytes each, then small things, then (D = 64 only,
+    // [A tile: qm chunk | B tile: k'] as SUB sub-tiles of (FEW: A 64) 128 rows x 128 bytes each (in this order: the MMA reads 128 rows
+    // from the start of every A sub-tile, which has to stay inside the block's shared memory), then small things, then (D = 64 only,
     // where the A tile is too small for it) the staging tile of the epilogue: 8 warps x 32 rows x 128 bytes
-    constexpr int oB = 0, oA = SUB * 16384, oMean = 2 * SUB * 16384, oSf = oMean + D * 4, oBar = oSf + SUB * 512;
+    constexpr int kARows = FEW ? 64 : 128, kASub = kARows * 128;
+    constexpr int oA = 0, oB = SUB * kASub, oMean = oB + SUB * 16384, oSf = oMean + D * 4, oBar = oSf + SUB * 512;
+    static_assert(oA + (SUB - 1) * kASub + 16384 <= oMean, "the MMA's 128 A rows stay inside the tiles");
     constexpr int oStg = (D == 128) ? oA : ((oBar + 64 + 1023) / 1024) * 1024;
     float* s_mean = reinterpret_cast<float*>(sgen + oMean);
     uint8_t* s_sf = sgen + oSf;
@@ -526,10 +532,10 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
     }
     // the first A tile (see below) comes in while K is quantized
     auto load_a = [&](int m0) {
-        mbar_expect_tx(bar_a, SUB * 16384);
+        mbar_expect_tx(bar_a, SUB * kASub);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
-            tma_load_3d(sbase + oA + sub * 16384, &tm_qm, bar_a, sub * 128, m0, bh);
+            tma_load_3d(sbase + oA + sub * kASub, &tm_qm, bar_a, sub * 128, m0, bh);
     };
     if (t == 0) load_a(0);
     tc_fence_before();
@@ -589,8 +595,8 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
             tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
-                const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-                tc_mma_f16(tmem, make_sdesc(sbase + oA + off, 16, 1024, kSwz128), make_sdesc(sbase + oB + off, 16, 1024, kSwz128),
+                const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32, off_a = (ks >> 2) * kASub + (ks & 3) * 32;
+                tc_mma_f16(tmem, make_sdesc(sbase + oA + off_a, 16, 1024, kSwz128), make_sdesc(sbase + oB + off, 16, 1024, kSwz128),
                            idesc, ks > 0);
             }
             tc_commit(bar);
@@ -604,7 +610,8 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
         // which is free once the MMAs have completed) and leave as one TMA tile store; the engine clips rows beyond nqm.
         if (m0 + quarter * 32 < rows) {
             const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + chalf * 64;
-            uint8_t* stg = sgen + oStg + warp * 4096;
+            const int stg_off = oStg + (chalf * (kARows / 32) + quarter) * 4096;
+                uint8_t* stg = sgen + stg_off;
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 float v[32];
@@ -622,7 +629,7 @@ __global__ void __launch_bounds__(256, 3) quant_k_delta_kernel(
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-                tma_store_3d(&tm_delta, sbase + oStg + warp * 4096, (row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
+                tma_store_3d(&tm_delta, sbase + stg_off, (row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
                 bulk_commit_group();
                 bulk_wait_group_read0();      // the engine has read the staging tile: it may be written again
             }
@@ -850,17 +857,19 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         s.means.wait = true;
         if ((e = launch_pdl(prepass_stage_kernel<T, D>, dim3(s.n_q), dim3(256), (size_t)StageCfg<T, D>::kSmem, st, s)) != cudaSuccess) return e;
     }
-    const size_t smem_k = 2 * (D / 64) * 16384 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + 32768 : 0);
-    e = allow_smem(reinterpret_cast<const void*>(quant_k_delta_kernel<T, D>), (int)smem_k);
-    if (e != cudaSuccess) return e;
     // tensor maps for the K kernel: the Q means and delta_s of a kv head's query heads follow one another, so both are byte
     // tensors [B*Hkv][group * nqm][...] and one MMA takes the blocks of several heads
     const uint64_t rows = (uint64_t)(a.Hq / a.Hkv) * a.nqm;
+    const bool few = rows <= 64;
+    const int a_rows = few ? 64 : 128;
+    const size_t smem_k = (D / 64) * (128 + a_rows) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + a_rows * 256 : 0);
     alignas(64) CUtensorMap tm_qm, tm_delta;
-    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, 128, 3) != 0 ||
+    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, few ? 64 : 128, 3) != 0 ||
         encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    return launch_pdl(quant_k_delta_kernel<T, D>, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
+    auto kern = few ? quant_k_delta_kernel<T, D, true> : quant_k_delta_kernel<T, D, false>;
+    if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
+    return launch_pdl(kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
                       a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status, tm_qm, tm_delta);
 }
 

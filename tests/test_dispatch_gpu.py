@@ -61,10 +61,12 @@ def test_means_inside_and_outside_the_kernels(cuda_device, Nk, block_mean):
     assert (lse.cpu() - ref_lse).abs().max() <= 1e-3       # log2 / exp2 approximations, as in the LSE tests of the whole path
 
 
-@pytest.mark.parametrize("heads,Nq", [(1, 128 * 128), (1, 128 * 128 + 1), (8, 16 * 128), (8, 16 * 128 + 1)])
-def test_query_blocks_of_a_kv_head_around_one_mma(cuda_device, heads, Nq):
-    """delta_s takes 128 query blocks of all heads of a kv head at a time: 128 blocks, and one more per head."""
-    q, k, v = _inputs(cuda_device, 1, heads, 1, Nq, 200, 64, seed=1000 + heads)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("heads,Nq", [(8, 8 * 128), (8, 8 * 128 + 1), (1, 128 * 128), (1, 128 * 128 + 1), (8, 16 * 128), (8, 16 * 128 + 1)])
+def test_query_blocks_of_a_kv_head_around_one_mma(cuda_device, heads, Nq, D):
+    """delta_s takes 128 query blocks of all heads of a kv head at a time, and a smaller tile serves up to 64: 64 and 128 blocks, and
+    one more per head."""
+    q, k, v = _inputs(cuda_device, 1, heads, 1, Nq, 200, D, seed=1000 + heads)
     out = sageattn3(q, k, v)
     for h in {0, heads - 1}:
         tail = sageattn3(q[:, h:h + 1, -(Nq % 128 or 128):], k, v)         # the last block alone has the same block mean
