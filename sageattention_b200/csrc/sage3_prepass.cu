@@ -240,12 +240,12 @@ __device__ __forceinline__ void colsum_chunk(const Src<T>& x, int64_t sb, int64_
 // One sum of a column's partial sums, in the order of the chunks.
 __device__ __forceinline__ float sum_chunks(const float* __restrict__ part, int chunks, int D) {
     float s = 0.f;
-    for (int c = 0; c < chunks; c += 8) {
-        float v[8];
+    for (int c = 0; c < chunks; c += 16) {
+        float v[16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = c + i < chunks ? part[(int64_t)(c + i) * D] : 0.f;
+        for (int i = 0; i < 16; ++i) v[i] = c + i < chunks ? part[(int64_t)(c + i) * D] : 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s += v[i];       // (+ 0 beyond the last chunk: no change)
+        for (int i = 0; i < 16; ++i) s += v[i];       // (+ 0 beyond the last chunk: no change)
     }
     return s;
 }
@@ -505,11 +505,13 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + oBar + 12);
 
     const uint32_t bar_a = bar + 16;        // "the A tile has landed" (the bytes between hold the abort flag and the tensor-memory slot)
-    if (t == 0) {
+    if (t == 224) {
         *abort_flag = 0;
         mbar_init(bar, 1);
         mbar_init(bar_a, 1);
         mbar_fence_init();
+        prefetch_tmap(&tm_qm);
+        prefetch_tmap(&tm_delta);
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(tmem_slot), kTmemCols);
@@ -521,6 +523,14 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     });
     pdl_launch_dependents();
     pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
+    // the first A tile (see below) comes in while K is quantized
+    auto load_a = [&](int m0) {
+        mbar_expect_tx(bar_a, SUB * kASub);
+#pragma unroll
+        for (int sub = 0; sub < SUB; ++sub)
+            tma_load_3d(sbase + oA + sub * kASub, &tm_qm, bar_a, sub * 128, m0, bh);
+    };
+    if (t == 224) load_a(0);       // (a warp with nothing else to do here)
     if (t < D) {
         if (part != nullptr) {
             const T m = Num<T>::from_f(sum_chunks(part + (int64_t)bh * chunks * D + t, chunks, D) * (N > 0 ? 1.0f / (float)N : 0.f));
@@ -530,14 +540,6 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
             s_mean[t] = Num<T>::to_f(km[(int64_t)bh * D + t]);
         }
     }
-    // the first A tile (see below) comes in while K is quantized
-    auto load_a = [&](int m0) {
-        mbar_expect_tx(bar_a, SUB * kASub);
-#pragma unroll
-        for (int sub = 0; sub < SUB; ++sub)
-            tma_load_3d(sbase + oA + sub * kASub, &tm_qm, bar_a, sub * 128, m0, bh);
-    };
-    if (t == 0) load_a(0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -562,9 +564,11 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
         // k' into the B tile: this item's 16 elements are the 16-byte chunks 2c, 2c+1 of row rt
 #pragma unroll
         for (int q2 = 0; q2 < 2; ++q2) {
-            const int chunk = 2 * c + q2, sub = chunk >> 3, cw = chunk & 7;
+            // (the two sub-tiles lie on the same banks: where one half of a row's threads store even chunks, the other store odd ones)
+            const bool odd = (q2 ^ (c >> 2)) & 1;
+            const int chunk = 2 * c + (odd ? 1 : 0), sub = chunk >> 3, cw = chunk & 7;
             *reinterpret_cast<uint4*>(sgen + oB + sub * 16384 + rt * 128 + ((cw ^ (rt & 7)) << 4)) =
-                make_uint4(w[4 * q2], w[4 * q2 + 1], w[4 * q2 + 2], w[4 * q2 + 3]);
+                make_uint4(odd ? w[4] : w[0], odd ? w[5] : w[1], odd ? w[6] : w[2], odd ? w[7] : w[3]);
         }
     }
     __syncthreads();
