@@ -21,8 +21,9 @@
 // nothing else connects the groups: four independent chains per scheduler, a quarter of an item apart.
 // What bounds it: the exp2 unit (16 results per clock and SM: 1 096 cycles per 128 x 128 block with the exponentials of the
 // scales) and, next to it, the instruction latency of the softmax warps; the tensor pipe needs 580 cycles.  Measured (B = 2,
-// H = 32, N = 16 384): 1 525 cycles per block at D = 128 and 1 490 at D = 64, the exp2 unit 77 % busy.  (With a row shared by two
-// threads and all warps of a tile in step, as this kernel was first: 1 640 and 1 590.)  Units in place of one CTA per pair took the
+// H = 32, N = 16 384, 1 965 MHz): 1 532 cycles per block at D = 128 and 1 477 at D = 64, the exp2 unit 77 % busy; the softmax code
+// without any wait and without the other warps takes 1 233.  (With a row shared by two threads and all warps of a tile in step,
+// as this kernel was first: 1 662 and 1 611.)  Units in place of one CTA per pair took the
 // drain and refill of the pipeline, 10 us per pair, out: B = 2, H = 32, N = 8 192 causal 960 -> 776 us, B = 4, H = 32, N = 1 024
 // 99 -> 77 us, two key blocks per tile (B = 2, H = 48, 17 550 queries x 226 keys, D = 64) 483 -> 250 us.
 // Halves of 64 keys because a thread's registers hold 64 scores, and because tensor memory has room for three 64-key buffers
