@@ -73,6 +73,22 @@ def test_query_blocks_of_a_kv_head_around_one_mma(cuda_device, heads, Nq, D):
         assert torch.equal(out[:, h:h + 1, -tail.shape[2]:], tail)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Nq,Nk,causal", [(130, n, False) for n in (63, 64, 65, 127, 191, 192, 193, 226)]
+                         + [(256, n, True) for n in (160, 192, 193, 255, 256, 257, 288, 319)])
+def test_mask_edges_of_half_blocks_and_warps(cuda_device, Nq, Nk, causal, D):
+    """Lengths around the 64 keys of a half block and causal shifts around the 32 rows of a warp.  A masked-out key that got
+    through would be the only large one: the keys past a row's limit point along its query."""
+    q, k, v = _inputs(cuda_device, 1, 2, 2, Nq, Nk, D, seed=950 + Nk)
+    if causal:
+        rows = torch.arange(Nk, device=q.device) - (Nk - Nq) - 1                  # the query whose first hidden key this is
+        hidden = (rows >= 0) & (rows < Nq)
+        k[:, :, hidden] += q[:, :, rows[hidden]]
+    out = sageattn3(q, k, v, is_causal=causal)
+    ref = O.sageattn3_oracle(q.cpu(), k.cpu(), v.cpu(), is_causal=causal)
+    assert O.cosine(out.cpu(), ref) >= 0.999 and O.rel_l1(out.cpu(), ref) <= 0.01
+
+
 @pytest.mark.parametrize("pad", [8, 16])
 def test_output_rows_on_16_and_32_byte_boundaries(cuda_device, pad):
     q, k, v = _inputs(cuda_device, 1, 3, 3, 200, 300, 64, seed=1100)
