@@ -82,27 +82,37 @@ constexpr int kUnitRing = 4;
 // PACK: few query rows and several query heads per kv head.  The rows of all these heads share one 128-row tile (row = head * Nq +
 // token), so the keys are walked once instead of once per head: 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv
 // heads 122 -> 64 us.
-template <int D, bool PACK>
+//
+// PACK == 2: at most 32 such rows.  A thread owns a row of scores, so one warp of the four would have work and do the exponentials
+// of all 128 keys for it.  The rows stand in every quarter of the tile instead (rows 0..31 = 32..63 = ...), and the warp of quarter
+// w takes keys 32 w .. 32 w + 31 of the block for all of them: a quarter of the exponentials per warp.  The four exchange their
+// maxima through shared memory; P, its scales and the accumulator are those of rows 0..31.  Same operations per score, and the row
+// sums are added in the same order, so the same bits.  D = 128, 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv heads:
+// 62 -> 44 us (about 980 cycles per block; neither the loads, nor more stages, nor fewer tcgen05 instructions change that).
+template <int D, int PACK>
 struct Cfg {
-    static constexpr int kStages = (D == 128) ? 4 : (PACK ? 6 : 8);        // K and V^T stages, each shared by the two query tiles
+    // K and V^T stages, each shared by the two query tiles (as many as fit: PACK, see oP)
+    static constexpr int kStages = PACK == 2 ? (D == 128 ? 7 : 11) : PACK ? (D == 128 ? 5 : 8) : (D == 128 ? 4 : 8);
+    static constexpr int kQTiles = PACK ? 1 : 2;              // query tiles per unit
     static constexpr int kThreads = 768;                      // 6 warpgroups, see the kernel
     // S buffers of 128 rows x 64 keys: a rotation for the first halves of the items and one for the second halves (D = 64 has room for
     // a second one of the latter: 1 % slower)
-    static constexpr int kSBufs0 = 2, kSBufs1 = 1, kSBufs = kSBufs0 + kSBufs1;
+    static constexpr int kSBufs0 = 2, kSBufs1 = PACK ? 2 : 1, kSBufs = kSBufs0 + kSBufs1;
     static constexpr int kQBytes = 128 * D / 2;               // per query tile
     static constexpr int kSfQkBytes = (D / 64) * 512;
     static constexpr int kKBytes = 128 * D / 2;
     static constexpr int kVBytes = D * 64;
     static constexpr int kSfVBytes = 1024;
     static constexpr int kDeltaBytes = 256;
-    static constexpr int kPBytes = 8192;
+    // P slot to slot. PACK == 2 writes rows 0 .. 31 only, and lets the other rows of the operand be the next slots' bytes: finite codes, and scales of 0
+    static constexpr int kPBytes = PACK == 2 ? 2048 : 8192;
     // shared-memory map (bytes from a 1024-aligned base)
     static constexpr int oQ = 0;                              // [buffer][tile] 8192
-    static constexpr int oK = oQ + 4 * 8192;
+    static constexpr int oK = oQ + 2 * kQTiles * 8192;
     static constexpr int oV = oK + kStages * kKBytes;
     static constexpr int oP = oV + kStages * kVBytes;            // [slot] 8192
-    static constexpr int oSfQ = oP + 8 * kPBytes;             // [buffer][tile] 1024
-    static constexpr int oSfK = oSfQ + 4 * 1024;
+    static constexpr int oSfQ = oP + 7 * kPBytes + 8192;      // [buffer][tile] 1024
+    static constexpr int oSfK = oSfQ + 2 * kQTiles * 1024;
     static constexpr int oSfV = oSfK + kStages * 1024;
     static constexpr int oSfP = oSfV + kStages * 1024;        // [slot] 1024
     // delta_s per stage: one row per tile, 256 B + 256 B that stay zero; PACK: [16 chunks of 8 keys][8 heads] 16 B + 128 B that stay zero
@@ -111,15 +121,17 @@ struct Cfg {
     static constexpr int oOnes = oDelta + kStages * kDeltaStage;   // 128 x 16 tile: 1.0 in column 0 (PACK: in the column of the row's head), rest 0
     static constexpr int oStat = oOnes + 4096;                // float2 [slot][128 rows]: running maximum, rescale factor
     static constexpr int oSum = oStat + 8192;                 // float2 [slot][128 rows]: row sums of the two key halves of a block
-    static constexpr int oL = oSum + 8192;                    // float2 [tile][128 rows]: running row sums of the two key halves
+    static constexpr int oMax = oSum + (PACK == 2 ? 16384 : 8192);      // PACK == 2: float [slot][quarter][32 rows]; oSum: float4 [slot][quarter][32 rows]
+    static constexpr int oL = oMax + (PACK == 2 ? 4096 : 0);                    // float2 [tile][128 rows]: running row sums of the two key halves
     static constexpr int oM = oL + 2048;                      // float [tile][128 rows]: running maximum
     static constexpr int oBar = oM + 1024;
-    static constexpr int kNumBars = 4 + 4 * kStages + kSBufs + 8 + 7 * 8 + 2 * kUnitRing;
+    static constexpr int kNumBars = 4 + 4 * kStages + kSBufs + 8 + 7 * 8 + (PACK == 2 ? 4 : 0) + 2 * kUnitRing;
     static constexpr int oUnit = (oBar + kNumBars * 8 + 15) / 16 * 16;      // descriptors of the units being worked on
     static constexpr int oMisc = oUnit + kUnitRing * 64;
     static constexpr int kSmemBytes = oMisc + 64 + 1024;      // + slack for the manual 1024-byte alignment
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory");
     // tensor-memory columns: the S buffers, one O accumulator per tile, scale factors (Q, K: one copy per issuer)
-    static constexpr uint32_t cS = 0, cO = 64 * kSBufs, cSfQ = cO + 2 * D, cSfK = cSfQ + 32, cSfV = cSfK + 16, cSfP = cSfV + 8;
+    static constexpr uint32_t cS = 0, cO = 64 * kSBufs, cSfQ = cO + (PACK ? 1 : 2) * D, cSfK = cSfQ + 32, cSfV = cSfK + 16, cSfP = cSfV + 8;
     static_assert(cSfP + 8 <= 512, "tensor memory");
     static constexpr uint64_t kSwzQK = (D == 128) ? kSwz64 : kSwz32;
     static constexpr uint32_t kSboQK = (D == 128) ? 512 : 256;
@@ -169,7 +181,7 @@ struct __align__(16) Unit {
 // Unit number u of the launch; false when it is empty (beyond a short sequence of a packed batch).
 // Order: without a mask pairs of tiles of one head are neighbours (its K and V are shared in L2); under a causal mask the
 // pairs with the most keys of all heads come first, so that the short ones level out the end of the launch.
-template <bool CAUSAL, bool VARLEN, bool PACK>
+template <bool CAUSAL, bool VARLEN, int PACK>
 __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
     if constexpr (PACK) {
         w.bhkv = u / p.pack_tiles;
@@ -240,7 +252,7 @@ __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
     return true;
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN, bool PACK>
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK>
 __global__ void __launch_bounds__(Cfg<D, PACK>::kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ AttnParams p) {
@@ -256,7 +268,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t bars = uniform(sbase + C::oBar);
     auto bar = [&](int i) { return bars + 8u * i; };
     constexpr int bQF = 0, bQE = 2, bKF = 4, bKE = bKF + S, bVF = bKE + S, bVE = bVF + S, bSF = bVE + S, bSE = bSF + 8, bM = bSE + C::kSBufs,
-                  bPF = bM + 32, bPV = bPF + 8, bOS = bPV + 8, bWF = bOS + 8, bWE = bWF + kUnitRing, bEnd = bWE + kUnitRing;
+                  bPF = bM + 32, bPV = bPF + 8, bOS = bPV + 8, bX = bOS + 8, bWF = bX + (PACK == 2 ? 4 : 0), bWE = bWF + kUnitRing, bEnd = bWE + kUnitRing;
     static_assert(bEnd == C::kNumBars, "barriers");
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + C::oMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + C::oMisc + 8);
@@ -265,11 +277,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (threadIdx.x < C::kNumBars) {
         const int i = threadIdx.x;
         uint32_t count = 1;                                      // copies landed, MMAs complete, one warp's statistics
-        if (i >= bQE && i < bKF) count = 2;                      // Q buffer free: both Q K^T issuers are done with it
-        if (i >= bKE && i < bKE + S) count = 2;                  // K stage free: likewise
+        if (i >= bQE && i < bKF) count = PACK == 2 ? 1 : 2;      // Q buffer free: the Q K^T issuers are done with it
+        if (i >= bKE && i < bKE + S) count = PACK == 2 ? 1 : 2;  // K stage free: likewise
         if (i >= bSE && i < bM) count = 4;                       // S buffer free: the four warps of its group hold the scores
         if (i >= bPF && i < bPV) count = 4;                      // P, its scales and the row sums written
-        if (i >= bOS && i < bWF) count = 4;                               // the correction warps are done with O (and have seen P written)
+        if (i >= bOS && i < bWF) count = 4;                      // the correction warps are done with O (and have seen P written); bX: maxima exchanged
         if (i >= bWE) count = C::kThreads / 32 - 1;              // unit descriptor free: every warp but the producer has finished the unit
         mbar_init(bar(i), count);
         mbar_fence_init();
@@ -287,15 +299,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int i = threadIdx.x; i < nd + 4096 / 16; i += C::kThreads) {
             uint4 v = make_uint4(0, 0, 0, 0);
             if (i >= nd && i < nd + 128) {
-                const int g = PACK ? (i - nd) / p.Nq : 0;
+                const int g = PACK ? (PACK == 2 ? (i - nd) & 31 : i - nd) / p.Nq : 0;
                 const uint32_t w = one << (16 * (g & 1));
                 if (!PACK || g < p.pack_heads) v = make_uint4(g >> 1 == 0 ? w : 0, g >> 1 == 1 ? w : 0, g >> 1 == 2 ? w : 0, g >> 1 == 3 ? w : 0);
             }
             z[i] = v;
         }
         if constexpr (PACK) {
-            for (int i = threadIdx.x; i < 4 * 8192 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oQ)[i] = make_uint4(0, 0, 0, 0);
-            for (int i = threadIdx.x; i < 4 * 1024 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oSfQ)[i] = make_uint4(0, 0, 0, 0);
+            for (int i = threadIdx.x; i < 2 * C::kQTiles * 8192 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oQ)[i] = make_uint4(0, 0, 0, 0);
+            for (int i = threadIdx.x; i < 2 * C::kQTiles * 1024 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oSfQ)[i] = make_uint4(0, 0, 0, 0);
+            // rows 32 .. 127 of P have no writer: scale 0
+            for (int i = threadIdx.x; PACK == 2 && i < 8 * 1024 / 16; i += C::kThreads) reinterpret_cast<uint4*>(sgen + C::oSfP)[i] = make_uint4(0, 0, 0, 0);
         }
         fence_proxy_async_smem();
     }
@@ -381,7 +395,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const float2 ma = stat[slot * 128];
               const float alpha = ma.y;
               // the first block has nothing to rescale unless the accumulator was carried in
-              if ((!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
+              if ((PACK != 2 || quarter == 0) && (!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
                   // the P V MMA of the tile's previous block must have landed first
                   if (!first) {
                       const int sp = sg - 1 - two;
@@ -405,7 +419,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               tc_fence_before();
               // P V issue waits for this warpgroup only, so its arrival also stands for "P is written"
               if (!warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
-              const float2 rs = sum[slot * 128];
+              float2 rs;
+              if constexpr (PACK == 2) {
+                  // scale and sum of every microblock, two per quarter
+                  const float4* mb = reinterpret_cast<const float4*>(sgen + C::oSum) + slot * 128 + lane;
+                  const float4 a = mb[0], b = mb[32], c = mb[64], e = mb[96];
+                  rs.x = fmaf(b.z, b.w, fmaf(b.x, b.y, fmaf(a.z, a.w, fmaf(a.x, a.y, 0.f))));
+                  rs.y = fmaf(e.z, e.w, fmaf(e.x, e.y, fmaf(c.z, c.w, fmaf(c.x, c.y, 0.f))));
+              } else {
+                  rs = sum[slot * 128];
+              }
               warp_arrive(bar(bOS + slot), lane);
               float2 l = l_s[t * 128];
               l.x = fmaf(l.x, alpha, rs.x);
@@ -515,21 +538,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 for (int r = lane; r < live; r += 32) {
                     const int g = r / p.Nq, i = r - g * p.Nq;
 #pragma unroll
-                    for (int a = 0; a < D / 64; ++a)
-                        *reinterpret_cast<uint32_t*>(sgen + C::oSfQ + qb * 2048 + sf_atom_offset(r, 4 * a)) =
-                            *reinterpret_cast<const uint32_t*>(p.q_sf + (size_t)(w.bhq + g) * C::kSfQkBytes + sf_atom_offset(i, 4 * a));
+                    for (int a = 0; a < D / 64; ++a) {
+                        const uint32_t sf = *reinterpret_cast<const uint32_t*>(p.q_sf + (size_t)(w.bhq + g) * C::kSfQkBytes + sf_atom_offset(i, 4 * a));
+#pragma unroll
+                        for (int c = 0; c < (PACK == 2 ? 4 : 1); ++c)
+                            *reinterpret_cast<uint32_t*>(sgen + C::oSfQ + qb * C::kQTiles * 1024 + sf_atom_offset(r + 32 * c, 4 * a)) = sf;
+                    }
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_expect_tx(bar(bQF + qb), p.pack_heads * p.Nq * (D / 2));
-                    tma_load_3d(sbase + C::oQ + qb * 2 * 8192, &tm_q, bar(bQF + qb), 0, 0, w.bhq);
+                    constexpr int copies = PACK == 2 ? 4 : 1;
+                    mbar_expect_tx(bar(bQF + qb), copies * p.pack_heads * p.Nq * (D / 2));
+                    for (int c = 0; c < copies; ++c)
+                        tma_load_3d(sbase + C::oQ + qb * C::kQTiles * 8192 + c * 32 * (D / 2), &tm_q, bar(bQF + qb), 0, 0, w.bhq);
                 }
             } else if (lane == 0) {
                 mbar_expect_tx(bar(bQF + qb), w.nv * (C::kQBytes + C::kSfQkBytes));
                 for (int t = 0; t < w.nv; ++t) {
-                    tma_load_3d(sbase + C::oQ + (qb * 2 + t) * 8192, &tm_q, bar(bQF + qb), 0, (w.mt0 + t) * kBlock, w.bhq);
-                    bulk_load(sbase + C::oSfQ + (qb * 2 + t) * 1024, p.q_sf + ((size_t)w.bhq * p.nqt + w.mt0 + t) * C::kSfQkBytes,
+                    tma_load_3d(sbase + C::oQ + (qb * C::kQTiles + t) * 8192, &tm_q, bar(bQF + qb), 0, (w.mt0 + t) * kBlock, w.bhq);
+                    bulk_load(sbase + C::oSfQ + (qb * C::kQTiles + t) * 1024, p.q_sf + ((size_t)w.bhq * p.nqt + w.mt0 + t) * C::kSfQkBytes,
                               C::kSfQkBytes, bar(bQF + qb));
                 }
             }
@@ -566,9 +594,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // ones, each into its own S buffers (issuing one half takes a few hundred cycles next to busy softmax warps: one
         // issuer for both would be the slowest part of the pipeline).  The whole warp walks the loop and one elected lane
         // issues, so loop state and descriptors stay in uniform registers.
+        // (PACK == 2: softmax is short there, and the tensor pipe's cost per instruction counts; warp 1 issues all 128 keys at once.)
         const int h = warp >> 1;
-        constexpr uint32_t idesc_qk = make_idesc_nvfp4(64);
-        constexpr uint32_t idesc_delta = make_idesc_f16_bmn(64, std::is_same<OutT, __nv_bfloat16>::value);
+        constexpr int kKeys = PACK == 2 ? 128 : 64;
+        constexpr uint32_t idesc_qk = make_idesc_nvfp4(kKeys);
+        constexpr uint32_t idesc_delta = make_idesc_f16_bmn(kKeys, std::is_same<OutT, __nv_bfloat16>::value);
         // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
         constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(PACK ? 128 : 16, kSwzNone);
         const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo0 = sdesc_lo(sbase + C::oQ, 16), sfq_lo0 = sdesc_lo(sbase + C::oSfQ, 0);
@@ -585,7 +615,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
             unit_done(i);
-            if (ns == 0) continue;
+            if (ns == 0 || (PACK == 2 && h == 1)) continue;
             const int qb = k & 1;
             if (!warp_wait(bar(bQF + qb), (k >> 1) & 1, abort_flag, p.status, kWaitQFull)) break;
             ++k;
@@ -594,7 +624,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 for (int t = 0; t < nv; ++t)
 #pragma unroll
                     for (int ks = 0; ks < D / 64; ++ks)
-                        tc_cp_sf(sfq_col0 + 8 * t + 4 * ks, sdesc(sfq_lo0 + (qb * 2 + t) * 64 + ks * 32, sdesc_hi(128, kSwzNone)));
+                        tc_cp_sf(sfq_col0 + 8 * t + 4 * ks, sdesc(sfq_lo0 + (qb * C::kQTiles + t) * 64 + ks * 32, sdesc_hi(128, kSwzNone)));
             }
             __syncwarp();
             for (int s = 0; s < ns; ++s) {
@@ -604,8 +634,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 if (!warp_wait(bar(bSE + buf0 + buf), buf_parity, abort_flag, p.status, kWaitSEmpty)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t k_lo = k_lo0 + st * (C::kKBytes / 16), delta_lo = delta_lo0 + st * (C::kDeltaStage / 16) + t * (C::kDeltaPitch / 16);
-                const uint32_t sfk_lo = sfk_lo0 + st * (1024 / 16), q_lo = q_lo0 + (qb * 2 + t) * (8192 / 16);
-                const uint32_t s_col = tmem + C::cS + 64 * (buf0 + buf), sfq_col = sfq_col0 + 8 * t;
+                const uint32_t sfk_lo = sfk_lo0 + st * (1024 / 16), q_lo = q_lo0 + (qb * C::kQTiles + t) * (8192 / 16);
+                const uint32_t s_col = tmem + C::cS + kKeys * (buf0 + buf), sfq_col = sfq_col0 + 8 * t;
                 if (elect_one()) {
                     if (opens) {
 #pragma unroll
@@ -671,6 +701,98 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         __syncwarp();
       }
+    } else if constexpr (PACK == 2) {
+        reg_alloc<96>();
+        // ------------------------------------------------------------------ softmax groups, at most 32 rows
+        // As below, but the thread's row is its lane and the warp's keys are 32 * quarter .. + 31 of the block.
+        const int g = (warp >> 2) - 1, quarter = warp & 3;
+        const uint32_t s_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + C::cS + 32 * quarter;
+        const int head = lane / p.Nq, tok = lane - head * p.Nq;
+        float* wmax = reinterpret_cast<float*>(sgen + C::oMax) + lane;
+        float2* stat = reinterpret_cast<float2*>(sgen + C::oStat) + quarter * 32 + lane;
+        uint8_t* prow = sgen + C::oP + lane * 64 + ((quarter ^ ((lane >> 1) & 3)) << 4);
+        bool alive = true;
+        const Unit* u;
+        for (int i = 0; alive && (u = next_unit(i)) != nullptr; ++i) {
+            const int ns = uniform(u->ns), Nk = uniform(u->Nk), shift = CAUSAL ? uniform(u->shift) : 0;
+            const float sl2 = p.sm_scale_per_head ? p.sm_scale_per_head[u->hq + min(head, u->nb[1] - 1)] * 1.4426950408889634f : p.sm_scale_log2;
+            const uint64_t sl2x2 = pack2f(sl2, sl2);
+            for (int s = (g - base) & 3; s < ns; s += 4) {
+                const int sg = base + s, slot = sg & 7, slot_prev = (sg - 1) & 7, buf = sg % C::kSBufs0;
+                const int key0 = (ns - 1 - s) * kBlock + 32 * quarter;
+                if (!warp_wait(bar(bSF + 2 * g), (sg >> 2) & 1, abort_flag, p.status, kWaitSFull)) { alive = false; break; }
+                tc_fence_after();
+                float x[32];
+                tmem_ld32(s_addr + 128 * buf, x);
+                tc_wait_ld();
+                tc_fence_before();
+                warp_arrive(bar(bSE + buf), lane);
+                if (key0 + 31 > (CAUSAL ? min(Nk - 1, shift) : Nk - 1)) {
+                    const float vis = (float)((CAUSAL ? min(Nk - 1, tok + shift) : Nk - 1) - key0);
+#pragma unroll
+                    for (int q = 0; q < 32; ++q)
+                        if ((float)q > vis) x[q] = -INFINITY;
+                }
+                float bm[2], se[2];
+                uint32_t codes[4];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float* y = x + 16 * b;
+                    const float a = fmax3(fmax3(y[0], y[1], y[2]), y[12], y[13]);
+                    const float c = fmax3(fmax3(y[3], y[4], y[5]), y[14], y[15]);
+                    bm[b] = fmax3(a, c, fmax3(fmax3(y[6], y[7], y[8]), fmax3(y[9], y[10], y[11]), kNoKey));
+                }
+                wmax[(slot * 4 + quarter) * 32] = fmaxf(bm[0], bm[1]);
+                warp_arrive(bar(bX + g), lane);
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float negc = fmaf(bm[b], -sl2, kLog2Of6);
+                    const uint64_t negc2 = pack2f(negc, negc);
+                    float e[16];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        float a, c;
+                        unpack2f(fma2(pack2f(x[16 * b + 2 * q], x[16 * b + 2 * q + 1]), sl2x2, negc2), a, c);
+                        e[2 * q] = ex2_approx(a);
+                        e[2 * q + 1] = ex2_approx(c);
+                    }
+                    uint64_t acc0 = pack2f(e[0], e[1]), acc1 = pack2f(e[2], e[3]);
+#pragma unroll
+                    for (int q = 4; q < 16; q += 4) {
+                        acc0 = add2(acc0, pack2f(e[q], e[q + 1]));
+                        acc1 = add2(acc1, pack2f(e[q + 2], e[q + 3]));
+                    }
+                    float se0, se1;
+                    unpack2f(add2(acc0, acc1), se0, se1);
+                    se[b] = se0 + se1;
+                    codes[2 * b] = cvt_e2m1x8(e[0], e[1], e[2], e[3], e[4], e[5], e[6], e[7]);
+                    codes[2 * b + 1] = cvt_e2m1x8(e[8], e[9], e[10], e[11], e[12], e[13], e[14], e[15]);
+                }
+                if (sg >= 8 && !warp_wait(bar(bPV + slot), ((sg >> 3) - 1) & 1, abort_flag, p.status, kWaitPEmpty)) { alive = false; break; }
+                *reinterpret_cast<uint4*>(prow + slot * C::kPBytes) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
+                if (!warp_wait(bar(bX + g), (sg >> 2) & 1, abort_flag, p.status, kWaitPair)) { alive = false; break; }
+                float m_old = -INFINITY;
+                if (s > 0) {
+                    if (!warp_wait(bar(bM + slot_prev * 4 + quarter), ((sg - 1) >> 3) & 1, abort_flag, p.status, kWaitPair)) { alive = false; break; }
+                    m_old = stat[slot_prev * 128].x;
+                }
+                const float* wm = wmax + slot * 128;
+                const float m_run = fmax3(fmax3(wm[0], wm[32], wm[64]), wm[96], m_old);
+                const float alpha = ex2_approx((m_old - m_run) * sl2);
+                stat[slot * 128] = make_float2(m_run, alpha);
+                warp_arrive(bar(bM + slot * 4 + quarter), lane);
+                const float max_scaled = (m_run == kNoKey) ? 0.f : fmaf(m_run, sl2, kPScaleLog2);
+                const float sf0 = ex2_approx(fmaf(bm[0], sl2, -max_scaled) - kLog2Of6), sf1 = ex2_approx(fmaf(bm[1], sl2, -max_scaled) - kLog2Of6);
+                *reinterpret_cast<uint16_t*>(sgen + C::oSfP + slot * 1024 + 512 * (quarter >> 1) + lane * 16 + 2 * (quarter & 1)) =
+                    static_cast<uint16_t>((cvt_e4m3x2(sf0, 0.f) & 0xffu) | (cvt_e4m3x2(sf1, 0.f) & 0xffu) << 8);
+                reinterpret_cast<float4*>(sgen + C::oSum)[slot * 128 + quarter * 32 + lane] = make_float4(sf0, se[0], sf1, se[1]);
+                fence_proxy_async_smem();
+                warp_arrive(bar(bPF + slot), lane);
+            }
+            unit_done(i);
+            base += ns;
+        }
+        __syncwarp();
     } else {
         reg_alloc<96>();
         // ------------------------------------------------------------------ softmax groups (4 x 4 warps)
@@ -880,7 +1002,7 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
     return (int)make_map(fn, static_cast<CUtensorMap*>(map64), base, n0, n1, n2, b0, b1, swz);
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN, bool PACK>
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK>
 static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int grid, cudaStream_t st) {
     auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK>;
@@ -892,11 +1014,12 @@ static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUte
 
 template <int D, bool CAUSAL, typename OutT>
 static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
-                            const AttnParams& p, int grid, cudaStream_t st) {
+                            const AttnParams& p, int pack_mode, int grid, cudaStream_t st) {
     // packed variable-length batches run their own instantiation, so that the uniform kernels carry none of it
-    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, false>(a, tq, tk, tv, td, p, grid, st)
-           : p.pack_heads > 1 ? launch_v<D, CAUSAL, OutT, false, true>(a, tq, tk, tv, td, p, grid, st)
-                              : launch_v<D, CAUSAL, OutT, false, false>(a, tq, tk, tv, td, p, grid, st);
+    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, 0>(a, tq, tk, tv, td, p, grid, st)
+           : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(a, tq, tk, tv, td, p, grid, st)
+           : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(a, tq, tk, tv, td, p, grid, st)
+                              : launch_v<D, CAUSAL, OutT, false, 0>(a, tq, tk, tv, td, p, grid, st);
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
@@ -906,20 +1029,23 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     CUtensorMap tq, tk, tv, td;
     const uint32_t rowb = a.D / 2;
     const CUtensorMapSwizzle swz_qk = (a.D == 128) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-    // Few query rows and several heads per kv head (token generation): as many heads as fit share a tile.  Two heads at least,
-    // eight at most (the operand that adds delta_s has eight rows), and no carried state.
+    // Few query rows and several heads per kv head (token generation): as many heads as fit share a tile, eight at
+    // most (the operand that adds delta_s has eight rows), without carried state.  Mode 2, where a warp takes a quarter of the keys
+    // for all rows, when the rows of these heads (of one head, too) fit one warp: it would need more tiles otherwise.
     const int group = a.Hq / a.Hkv;
+    const bool plain = a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr;
     int pack = 1;
-    if (a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr && a.Nq <= kBlock / 2) {
+    if (plain && a.Nq <= kBlock / 2) {
         pack = kBlock / a.Nq < group ? kBlock / a.Nq : group;
         if (pack > 8) pack = 8;
     }
-    CUresult r = make_map(fn, &tq, a.q_codes, rowb, a.Nq_p, (uint64_t)a.B * a.Hq, rowb, pack > 1 ? a.Nq : kBlock, swz_qk, pack);
+    const int mode = plain && a.Nq * (group < 8 ? group : 8) <= 32 ? 2 : pack > 1 ? 1 : 0;
+    CUresult r = make_map(fn, &tq, a.q_codes, rowb, a.Nq_p, (uint64_t)a.B * a.Hq, rowb, mode ? a.Nq : kBlock, swz_qk, pack);
     if (r == CUDA_SUCCESS) r = make_map(fn, &tk, a.k_codes, rowb, a.Nk_p, (uint64_t)a.B * a.Hkv, rowb, kBlock, swz_qk);
     if (r == CUDA_SUCCESS)
         r = make_map(fn, &tv, a.v_codes, a.Nk_p / 2, a.D, (uint64_t)a.B * a.Hkv, 64, a.D, CU_TENSOR_MAP_SWIZZLE_64B);
     td = tv;                            // (only the PACK kernels use it)
-    if (r == CUDA_SUCCESS && pack > 1) {
+    if (r == CUDA_SUCCESS && mode) {
         // delta_s as [Nk_p / 8][B * Hq][8 keys]: eight keys of eight heads are one core matrix
         const cuuint64_t dims[3] = {16, (cuuint64_t)a.B * a.Hq, (cuuint64_t)a.Nk_p / 8}, strides[2] = {(cuuint64_t)a.Nk_p * 2, 16};
         const cuuint32_t box[3] = {16, 8, kBlock / 8}, estr[3] = {1, 1, 1};
@@ -944,7 +1070,7 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.whole_units = split ? pairs - rest : pairs;
     p.pack_heads = pack;
     p.pack_tiles = (group + pack - 1) / pack;
-    p.units = pack > 1 ? a.B * a.Hkv * p.pack_tiles : split ? pairs + rest : pairs;
+    p.units = mode ? a.B * a.Hkv * p.pack_tiles : split ? pairs + rest : pairs;
     const int grid = p.units < sms ? p.units : sms;
     p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;
@@ -966,15 +1092,15 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.causal_shift = a.causal_shift;
     p.cu_q = a.cu_q; p.cu_k = a.cu_k;
     if (a.is_bf16) {
-        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st)
-                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st);
-        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st)
-                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, td, p, grid, st);
+        if (a.D == 128) return a.is_causal ? launch_t<128, true, __nv_bfloat16>(a, tq, tk, tv, td, p, mode, grid, st)
+                                           : launch_t<128, false, __nv_bfloat16>(a, tq, tk, tv, td, p, mode, grid, st);
+        return a.is_causal ? launch_t<64, true, __nv_bfloat16>(a, tq, tk, tv, td, p, mode, grid, st)
+                           : launch_t<64, false, __nv_bfloat16>(a, tq, tk, tv, td, p, mode, grid, st);
     }
-    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, td, p, grid, st)
-                                       : launch_t<128, false, __half>(a, tq, tk, tv, td, p, grid, st);
-    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, td, p, grid, st)
-                       : launch_t<64, false, __half>(a, tq, tk, tv, td, p, grid, st);
+    if (a.D == 128) return a.is_causal ? launch_t<128, true, __half>(a, tq, tk, tv, td, p, mode, grid, st)
+                                       : launch_t<128, false, __half>(a, tq, tk, tv, td, p, mode, grid, st);
+    return a.is_causal ? launch_t<64, true, __half>(a, tq, tk, tv, td, p, mode, grid, st)
+                       : launch_t<64, false, __half>(a, tq, tk, tv, td, p, mode, grid, st);
 }
 
 }  // namespace sage3

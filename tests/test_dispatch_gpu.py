@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import sage3_oracle as O
-from sageattention_b200 import Sage3Problem, sageattn3
+from sageattention_b200 import Sage3Problem, sageattn3, sageattn_varlen
 
 pytestmark = pytest.mark.gpu
 
@@ -45,6 +45,19 @@ def test_heads_sharing_a_tile(cuda_device, Nq, Hq, Hkv, Nk, D, causal):
     assert torch.equal(out, rep) and torch.equal(lse, rep_lse)
     ref = O.sageattn3_oracle(q.cpu(), k.cpu(), v.cpu(), is_causal=causal, sm_scale=scale)
     assert O.cosine(out.cpu(), ref) >= 0.999 and O.rel_l1(out.cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("B,Nq,Hq,Hkv,D", [(2, 1, 4, 1, 128), (1, 4, 14, 2, 64), (1, 32, 2, 2, 128), (1, 33, 2, 2, 64), (2, 2, 32, 2, 64),
+                                           (1, 4, 8, 1, 128), (1, 5, 8, 1, 128), (3, 1, 60, 60, 64)])
+@pytest.mark.parametrize("Nk,causal", [(31, False), (32, True), (33, False), (97, True), (128, True), (129, False), (1300, True)])
+def test_few_rows_split_by_keys(cuda_device, B, Nq, Hq, Hkv, D, Nk, causal):
+    """Up to 32 rows per kv head: a warp takes 32 keys of a block for all rows.  Row counts around 32, lengths around a
+    warp's keys, more units than SMs: the bits of the packed variable-length path, where a warp has rows of its own."""
+    q, k, v = _inputs(cuda_device, B, Hq, Hkv, Nq, Nk, D, seed=850 + Nq + Nk)
+    out, lse = sageattn3(q, k, v, is_causal=causal, return_lse=True)
+    cq, ck = (torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * n for n in (Nq, Nk))
+    ref, ref_lse = sageattn_varlen(*(x.transpose(1, 2).flatten(0, 1) for x in (q, k, v)), cq, ck, Nq, Nk, is_causal=causal, return_lse=True)
+    assert torch.equal(out.transpose(1, 2).flatten(0, 1), ref) and torch.equal(lse, ref_lse)
 
 
 @pytest.mark.parametrize("Nk", [1, 512, 513, 16384, 16385])
