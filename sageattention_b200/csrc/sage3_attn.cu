@@ -88,7 +88,7 @@ constexpr int kUnitRing = 4;
 // w takes keys 32 w .. 32 w + 31 of the block for all of them: a quarter of the exponentials per warp.  The four exchange their
 // maxima through shared memory; P, its scales and the accumulator are those of rows 0..31.  Same operations per score, and the row
 // sums are added in the same order, so the same bits.  D = 128, 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv heads:
-// 62 -> 44 us (about 980 cycles per block; neither the loads, nor more stages, nor fewer tcgen05 instructions change that).
+// 62 -> 40 us, 780 cycles per block (D = 64: 33 us); the copy warp's and the MMA issuer's instructions bound it now.
 template <int D, int PACK>
 struct Cfg {
     // K and V^T stages, each shared by the two query tiles (as many as fit: PACK, see oP)
@@ -281,7 +281,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (i >= bKE && i < bKE + S) count = PACK == 2 ? 1 : 2;  // K stage free: likewise
         if (i >= bSE && i < bM) count = 4;                       // S buffer free: the four warps of its group hold the scores
         if (i >= bPF && i < bPV) count = 4;                      // P, its scales and the row sums written
-        if (i >= bOS && i < bWF) count = 4;                      // the correction warps are done with O (and have seen P written); bX: maxima exchanged
+        if (i >= bOS && i < bX) count = PACK == 2 ? 1 : 4;       // the correction warps are done with O (and have seen P written)
+        if (i >= bX && i < bWF) count = 4;                       // maxima exchanged
         if (i >= bWE) count = C::kThreads / 32 - 1;              // unit descriptor free: every warp but the producer has finished the unit
         mbar_init(bar(i), count);
         mbar_fence_init();
@@ -387,7 +388,43 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   tc_wait_st();
               }
           }
-          for (int s = 0; s < ns; ++s) {
+          if constexpr (PACK == 2) {
+              // One warp holds all rows: it waits for P alone (the factor was written before), reads all it needs, and keeps the sums in
+              // registers.  (Waiting for the factor and for P with the sums in shared memory took it 1 000 cycles per block.)
+              float2 l = make_float2(0.f, 0.f);
+              float m = -INFINITY;
+              const uint32_t o_addr = tmem + C::cO;
+              for (int s = 0; quarter == 0 && s < ns; ++s) {
+                  const int sg = base + s, slot = sg & 7;
+                  if (!warp_wait(bar(bPF + slot), (sg >> 3) & 1, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
+                  const float2 ma = stat[slot * 128];
+                  // scale and sum of every microblock, two per softmax warp
+                  const float4* mb = reinterpret_cast<const float4*>(sgen + C::oSum) + slot * 128 + lane;
+                  const float4 a = mb[0], b = mb[32], c = mb[64], e = mb[96];
+                  if (s > 0 && __any_sync(0xffffffffu, ma.y != 1.0f)) {
+                      if (!warp_wait(bar(bPV + ((sg - 1) & 7)), ((sg - 1) >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
+                      tc_fence_after();
+#pragma unroll
+                      for (int cc = 0; cc < D / 16; ++cc) {
+                          float o0[16];
+                          tmem_ld16(o_addr + cc * 16, o0);
+                          tc_wait_ld();
+#pragma unroll
+                          for (int q = 0; q < 16; ++q) o0[q] *= ma.y;
+                          tmem_st16(o_addr + cc * 16, o0);
+                      }
+                      tc_wait_st();
+                      tc_fence_before();
+                  }
+                  warp_arrive(bar(bOS + slot), lane);
+                  l.x = fmaf(l.x, ma.y, fmaf(b.z, b.w, fmaf(b.x, b.y, fmaf(a.z, a.w, fmaf(a.x, a.y, 0.f)))));
+                  l.y = fmaf(l.y, ma.y, fmaf(e.z, e.w, fmaf(e.x, e.y, fmaf(c.z, c.w, fmaf(c.x, c.y, 0.f)))));
+                  m = ma.x;
+              }
+              l_s[0] = l;
+              m_s[0] = m;
+          }
+          for (int s = 0; PACK != 2 && s < ns; ++s) {
               const int sg = base + s, slot = sg & 7, ph = (sg >> 3) & 1;
               const int t = (s + d) & two;
               const bool first = s <= two;                            // the tile's first block
@@ -395,7 +432,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const float2 ma = stat[slot * 128];
               const float alpha = ma.y;
               // the first block has nothing to rescale unless the accumulator was carried in
-              if ((PACK != 2 || quarter == 0) && (!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
+              if ((!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
                   // the P V MMA of the tile's previous block must have landed first
                   if (!first) {
                       const int sp = sg - 1 - two;
@@ -419,16 +456,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               tc_fence_before();
               // P V issue waits for this warpgroup only, so its arrival also stands for "P is written"
               if (!warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
-              float2 rs;
-              if constexpr (PACK == 2) {
-                  // scale and sum of every microblock, two per quarter
-                  const float4* mb = reinterpret_cast<const float4*>(sgen + C::oSum) + slot * 128 + lane;
-                  const float4 a = mb[0], b = mb[32], c = mb[64], e = mb[96];
-                  rs.x = fmaf(b.z, b.w, fmaf(b.x, b.y, fmaf(a.z, a.w, fmaf(a.x, a.y, 0.f))));
-                  rs.y = fmaf(e.z, e.w, fmaf(e.x, e.y, fmaf(c.z, c.w, fmaf(c.x, c.y, 0.f))));
-              } else {
-                  rs = sum[slot * 128];
-              }
+              const float2 rs = sum[slot * 128];
               warp_arrive(bar(bOS + slot), lane);
               float2 l = l_s[t * 128];
               l.x = fmaf(l.x, alpha, rs.x);
@@ -507,6 +535,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
     } else if (warp < 4) {
       reg_dealloc<kRoleRegs>();
+      auto load_v = [&](int st, int n, int bhkv) {
+          mbar_expect_tx(bar(bVF + st), C::kVBytes + C::kSfVBytes);
+          tma_load_3d(sbase + C::oV + st * C::kVBytes, &tm_v, bar(bVF + st), n * 64, 0, bhkv);
+          bulk_load(sbase + C::oSfV + st * 1024, p.v_sf + ((size_t)bhkv * p.nkb + n) * C::kSfVBytes, C::kSfVBytes, bar(bVF + st));
+      };
       if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
@@ -575,17 +608,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         bulk_load(sbase + C::oDelta + (st * 2 + t) * C::kDeltaPitch, dptr0 + t * dstep + (size_t)n * kBlock,
                                   C::kDeltaBytes, bar(bKF + st));
                 }
-                if (!warp_wait<true>(bar(bVE + st), st_parity, abort_flag, p.status, kWaitVEmpty)) { ok = false; break; }
-                if (lane == 0) {
-                    mbar_expect_tx(bar(bVF + st), C::kVBytes + C::kSfVBytes);
-                    tma_load_3d(sbase + C::oV + st * C::kVBytes, &tm_v, bar(bVF + st), n * 64, 0, w.bhkv);
-                    bulk_load(sbase + C::oSfV + st * 1024, p.v_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfVBytes,
-                              C::kSfVBytes, bar(bVF + st));
+                if constexpr (PACK != 2) {
+                    if (!warp_wait<true>(bar(bVE + st), st_parity, abort_flag, p.status, kWaitVEmpty)) { ok = false; break; }
+                    if (lane == 0) load_v(st, n, w.bhkv);
                 }
                 __syncwarp();
                 if (++st == S) { st = 0; st_parity ^= 1; }
             }
             u = uniform(next);
+        }
+        __syncwarp();
+      } else if (PACK == 2 && warp == 3) {
+        // ------------------------------------------------------------------ TMA producer of V
+        // The waits and five copies of a block cost one producer 1 100 cycles, more than anything else does per block here (8 192
+        // keys, 64 kv heads: 44 -> 40 us with a warp for K and one for V, D = 64 43 -> 33).
+        int st = 0, st_parity = 1;
+        bool ok = true;
+        const Unit* u;
+        for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
+            const int nbmax = uniform(u->nbmax), bhkv = uniform(u->bhkv);
+            unit_done(i);
+            for (int n = nbmax - 1; n >= 0; --n) {
+                if (!warp_wait<true>(bar(bVE + st), st_parity, abort_flag, p.status, kWaitVEmpty)) { ok = false; break; }
+                if (lane == 0) load_v(st, n, bhkv);
+                __syncwarp();
+                if (++st == S) { st = 0; st_parity ^= 1; }
+            }
         }
         __syncwarp();
       } else if (warp == 1 || warp == 3) {
@@ -615,7 +663,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
             unit_done(i);
-            if (ns == 0 || (PACK == 2 && h == 1)) continue;
+            if (ns == 0) continue;
             const int qb = k & 1;
             if (!warp_wait(bar(bQF + qb), (k >> 1) & 1, abort_flag, p.status, kWaitQFull)) break;
             ++k;
