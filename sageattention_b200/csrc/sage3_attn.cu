@@ -21,7 +21,7 @@
 // nothing else connects the groups: four independent chains per scheduler, a quarter of an item apart.
 // What bounds it: the exp2 unit (16 results per clock and SM: 1 096 cycles per 128 x 128 block with the exponentials of the
 // scales) and, next to it, the instruction latency of the softmax warps; the tensor pipe needs 580 cycles.  Measured (B = 2,
-// H = 32, N = 16 384, 1 965 MHz): 1 532 cycles per block at D = 128 and 1 477 at D = 64, the exp2 unit 77 % busy; the softmax code
+// H = 32, N = 16 384, 1 965 MHz): 1 532 cycles per block at D = 128 and 1 460 at D = 64, the exp2 unit 77 % busy; the softmax code
 // without any wait and without the other warps takes 1 233.  (With a row shared by two threads and all warps of a tile in step,
 // as this kernel was first: 1 662 and 1 611.)  Units in place of one CTA per pair took the
 // drain and refill of the pipeline, 10 us per pair, out: B = 2, H = 32, N = 8 192 causal 960 -> 776 us, B = 4, H = 32, N = 1 024
