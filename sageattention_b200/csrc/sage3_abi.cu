@@ -64,6 +64,10 @@ constexpr size_t kAlign = 1024;     // every workspace region starts at a multip
 constexpr size_t kWsAlign = 256;    // required alignment of the workspace base pointer
 inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
+// Words of the status region: behind the 64 status words the attention kernel's work counter, then one word per (batch, kv head) that
+// the pre-pass sets when a value of its delta_s is not finite.
+constexpr int kStatusWords = 64, kAttnStatusWord = 32, kUnitCounterWord = 64, kNonfiniteWord = 65;
+
 int validate(const Sage3Desc* d) {
     if (!d) return SAGE3_E_NULL;
     if (d->B <= 0 || d->Hq <= 0 || d->Hkv <= 0 || d->Nq <= 0 || d->Nk <= 0) return SAGE3_E_SHAPE;
@@ -95,7 +99,7 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     const size_t kch_q = ((size_t)d->Nq + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t part = B * Hkv * kch_k + (d->per_block_mean ? 0 : B * Hq * kch_q);
     size_t off = 0;
-    w->status = off;  off += align_up(64 * sizeof(int32_t));
+    w->status = off;  off += align_up((kNonfiniteWord + B * Hkv) * sizeof(int32_t));
     w->kpart = off;   off += align_up(part * D * sizeof(float));
     w->km = off;      off += align_up(B * Hkv * D * 2);
     w->qm = off;      off += align_up(B * Hq * nqm * D * 2);
@@ -126,8 +130,6 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 
 // Status words: [0, 32) belong to the pre-pass, [32, 64) to the attention kernel.  Each stage clears its own half only,
 // so a wait the pre-pass gave up on is still there after the attention launch (whose CTAs read it and exit at once).
-// Behind them (the region is 1 024 bytes) lies the attention kernel's work counter, cleared with its half.
-constexpr int kStatusWords = 64, kAttnStatusWord = 32, kUnitCounterWord = 64;
 
 // checks a Sage3Parts argument and converts it; `align`: required alignment of every base pointer
 int to_parts(const Sage3Parts* in, int64_t rows_total, sage3::PartsPtr* out) {
@@ -197,6 +199,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.status = reinterpret_cast<int*>(base + w.status) + kAttnStatusWord;
     a.unit_counter = reinterpret_cast<int*>(base + w.status) + kUnitCounterWord;
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
+    a.nonfinite = reinterpret_cast<const int*>(base + w.status) + kNonfiniteWord;
     a.cu_q = cu_q; a.cu_k = cu_k;
     int drv = 0;
     return sage3::launch_attn(a, st, &drv) == cudaSuccess ? SAGE3_OK : SAGE3_E_CUDA;
@@ -350,7 +353,10 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     a.want_qkm = want_qkm;
     a.clear = a.status;
-    a.n_clear = kUnitCounterWord + 1;
+    // (without carried state, which only the attention call knows about: a word more or less per head costs nothing)
+    const bool shared = sage3::PackRule(desc->Nq, desc->Hq / desc->Hkv, cu_q == nullptr).heads > 1;
+    a.nonfinite = shared ? a.status + kNonfiniteWord : nullptr;
+    a.n_clear = kNonfiniteWord + (shared ? desc->B * desc->Hkv : 0);
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
         cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st) != cudaSuccess)

@@ -70,6 +70,7 @@ struct AttnParams {
     float sm_scale;
     int* status;
     const int* prepass_status;
+    const int* nonfinite;               // PACK: per (batch, kv head), delta_s holds values that are not finite
     // accumulator state carried between calls that walk consecutive key ranges of one attention (nullptr: none)
     const float *carry_o_in, *carry_m_in, *carry_l_in;   // fp32 [B*Hq][Nq][D] unnormalized O; [B*Hq][Nq] running max; [B*Hq][Nq][2] partial row sums
     float *carry_o_out, *carry_m_out, *carry_l_out;
@@ -115,7 +116,8 @@ struct Cfg {
     static constexpr int oSfK = oSfQ + 2 * kQTiles * 1024;
     static constexpr int oSfV = oSfK + kStages * 1024;
     static constexpr int oSfP = oSfV + kStages * 1024;        // [slot] 1024
-    // delta_s per stage: one row per tile, 256 B + 256 B that stay zero; PACK: [16 chunks of 8 keys][8 heads] 16 B + 128 B that stay zero
+    // delta_s per stage: one row per tile, 256 B + 256 B that stay zero; PACK: [16 chunks of 8 keys][8 heads] 16 B, all finite, + 128 B that
+    // stay zero, or the row of one head over the first 256 B
     static constexpr int kDeltaPitch = 512, kDeltaStage = PACK ? 16 * 128 + 128 : 2 * kDeltaPitch;
     static constexpr int oDelta = oSfP + 8 * 1024;            // [stage] kDeltaStage
     static constexpr int oOnes = oDelta + kStages * kDeltaStage;   // 128 x 16 tile: 1.0 in column 0 (PACK: in the column of the row's head), rest 0
@@ -544,14 +546,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
         int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
+        int next = 0, head = 0;                   // the unit after this one (lane 0); PACK: next head of a unit whose heads go one by one
         bool ok = true;
         while (ok) {
-            int next = 0;
-            if (lane == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
+            if (lane == 0 && head == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
             Unit w;
             const bool more = u < p.units;
             if (!more) w.ns = -1;
             else if (!make_unit<CAUSAL, VARLEN, PACK>(p, u, w)) { u = uniform(next); continue; }
+            // Heads that share a tile share the operand that adds delta_s (eight rows of it, the next heads' too), and 0 x NaN is NaN: where
+            // one of the kv heads behind these rows has a delta_s that is not finite, the unit's heads are published one by one.
+            bool last_head = true;
+            if constexpr (PACK) {
+                if (more && w.ns > 0 && w.nb[1] > 1) {
+                    const int kv = min(w.bhq + 7, p.BHq - 1) / (p.Hq / p.Hkv) - w.bhkv;
+                    if (__any_sync(0xffffffffu, lane <= kv && p.nonfinite[w.bhkv + lane] != 0)) {
+                        last_head = head + 1 == w.nb[1];
+                        w.bhq += head;
+                        w.hq += head;
+                        w.nb[1] = 1;
+                    }
+                }
+            }
+            auto advance = [&] {
+                if (last_head) u = uniform(next);
+                head = last_head ? 0 : head + 1;
+            };
             if (!warp_wait<true>(bar(bWE + k % kUnitRing), ((k / kUnitRing) & 1) ^ 1, abort_flag, p.status, kWaitUnit)) break;
             if (lane == 0) {
                 *reinterpret_cast<Unit*>(sgen + C::oUnit + (k % kUnitRing) * 64) = w;
@@ -559,12 +579,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
             ++k;
             if (!more) break;
-            if (w.ns == 0) { u = uniform(next); continue; }
+            if (w.ns == 0) { advance(); continue; }
             const int qb = kq & 1;                // Q buffer
             if (!warp_wait<true>(bar(bQE + qb), ((kq >> 1) & 1) ^ 1, abort_flag, p.status, kWaitKEmpty)) break;
             ++kq;
             const uint16_t* dptr0 = p.delta + ((size_t)w.bhq * p.nqm + ((p.nqm > 1) ? w.mt0 : 0)) * ((size_t)p.nkb * kBlock);
             const size_t dstep = (p.nqm > 1) ? (size_t)p.nkb * kBlock : 0;
+            const bool box = PACK && w.nb[1] > 1;        // (a head on its own brings its delta_s as a plain row, as a tile does)
             if constexpr (PACK) {
                 // one box holds the rows of all heads; the scales move one word (four scales of a row) at a time into the packed row's place
                 const int live = w.nb[1] * p.Nq;
@@ -597,15 +618,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int n = w.nbmax - 1; n >= 0; --n) {
                 if (!warp_wait<true>(bar(bKE + st), st_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
                 if (lane == 0) {
-                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (PACK ? 8 : w.nv) * C::kDeltaBytes);
+                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (box ? 8 : w.nv) * C::kDeltaBytes);
                     tma_load_3d(sbase + C::oK + st * C::kKBytes, &tm_k, bar(bKF + st), 0, n * kBlock, w.bhkv);
                     bulk_load(sbase + C::oSfK + st * 1024, p.k_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfQkBytes,
                               C::kSfQkBytes, bar(bKF + st));
-                    // PACK: [16 chunks of 8 keys][8 heads], the canonical core matrices of an MN-major operand (heads beyond the packed ones
-                    // bring data that meets zeros).  One tensor copy: 64 copies of 16 bytes took 2.9 us per key block.
-                    if constexpr (PACK) tma_load_3d(sbase + C::oDelta + st * C::kDeltaStage, &tm_d, bar(bKF + st), 0, w.bhq, n * (kBlock / 8));
-                    for (int t = 0; !PACK && t < w.nv; ++t)
-                        bulk_load(sbase + C::oDelta + (st * 2 + t) * C::kDeltaPitch, dptr0 + t * dstep + (size_t)n * kBlock,
+                    // box: [16 chunks of 8 keys][8 heads], the canonical core matrices of an MN-major operand (heads beyond the packed ones
+                    // bring finite data that meets zeros).  One tensor copy: 64 copies of 16 bytes took 2.9 us per key block.
+                    if (box) tma_load_3d(sbase + C::oDelta + st * C::kDeltaStage, &tm_d, bar(bKF + st), 0, w.bhq, n * (kBlock / 8));
+                    for (int t = 0; !box && t < w.nv; ++t)
+                        bulk_load(sbase + C::oDelta + st * C::kDeltaStage + t * C::kDeltaPitch, dptr0 + t * dstep + (size_t)n * kBlock,
                                   C::kDeltaBytes, bar(bKF + st));
                 }
                 if constexpr (PACK != 2) {
@@ -615,7 +636,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 __syncwarp();
                 if (++st == S) { st = 0; st_parity ^= 1; }
             }
-            u = uniform(next);
+            advance();
         }
         __syncwarp();
       } else if (PACK == 2 && warp == 3) {
@@ -648,9 +669,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         constexpr uint32_t idesc_qk = make_idesc_nvfp4(kKeys);
         constexpr uint32_t idesc_delta = make_idesc_f16_bmn(kKeys, std::is_same<OutT, __nv_bfloat16>::value);
         // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
-        constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone), hi_delta = sdesc_hi(PACK ? 128 : 16, kSwzNone);
+        constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone);
         const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo0 = sdesc_lo(sbase + C::oQ, 16), sfq_lo0 = sdesc_lo(sbase + C::oSfQ, 0);
-        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_lo0 = sdesc_lo(sbase + C::oDelta + h * (PACK ? 1024 : 128), PACK ? 128 : 16);
+        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16);
         const uint32_t sfk_lo0 = sdesc_lo(sbase + C::oSfK, 0);
         // each issuer has its own copies of the scale factors in tensor memory, so that its MMAs and copies stay in one order
         const uint32_t sfk_col = tmem + C::cSfK + 8 * h;        // the 128-key atoms; keys 64 .. 127 start two columns in
@@ -662,6 +683,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const Unit* u;
         for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
+            const int chunk = PACK && uniform(u->nb[1]) > 1 ? 128 : 16;           // bytes from 8 keys of delta_s to the next 8
+            const uint32_t delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 8 * chunk, chunk), hi_delta = sdesc_hi(chunk, kSwzNone);
             unit_done(i);
             if (ns == 0) continue;
             const int qb = k & 1;
@@ -690,7 +713,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         for (int ks = 0; ks < D / 64; ++ks) tc_cp_sf(sfk_col + 4 * ks, sdesc(sfk_lo + ks * 32, sdesc_hi(128, kSwzNone)));
                     }
                     // S <- 1 (x) delta_s: A = [128 x 16] with ones in column 0 (K-major), B = 64 elements of the delta_s row read as an
-                    // MN-major [16 x 64] operand whose rows 1..15 alias finite data and meet zeros in A (PACK: rows 0..7 are the heads')
+                    // MN-major [16 x 64] operand whose rows 1..15 alias later keys of the row or finite data and meet zeros in A (PACK, several
+                    // heads: rows 0..7 are the heads', all finite)
                     tc_mma_f16(s_col, sdesc(ones_lo, hi_ones), sdesc(delta_lo, hi_delta), idesc_delta, false);
 #pragma unroll
                     for (int ks = 0; ks < D / 64; ++ks)
@@ -1077,17 +1101,9 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     CUtensorMap tq, tk, tv, td;
     const uint32_t rowb = a.D / 2;
     const CUtensorMapSwizzle swz_qk = (a.D == 128) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-    // Few query rows and several heads per kv head (token generation): as many heads as fit share a tile, eight at
-    // most (the operand that adds delta_s has eight rows), without carried state.  Mode 2, where a warp takes a quarter of the keys
-    // for all rows, when the rows of these heads (of one head, too) fit one warp: it would need more tiles otherwise.
     const int group = a.Hq / a.Hkv;
-    const bool plain = a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr;
-    int pack = 1;
-    if (plain && a.Nq <= kBlock / 2) {
-        pack = kBlock / a.Nq < group ? kBlock / a.Nq : group;
-        if (pack > 8) pack = 8;
-    }
-    const int mode = plain && a.Nq * (group < 8 ? group : 8) <= 32 ? 2 : pack > 1 ? 1 : 0;
+    const PackRule rule(a.Nq, group, a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr);
+    const int pack = rule.heads, mode = rule.mode;
     CUresult r = make_map(fn, &tq, a.q_codes, rowb, a.Nq_p, (uint64_t)a.B * a.Hq, rowb, mode ? a.Nq : kBlock, swz_qk, pack);
     if (r == CUDA_SUCCESS) r = make_map(fn, &tk, a.k_codes, rowb, a.Nk_p, (uint64_t)a.B * a.Hkv, rowb, kBlock, swz_qk);
     if (r == CUDA_SUCCESS)
@@ -1135,6 +1151,7 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.os0 = a.os[0]; p.os1 = a.os[1]; p.os2 = a.os[2];
     p.status = a.status;
     p.prepass_status = a.prepass_status;
+    p.nonfinite = a.nonfinite;
     p.carry_o_in = a.carry_o_in; p.carry_m_in = a.carry_m_in; p.carry_l_in = a.carry_l_in;
     p.carry_o_out = a.carry_o_out; p.carry_m_out = a.carry_m_out; p.carry_l_out = a.carry_l_out;
     p.causal_shift = a.causal_shift;

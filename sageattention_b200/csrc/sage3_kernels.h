@@ -30,8 +30,9 @@ struct PrepassArgs {
     float* qkm;                    // fp32 [B][Hq][Nq_p]: q . km per query row
     int* status;                   // device status words (bounded waits report here)
     int want_qkm;                  // q . km per query row is wanted (the LSE output needs it)
-    int* clear;                    // words the first kernel zeroes: all status words and the attention kernel's work counter
+    int* clear;                    // words the first kernel zeroes: status words, the attention kernel's work counter, `nonfinite`
     int n_clear;
+    int* nonfinite;                // per (batch, kv head): set when a delta_s value is not finite; nullptr: nobody asks (see PackRule)
     // packed variable-length sequences (both nullptr: every batch entry has Nq / Nk tokens): device int32 [B + 1], entry b
     // owns rows cu[b] .. cu[b + 1] of the packed tensor; Nq / Nk are then the maximum lengths, stride 0 is unused
     const int *cu_q, *cu_k;
@@ -55,7 +56,21 @@ struct AttnArgs {
     float *carry_o_out, *carry_m_out, *carry_l_out;
     int causal_shift;               // key j visible to query i iff j <= i + causal_shift (Nk - Nq unless the caller offsets it)
     const int* prepass_status;      // the pre-pass's status word (non-zero: the workspace is incomplete, do nothing)
+    const int* nonfinite;           // per (batch, kv head), from the pre-pass: delta_s holds values that are not finite
     const int *cu_q, *cu_k;         // packed variable-length sequences, as in PrepassArgs (nullptr: uniform lengths)
+};
+
+// Few query rows and several heads per kv head (token generation): as many heads as fit share a 128-row tile, eight at most (the
+// operand that adds delta_s has eight rows); uniform lengths and no carried state only (`plain`).  Mode 2, where a warp takes a
+// quarter of the keys for all rows, when the rows of these heads (of one head, too) fit one warp: it would need more tiles otherwise.
+struct PackRule {
+    int heads = 1, mode = 0;       // query heads per tile; kernel: 0 pairs of tiles, 1 packed, 2 packed with at most 32 rows
+    PackRule(int Nq, int group, bool plain) {
+        if (!plain) return;
+        const int most = group < 8 ? group : 8;
+        if (Nq <= 64) heads = 128 / Nq < most ? 128 / Nq : most;
+        mode = Nq * most <= 32 ? 2 : heads > 1 ? 1 : 0;
+    }
 };
 
 // Device the calling thread has current, its SM count and whether it is compute capability 10.0 (looked up once per device).

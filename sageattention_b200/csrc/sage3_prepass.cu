@@ -64,6 +64,10 @@ template <> struct Num<__nv_bfloat16> {
         const __nv_bfloat162 r = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&m), __habs2(*reinterpret_cast<const __nv_bfloat162*>(&a)));
         return *reinterpret_cast<const uint32_t*>(&r);
     }
+    static __device__ __forceinline__ uint32_t zero_fma2(uint32_t a, uint32_t z) {   // 0 a + z: stays 0 while every a is finite, then NaN
+        const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&a), __floats2bfloat162_rn(0.f, 0.f), *reinterpret_cast<const __nv_bfloat162*>(&z));
+        return *reinterpret_cast<const uint32_t*>(&r);
+    }
 };
 template <> struct Num<__half> {
     using T2 = __half2;
@@ -87,6 +91,10 @@ template <> struct Num<__half> {
     }
     static __device__ __forceinline__ uint32_t absmax2(uint32_t m, uint32_t a) {
         const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&m), __habs2(*reinterpret_cast<const __half2*>(&a)));
+        return *reinterpret_cast<const uint32_t*>(&r);
+    }
+    static __device__ __forceinline__ uint32_t zero_fma2(uint32_t a, uint32_t z) {
+        const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&a), __floats2half2_rn(0.f, 0.f), *reinterpret_cast<const __half2*>(&z));
         return *reinterpret_cast<const uint32_t*>(&r);
     }
 };
@@ -470,6 +478,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     uint8_t* __restrict__ sfs,         // [B*H][Np/128][D/64][512]
     int rows,                          // query blocks of all query heads of a kv head
     int* __restrict__ status,
+    int* __restrict__ nonfinite,       // [B*H]: set when a delta_s value is not finite; nullptr: not wanted
     const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 (FEW: 64) rows x 128 bytes, 128-byte swizzle
     const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*H][rows][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
     constexpr int CH = D / 16;            // microblocks per row
@@ -615,7 +624,8 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
         if (m0 + quarter * 32 < rows) {
             const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + chalf * 64;
             const int stg_off = oStg + (chalf * (kARows / 32) + quarter) * 4096;
-                uint8_t* stg = sgen + stg_off;
+            uint8_t* stg = sgen + stg_off;
+            uint32_t z = 0;
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 float v[32];
@@ -628,8 +638,13 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
                     for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
                     *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
                         make_uint4(p4[0], p4[1], p4[2], p4[3]);
+                    if (nonfinite != nullptr) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) z = Num<T>::zero_fma2(p4[e], z);
+                    }
                 }
             }
+            if (nonfinite != nullptr && (z & 0x7fff7fffu) != 0 && m0 + quarter * 32 + lane < rows) nonfinite[bh] = 1;
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -752,7 +767,7 @@ struct StageArgs {
     uint8_t *q_codes, *q_sf, *v_codes, *v_sf;
     float* qkm;                        // nullptr: not wanted
     MeanParts means;
-    int* clear;                        // status words and work counter to zero (nullptr: not in this launch)
+    int* clear;                        // words to zero: status, work counter, `nonfinite` (nullptr: not in this launch)
     int n_clear;
 };
 
@@ -771,7 +786,8 @@ __global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(con
     extern __shared__ __align__(16) uint8_t smem_raw[];
     pdl_launch_dependents();
     int i = blockIdx.x;
-    if (a.clear != nullptr && i == 0 && threadIdx.x < a.n_clear) a.clear[threadIdx.x] = 0;
+    if (a.clear != nullptr && i == 0)
+        for (int j = threadIdx.x; j < a.n_clear; j += 256) a.clear[j] = 0;
     int tile, bh;
     if (i < a.n_colk) {
         bh = a.chunks_k.divmod(i, tile);
@@ -874,7 +890,8 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     auto kern = few ? quant_k_delta_kernel<T, D, true> : quant_k_delta_kernel<T, D, false>;
     if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
     return launch_pdl(kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
-                      a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status, tm_qm, tm_delta);
+                      a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status,
+                      a.nonfinite, tm_qm, tm_delta);
 }
 
 cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t st) {

@@ -156,3 +156,31 @@ def test_scale_of_every_microblock_maximum(cuda_device, dtype):
     ws, ref = read_workspace(prob), O.prepass(q, k, v)
     assert torch.equal(ws["vt_sf"], ref.vt_sf)
     assert torch.equal(canon(ws["vt_codes"]), canon(ref.vt_codes))
+
+
+@pytest.mark.parametrize("what", ["k_nan", "q_inf", "delta_overflow"])
+@pytest.mark.parametrize("Nq,Hq,Hkv,D", [(1, 32, 8, 128), (1, 4, 4, 64), (9, 14, 2, 128), (40, 6, 2, 64), (4, 18, 2, 128), (2, 32, 4, 64)])
+def test_non_finite_values_stay_with_their_head(cuda_device, Nq, Hq, Hkv, D, what):
+    """Heads that share a tile share the operand that adds delta_s, where 0 x NaN and 0 x Inf are NaN.  One query head, or one kv
+    head, of sequence 1 is not finite (a NaN key, an Inf query, an fp16 delta_s that overflows): sequence 0 and the other heads
+    get the bits of a call without it, and the head itself what the packed variable-length path, one head per tile, gives it."""
+    dtype = torch.float16 if what == "delta_overflow" else torch.bfloat16
+    Nk, B, g = 400, 2, Hq // Hkv
+    q, k, v = _inputs(cuda_device, B, Hq, Hkv, Nq, Nk, D, seed=1300 + Nq + Hq, dtype=dtype)
+    good = sageattn3(q, k, v, return_lse=True)
+    if what == "k_nan":
+        k[1, 0, 5, 3] = float("nan")
+    elif what == "q_inf":
+        q[1, min(1, g - 1), 0, 3] = float("inf")
+    else:
+        q[1, min(1, g - 1)] = 6.0e4
+        k[1, 0, 5] = 200.0
+    out, lse = sageattn3(q, k, v, return_lse=True)
+    cq, ck = (torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * n for n in (Nq, Nk))
+    ref, ref_lse = sageattn_varlen(*(x.transpose(1, 2).flatten(0, 1) for x in (q, k, v)), cq, ck, Nq, Nk, return_lse=True)
+    assert not torch.isfinite(ref_lse).all() or (ref == 0).all(-1).any()          # the values do reach that head
+    healthy = torch.ones(B, Hq, dtype=torch.bool, device=cuda_device)
+    healthy[1, :g] = False                                                        # (in the third case their K differs)
+    assert torch.equal(out[healthy], good[0][healthy]) and torch.equal(lse[healthy], good[1][healthy])
+    assert torch.equal(out.transpose(1, 2).flatten(0, 1).nan_to_num(7.0), ref.nan_to_num(7.0))
+    assert torch.equal(lse.nan_to_num(7.0), ref_lse.nan_to_num(7.0))
