@@ -225,7 +225,8 @@ SAGE3_API int sage3_shared_open(const unsigned char handle[64], void** ptr);
 SAGE3_API int sage3_shared_close(void* ptr);
 SAGE3_API int sage3_shared_free(void* ptr);
 
-/* sage3_prepass followed by sage3_attn_fwd on the same stream. */
+/* sage3_prepass followed by sage3_attn_fwd on the same stream.  Calls of several threads with one workspace and one stream are
+ * enqueued one after the other (this and sage3_fwd_varlen; the single stages are the caller's to order). */
 SAGE3_API int sage3_fwd(const Sage3Desc* desc, const void* q, const void* k, const void* v, void* ws, void* out,
               float* lse, void* stream);
 

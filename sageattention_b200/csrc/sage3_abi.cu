@@ -131,6 +131,15 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 // Status words: [0, 32) belong to the pre-pass, [32, 64) to the attention kernel.  Each stage clears its own half only,
 // so a wait the pre-pass gave up on is still there after the attention launch (whose CTAs read it and exit at once).
 
+// Held while a whole call (pre-pass and attention) is enqueued: its launches hand their results on through the workspace, so the calls
+// of several threads on one workspace and stream may follow one another but not interleave.  One of a few locks by address: threads
+// with workspaces of their own seldom meet, and then for microseconds.
+std::mutex& enqueue_mutex(const void* ws) {
+    static std::mutex mutexes[16];
+    const uintptr_t a = reinterpret_cast<uintptr_t>(ws) >> 8;      // (256-byte aligned; blocks of an allocator differ in some bits above 9)
+    return mutexes[(a ^ (a >> 4) ^ (a >> 13) ^ (a >> 21)) & 15];
+}
+
 // checks a Sage3Parts argument and converts it; `align`: required alignment of every base pointer
 int to_parts(const Sage3Parts* in, int64_t rows_total, sage3::PartsPtr* out) {
     if (!in) return SAGE3_E_NULL;
@@ -377,6 +386,7 @@ SAGE3_API int sage3_fwd_varlen(const Sage3Desc* desc, const int32_t* cu_seqlens_
                                const void* k, const void* v, void* out, float* lse, void* ws, void* stream) {
     if (!desc || !cu_seqlens_q || !cu_seqlens_k || !q || !k || !v || !out) return SAGE3_E_NULL;
     if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16) || !aligned(cu_seqlens_q, 4) || !aligned(cu_seqlens_k, 4)) return SAGE3_E_ALIGN;
+    std::lock_guard<std::mutex> lock(enqueue_mutex(ws));
     const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, lse != nullptr, cu_seqlens_q, cu_seqlens_k);
     if (rc != SAGE3_OK) return rc;
     return attn_impl(desc, ws, one_part(out), lse, stream, true, nullptr, cu_seqlens_q, cu_seqlens_k);
@@ -453,6 +463,7 @@ SAGE3_API int sage3_fwd(const Sage3Desc* desc, const void* q, const void* k, con
               void* stream) {
     if (!q || !k || !v) return SAGE3_E_NULL;
     if (!aligned(q, 16) || !aligned(k, 16) || !aligned(v, 16)) return SAGE3_E_ALIGN;
+    std::lock_guard<std::mutex> lock(enqueue_mutex(ws));
     const int rc = prepass_impl(desc, one_part(q), one_part(k), one_part(v), nullptr, ws, stream, lse != nullptr);
     if (rc != SAGE3_OK) return rc;
     return attn_impl(desc, ws, one_part(out), lse, stream, true);

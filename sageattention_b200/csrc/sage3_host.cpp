@@ -27,8 +27,9 @@ VarlenFn g_varlen = nullptr;
 BytesFn g_bytes = nullptr;
 
 // One workspace per (device, stream), grown on demand and reused by later calls: kernels of successive calls on one stream
-// run in order, so they may share it; calls on different streams get different buffers.  (Allocating 3.4 GB anew on every
-// call of the 4 x 32 x 32 768 shape costs more than the pre-pass.)
+// run in order, so they may share it (sage3_fwd and sage3_fwd_varlen enqueue a call as a whole, also when several threads use the
+// stream; a buffer that was replaced meanwhile lives as long as the call that holds it); calls on different streams get different
+// buffers.  (Allocating 3.4 GB anew on every call of the 4 x 32 x 32 768 shape costs more than the pre-pass.)
 std::mutex g_mutex;
 std::map<std::pair<int, cudaStream_t>, at::Tensor>* g_workspaces = nullptr;      // never destroyed: the CUDA context may go first
 

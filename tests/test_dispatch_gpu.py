@@ -184,3 +184,32 @@ def test_non_finite_values_stay_with_their_head(cuda_device, Nq, Hq, Hkv, D, wha
     assert torch.equal(out[healthy], good[0][healthy]) and torch.equal(lse[healthy], good[1][healthy])
     assert torch.equal(out.transpose(1, 2).flatten(0, 1).nan_to_num(7.0), ref.nan_to_num(7.0))
     assert torch.equal(lse.nan_to_num(7.0), ref_lse.nan_to_num(7.0))
+
+
+def test_threads_on_one_stream_share_a_workspace(cuda_device):
+    """Several threads, all on the default stream and so on one workspace, through the host extension, the Python path (a scale per
+    head) and the packed entry; more units than SMs, so that a work counter another call has used up would leave rows unwritten."""
+    import threading
+    N, H = 260, 160
+    cu = torch.tensor([0, N], dtype=torch.int32, device=cuda_device)
+    per_head = torch.full((H,), 0.2, device=cuda_device)
+
+    def call(i, q, k, v):
+        if i == 2:
+            return sageattn_varlen(*(x[0].transpose(0, 1) for x in (q, k, v)), cu, cu, N, N, sm_scale=0.2).transpose(0, 1)[None]
+        return sageattn3(q, k, v, sm_scale=per_head if i == 1 else 0.2)
+    inputs = [_inputs(cuda_device, 1, H, H, N, N, 64, seed=1600 + i) for i in range(3)]
+    refs = [call(i, *x) for i, x in enumerate(inputs)]
+    torch.cuda.synchronize()
+    outs, start = [[] for _ in inputs], threading.Barrier(len(inputs))
+
+    def work(i):
+        start.wait()
+        for _ in range(30):
+            outs[i].append(call(i, *inputs[i]))
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(inputs))]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    torch.cuda.synchronize()
+    for i, ref in enumerate(refs):
+        assert len(outs[i]) == 30 and all(torch.equal(o, ref) for o in outs[i])

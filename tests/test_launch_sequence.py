@@ -1,0 +1,80 @@
+"""CPU tests of what the library's host code enqueues: its own object files, linked with a CUDA runtime that records the launches
+instead of making them (tests/fake_cudart.cpp)."""
+import ctypes as C
+import os
+import pathlib
+import subprocess
+import threading
+
+import pytest
+
+from sageattention_b200 import _cabi, build
+
+WS = 1 << 20              # "device" addresses: never dereferenced by host code
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    objs = [build.PKG / "build" / (s + ".o") for s in build.SOURCES]
+    srcs = [build.CSRC / s for s in build.SOURCES + build.HEADERS]
+    tmp = tmp_path_factory.mktemp("fake")
+    if not all(o.exists() for o in objs) or max(s.stat().st_mtime for s in srcs) > min(o.stat().st_mtime for o in objs):
+        objs = [tmp / (s + ".o") for s in build.SOURCES]
+        procs = [subprocess.Popen(["nvcc", *build.NVCC_FLAGS, "-c", str(build.CSRC / s), "-o", str(o)]) for s, o in zip(build.SOURCES, objs)]
+        assert [p.wait() for p in procs] == [0] * len(procs)
+    so = tmp / "libsage3_fake.so"
+    cuda = pathlib.Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", f"-isystem{cuda / 'include'}",
+                           str(pathlib.Path(__file__).with_name("fake_cudart.cpp")), *map(str, objs), "-o", str(so), "-lpthread"])
+    lib = C.CDLL(str(so))
+    lib.fake_log.restype = C.c_char_p
+    return lib
+
+
+def _desc(**kw):
+    d = _cabi.Sage3Desc()
+    base = dict(B=1, Hq=4, Hkv=2, Nq=300, Nk=700, D=64, dtype=_cabi.SAGE3_BF16, is_causal=0, per_block_mean=1)
+    base.update(kw)
+    for k, v in base.items():
+        setattr(d, k, v)
+    n = max(base["Nq"], base["Nk"])
+    for name in ("q_stride", "k_stride", "v_stride", "o_stride"):
+        setattr(d, name, (C.c_int64 * 3)(base["Hq"] * n * base["D"], n * base["D"], base["D"]))
+    return d
+
+
+def _fwd(lib, d, ws=WS, lse=None):
+    p = C.c_void_p
+    return lib.sage3_fwd(C.byref(d), p(1 << 12), p(1 << 13), p(1 << 14), p(ws), p(1 << 15), p(lse), None)
+
+
+def _varlen(lib, d, ws=WS, lse=None):
+    p = C.c_void_p
+    return lib.sage3_fwd_varlen(C.byref(d), p(1 << 10), p(1 << 11), p(1 << 12), p(1 << 13), p(1 << 14), p(1 << 15), p(lse), p(ws), None)
+
+
+def _log(lib):
+    return [line.split(":") for line in lib.fake_log().decode().splitlines()]
+
+
+@pytest.mark.parametrize("call", [_fwd, _varlen])
+@pytest.mark.parametrize("kw,lse", [({}, None), (dict(per_block_mean=0, Nk=20000), 1 << 16)])
+def test_calls_of_two_threads_on_one_workspace_do_not_interleave(fake, call, kw, lse):
+    """The kernels of a call hand their results on through the workspace: another call that uses it may come before or after all
+    of them only.  (Every launch pauses, so that threads that may interleave do.)"""
+    fake.fake_start(-1, 2000)
+    start, rcs = threading.Barrier(3), []
+
+    def work():
+        start.wait()
+        for _ in range(3):
+            rcs.append(call(fake, _desc(**kw), lse=lse))
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    log = _log(fake)
+    assert rcs == [0] * 9 and len(log) % 9 == 0
+    per_call = len(log) // 9
+    assert per_call >= 3
+    for i in range(0, len(log), per_call):
+        assert len({entry[0] for entry in log[i:i + per_call]}) == 1, log[i:i + per_call]
