@@ -48,7 +48,7 @@ cudaError_t allow_smem(const void* kernel, int bytes) {
             break;
         }
     if (slot && dev < kMaxDevices && (slot->devices >> dev & 1)) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    e = checked(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     if (e == cudaSuccess && slot && dev < kMaxDevices) {
         slot->kernel = kernel;
         slot->devices |= 1ull << dev;
@@ -83,8 +83,12 @@ int validate(const Sage3Desc* d) {
     const int64_t nqp = ((int64_t)d->Nq + 127) / 128 * 128, nkp = ((int64_t)d->Nk + 127) / 128 * 128;
     if (nqp > (1 << 24) || nkp > (1 << 24)) return SAGE3_E_TOO_LARGE;
     if ((int64_t)d->B * d->Hq * (nqp / 128) > 0x7fffffffLL) return SAGE3_E_TOO_LARGE;
-    // the pre-pass kernels put the (batch, head) index in gridDim.y
+    // a pre-pass kernel puts the (batch, kv head) index in gridDim.y
     if ((int64_t)d->B * d->Hq > 65535) return SAGE3_E_TOO_LARGE;
+    // the pieces of the first pre-pass kernel (at most: chunks of K and Q, tiles of Q and V) are the blocks of one grid
+    const int64_t chunks_k = ((int64_t)d->Nk + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
+    const int64_t chunks_q = d->per_block_mean ? 0 : ((int64_t)d->Nq + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
+    if ((int64_t)d->B * d->Hkv * (chunks_k + nkp / 128) + (int64_t)d->B * d->Hq * (chunks_q + nqp / 128) > 0x7fffffffLL) return SAGE3_E_TOO_LARGE;
     return SAGE3_OK;
 }
 
@@ -184,8 +188,8 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     if (rc != SAGE3_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* base = static_cast<uint8_t*>(ws);
-    if (!cleared && cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0, (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st) !=
-        cudaSuccess)
+    if (!cleared && sage3::checked(cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0,
+                                                   (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st)) != cudaSuccess)
         return SAGE3_E_CUDA;
     sage3::AttnArgs a;
     a.B = desc->B; a.Hq = desc->Hq; a.Hkv = desc->Hkv; a.Nq = desc->Nq; a.Nk = desc->Nk; a.D = desc->D;
@@ -368,7 +372,7 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     a.n_clear = kNonfiniteWord + (shared ? desc->B * desc->Hkv : 0);
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
-        cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        sage3::checked(cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
         return SAGE3_E_CUDA;
     return sage3::launch_prepass(a, st) == cudaSuccess ? SAGE3_OK : SAGE3_E_CUDA;
 }

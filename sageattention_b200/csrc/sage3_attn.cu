@@ -1081,7 +1081,7 @@ static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUte
     using C = Cfg<D, PACK>;
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), C::kSmemBytes);
     if (e != cudaSuccess) return e;
-    return launch_pdl(kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, p);
+    return launch(true, kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, p);
 }
 
 template <int D, bool CAUSAL, typename OutT>

@@ -80,9 +80,16 @@ cudaError_t current_device(int* dev, DeviceInfo* info);
 // Dynamic shared memory of a kernel beyond 48 KB (set once per kernel and device).
 cudaError_t allow_smem(const void* kernel, int bytes);
 
-// Launch that may begin (up to its griddepcontrol.wait) while the kernel before it in the stream is still running.
+// Result of a runtime call, an error taken off the thread's record: the caller gets it as a return code, and whoever asks the runtime
+// next must not find it.
+inline cudaError_t checked(cudaError_t e) {
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
+// Launch, with its result.  `early`: it may begin (up to its griddepcontrol.wait) while the kernel before it in the stream is still running.
 template <typename... P, typename... A>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -92,8 +99,8 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    cfg.numAttrs = early ? 1 : 0;
+    return checked(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
 // Encodes a tensor map over a byte tensor [n2][n1][n0] (n0 contiguous) with box [1][b1][b0]; swizzle: 0 none, 1 32 B, 2 64 B,

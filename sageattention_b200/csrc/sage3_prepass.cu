@@ -858,11 +858,15 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     s.n_colq = a.per_block_mean ? 0 : a.kchunks_q * BHq;
     s.n_q = q_late ? 0 : tiles_q * BHq;
     s.n_v = tiles_k * BHkv;
-    prepass_stage_kernel<T, D><<<s.n_colk + s.n_colq + s.n_q + s.n_v, 256, StageCfg<T, D>::kSmem, st>>>(s);
-    if (km_here && !km_inline)
-        colmean_finalize_kernel<T, D><<<BHkv, D, 0, st>>>(s.part_k, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0);
-    if (!a.per_block_mean && !qm_inline)
-        colmean_finalize_kernel<T, D><<<BHq, D, 0, st>>>(s.part_q, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1);
+    // Every launch is checked: the ones behind a failed one would work on what an earlier call left (the work counter among it).
+    if ((e = launch(false, prepass_stage_kernel<T, D>, dim3(s.n_colk + s.n_colq + s.n_q + s.n_v), dim3(256), (size_t)StageCfg<T, D>::kSmem, st, s)) != cudaSuccess)
+        return e;
+    if (km_here && !km_inline &&
+        (e = launch(false, colmean_finalize_kernel<T, D>, dim3(BHkv), dim3(D), 0, st, (const float*)s.part_k, a.kchunks_k, 1.0f / (float)a.Nk, km, a.cu_k, a.Hkv, 0)) != cudaSuccess)
+        return e;
+    if (!a.per_block_mean && !qm_inline &&
+        (e = launch(false, colmean_finalize_kernel<T, D>, dim3(BHq), dim3(D), 0, st, (const float*)s.part_q, a.kchunks_q, 1.0f / (float)a.Nq_p, qm, a.cu_q, a.Hq, 1)) != cudaSuccess)
+        return e;
     if (q_late) {
         s.n_colk = s.n_colq = s.n_v = 0;
         s.n_q = tiles_q * BHq;
@@ -875,7 +879,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         s.means.Nk = a.Nk;
         s.means.cu_k = a.cu_k;
         s.means.wait = true;
-        if ((e = launch_pdl(prepass_stage_kernel<T, D>, dim3(s.n_q), dim3(256), (size_t)StageCfg<T, D>::kSmem, st, s)) != cudaSuccess) return e;
+        if ((e = launch(true, prepass_stage_kernel<T, D>, dim3(s.n_q), dim3(256), (size_t)StageCfg<T, D>::kSmem, st, s)) != cudaSuccess) return e;
     }
     // tensor maps for the K kernel: the Q means and delta_s of a kv head's query heads follow one another, so both are byte
     // tensors [B*Hkv][group * nqm][...] and one MMA takes the blocks of several heads
@@ -889,7 +893,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         return cudaErrorInvalidValue;
     auto kern = few ? quant_k_delta_kernel<T, D, true> : quant_k_delta_kernel<T, D, false>;
     if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
-    return launch_pdl(kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
+    return launch(true, kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
                       a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status,
                       a.nonfinite, tm_qm, tm_delta);
 }
@@ -937,10 +941,11 @@ cudaError_t launch_kmean_t(const Sage3Desc* d, const void* k, void* km, float* s
     const int BH = d->B * d->Hkv;
     sage3::PartsPtr one = {};
     one.base[0] = const_cast<void*>(k);
-    sage3::colsum_partial_kernel<T, D><<<dim3(chunks, BH), 256, 0, st>>>(
-        sage3::make_src<T>(one), d->k_stride[0], d->k_stride[1], d->k_stride[2], sage3::FastDiv(d->Hkv), d->Nk, scratch, chunks);
-    sage3::colmean_finalize_kernel<T, D><<<BH, D, 0, st>>>(scratch, chunks, 1.0f / (float)d->Nk, static_cast<T*>(km), nullptr, d->Hkv, 0);
-    return cudaGetLastError();
+    const cudaError_t e = sage3::launch(false, sage3::colsum_partial_kernel<T, D>, dim3(chunks, BH), dim3(256), 0, st, sage3::make_src<T>(one),
+                                        d->k_stride[0], d->k_stride[1], d->k_stride[2], sage3::FastDiv(d->Hkv), d->Nk, scratch, chunks);
+    if (e != cudaSuccess) return e;
+    return sage3::launch(false, sage3::colmean_finalize_kernel<T, D>, dim3(BH), dim3(D), 0, st, (const float*)scratch, chunks,
+                         1.0f / (float)d->Nk, static_cast<T*>(km), (const int*)nullptr, d->Hkv, 0);
 }
 
 }  // namespace

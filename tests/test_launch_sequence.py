@@ -78,3 +78,31 @@ def test_calls_of_two_threads_on_one_workspace_do_not_interleave(fake, call, kw,
     assert per_call >= 3
     for i in range(0, len(log), per_call):
         assert len({entry[0] for entry in log[i:i + per_call]}) == 1, log[i:i + per_call]
+
+
+CALLS = [(_fwd, {}, None), (_fwd, {}, 1 << 16), (_fwd, dict(Nk=20000), None), (_fwd, dict(Nk=20000, Nq=20000, per_block_mean=0), None),
+         (_varlen, dict(per_block_mean=0, Nk=20000), 1 << 16)]
+
+
+@pytest.mark.parametrize("call,kw,lse", CALLS)
+def test_a_refused_launch_is_reported_and_ends_the_call(fake, call, kw, lse):
+    """Whichever launch of a call the runtime refuses: the call returns SAGE3_E_CUDA, enqueues nothing after it (the kernels behind
+    it would work on what an earlier call left), and leaves no error behind for whoever asks the runtime next."""
+    fake.fake_start(-1, 0)
+    assert call(fake, _desc(**kw), lse=lse) == 0
+    n = len(_log(fake))
+    for i in range(n):
+        fake.fake_start(i, 0)
+        assert call(fake, _desc(**kw), lse=lse) == -7, i
+        log = _log(fake)
+        assert len(log) == i + 1 and log[-1][-1] == "refused", log
+        assert fake.fake_last_error() == 0, i
+
+
+def test_a_launch_of_too_many_blocks_is_refused():
+    """All pieces of the first pre-pass kernel are one grid: their number, not that of one kind, has to stay below 2^31."""
+    d = _desc(B=60000, Hq=1, Hkv=1, Nq=128, Nk=6000000)       # 2.8e9 tiles of V
+    assert _cabi.lib().sage3_workspace_bytes(C.byref(d)) == 0
+    assert _cabi.lib().sage3_workspace_layout(C.byref(d), C.byref(_cabi.Sage3Workspace())) == -8
+    d = _desc(B=60000, Hq=1, Hkv=1, Nq=128, Nk=3000000)
+    assert _cabi.lib().sage3_workspace_bytes(C.byref(d)) > 0
