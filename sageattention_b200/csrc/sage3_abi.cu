@@ -66,7 +66,7 @@ inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 // Words of the status region: behind the 64 status words the attention kernel's work counter, then one word per (batch, kv head) that
 // the pre-pass sets when a value of its delta_s is not finite.
-constexpr int kStatusWords = 64, kAttnStatusWord = 32, kUnitCounterWord = 64, kNonfiniteWord = 65;
+constexpr int kAttnStatusWord = 32, kUnitCounterWord = 64, kNonfiniteWord = 65;
 
 int validate(const Sage3Desc* d) {
     if (!d) return SAGE3_E_NULL;

@@ -671,7 +671,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // descriptors: constant high words, low words that move with the stage, tile and key half (bytes / 16)
         constexpr uint32_t hi_qk = sdesc_hi(C::kSboQK, C::kSwzQK), hi_ones = sdesc_hi(128, kSwzNone);
         const uint32_t ones_lo = sdesc_lo(sbase + C::oOnes, 2048), q_lo0 = sdesc_lo(sbase + C::oQ, 16), sfq_lo0 = sdesc_lo(sbase + C::oSfQ, 0);
-        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16);
+        const uint32_t k_lo0 = sdesc_lo(sbase + C::oK + h * (64 * D / 2), 16), delta_row_lo = sdesc_lo(sbase + C::oDelta + h * 128, 16);
         const uint32_t sfk_lo0 = sdesc_lo(sbase + C::oSfK, 0);
         // each issuer has its own copies of the scale factors in tensor memory, so that its MMAs and copies stay in one order
         const uint32_t sfk_col = tmem + C::cSfK + 8 * h;        // the 128-key atoms; keys 64 .. 127 start two columns in
@@ -683,8 +683,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const Unit* u;
         for (int i = 0, k = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d), nv = uniform(u->nv);
-            const int chunk = PACK && uniform(u->nb[1]) > 1 ? 128 : 16;           // bytes from 8 keys of delta_s to the next 8
-            const uint32_t delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 8 * chunk, chunk), hi_delta = sdesc_hi(chunk, kSwzNone);
+            uint32_t delta_lo0 = delta_row_lo, hi_delta = sdesc_hi(16, kSwzNone);
+            if constexpr (PACK) {
+                if (uniform(u->nb[1]) > 1) {       // the box of several heads: 128 bytes from 8 keys to the next 8
+                    delta_lo0 = sdesc_lo(sbase + C::oDelta + h * 1024, 128);
+                    hi_delta = sdesc_hi(128, kSwzNone);
+                }
+            }
             unit_done(i);
             if (ns == 0) continue;
             const int qb = k & 1;

@@ -468,7 +468,8 @@ __device__ __forceinline__ void quant_q_tile(
 // FEW: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
 // looks at), which makes room for a fourth block per SM:
 // 1 000 queries of 32 heads against 9 192 keys 143.9 -> 141.9 us per call, 4 250 tokens of 48 heads 359.0 -> 356.9 us.
-template <typename T, int D, bool FEW>
+// FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
+template <typename T, int D, bool FEW, bool FLAG>
 __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     T* __restrict__ km,                // [B*H][D]
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     uint8_t* __restrict__ sfs,         // [B*H][Np/128][D/64][512]
     int rows,                          // query blocks of all query heads of a kv head
     int* __restrict__ status,
-    int* __restrict__ nonfinite,       // [B*H]: set when a delta_s value is not finite; nullptr: not wanted
+    int* __restrict__ nonfinite,       // FLAG: [B*H], set when a delta_s value is not finite
     const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 (FEW: 64) rows x 128 bytes, 128-byte swizzle
     const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*H][rows][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
     constexpr int CH = D / 16;            // microblocks per row
@@ -625,7 +626,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
             const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + chalf * 64;
             const int stg_off = oStg + (chalf * (kARows / 32) + quarter) * 4096;
             uint8_t* stg = sgen + stg_off;
-            uint32_t z = 0;
+            uint32_t z = 0;               // FLAG: 0 while all values are finite
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 float v[32];
@@ -638,13 +639,13 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
                     for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
                     *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
                         make_uint4(p4[0], p4[1], p4[2], p4[3]);
-                    if (nonfinite != nullptr) {
+                    if constexpr (FLAG) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e) z = Num<T>::zero_fma2(p4[e], z);
                     }
                 }
             }
-            if (nonfinite != nullptr && (z & 0x7fff7fffu) != 0 && m0 + quarter * 32 + lane < rows) nonfinite[bh] = 1;
+            if (FLAG && (z & 0x7fff7fffu) != 0 && m0 + quarter * 32 + lane < rows) nonfinite[bh] = 1;
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -786,8 +787,7 @@ __global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(con
     extern __shared__ __align__(16) uint8_t smem_raw[];
     pdl_launch_dependents();
     int i = blockIdx.x;
-    if (a.clear != nullptr && i == 0)
-        for (int j = threadIdx.x; j < a.n_clear; j += 256) a.clear[j] = 0;
+    if (a.clear != nullptr && i == 0 && threadIdx.x < a.n_clear) a.clear[threadIdx.x] = 0;
     int tile, bh;
     if (i < a.n_colk) {
         bh = a.chunks_k.divmod(i, tile);
@@ -849,7 +849,8 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     s.part_k = a.kpart; s.part_q = a.kpart + (size_t)BHkv * a.kchunks_k * D;
     s.km = km; s.qm = qm;
     s.q_codes = a.q_codes; s.q_sf = a.q_sf; s.v_codes = a.v_codes; s.v_sf = a.v_sf;
-    s.clear = a.clear; s.n_clear = a.n_clear;
+    s.clear = a.clear; s.n_clear = a.n_clear < 256 ? a.n_clear : 256;      // by the threads of one block
+    if (a.n_clear > 256 && (e = checked(cudaMemsetAsync(a.clear + 256, 0, (a.n_clear - 256) * sizeof(int), st))) != cudaSuccess) return e;
     // Q waits for the means when it is smoothed by one mean per head (api.py:88-90) or when q . km is wanted
     const bool q_late = !a.per_block_mean || a.want_qkm;
     const bool km_here = !a.km_given;
@@ -891,7 +892,8 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, few ? 64 : 128, 3) != 0 ||
         encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    auto kern = few ? quant_k_delta_kernel<T, D, true> : quant_k_delta_kernel<T, D, false>;
+    auto kern = a.nonfinite != nullptr ? (few ? quant_k_delta_kernel<T, D, true, true> : quant_k_delta_kernel<T, D, false, true>)
+                                       : (few ? quant_k_delta_kernel<T, D, true, false> : quant_k_delta_kernel<T, D, false, false>);
     if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
     return launch(true, kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
                       a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status,
