@@ -467,8 +467,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               m_s[t * 128] = ma.x;
           }
           // ---------------------------------------------------------------- O / l of the unit's tiles
-          // (The accumulators belong to the next unit once this warpgroup arrives for its first items.)
-          for (int t = 0; ok && broken == 0 && t < w.nv; ++t) {
+          // (The accumulators belong to the next unit once this warpgroup arrives for its first items.  PACK == 2: the warps without rows
+          // stay away, the pipeline does not wait for them, and the barrier below may be two phases on by the time they look.)
+          for (int t = 0; ok && broken == 0 && (PACK != 2 || quarter == 0) && t < w.nv; ++t) {
               const int grow = PACK ? prow_tok : (w.mt0 + t) * kBlock + row;
               const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq;
               const int bhq = w.bhq + prow_head, hq = w.hq + prow_head;

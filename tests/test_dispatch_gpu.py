@@ -60,6 +60,22 @@ def test_few_rows_split_by_keys(cuda_device, B, Nq, Hq, Hkv, D, Nk, causal):
     assert torch.equal(out.transpose(1, 2).flatten(0, 1), ref) and torch.equal(lse, ref_lse)
 
 
+@pytest.mark.parametrize("Nk", [128, 1030, 2400])
+@pytest.mark.parametrize("D", [64, 128])
+def test_few_rows_in_many_units(cuda_device, D, Nk):
+    """At most 32 rows per kv head, four units and more per CTA, of 1 to 19 key blocks: one warp of the output group does the work and the
+    other three pass units by.  No wait gives up, and the bits are those of the packed variable-length path."""
+    B, H, Nq = 8, 80, 2
+    q, k, v = _inputs(cuda_device, B, H, H, Nq, Nk, D, seed=870 + Nk)
+    prob = Sage3Problem(q, k, v)
+    for _ in range(5):
+        out = prob.run()
+    assert prob.check_status() == 0
+    cq, ck = (torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * n for n in (Nq, Nk))
+    ref = sageattn_varlen(*(x.transpose(1, 2).flatten(0, 1) for x in (q, k, v)), cq, ck, Nq, Nk)
+    assert torch.equal(out.transpose(1, 2).flatten(0, 1), ref)
+
+
 @pytest.mark.parametrize("Nk", [1, 512, 513, 16384, 16385])
 @pytest.mark.parametrize("block_mean", [True, False])
 def test_means_inside_and_outside_the_kernels(cuda_device, Nk, block_mean):
