@@ -320,7 +320,7 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
                     sm_scale=None, per_block_mean: bool = True, return_lse: bool = False, **kwargs):
     """Signature of the reference's packed variable-length entry (sageattention/core.py:334-345): q
     [total_q, Hq, D], k, v [total_k, Hkv, D]; sequence i owns rows cu_seqlens[i]:cu_seqlens[i+1].  Returns
-    [total_q, Hq, D].
+    [total_q, Hq, D] (strides like q's when q is a permuted view).
 
     The whole batch is ONE launch of every kernel (`sage3_fwd_varlen`): the kernels read cu_seqlens on the device, every
     sequence is smoothed, quantized and attended exactly as a call on it alone would be, and a sequence without keys
@@ -374,6 +374,11 @@ def sageattn_varlen(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlen
     return _varlen_impl(q, k, v, cq, ck, max_seqlen_q, max_seqlen_k, is_causal, sm_scale, per_block_mean, return_lse)
 
 
+def _varlen_out(q):
+    """The output of sageattn_varlen: q's strides (a permuted view gives a permuted result) where rows the kernels can store allow it."""
+    return torch.empty_like(q) if q.stride(-1) == 1 and all(s % 8 == 0 for s in q.stride()[:-1]) else torch.empty(q.shape, dtype=q.dtype, device=q.device)
+
+
 def _varlen_impl(q, k, v, cq, ck, max_seqlen_q, max_seqlen_k, is_causal, sm_scale, per_block_mean, return_lse=False):
     dev = q.device
     Hq, Hkv, D = q.shape[1], k.shape[1], q.shape[2]
@@ -387,7 +392,7 @@ def _varlen_impl(q, k, v, cq, ck, max_seqlen_q, max_seqlen_k, is_causal, sm_scal
         max_seqlen_q = max(b - a for a, b in zip(hq, hq[1:]))
         max_seqlen_k = max(b - a for a, b in zip(hk, hk[1:]))
     qc, kc, vc = (t if _usable(t) else t.contiguous() for t in (q, k, v))
-    out = torch.empty_like(qc)
+    out = _varlen_out(q)
     max_seqlen_q, max_seqlen_k = max(int(max_seqlen_q), 1), max(int(max_seqlen_k), 1)
     lse = torch.full((nseq, Hq, max_seqlen_q), float("-inf"), dtype=torch.float32, device=dev) if return_lse else None
     if q.shape[0] == 0:
@@ -427,7 +432,7 @@ def _fwd_varlen_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens
 
 @_fwd_varlen_op.register_fake
 def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, is_causal, sm_scale, per_block_mean):
-    return torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    return _varlen_out(q)
 
 
 _OFFLOAD_STATE: dict = {}

@@ -4,6 +4,7 @@
 // Anything unusual (copies needed, per-head scale, wrong types or shapes) returns None: the Python path deals with it and raises
 // what there is to raise.
 #include <ATen/ops/empty.h>
+#include <ATen/ops/empty_like.h>
 #include <ATen/ops/full.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -154,7 +155,7 @@ PyObject* fwd_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
     d.per_block_mean = block_mean;
     d.sm_scale = (float)scale;
     const c10::cuda::CUDAGuard guard(q.device());
-    const at::Tensor out = at::empty(q.sizes(), q.options());
+    const at::Tensor out = at::empty_like(q);          // (the strides of a permuted q, as on the Python path)
     const at::Tensor lse = want_lse ? at::full({nseq, Hq, (int64_t)max_q}, -std::numeric_limits<double>::infinity(), q.options().dtype(at::kFloat))
                                     : at::Tensor();
     auto strides = [&](const at::Tensor& t, int64_t* s) {

@@ -231,3 +231,19 @@ def test_threads_on_one_stream_share_a_workspace(cuda_device):
     torch.cuda.synchronize()
     for i, ref in enumerate(refs):
         assert len(outs[i]) == 30 and all(torch.equal(o, ref) for o in outs[i])
+
+
+@pytest.mark.parametrize("maxima", [(), (230, 230)])
+def test_varlen_output_keeps_the_strides_of_q(cuda_device, maxima):
+    """A packed q that is a permuted view, or a slice of a wider tensor: the output is laid out like torch.empty_like(q), whether the
+    maxima are given (host extension) or not (Python path)."""
+    lens = torch.tensor([0, 70, 300], dtype=torch.int32, device=cuda_device)
+    q, k, v = (x[0].transpose(0, 1) for x in _inputs(cuda_device, 1, 4, 2, 300, 300, 64, seed=1400))
+    ref = sageattn_varlen(q.contiguous(), k, v, lens, lens, *maxima)
+    assert ref.is_contiguous()
+    wide = torch.empty(300, 7, 64, dtype=q.dtype, device=cuda_device)
+    wide[:, :4] = q
+    for view in (q, wide[:, :4]):
+        out = sageattn_varlen(view, k, v, lens, lens, *maxima)
+        assert out.stride() == torch.empty_like(view).stride()
+        assert torch.equal(out, ref)

@@ -147,6 +147,21 @@ def test_custom_op_traces_with_fake_tensors():
         assert o.shape == qp.shape and o.dtype == qp.dtype
 
 
+def test_fake_varlen_output_has_the_strides_of_the_real_one():
+    """A compiler lays its code out by the fake result: like torch.empty_like(q) where q's rows can be stored to, else contiguous."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    import sageattention_b200  # noqa: F401  (registers the ops)
+    with FakeTensorMode():
+        kp = torch.empty(120, 2, 64, dtype=torch.bfloat16, device="cuda")
+        cu = torch.empty(3, dtype=torch.int32, device="cuda")
+        permuted = torch.empty(4, 100, 64, dtype=torch.bfloat16, device="cuda").transpose(0, 1)
+        slice_ = torch.empty(100, 9, 64, dtype=torch.bfloat16, device="cuda")[:, :4]
+        columns = torch.empty(64, 100, 4, dtype=torch.bfloat16, device="cuda").permute(1, 2, 0)
+        for q, strides in ((permuted, (64, 6400, 1)), (slice_, (256, 64, 1)), (columns, (256, 64, 1))):
+            o = torch.ops.sageattention_b200.fwd_varlen(q, kp, kp, cu, cu, 60, 70, True, None, True)
+            assert o.shape == q.shape and o.stride() == strides
+
+
 # ------------------------------------------------------------------------------------------------------ GPU
 @pytest.mark.gpu
 def test_processor_with_fp4_kernel_matches_oracle(cuda_device):
