@@ -67,6 +67,9 @@ bool same_kind(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v) {
     return k.device() == q.device() && v.device() == q.device();
 }
 
+// 0 asks for the default; any other scale has to be positive as the 32-bit value of the descriptor, too (1e-60 is not)
+bool scale_ok(double scale) { return scale == 0 || (float)scale > 0; }
+
 PyObject* result(const at::Tensor& out, const at::Tensor& lse) {
     if (!lse.defined()) return THPVariable_Wrap(out);
     PyObject* t = PyTuple_New(2);
@@ -93,7 +96,7 @@ PyObject* fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!truth(args[3], &nhd) || !truth(args[4], &causal) || !truth(args[6], &block_mean) || !truth(args[7], &want_lse)) return nullptr;
     const double scale = PyFloat_AsDouble(args[5]);
     if (scale == -1.0 && PyErr_Occurred()) return nullptr;
-    if (!(scale >= 0) || q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || !same_kind(q, k, v)) Py_RETURN_NONE;
+    if (!scale_ok(scale) || q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || !same_kind(q, k, v)) Py_RETURN_NONE;
     const int hd = nhd ? 2 : 1, nd = nhd ? 1 : 2;
     const auto qs = q.sizes(), ks = k.sizes();
     const int64_t B = qs[0], Hq = qs[hd], Nq = qs[nd], D = qs[3], Hkv = ks[hd], Nk = ks[nd];
@@ -140,7 +143,7 @@ PyObject* fwd_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     bool causal, block_mean, want_lse;
     if (!truth(args[7], &causal) || !truth(args[9], &block_mean) || !truth(args[10], &want_lse)) return nullptr;
-    if (!(scale >= 0) || q.dim() != 3 || k.dim() != 3 || v.dim() != 3 || !same_kind(q, k, v)) Py_RETURN_NONE;
+    if (!scale_ok(scale) || q.dim() != 3 || k.dim() != 3 || v.dim() != 3 || !same_kind(q, k, v)) Py_RETURN_NONE;
     for (const at::Tensor* c : {&cq, &ck})
         if (!c->is_cuda() || c->device() != q.device() || c->scalar_type() != at::kInt || c->dim() != 1 || !c->is_contiguous()) Py_RETURN_NONE;
     const int64_t Hq = q.size(1), Hkv = k.size(1), D = q.size(2), nseq = cq.size(0) - 1;

@@ -247,3 +247,16 @@ def test_varlen_output_keeps_the_strides_of_q(cuda_device, maxima):
         out = sageattn_varlen(view, k, v, lens, lens, *maxima)
         assert out.stride() == torch.empty_like(view).stride()
         assert torch.equal(out, ref)
+
+
+def test_scale_that_is_zero_in_fp32_is_refused(cuda_device):
+    """1e-60 is positive but 0 as the 32-bit scale of the descriptor, where 0 stands for the default; 1e-38 is a scale."""
+    q, k, v = _inputs(cuda_device, 1, 2, 2, 100, 100, 64, seed=1500)
+    packed = [x[0].transpose(0, 1) for x in (q, k, v)]
+    cu = torch.tensor([0, 100], dtype=torch.int32, device=cuda_device)
+    for scale in (1e-60, 0.0, float("nan")):
+        with pytest.raises(ValueError):
+            sageattn3(q, k, v, sm_scale=scale)
+        with pytest.raises(ValueError):
+            sageattn_varlen(*packed, cu, cu, 100, 100, sm_scale=scale)
+    assert not torch.equal(sageattn3(q, k, v, sm_scale=1e-38), sageattn3(q, k, v))
