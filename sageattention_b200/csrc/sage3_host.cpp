@@ -6,6 +6,7 @@
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <ATen/ops/full.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -34,13 +35,15 @@ BytesFn g_bytes = nullptr;
 std::mutex g_mutex;
 std::map<std::pair<int, cudaStream_t>, at::Tensor>* g_workspaces = nullptr;      // never destroyed: the CUDA context may go first
 
-at::Tensor workspace(int device, cudaStream_t stream, size_t bytes) {
+at::Tensor workspace(int device, cudaStream_t stream, size_t bytes) {      // (the device and its stream are the current ones)
+    const auto options = at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, device));
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return at::empty({(int64_t)bytes}, options);
     std::lock_guard<std::mutex> lock(g_mutex);
     if (!g_workspaces) g_workspaces = new std::map<std::pair<int, cudaStream_t>, at::Tensor>();
     at::Tensor& t = (*g_workspaces)[{device, stream}];
     if (!t.defined() || (size_t)t.numel() < bytes) {
         t = at::Tensor();                             // give the old one back first
-        t = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, device)));
+        t = at::empty({(int64_t)bytes}, options);
     }
     return t;
 }
@@ -188,6 +191,7 @@ PyObject* shared_buffer(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const long dev = PyLong_AsLong(args[0]);
     const long long bytes = PyLong_AsLongLong(args[1]);
     if (PyErr_Occurred()) return nullptr;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)dev);
     return THPVariable_Wrap(workspace((int)dev, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(), (size_t)bytes));
     END_HANDLE_TH_ERRORS
 }

@@ -260,3 +260,29 @@ def test_scale_that_is_zero_in_fp32_is_refused(cuda_device):
         with pytest.raises(ValueError):
             sageattn_varlen(*packed, cu, cu, 100, 100, sm_scale=scale)
     assert not torch.equal(sageattn3(q, k, v, sm_scale=1e-38), sageattn3(q, k, v))
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+def test_a_captured_call_keeps_its_workspace(cuda_device, per_head):
+    """A functional call captured on a stream that has made calls before: a larger call replaces the stream's workspace, and
+    the memory it had goes to other tensors.  Replays write to none of them and still give the call's result."""
+    q, k, v = _inputs(cuda_device, 1, 8, 8, 500, 500, 64, seed=1700)
+    big = _inputs(cuda_device, 1, 32, 32, 1000, 1000, 64, seed=1701)
+    scale = torch.full((8,), 0.2, device=cuda_device) if per_head else 0.2              # through Python / the host extension
+    s = torch.cuda.Stream(cuda_device)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        ref = sageattn3(q, k, v, sm_scale=scale)
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            out = sageattn3(q, k, v, sm_scale=scale)
+        big_ref = sageattn3(*big)
+        fill = [torch.full((1 << 20,), 7, dtype=torch.uint8, device=cuda_device) for _ in range(64)]
+        for _ in range(3):
+            out.zero_()
+            g.replay()
+        again = sageattn3(*big)
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref) and torch.equal(again, big_ref)
+    assert all((f == 7).all() for f in fill)
