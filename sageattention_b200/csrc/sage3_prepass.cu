@@ -251,7 +251,7 @@ __device__ __forceinline__ float sum_chunks(const float* __restrict__ part, int 
     for (int c = 0; c < chunks; c += 16) {
         float v[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = c + i < chunks ? part[(int64_t)(c + i) * D] : 0.f;
+        for (int i = 0; i < 16; ++i) v[i] = c + i < chunks ? load_written(part + (int64_t)(c + i) * D) : 0.f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) s += v[i];       // (+ 0 beyond the last chunk: no change)
     }
@@ -342,8 +342,8 @@ __device__ __forceinline__ void quant_q_tile(
             for (int j = 0; j < 16; ++j) kf[j] = s_mean[c * 16 + j];
             __syncthreads();               // s_mean takes the Q mean next
         } else {
-            uint4 k0, k1;
-            load16_packed<T>(km + (int64_t)bhk * D + c * 16, true, k0, k1);
+            const uint4* km4 = reinterpret_cast<const uint4*>(km + (int64_t)bhk * D + c * 16);
+            const uint4 k0 = load_written(km4), k1 = load_written(km4 + 1);
             unpack16<T>(k0, k1, kf);
         }
 #pragma unroll
