@@ -526,12 +526,14 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     if (warp == 0) {
         tmem_alloc(smem_u32(tmem_slot), kTmemCols);
         tmem_relinquish();
+        // Not before this block has its tensor memory: a dependent that takes all of it and then waits for this launch would keep it from
+        // going on.  (The attention kernel's shared memory leaves no room next to a block of this one; another's may.)
+        pdl_launch_dependents();
     }
     uint4 raw[ITEMS][2];
     x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
         load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
     });
-    pdl_launch_dependents();
     pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
     // the first A tile (see below) comes in while K is quantized
     auto load_a = [&](int m0) {
