@@ -18,13 +18,16 @@ def _inputs(device, B, Hq, Hkv, Nq, Nk, D, seed, dtype=torch.bfloat16):
 
 
 @pytest.mark.parametrize("D,causal", [(128, False), (64, True)])
-@pytest.mark.parametrize("extra", [-1, 0, 1, 74, 76])
-def test_units_around_the_sm_count(cuda_device, D, causal, extra):
-    """Three query tiles per head (a pair and a single one); two units per head, 2 x heads around one round of all SMs: one
-    round less a unit, full, and a second round that is dealt out as single tiles (up to half of the SMs) or not."""
+@pytest.mark.parametrize("tiles,half,extra", [(3, 0, -2), (3, 0, 0), (3, 0, 2), (3, 1, 0), (3, 1, 2), (2, 0, -1), (2, 0, 0), (2, 0, 1), (2, 1, 0), (2, 1, 1)])
+def test_units_around_the_sm_count(cuda_device, D, causal, tiles, half, extra):
+    """Two query tiles per head are one unit, three are two (a pair and a single one).  The units number one round of all SMs, or a round
+    and a half, plus `extra`: a round that is not full, a full one, and a second one that is dealt out as single tiles (up to half of the
+    SMs) or not."""
     sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
-    H = (sms + extra + 1) // 2
-    q, k, v = _inputs(cuda_device, 1, H, H, 300, 260, D, seed=700 + extra)
+    units = sms + half * (sms // 2) + extra
+    H = units // (tiles - 1)
+    assert H * (tiles - 1) == units
+    q, k, v = _inputs(cuda_device, 1, H, H, 128 * tiles - 84, 260, D, seed=700 + extra)
     out = sageattn3(q, k, v, is_causal=causal)
     for h in sorted({0, 1, H // 2, H - 2, H - 1}):
         one = sageattn3(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], is_causal=causal)
