@@ -73,7 +73,8 @@ typedef struct Sage3Desc {
 /*
  * Byte offsets of the regions inside the workspace (all multiples of 1024).  Np = N rounded up to 128.
  *   status   int32[64]                        device-written status words (0 = fine): [0, 32) pre-pass, [32, 64) attention;
- *                                             each stage clears its own half, so sage3_check_status after sage3_fwd sees both
+ *                                             the pre-pass clears all, attention on its own its half only, so that
+ *                                             sage3_check_status after sage3_fwd sees what either stage reported
  *                                             (behind them, word 64: the attention kernel's work counter; words 65 ...: per
  *                                             (batch, kv head), delta_s holds a value that is not finite)
  *   kpart    fp32 [B*Hkv][chunks][D]          scratch: partial column sums of K (followed by those of Q when per_block_mean = 0)

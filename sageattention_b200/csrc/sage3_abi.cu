@@ -35,7 +35,7 @@ cudaError_t current_device(int* dev, DeviceInfo* info) {
 
 cudaError_t allow_smem(const void* kernel, int bytes) {
     struct Entry { const void* kernel; uint64_t devices; };
-    static Entry done[64];                            // one per kernel instantiation (fewer than 32 exist)
+    static Entry done[64];                            // one per kernel instantiation (52 exist)
     static std::mutex mutex;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -64,8 +64,8 @@ constexpr size_t kAlign = 1024;     // every workspace region starts at a multip
 constexpr size_t kWsAlign = 256;    // required alignment of the workspace base pointer
 inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
-// Words of the status region: behind the 64 status words the attention kernel's work counter, then one word per (batch, kv head) that
-// the pre-pass sets when a value of its delta_s is not finite.
+// Words of the status region: [0, 32) what the pre-pass reports, [32, 64) what the attention kernel reports, then its work counter, then
+// one word per (batch, kv head) that the pre-pass sets when a value of its delta_s is not finite.  The first pre-pass kernel clears all.
 constexpr int kAttnStatusWord = 32, kUnitCounterWord = 64, kNonfiniteWord = 65;
 
 int validate(const Sage3Desc* d) {
@@ -132,9 +132,6 @@ int check_arch() {
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
-// Status words: [0, 32) belong to the pre-pass, [32, 64) to the attention kernel.  Each stage clears its own half only,
-// so a wait the pre-pass gave up on is still there after the attention launch (whose CTAs read it and exit at once).
-
 // Held while a whole call (pre-pass and attention) is enqueued: its launches hand their results on through the workspace, so the calls
 // of several threads on one workspace and stream may follow one another but not interleave.  One of a few locks by address: threads
 // with workspaces of their own seldom meet, and then for microseconds.
@@ -167,7 +164,9 @@ sage3::PartsPtr one_part(const void* p) {
     return r;
 }
 
-// `cleared`: the pre-pass of the same call has already zeroed the attention half of the status words and the work counter
+// `cleared`: the pre-pass of the same call has already zeroed the attention half of the status words and the work counter.  An attention
+// call on its own zeroes these and leaves the pre-pass half alone, so that a wait the pre-pass gave up on stays on record (the kernel
+// then walks its units without writing anything).
 int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, void* stream, bool cleared = false,
               const Sage3Carry* carry = nullptr, const int32_t* cu_q = nullptr, const int32_t* cu_k = nullptr) {
     Sage3Workspace w;

@@ -81,15 +81,16 @@ struct AttnParams {
 constexpr int kUnitRing = 4;
 
 // PACK: few query rows and several query heads per kv head.  The rows of all these heads share one 128-row tile (row = head * Nq +
-// token), so the keys are walked once instead of once per head: 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv
-// heads 122 -> 64 us.
+// token), so the keys are walked once instead of once per head.  Mode 1: 2 sequences x 32 heads x 16 tokens against 8 192 keys of 8
+// kv heads 90.1 -> 88.3 us per call (without packing its 64 tiles leave SMs idle too; 8 sequences x 32 heads x 1 token, which
+// mode 2 has now: 225.8 -> 166.4 us).
 //
 // PACK == 2: at most 32 such rows.  A thread owns a row of scores, so one warp of the four would have work and do the exponentials
 // of all 128 keys for it.  The rows stand in every quarter of the tile instead (rows 0..31 = 32..63 = ...), and the warp of quarter
 // w takes keys 32 w .. 32 w + 31 of the block for all of them: a quarter of the exponentials per warp.  The four exchange their
 // maxima through shared memory; P, its scales and the accumulator are those of rows 0..31.  Same operations per score, and the row
 // sums are added in the same order, so the same bits.  D = 128, 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv heads:
-// 62 -> 40 us, 780 cycles per block (D = 64: 33 us); the copy warp's and the MMA issuer's instructions bound it now.
+// 166.4 -> 143.1 us per call, pre-pass included (D = 64: 116.8 -> 92.2 us).  The copy warp's and the MMA issuer's instructions bound it.
 template <int D, int PACK>
 struct Cfg {
     // K and V^T stages, each shared by the two query tiles (as many as fit: PACK, see oP)
@@ -1082,7 +1083,7 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
 }
 
 template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK>
-static cudaError_t launch_v(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
+static cudaError_t launch_v(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int grid, cudaStream_t st) {
     auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK>;
     using C = Cfg<D, PACK>;
@@ -1095,10 +1096,10 @@ template <int D, bool CAUSAL, typename OutT>
 static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int pack_mode, int grid, cudaStream_t st) {
     // packed variable-length batches run their own instantiation, so that the uniform kernels carry none of it
-    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, 0>(a, tq, tk, tv, td, p, grid, st)
-           : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(a, tq, tk, tv, td, p, grid, st)
-           : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(a, tq, tk, tv, td, p, grid, st)
-                              : launch_v<D, CAUSAL, OutT, false, 0>(a, tq, tk, tv, td, p, grid, st);
+    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, 0>(tq, tk, tv, td, p, grid, st)
+           : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(tq, tk, tv, td, p, grid, st)
+           : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(tq, tk, tv, td, p, grid, st)
+                              : launch_v<D, CAUSAL, OutT, false, 0>(tq, tk, tv, td, p, grid, st);
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
@@ -1134,7 +1135,9 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     const int sms = info.sms;
     AttnParams p;
     // Units of work: pairs of query tiles; when the last round of pairs fills at most half of the SMs it is dealt out as
-    // single tiles (half the time for the round, twice the SMs).
+    // single tiles (half the time for the round, twice the SMs).  With more than that single tiles need two rounds and lose the shared
+    // K and V stages.  148 SMs, heads x 2 048 tokens, D = 128, never / this rule / always single: 68 pairs over 81.8 / 71.8 / 71.7 us,
+    // 76 over 82.8 / 82.8 / 85.9 us, 140 over 87.5 / 87.4 / 92.9 us.
     const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), rest = pairs % sms;
     const bool split = nqt > 1 && 2 * rest <= sms;
     p.unit_counter = a.unit_counter;

@@ -97,16 +97,6 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 // ------------------------------------------------------------------------------------------------
 // number formats
 // ------------------------------------------------------------------------------------------------
-// Two fp32 -> one byte of two E2M1 codes; `lo` lands in bits 0-3, `hi` in bits 4-7.
-__device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
-    uint32_t r;
-    asm("{\n\t.reg .b8 b;\n\t"
-        "cvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n\t"
-        "cvt.u32.u8 %0, b;\n\t}"
-        : "=r"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-
 // Eight fp32 -> 32 bits of E2M1 codes, element i in nibble i.
 __device__ __forceinline__ uint32_t cvt_e2m1x8(float f0, float f1, float f2, float f3, float f4, float f5,
                                                float f6, float f7) {
@@ -163,17 +153,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-// one non-blocking look
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
@@ -353,19 +332,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
           "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
-    const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
-        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]),
-          "r"(taddr) : "memory");
-}
-
 // byte offset of scale (row r, scale column c) inside a group of 128-row x 4-scale atoms
 __host__ __device__ constexpr uint32_t sf_atom_offset(uint32_t r, uint32_t c) {
     return (c >> 2) * 512u + (r & 31u) * 16u + ((r >> 5) & 3u) * 4u + (c & 3u);
