@@ -162,22 +162,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // CTA (abort flag in shared memory) or another CTA (status word in global memory) has given up.
 // On giving up it records `code` in the status word, raises the CTA's abort flag and returns false;
 // the caller must then leave its loop.  Nothing ever spins without a limit.
-constexpr long long kWaitLimitCycles = 2000000000LL;   // about a second
+constexpr uint32_t kWaitLimitCycles = 2000000000u;   // about a second (of a 32-bit clock)
 
 // kBackoff: sleep a little between polls (single-lane roles, so that polling does not take issue slots
 // from the math warps of the same scheduler).
 template <bool kBackoff = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status_word, int code, long long limit_cycles = kWaitLimitCycles) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
+                                          int* status_word, int code, uint32_t limit_cycles = kWaitLimitCycles) {
+    const uint32_t t0 = clock();
     uint32_t spins = 0;
     while (true) {
         if (mbar_try_wait(bar, parity)) return true;
         if (kBackoff) __nanosleep(40);
         if ((++spins & 0x3f) == 0) {
             if (*abort_flag != 0) return false;
-            if (clock64() - t0 > limit_cycles || *reinterpret_cast<volatile int*>(status_word) != 0) {
+            if ((uint32_t)clock() - t0 > limit_cycles || *reinterpret_cast<volatile int*>(status_word) != 0) {
                 atomicCAS(status_word, 0, code);
                 *abort_flag = 1;
                 return false;
