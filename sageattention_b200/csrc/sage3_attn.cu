@@ -493,11 +493,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq;
               const int bhq = w.bhq + prow_head, hq = w.hq + prow_head;
               const bool have = w.nb[t] > 0 || carry_in;
-              if (w.nb[t] > 0) {
-                  const int sl = base + (w.two ? 2 * (w.nbmax - 1) + t - w.d : w.nb[t] - 1);       // the tile's last item
-                  if (!warp_wait(bar(bPV + (sl & 7)), (sl >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
-              }
-              tc_fence_after();
               const float2 l2 = l_s[t * 128];
               const float l_tot = l2.x + l2.y;
               if (live && (p.lse != nullptr || carry_out)) {
@@ -523,6 +518,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const int opart = (p.out_rows == 0) ? 0 : min(grow / p.out_rows, kMaxParts - 1);
               OutT* orow = p.out[opart] == nullptr || !live ? nullptr
                          : static_cast<OutT*>(p.out[opart]) + w.out_base + hq * p.os1 + (int64_t)(grow - opart * p.out_rows) * p.os2;
+              if (w.nb[t] > 0) {
+                  const int sl = base + (w.two ? 2 * (w.nbmax - 1) + t - w.d : w.nb[t] - 1);       // the tile's last item
+                  if (!warp_wait(bar(bPV + (sl & 7)), (sl >> 3) & 1, abort_flag, p.status, kWaitOReady)) { ok = false; break; }
+              }
+              tc_fence_after();
+              // All address arithmetic ahead of the wait for the last P V, products in pairs: the warp shares its scheduler with four softmax
+              // warps, so what is behind the wait costs several cycles an instruction (300 keys at D = 128 191.9 -> 190.7 us, packed prompts
+              // 610.3 -> 607.6, 226 keys 247.6 -> 246.1).  Its stores cost nothing that shows, wider loads did not help.
+              const uint64_t inv2 = pack2f(inv_l, inv_l);
 #pragma unroll (PACK == 2 ? 8 : 1)
               for (int c = 0; c < D; c += 16) {
                   float o[16];
@@ -542,7 +546,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   if (orow != nullptr) {
                       uint32_t v[8];
 #pragma unroll
-                      for (int q = 0; q < 8; ++q) v[q] = pack2<OutT>(o[2 * q] * inv_l, o[2 * q + 1] * inv_l);
+                      for (int q = 0; q < 8; ++q) {
+                          float x, y;
+                          unpack2f(mul2(pack2f(o[2 * q], o[2 * q + 1]), inv2), x, y);
+                          v[q] = pack2<OutT>(x, y);
+                      }
                       if (p.out_wide) {
                           store_32b(orow + c, v);
                       } else {
