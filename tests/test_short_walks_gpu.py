@@ -1,0 +1,47 @@
+"""Walks of few key blocks, many of them per SM: V is loaded two blocks behind K (D = 128), across units too; P slots, running maxima and
+barrier phases run on from unit to unit; and the number of key blocks at which D = 64 without a mask changes kernels.  A head's result
+depends on its own q, k, v alone, so every comparison is for equal bits; against the oracle the gate is the one of the whole path
+(cosine >= 0.999, relative L1 <= 1 %)."""
+import pytest
+import torch
+
+from oracle import sage3_oracle as O
+from sageattention_b200 import sageattn3, sageattn_varlen
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(device, B, H, Nq, Nk, D, seed):
+    q, k, v = O.make_inputs(B, H, H, Nq, Nk, D, seed=seed, dtype=torch.bfloat16, k_offset_std=1.0)
+    return q.to(device), k.to(device), v.to(device)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Nq,Nk,causal", [(130, 1, False), (1, 128, False), (130, 129, False), (257, 300, False), (130, 650, False),
+                                          (130, 130, True), (300, 300, True), (257, 100, True), (640, 640, True)])
+def test_units_of_few_key_blocks(cuda_device, D, Nq, Nk, causal):
+    """Some five units per SM, single tiles and pairs, of one to five key blocks (causal: none to five, the tiles of a pair with
+    different numbers): the same bits as the heads alone, where each is the first unit of its SM."""
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    pairs = (Nq + 255) // 256
+    H = 5 * sms // pairs + 3
+    q, k, v = _inputs(cuda_device, 1, H, Nq, Nk, D, seed=1300 + Nq + Nk)
+    out, lse = sageattn3(q, k, v, is_causal=causal, return_lse=True)
+    for h in sorted({0, 1, H // 3, H // 2, H - 2, H - 1}):
+        one, one_lse = sageattn3(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], is_causal=causal, return_lse=True)
+        assert torch.equal(out[:, h:h + 1], one) and torch.equal(lse[:, h:h + 1], one_lse), f"head {h} of {H}"
+    h = H // 2
+    ref = O.sageattn3_oracle(q[:, h:h + 1].cpu(), k[:, h:h + 1].cpu(), v[:, h:h + 1].cpu(), is_causal=causal)
+    assert O.cosine(out[:, h:h + 1].cpu(), ref) >= 0.999 and O.rel_l1(out[:, h:h + 1].cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("Nk", [1023, 1024, 1025, 1152, 2049])
+def test_halves_rolled_and_unrolled_at_64_channels(cuda_device, Nk, causal):
+    """Beyond eight key blocks the uniform kernel without a mask has the halves of an item unrolled; the packed variable-length kernel
+    has them rolled at every length: the same bits."""
+    H, Nq = 5, 300
+    q, k, v = _inputs(cuda_device, 1, H, Nq, Nk, 64, seed=1400 + Nk)
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (Nq, Nk))
+    packed = sageattn_varlen(*(x[0].transpose(0, 1).contiguous() for x in (q, k, v)), cu_q, cu_k, Nq, Nk, is_causal=causal)
+    assert torch.equal(sageattn3(q, k, v, is_causal=causal)[0].transpose(0, 1), packed)
