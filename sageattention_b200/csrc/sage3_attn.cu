@@ -21,7 +21,8 @@
 // nothing else connects the groups: four independent chains per scheduler, a quarter of an item apart.
 // What bounds it: the exp2 unit (16 results per clock and SM: 1 096 cycles per 128 x 128 block with the exponentials of the
 // scales), the other instructions of the softmax warps (some 700 issue slots per block and scheduler) and fetching them; the tensor pipe
-// needs 580 cycles.  Measured (B = 2, H = 32, N = 16 384, 1 965 MHz): 1 505 cycles per block at D = 128 and 1 425 at D = 64.
+// needs 580 cycles.  Measured (1 965 MHz): 1 522 cycles per block at D = 128 and 1 458 at D = 64 for N = 16 384, 1 483 and 1 425 for N = 32 768;
+// the exp2 unit 78 %, issue slots 63 % busy.
 // Code size is a cost of its own: the softmax warps of a scheduler are in different places of their loop, and the issuers' and correction
 // warps' loops come on top.  Taking out code that never ran (carried state, masks, second copies of waits) and rolling the two halves of
 // an item into one loop gave more than any instruction saved in it: 2 x 48 heads, 17 550 queries x 226 keys, D = 64 298 -> 246 us per call, 2 x 40
