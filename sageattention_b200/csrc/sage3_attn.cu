@@ -4,9 +4,11 @@
 // One CTA per SM; each draws units of work from a counter.  A unit is a PAIR of 128-row query tiles of one head (every K / V^T
 // stage in shared memory serves both tiles), a stream of items (key block, tile), the two tiles in turn; all pipelines run on
 // from unit to unit.  Six warpgroups (setmaxnreg moves registers to the softmax warpgroups):
-//   warp 0       draws and publishes the units; TMA producer: Q tiles, then K (+ one delta_s row per tile) / V^T / scale atoms per block
-//   warps 1, 3   Q K^T MMA issuers, for keys [0, 64) and [64, 128) of every item; warp 1 owns the tensor-memory allocation
+//   warps 0, 1   Q K^T MMA issuers, for keys [0, 64) and [64, 128) of every item; warp 1 owns the tensor-memory allocation
 //   warp 2       P V MMA issuer
+//   warp 3       draws and publishes the units; TMA producer: Q tiles, then K (+ one delta_s row per tile) / V^T / scale atoms per block
+//                (Each on a scheduler of its own.  With the producer as warp 0 and the issuers as 1 and 3 nothing was faster and most
+//                calls 0.1 to 0.6 % slower: packed prompts 607.0 / 603.5 us, 3 001 tokens 90.6 / 90.3, 16 384 keys 5 788 / 5 780.)
 //   warps 4-19   four softmax groups of four warps; group g takes the items g, g + 4, ...  A thread owns one row of the block
 //                and walks its 128 keys in two halves of 64 (the scores of a half live in registers).
 //   warps 20-23  O rescale ("correction"), one warp per tensor-memory lane quarter, one wait per item: when a row of the quarter moved
@@ -572,7 +574,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tma_load_3d(sbase + C::oV + st * C::kVBytes, &tm_v, bar(bVF + st), n * 64, 0, bhkv);
           bulk_load(sbase + C::oSfV + st * 1024, p.v_sf + ((size_t)bhkv * p.nkb + n) * C::kSfVBytes, C::kSfVBytes, bar(bVF + st));
       };
-      if (warp == 0) {
+      if (warp == 3) {
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
         int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
@@ -696,7 +698,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             advance();
         }
         __syncwarp();
-      } else if (PACK == 2 && warp == 3) {
+      } else if (PACK == 2 && warp == 1) {
         // ------------------------------------------------------------------ TMA producer of V
         // The waits and five copies of a block cost one producer 1 100 cycles, more than anything else does per block here (8 192
         // keys, 64 kv heads: 44 -> 40 us with a warp for K and one for V, D = 64 43 -> 33).
@@ -714,14 +716,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
         }
         __syncwarp();
-      } else if (warp == 1 || warp == 3) {
+      } else if (warp == 0 || warp == 1) {
         // ------------------------------------------------------------------ Q K^T MMA issuers
-        // The scores of an item are formed in two halves of 64 keys; warp 1 issues the first halves, warp 3 the second
+        // The scores of an item are formed in two halves of 64 keys; warp 0 issues the first halves, warp 1 the second
         // ones, each into its own S buffers (issuing one half takes a few hundred cycles next to busy softmax warps: one
         // issuer for both would be the slowest part of the pipeline).  The whole warp walks the loop and one elected lane
         // issues, so loop state and descriptors stay in uniform registers.
-        // (PACK == 2: softmax is short there, and the tensor pipe's cost per instruction counts; warp 1 issues all 128 keys at once.)
-        const int h = warp >> 1;
+        // (PACK == 2: softmax is short there, and the tensor pipe's cost per instruction counts; warp 0 issues all 128 keys at once, warp 1 loads V.)
+        const int h = warp;
         constexpr int kKeys = PACK == 2 ? 128 : 64;
         constexpr uint32_t idesc_qk = make_idesc_nvfp4(kKeys);
         constexpr uint32_t idesc_delta = make_idesc_f16_bmn(kKeys, std::is_same<OutT, __nv_bfloat16>::value);
