@@ -462,12 +462,23 @@ __device__ __forceinline__ void quant_q_tile(
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
 // ------------------------------------------------------------------------------------------------
-// FEW: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
+// AROWS = 64: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
 // looks at), which makes room for a fourth block per SM:
 // 1 000 queries of 32 heads against 9 192 keys 143.9 -> 141.9 us per call, 4 250 tokens of 48 heads 359.0 -> 356.9 us.
+// AROWS = 32: up to eight query blocks and many tiles (token generation).  A block takes two (D = 64: three) tiles one after the other: its tensor
+// memory, mean and A tile are set up once, and the next tile's rows come in under this one's MMAs and read-out, which takes 80
+// registers at D = 128 (three blocks per SM; with four, spilled rows: 137.4 -> 147.1).  us per call, before / after: one token of 8 x 32 heads
+// against 8 192 keys of 8 kv heads 137.2 / 134.2 (D = 64 89.4 / 87.7), of 32 kv heads 464 / 432, four tokens of 16 x 64 heads against 16 000 472 / 451,
+// one against 12 000 at D = 64 212 / 195.
 // FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
-template <typename T, int D, bool FEW, bool FLAG>
-__global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
+// Tiles that a block of the AROWS = 32 kernel takes, and the tiles of a call from which it is used: with fewer than some ten rounds of resident
+// blocks the coarser last round costs as much (148 SMs, 2 048 tiles 87.5 / 88.0 us at D = 128, 59.2 / 59.4 at D = 64; 3 008 109.7 / 109.7 and
+// 69.6 / 67.5).
+__host__ __device__ constexpr int tiles_in_turn(int D) { return D == 128 ? 2 : 3; }
+constexpr int tiles_in_turn_from(int D) { return D == 128 ? 4000 : 3000; }
+
+template <typename T, int D, int AROWS, bool FLAG>
+__global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128) ? 3 : 4) quant_k_delta_kernel(
     const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     T* __restrict__ km,                // [B*H][D]
     const float* __restrict__ part,    // partial column sums to form the mean from ([B*H][chunks][D]), or nullptr: `km` holds it
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     int rows,                          // query blocks of all query heads of a kv head
     int* __restrict__ status,
     int* __restrict__ nonfinite,       // FLAG: [B*H], set when a delta_s value is not finite
-    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box 128 (FEW: 64) rows x 128 bytes, 128-byte swizzle
+    const __grid_constant__ CUtensorMap tm_qm,       // bytes [B*H][rows][2 D], box AROWS rows x 128 bytes, 128-byte swizzle
     const __grid_constant__ CUtensorMap tm_delta) {  // bytes [B*H][rows][2 Np], box 32 rows x 128 bytes, 128-byte swizzle
     constexpr int CH = D / 16;            // microblocks per row
     constexpr int RPP = 256 / CH;         // rows per pass
@@ -486,25 +497,26 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     constexpr uint32_t kTmemCols = 128;
     constexpr bool kBf16 = sizeof(T) == 2 && Num<T>::kIsBf16;
 
-    const int tile = blockIdx.x, bh = blockIdx.y;
+    constexpr int TILES = AROWS == 32 ? tiles_in_turn(D) : 1;
+    const int tile0 = blockIdx.x * TILES, bh = blockIdx.y;
     int h;
     const int b = H.divmod(bh, h);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int c = t % CH, rl = t / CH;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
-    const int row0 = tile * kBlock;
+    int row0 = tile0 * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
 
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t sbase = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     uint8_t* sgen = smem_dyn + (sbase - smem_u32(smem_dyn));
-    // [A tile: qm chunk | B tile: k'] as SUB sub-tiles of (FEW: A 64) 128 rows x 128 bytes each (in this order: the MMA reads 128 rows
-    // from the start of every A sub-tile, which has to stay inside the block's shared memory), then small things, then (D = 64 only,
-    // where the A tile is too small for it) the staging tile of the epilogue: 8 warps x 32 rows x 128 bytes
-    constexpr int kARows = FEW ? 64 : 128, kASub = kARows * 128;
+    // [A tile: qm chunk | B tile: k'] as SUB sub-tiles of (A: AROWS) 128 rows x 128 bytes each (in this order: the MMA reads 128 rows
+    // from the start of every A sub-tile, which has to stay inside the block's shared memory), then small things, then (where the
+    // A tile is too small for it, or stays) the staging tile of the epilogue: 32 rows x 128 bytes per warp that has rows
+    constexpr int kARows = AROWS, kASub = kARows * 128;
     constexpr int oA = 0, oB = SUB * kASub, oMean = oB + SUB * 16384, oSf = oMean + D * 4, oBar = oSf + SUB * 512;
     static_assert(oA + (SUB - 1) * kASub + 16384 <= oMean, "the MMA's 128 A rows stay inside the tiles");
-    constexpr int oStg = (D == 128) ? oA : ((oBar + 64 + 1023) / 1024) * 1024;
+    constexpr int oStg = (D == 128 && TILES == 1) ? oA : ((oBar + 64 + 1023) / 1024) * 1024;
     T* s_mean = reinterpret_cast<T*>(sgen + oMean);
     uint8_t* s_sf = sgen + oSf;
     const uint32_t bar = sbase + oBar;
@@ -528,9 +540,12 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
         pdl_launch_dependents();
     }
     uint4 raw[ITEMS][2];
-    x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
-        load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
-    });
+    auto load_rows = [&]() {
+        x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
+            load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
+        });
+    };
+    load_rows();
     pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
     // the first A tile (see below) comes in while K is quantized
     auto load_a = [&](int m0) {
@@ -543,7 +558,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     if (t < D) {
         if (part != nullptr) {
             const T m = Num<T>::from_f(sum_chunks(part + (int64_t)bh * chunks * D + t, chunks, D) * (N > 0 ? 1.0f / (float)N : 0.f));
-            if (tile == 0) km[(int64_t)bh * D + t] = m;
+            if (tile0 == 0) km[(int64_t)bh * D + t] = m;
             s_mean[t] = m;
         } else {
             s_mean[t] = km[(int64_t)bh * D + t];
@@ -557,6 +572,9 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     uint32_t mu2[8];       // the 16 means of this thread's columns, packed (they are values of the input type)
     *reinterpret_cast<uint4*>(mu2) = reinterpret_cast<const uint4*>(s_mean)[2 * c];
     *reinterpret_cast<uint4*>(mu2 + 4) = reinterpret_cast<const uint4*>(s_mean)[2 * c + 1];
+    uint32_t iter = 0;
+    bool alive = true;
+    for (int it = 0; it < TILES; ++it) {
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const int rt = rl + RPP * i;          // row inside the tile
@@ -582,15 +600,20 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
     }
     __syncthreads();
     {
-        uint8_t* dst = sfs + ((int64_t)bh * (Np / kBlock) + tile) * (D / 64) * 512;
+        uint8_t* dst = sfs + ((int64_t)bh * (Np / kBlock) + tile0 + it) * (D / 64) * 512;
         if (t < (D / 64) * 32) reinterpret_cast<uint4*>(dst)[t] = reinterpret_cast<const uint4*>(s_sf)[t];
     }
 
+    const int tile_row0 = row0;
+    bool more = false;                    // the block's next tile: its rows come in under this one's MMAs
+    if constexpr (TILES > 1) {
+        row0 += kBlock;
+        more = it + 1 < TILES && row0 < N;
+        if (more) load_rows();
+    }
     // delta_s of all query heads of this kv head, 128 query blocks per MMA group
     constexpr uint32_t idesc = make_idesc_f16_kk(128, kBf16);
     const int quarter = warp & 3, chalf = warp >> 2;       // tensor-memory lane quarter, column half of the epilogue
-    uint32_t iter = 0;
-    bool alive = true;
     for (int m0 = 0; m0 < rows && alive; m0 += 128, ++iter) {
         // A tile: 128 query-block means, fetched by the copy engine in the 128-byte swizzle the MMA reads.  Rows beyond
         // the tensor arrive as zeros; rows of a shorter sequence of a packed batch only feed accumulator rows
@@ -600,7 +623,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
             __syncthreads();
             if (t == 0) load_a(m0);
         }
-        alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);
+        if (TILES == 1 || it == 0) alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);      // (several tiles: the A tile stays)
         tc_fence_before();
         alive = __syncthreads_and(alive ? 1 : 0) != 0;
         if (!alive) break;
@@ -626,17 +649,19 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
             const int stg_off = oStg + (chalf * (kARows / 32) + quarter) * 4096;
             uint8_t* stg = sgen + stg_off;
             uint32_t z = 0;               // FLAG: 0 while all values are finite
+            constexpr int kCols = TILES > 1 ? 16 : 32;      // (several tiles: the registers hold the next one's rows)
 #pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                float v[32];
-                tmem_ld32(acc + cc * 32, v);
+            for (int cc = 0; cc < 64 / kCols; ++cc) {
+                float v[kCols];
+                if constexpr (kCols == 32) tmem_ld32(acc + cc * 32, v);
+                else tmem_ld16(acc + cc * 16, v);
                 tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < kCols / 8; ++i) {
                     uint32_t p4[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
-                    *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
+                    *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * (kCols / 8) + i) ^ (lane & 7)) << 4)) =
                         make_uint4(p4[0], p4[1], p4[2], p4[3]);
                     if constexpr (FLAG) {
 #pragma unroll
@@ -648,7 +673,7 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-                tma_store_3d(&tm_delta, sbase + stg_off, (row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
+                tma_store_3d(&tm_delta, sbase + stg_off, (tile_row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
                 bulk_commit_group();
                 bulk_wait_group_read0();      // the engine has read the staging tile: it may be written again
             }
@@ -656,6 +681,8 @@ __global__ void __launch_bounds__(256, FEW ? 4 : 3) quant_k_delta_kernel(
         }
         tc_fence_before();
         __syncthreads();      // the accumulator and the A tile are free again
+    }
+    if (!more || !alive) break;
     }
     tc_fence_before();
     __syncthreads();
@@ -887,17 +914,18 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     // tensor maps for the K kernel: the Q means and delta_s of a kv head's query heads follow one another, so both are byte
     // tensors [B*Hkv][group * nqm][...] and one MMA takes the blocks of several heads
     const uint64_t rows = (uint64_t)(a.Hq / a.Hkv) * a.nqm;
-    const bool few = rows <= 64;
-    const int a_rows = few ? 64 : 128;
-    const size_t smem_k = (D / 64) * (128 + a_rows) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + a_rows * 256 : 0);
+    const bool few = rows <= 64, in_turn = rows <= 8 && (int64_t)tiles_k * BHkv >= tiles_in_turn_from(D);
+    const int a_rows = in_turn ? 32 : few ? 64 : 128;
+    const size_t smem_k = (D / 64) * (128 + a_rows) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 || in_turn ? 1024 + a_rows * 256 : 0);
     alignas(64) CUtensorMap tm_qm, tm_delta;
-    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, few ? 64 : 128, 3) != 0 ||
+    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, a_rows, 3) != 0 ||
         encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    auto kern = a.nonfinite != nullptr ? (few ? quant_k_delta_kernel<T, D, true, true> : quant_k_delta_kernel<T, D, false, true>)
-                                       : (few ? quant_k_delta_kernel<T, D, true, false> : quant_k_delta_kernel<T, D, false, false>);
+    auto kern = a.nonfinite != nullptr
+                    ? (in_turn ? quant_k_delta_kernel<T, D, 32, true> : few ? quant_k_delta_kernel<T, D, 64, true> : quant_k_delta_kernel<T, D, 128, true>)
+                    : (in_turn ? quant_k_delta_kernel<T, D, 32, false> : few ? quant_k_delta_kernel<T, D, 64, false> : quant_k_delta_kernel<T, D, 128, false>);
     if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
-    return launch(true, kern, dim3(a.Nk_p / kBlock, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
+    return launch(true, kern, dim3(in_turn ? (tiles_k + tiles_in_turn(D) - 1) / tiles_in_turn(D) : tiles_k, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
                       a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status,
                       a.nonfinite, tm_qm, tm_delta);
 }

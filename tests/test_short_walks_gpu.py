@@ -45,3 +45,22 @@ def test_halves_rolled_and_unrolled_at_64_channels(cuda_device, Nk, causal):
     cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (Nq, Nk))
     packed = sageattn_varlen(*(x[0].transpose(0, 1).contiguous() for x in (q, k, v)), cu_q, cu_k, Nq, Nk, is_causal=causal)
     assert torch.equal(sageattn3(q, k, v, is_causal=causal)[0].transpose(0, 1), packed)
+
+
+@pytest.mark.parametrize("D,tiles,kv_heads", [(128, 101, 40), (128, 100, 40), (64, 76, 40), (64, 77, 40), (64, 78, 40)])
+def test_key_tiles_in_turn(cuda_device, D, tiles, kv_heads):
+    """Few query blocks and many key tiles: a block of the K kernel takes two (D = 64: three) tiles one after the other.  Numbers of tiles that it
+    divides and does not, a ragged last tile: the same bits as with two kv heads, where every tile has a block of its own.  One head
+    has a key that is not finite in a block's second tile: it stays there."""
+    g = torch.Generator(device=cuda_device).manual_seed(1500 + tiles)
+    Nk, group = tiles * 128 - 5, 4
+    k, v = (torch.randn(1, kv_heads, Nk, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
+    q = torch.randn(1, kv_heads * group, 1, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+    for bad in (False, True):
+        if bad:
+            k[0, 5, 130] = float("nan")
+        out = sageattn3(q, k, v, is_causal=True)
+        for h in (0, 5, kv_heads - 2):
+            few = sageattn3(q[:, h * group:(h + 2) * group], k[:, h:h + 2], v[:, h:h + 2], is_causal=True)
+            assert torch.equal(out[:, h * group:(h + 2) * group].nan_to_num(7.0), few.nan_to_num(7.0)), (h, bad)
+        assert torch.isfinite(out[:, 6 * group:]).all() and torch.isfinite(out[:, :5 * group]).all()
