@@ -582,6 +582,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // V is loaded kLag blocks behind K.  A V stage is free four blocks after its K stage (scores, softmax and P lie between), and
         // with as few stages as D = 128 has room for, the K that the issuers want next would otherwise queue behind a V that
         // nobody is waiting for yet: they waited 740 cycles for every second item.
+        // What is held back must not keep the producer itself waiting: a ring entry is free when the unit four before it is finished, which
+        // takes all of that unit's V.  Behind units with keys every block loaded brings a V in; an empty unit and the end marker load
+        // nothing, so ahead of publishing one of these all V that is pending is loaded.
         constexpr int kLag = PACK == 2 || D == 64 ? 0 : 2;
         int vst = 0, vst_parity = 1, pend = 0;    // V stage; blocks whose V is still to be loaded: key block, kv head, oldest first
         int pend_n[2], pend_kv[2];
@@ -617,19 +620,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 if (last_head) u = uniform(next);
                 head = last_head ? 0 : head + 1;
             };
+            if constexpr (kLag == 2) {
+                if (w.ns <= 0) {
+                    for (; ok && pend > 0; --pend) ok = next_v(pend == 2 ? pend_n[0] : pend_n[1], pend == 2 ? pend_kv[0] : pend_kv[1]);
+                    if (!ok) break;
+                }
+            }
             if (!warp_wait<true>(bar(bWE + k % kUnitRing), ((k / kUnitRing) & 1) ^ 1, abort_flag, p.status, kWaitUnit)) break;
             if (lane == 0) {
                 *reinterpret_cast<Unit*>(sgen + C::oUnit + (k % kUnitRing) * 64) = w;
                 mbar_arrive(bar(bWF + k % kUnitRing));
             }
             ++k;
-            if (!more) {
-                if constexpr (kLag == 2) {
-                    for (int q = 2 - pend; q < 2; ++q)
-                        if (!next_v(q == 0 ? pend_n[0] : pend_n[1], q == 0 ? pend_kv[0] : pend_kv[1])) break;
-                }
-                break;
-            }
+            if (!more) break;
             if (w.ns == 0) { advance(); continue; }
             const int qb = kq & 1;                // Q buffer
             if (!warp_wait<true>(bar(bQE + qb), ((kq >> 1) & 1) ^ 1, abort_flag, p.status, kWaitKEmpty)) break;

@@ -91,6 +91,7 @@ def _carry(o_in=None, m_in=None, l_in=None, o_out=None, m_out=None, l_out=None, 
     (1, 2, 2, 384, [0, 256, 640, 1000], 128, False),       # three key ranges, the last one ragged
     (2, 4, 2, 300, [0, 128, 300], 64, True),               # causal, GQA, Nq == Nk
     (1, 2, 1, 200, [0, 384, 768], 128, True),              # causal, Nk > Nq (bottom-right aligned)
+    (1, 95, 95, 2048, [0, 1792, 2048], 128, True),         # the last range is hidden from seven eighths of the queries: units without keys
 ])
 def test_key_ranges_with_carried_state_equal_one_call(cuda_device, B, Hq, Hkv, Nq, cuts, D, causal):
     """One attention computed as several calls over consecutive key ranges, walked from the last range to the first

@@ -2,11 +2,13 @@
 barrier phases run on from unit to unit; and the number of key blocks at which D = 64 without a mask changes kernels.  A head's result
 depends on its own q, k, v alone, so every comparison is for equal bits; against the oracle the gate is the one of the whole path
 (cosine >= 0.999, relative L1 <= 1 %)."""
+import ctypes as C
+
 import pytest
 import torch
 
 from oracle import sage3_oracle as O
-from sageattention_b200 import sageattn3, sageattn_varlen
+from sageattention_b200 import Sage3Problem, _cabi, sageattn3, sageattn_varlen
 
 pytestmark = pytest.mark.gpu
 
@@ -20,8 +22,8 @@ def _inputs(device, B, H, Nq, Nk, D, seed):
 @pytest.mark.parametrize("Nq,Nk,causal", [(130, 1, False), (1, 128, False), (130, 129, False), (257, 300, False), (130, 650, False),
                                           (130, 130, True), (300, 300, True), (257, 100, True), (640, 640, True)])
 def test_units_of_few_key_blocks(cuda_device, D, Nq, Nk, causal):
-    """Some five units per SM, single tiles and pairs, of one to five key blocks (causal: none to five, the tiles of a pair with
-    different numbers): the same bits as the heads alone, where each is the first unit of its SM."""
+    """Some five units per SM, single tiles and pairs, of one to five key blocks (causal: the tiles of a pair with different numbers, one of them
+    none, but no unit without any): the same bits as the heads alone, where each is the first unit of its SM."""
     sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
     pairs = (Nq + 255) // 256
     H = 5 * sms // pairs + 3
@@ -33,6 +35,58 @@ def test_units_of_few_key_blocks(cuda_device, D, Nq, Nk, causal):
     h = H // 2
     ref = O.sageattn3_oracle(q[:, h:h + 1].cpu(), k[:, h:h + 1].cpu(), v[:, h:h + 1].cpu(), is_causal=causal)
     assert O.cosine(out[:, h:h + 1].cpu(), ref) >= 0.999 and O.rel_l1(out[:, h:h + 1].cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Nq,Nk", [(2048, 512), (1000, 100), (1300, 640)])
+def test_units_without_keys(cuda_device, D, Nq, Nk):
+    """Causal, more queries than keys: most units have no keys, and an SM draws three and more of them behind its full ones.  No wait gives up,
+    every row is written, those without keys with zeros, and the bits are those of the heads alone."""
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    H = 5 * sms // ((Nq + 255) // 256) + 3
+    q, k, v = _inputs(cuda_device, 1, H, Nq, Nk, D, seed=1350 + Nq)
+    prob = Sage3Problem(q, k, v, is_causal=True, return_lse=True, out=torch.full_like(q, float("nan")))
+    prob.lse.fill_(float("nan"))
+    out, lse = prob.run(), prob.lse
+    assert prob.check_status() == 0
+    blind = Nq - Nk                                # the first rows
+    assert (out[:, :, :blind] == 0).all() and (lse[:, :, :blind] == float("-inf")).all() and torch.isfinite(lse[:, :, blind:]).all()
+    for h in sorted({0, 1, H // 3, H // 2, H - 2, H - 1}):
+        one, one_lse = sageattn3(q[:, h:h + 1], k[:, h:h + 1], v[:, h:h + 1], is_causal=True, return_lse=True)
+        assert torch.equal(out[:, h:h + 1], one) and torch.equal(lse[:, h:h + 1], one_lse), f"head {h} of {H}"
+    h = H // 2
+    ref = O.sageattn3_oracle(q[:, h:h + 1].cpu(), k[:, h:h + 1].cpu(), v[:, h:h + 1].cpu(), is_causal=True)
+    assert O.cosine(out[:, h:h + 1].cpu(), ref) >= 0.999 and O.rel_l1(out[:, h:h + 1].cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+def test_packed_batch_of_mostly_empty_sequences(cuda_device, D, causal):
+    """Sequences without keys, ten or eleven in a row between two that have some (causal: one of these with more queries than keys): several units without
+    keys in a row on every SM, between units with keys.  No wait gives up, and every sequence is as it is alone."""
+    B, H, Nq = 40, 24, 300
+    lens_k = [0] * B
+    for i in range(0, B, 13):
+        lens_k[i], lens_k[i + (1 if i < 39 else -1)] = 300 + i, 100
+    g = torch.Generator(device=cuda_device).manual_seed(1370)
+    q = torch.randn(B * Nq, H, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+    k, v = (torch.randn(sum(lens_k), H, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
+    cu_q = torch.arange(B + 1, dtype=torch.int32, device=cuda_device) * Nq
+    cu_k = torch.tensor([0] + lens_k).cumsum(0).to(device=cuda_device, dtype=torch.int32)
+    prob = Sage3Problem.for_shape(B, H, H, Nq, max(lens_k), D, torch.bfloat16, cuda_device, is_causal=causal, q_stride=(0, D, H * D), k_stride=(0, D, H * D))
+    out = torch.full_like(q, float("nan"))
+    rc = _cabi.lib().sage3_fwd_varlen(C.byref(prob.desc), *(t.data_ptr() for t in (cu_q, cu_k, q, k, v, out)), None, prob.ws.buf.data_ptr(),
+                                      torch.cuda.current_stream(cuda_device).cuda_stream)
+    assert rc == 0 and prob.check_status() == 0
+    k0 = 0
+    for i, n in enumerate(lens_k):
+        mine = out[i * Nq:(i + 1) * Nq]
+        if n == 0:
+            assert (mine == 0).all(), i
+        else:
+            alone = sageattn3(q[None, i * Nq:(i + 1) * Nq], k[None, k0:k0 + n], v[None, k0:k0 + n], tensor_layout="NHD", is_causal=causal)[0]
+            assert torch.equal(mine, alone), i
+        k0 += n
 
 
 @pytest.mark.parametrize("causal", [False, True])
