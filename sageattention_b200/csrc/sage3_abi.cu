@@ -33,29 +33,6 @@ cudaError_t current_device(int* dev, DeviceInfo* info) {
     return cudaSuccess;
 }
 
-cudaError_t allow_smem(const void* kernel, int bytes) {
-    struct Entry { const void* kernel; uint64_t devices; };
-    static Entry done[64];                            // one per kernel instantiation (52 exist)
-    static std::mutex mutex;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mutex);
-    Entry* slot = nullptr;
-    for (Entry& d : done)
-        if (d.kernel == kernel || d.kernel == nullptr) {
-            slot = &d;
-            break;
-        }
-    if (slot && dev < kMaxDevices && (slot->devices >> dev & 1)) return cudaSuccess;
-    e = checked(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (e == cudaSuccess && slot && dev < kMaxDevices) {
-        slot->kernel = kernel;
-        slot->devices |= 1ull << dev;
-    }
-    return e;
-}
-
 }  // namespace sage3
 
 namespace {

@@ -1164,9 +1164,9 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
 template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK, bool CARRY = false, bool ROLL = true>
 static cudaError_t launch_v(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int grid, cudaStream_t st) {
-    auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK, CARRY, ROLL>;
+    constexpr auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK, CARRY, ROLL>;
     using C = Cfg<D, PACK>;
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), C::kSmemBytes);
+    cudaError_t e = allow_smem<kern>(C::kSmemBytes);
     if (e != cudaSuccess) return e;
     return launch(true, kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, p);
 }

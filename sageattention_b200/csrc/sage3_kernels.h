@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace sage3 {
 
 constexpr int kRowsPerChunk = 512;   // rows per partial column sum (fixes the summation order)
@@ -77,13 +79,25 @@ struct PackRule {
 struct DeviceInfo { int sms; bool ok; };
 cudaError_t current_device(int* dev, DeviceInfo* info);
 
-// Dynamic shared memory of a kernel beyond 48 KB (set once per kernel and device).
-cudaError_t allow_smem(const void* kernel, int bytes);
-
 // Result of a runtime call, an error taken off the thread's record: the caller gets it as a return code, and whoever asks the runtime
 // next must not find it.
 inline cudaError_t checked(cudaError_t e) {
     if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
+// Dynamic shared memory of a kernel beyond 48 KB: set once per kernel and device, which every kernel remembers for itself (the call into
+// the runtime would come on top of every launch).
+template <auto Kernel>
+cudaError_t allow_smem(int bytes) {
+    static std::atomic<uint64_t> devices{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (devices.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = checked(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
     return e;
 }
 

@@ -10,6 +10,7 @@
 //   quantization/fp4_quantization_4d.cu:300-349   V: microblocks are 16 consecutive tokens of one channel
 // Quotients and reciprocals are those of IEEE arithmetic (see micro_scale), so the result can be checked bit for bit.
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/sage3_b200.h"
 #include <cuda.h>
@@ -858,7 +859,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     T* qm = static_cast<T*>(a.qm);
     T* delta = static_cast<T*>(a.delta);
     const int BHq = a.B * a.Hq, BHkv = a.B * a.Hkv;
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(prepass_stage_kernel<T, D>), StageCfg<T, D>::kSmem);
+    cudaError_t e = allow_smem<prepass_stage_kernel<T, D>>(StageCfg<T, D>::kSmem);
     if (e != cudaSuccess) return e;
 
     StageArgs<T> s = {};
@@ -921,13 +922,20 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, a_rows, 3) != 0 ||
         encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
         return cudaErrorInvalidValue;
-    auto kern = a.nonfinite != nullptr
-                    ? (in_turn ? quant_k_delta_kernel<T, D, 32, true> : few ? quant_k_delta_kernel<T, D, 64, true> : quant_k_delta_kernel<T, D, 128, true>)
-                    : (in_turn ? quant_k_delta_kernel<T, D, 32, false> : few ? quant_k_delta_kernel<T, D, 64, false> : quant_k_delta_kernel<T, D, 128, false>);
-    if ((e = allow_smem(reinterpret_cast<const void*>(kern), (int)smem_k)) != cudaSuccess) return e;
-    return launch(true, kern, dim3(in_turn ? (tiles_k + tiles_in_turn(D) - 1) / tiles_in_turn(D) : tiles_k, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2], s.Hkv, a.Nk,
-                      a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows, a.status,
-                      a.nonfinite, tm_qm, tm_delta);
+    auto k_kernel = [&](auto a_rows_, auto flag_) {
+        constexpr auto kern = quant_k_delta_kernel<T, D, decltype(a_rows_)::value, decltype(flag_)::value>;
+        const cudaError_t allowed = allow_smem<kern>((int)smem_k);
+        if (allowed != cudaSuccess) return allowed;
+        return launch(true, kern, dim3(in_turn ? (tiles_k + tiles_in_turn(D) - 1) / tiles_in_turn(D) : tiles_k, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2],
+                      s.Hkv, a.Nk, a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows,
+                      a.status, a.nonfinite, tm_qm, tm_delta);
+    };
+    auto by_rows = [&](auto flag_) {
+        return in_turn ? k_kernel(std::integral_constant<int, 32>(), flag_)
+               : few   ? k_kernel(std::integral_constant<int, 64>(), flag_)
+                       : k_kernel(std::integral_constant<int, 128>(), flag_);
+    };
+    return a.nonfinite != nullptr ? by_rows(std::true_type()) : by_rows(std::false_type());
 }
 
 cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t st) {

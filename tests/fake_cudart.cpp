@@ -13,6 +13,7 @@ std::mutex g_mutex;
 std::map<const void*, std::string>* g_names;      // host stub -> device function
 std::string g_log;                                // one "thread:kernel" line per piece of work
 int g_refuse = -1, g_count = 0, g_pause_us = 0;
+std::atomic<int> g_attributes{0};                 // kernel attributes set
 std::atomic<int> g_threads{0};
 thread_local int t_id = -1;
 thread_local cudaError_t t_last = cudaSuccess;
@@ -47,9 +48,11 @@ void fake_start(int refuse, int pause_us) {
     g_refuse = refuse;
     g_pause_us = pause_us;
     g_count = 0;
+    g_attributes = 0;
 }
 const char* fake_log() { return g_log.c_str(); }
 int fake_last_error() { return t_last; }
+int fake_attributes() { return g_attributes; }
 
 void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
 void __cudaRegisterFatBinaryEnd(void**) {}
@@ -77,7 +80,7 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrComputeCapabilityMajor ? 10 : 0;
     return cudaSuccess;
 }
-cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { ++g_attributes; return cudaSuccess; }
 cudaError_t cudaGetDriverEntryPoint(const char*, void** f, unsigned long long, cudaDriverEntryPointQueryResult* r) {
     *f = reinterpret_cast<void*>(fake_encode);
     if (r) *r = cudaDriverEntryPointSuccess;

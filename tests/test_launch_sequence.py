@@ -99,6 +99,30 @@ def test_a_refused_launch_is_reported_and_ends_the_call(fake, call, kw, lse):
         assert fake.fake_last_error() == 0, i
 
 
+def test_shared_memory_is_asked_for_once_per_kernel(fake):
+    """Calls that between them launch every attention and every K kernel: in a second round no kernel's attributes are set again (that is a call into the
+    runtime for every launch, paid by the shortest calls)."""
+    p, carry = C.c_void_p, _cabi.Sage3Carry()
+    carry.o_out, carry.m_out, carry.l_out = (1 << 20,) * 3
+
+    def carried(lib, d):
+        return lib.sage3_attn_fwd_carry(C.byref(d), p(WS), C.byref(carry), None, None, None)
+    full = [dict(Nk=700), dict(Nk=3000), dict(Nq=128 * 33)]                                # whole tiles; many query blocks
+    few = [dict(Nq=16, Hq=16), dict(Nq=1, Hq=8), dict(Nq=1, Hq=66, Hkv=1),                 # heads that share a tile, of 8, 4 and 66 query blocks
+           dict(B=8, Nq=1, Hq=32, Hkv=8, Nk=20000), dict(B=8, Nq=1, Hq=8, Hkv=8, Nk=20000)]      # many key tiles
+    kernels = set()
+    for _ in range(2):
+        fake.fake_start(-1, 0)
+        for dtype in (_cabi.SAGE3_BF16, _cabi.SAGE3_FP16):
+            for D in (64, 128):
+                for causal in (0, 1):
+                    kw = dict(dtype=dtype, D=D, is_causal=causal)
+                    assert [_fwd(fake, _desc(**kw, **c)) for c in full + few] == [0] * (len(full) + len(few))
+                    assert [f(fake, _desc(**kw, Nk=n)) for f in (_varlen, carried) for n in (700, 3000, 9000)] == [0] * 6
+        kernels |= {entry[1] for entry in _log(fake) if "attn_fwd" in entry[1] or "quant_k_delta" in entry[1]}
+    assert len(kernels) >= 66 and fake.fake_attributes() == 0
+
+
 def test_a_launch_of_too_many_blocks_is_refused():
     """All pieces of the first pre-pass kernel are one grid: their number, not that of one kind, has to stay below 2^31."""
     d = _desc(B=60000, Hq=1, Hkv=1, Nq=128, Nk=6000000)       # 2.8e9 tiles of V
