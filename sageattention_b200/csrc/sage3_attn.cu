@@ -1174,19 +1174,24 @@ static cudaError_t launch_v(const CUtensorMap& tq, const CUtensorMap& tk, const 
 // D = 64 without a mask, more key blocks than this: the halves of an item unrolled.  us per call, rolled / unrolled: 226 keys (2 x 48 heads,
 // 17 550 queries) 245.5 / 282.2, 512 (4 x 24 x 2 000) 60.8 / 62.4, 1 024 98.6 / 98.8, 2 048 (2 x 24 x 2 048) 100.3 / 98.7, 4 250 356.3 / 351.1, 16 384
 // (2 x 32 heads) 5 542 / 5 441.  Under a causal mask rolled is faster throughout (1 024: 45.3 / 47.4, 6 000: 328.4 / 335.1), as it is at D = 128.
-constexpr int kRolledBlocks = 8;
+// Packed batches hold sequences shorter than the longest, which is what the host knows: 24 heads, 24 sequences of 300 to 2 048 tokens 522.8 / 545.1,
+// of 400 to 3 072 948.7 / 973.6, of 500 to 4 096 1 620 / 1 641, 12 of 1 000 to 8 192 3 597 / 3 556; of one length, 8 x 3 072 684.5 / 678.1,
+// 8 x 4 096 1 150 / 1 137, 8 x 6 144 2 464 / 2 424, 4 x 16 384 (12 heads) 4 161 / 4 089.
+constexpr int kRolledBlocks = 8, kRolledBlocksPacked = 32;
 
 template <int D, bool CAUSAL, typename OutT>
 static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
                             const AttnParams& p, int pack_mode, int grid, cudaStream_t st) {
     // packed variable-length batches and carried state run their own instantiations, so that the other kernels carry none of it
     const bool carry = a.carry_o_in != nullptr || a.carry_o_out != nullptr;
-    return a.cu_q != nullptr  ? launch_v<D, CAUSAL, OutT, true, 0>(tq, tk, tv, td, p, grid, st)
+    constexpr bool roll = D == 128 || CAUSAL;        // at every length
+    return a.cu_q != nullptr && !roll && p.nkb > kRolledBlocksPacked ? launch_v<D, CAUSAL, OutT, true, 0, false, roll>(tq, tk, tv, td, p, grid, st)
+           : a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true, 0>(tq, tk, tv, td, p, grid, st)
            : carry            ? launch_v<D, CAUSAL, OutT, false, 0, true>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(tq, tk, tv, td, p, grid, st)
-           : D == 64 && !CAUSAL && p.nkb > kRolledBlocks ? launch_v<D, CAUSAL, OutT, false, 0, false, D == 128 || CAUSAL>(tq, tk, tv, td, p, grid, st)
-                                              : launch_v<D, CAUSAL, OutT, false, 0>(tq, tk, tv, td, p, grid, st);
+           : !roll && p.nkb > kRolledBlocks ? launch_v<D, CAUSAL, OutT, false, 0, false, roll>(tq, tk, tv, td, p, grid, st)
+                              : launch_v<D, CAUSAL, OutT, false, 0>(tq, tk, tv, td, p, grid, st);
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {

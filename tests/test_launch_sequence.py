@@ -123,6 +123,16 @@ def test_shared_memory_is_asked_for_once_per_kernel(fake):
     assert len(kernels) >= 66 and fake.fake_attributes() == 0
 
 
+@pytest.mark.parametrize("call,Nk,causal,D,rolled", [(_fwd, 1024, 0, 64, 1), (_fwd, 1025, 0, 64, 0), (_fwd, 9000, 1, 64, 1), (_fwd, 9000, 0, 128, 1),
+                                                     (_varlen, 4096, 0, 64, 1), (_varlen, 4097, 0, 64, 0), (_varlen, 9000, 1, 64, 1), (_varlen, 9000, 0, 128, 1)])
+def test_halves_are_unrolled_where_that_is_faster(fake, call, Nk, causal, D, rolled):
+    """The attention kernel's last template argument: its halves rolled, except at 64 channels without a mask over many key blocks."""
+    fake.fake_start(-1, 0)
+    assert call(fake, _desc(Nk=Nk, Nq=Nk, is_causal=causal, D=D)) == 0
+    name = [entry[1] for entry in _log(fake) if "attn_fwd" in entry[1]][0]
+    assert f"ELb{rolled}EEEv" in name, name
+
+
 def test_a_launch_of_too_many_blocks_is_refused():
     """All pieces of the first pre-pass kernel are one grid: their number, not that of one kind, has to stay below 2^31."""
     d = _desc(B=60000, Hq=1, Hkv=1, Nq=128, Nk=6000000)       # 2.8e9 tiles of V

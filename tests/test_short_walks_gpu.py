@@ -93,12 +93,27 @@ def test_packed_batch_of_mostly_empty_sequences(cuda_device, D, causal):
 @pytest.mark.parametrize("Nk", [1023, 1024, 1025, 1152, 2049])
 def test_halves_rolled_and_unrolled_at_64_channels(cuda_device, Nk, causal):
     """Beyond eight key blocks the uniform kernel without a mask has the halves of an item unrolled; the packed variable-length kernel
-    has them rolled at every length: the same bits."""
+    has them rolled up to 32: the same bits."""
     H, Nq = 5, 300
     q, k, v = _inputs(cuda_device, 1, H, Nq, Nk, 64, seed=1400 + Nk)
     cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device=cuda_device) for n in (Nq, Nk))
     packed = sageattn_varlen(*(x[0].transpose(0, 1).contiguous() for x in (q, k, v)), cu_q, cu_k, Nq, Nk, is_causal=causal)
     assert torch.equal(sageattn3(q, k, v, is_causal=causal)[0].transpose(0, 1), packed)
+
+
+@pytest.mark.parametrize("longest", [4096, 4097])
+def test_packed_batch_around_the_length_that_unrolls(cuda_device, longest):
+    """A packed batch at 64 channels without a mask is walked unrolled, its short sequences too, when the longest has more than 32 key blocks: the
+    bits of the sequences alone, some of which are walked the other way."""
+    H, lens = 3, [200, longest, 1, 1100]
+    g = torch.Generator(device=cuda_device).manual_seed(longest)
+    q, k, v = (torch.randn(sum(lens), H, 64, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(3))
+    out = sageattn_varlen(q, k, v, *(torch.tensor([0] + lens).cumsum(0).to(device=cuda_device, dtype=torch.int32),) * 2, longest, longest)
+    r0 = 0
+    for n in lens:
+        alone = sageattn3(*(x[None, r0:r0 + n] for x in (q, k, v)), tensor_layout="NHD")[0]
+        assert torch.equal(out[r0:r0 + n], alone), n
+        r0 += n
 
 
 @pytest.mark.parametrize("D,tiles,kv_heads", [(128, 101, 40), (128, 100, 40), (64, 76, 40), (64, 77, 40), (64, 78, 40)])
