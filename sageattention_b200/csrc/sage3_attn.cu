@@ -348,6 +348,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     constexpr int kCorrRegs = PACK == 2 || !ROLL ? 48 : 64;
     static_assert(128 * (kRoleRegs + kCorrRegs + C::kGroups * kSoftRegs) <= C::kThreads * 80, "registers");
     constexpr int kRescaleUnroll = D == 128 ? 2 : 8;
+    // Carried state, us per three ranges attended (16 heads, 8 192 queries, ranges of 8 192 keys; D = 128 without / with a mask, D = 64 likewise): halves rolled, one
+    // wait per item, row sums in registers 1 134, 676, 1 061, 603.  Sums in shared memory and, at D = 128, the halves unrolled 1 129, 660; at D = 64 rolled, the
+    // factor waited for ahead of P and the output loop unrolled 1 048, 594.  Across: D = 128 rolled with the rest 1 130, 672, D = 64 unrolled 1 057, 610.
+    constexpr bool kFactorFirst = CARRY && ROLL;
     // A CTA runs unit after unit (the grid is one CTA per SM): the producer draws the next unit's number from a counter and
     // publishes the unit in shared memory, so the loads, scores and exponentials of the next unit fill in while the last one
     // drains, and uneven units (causal masks, packed batches) level out.
@@ -438,19 +442,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               l_s[0] = l;
               m_s[0] = m;
           }
-          float2 l0 = make_float2(0.f, 0.f), l1 = l0;              // running row sums of the two tiles
-          if (carry_in) {
-              l0 = l_s[0];
-              l1 = l_s[128];
-          }
+          float2 l0 = make_float2(0.f, 0.f), l1 = l0;              // running row sums of the two tiles (carried state: in l_s)
           for (int s = 0; PACK != 2 && s < ns; ++s) {
               const int sg = base + s, slot = sg & 7, ph = (sg >> 3) & 1;
               const int t = (s + d) & two;
               const bool first = s <= two;                            // the tile's first block
-              // One wait per item: P, its scales, the row sums and the factor are all written.  (A wait for the factor first, so that the rescale
+              // One wait per item: P, its scales, the row sums and the factor are all written.  (kFactorFirst elsewhere, a wait for the factor first, so that the rescale
               // runs under the rest of the softmax: 226 keys 255 instead of 248 us, 300 keys at D = 128 202 instead of 198.)
-              if (!warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
-              const float2 rs = sum[slot * 128];
+              if (kFactorFirst && !warp_wait(bar(bM + slot * 4 + quarter), ph, abort_flag, p.status, kWaitAlpha)) { ok = false; break; }
+              if (!kFactorFirst && !warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
+              float2 rs = make_float2(0.f, 0.f);
+              if (!kFactorFirst) rs = sum[slot * 128];
               const float2 ma = stat[slot * 128];
               const float alpha = ma.y;
               // the first block has nothing to rescale unless the accumulator was carried in
@@ -477,14 +479,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               }
               tc_fence_before();
               // P V issue waits for this warpgroup only, so its arrival also stands for "P is written"
+              if (kFactorFirst) {
+                  if (!warp_wait(bar(bPF + slot), ph, abort_flag, p.status, kWaitPFull)) { ok = false; break; }
+                  rs = sum[slot * 128];
+              }
               warp_arrive(bar(bOS + slot), lane);
-              float2 l = t ? l1 : l0;
+              float2 l = CARRY ? l_s[t * 128] : t ? l1 : l0;
               l.x = fmaf(l.x, alpha, rs.x);
               l.y = fmaf(l.y, alpha, rs.y);
-              if (t) l1 = l; else l0 = l;
+              if (CARRY) l_s[t * 128] = l; else if (t) l1 = l; else l0 = l;
               m_s[t * 128] = ma.x;
           }
-          if (PACK != 2) {
+          if (PACK != 2 && !CARRY) {
               l_s[0] = l0;
               l_s[128] = l1;
           }
@@ -530,7 +536,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               // warps, so what is behind the wait costs several cycles an instruction (300 keys at D = 128 191.9 -> 190.7 us, packed prompts
               // 610.3 -> 607.6, 226 keys 247.6 -> 246.1).  Its stores cost nothing that shows, wider loads did not help.
               const uint64_t inv2 = pack2f(inv_l, inv_l);
-#pragma unroll (PACK == 2 ? 8 : 1)
+#pragma unroll (kFactorFirst ? D / 16 : PACK == 2 ? 8 : 1)
               for (int c = 0; c < D; c += 16) {
                   float o[16];
                   if (have) {
@@ -1187,7 +1193,7 @@ static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUte
     constexpr bool roll = D == 128 || CAUSAL;        // at every length
     return a.cu_q != nullptr && !roll && p.nkb > kRolledBlocksPacked ? launch_v<D, CAUSAL, OutT, true, 0, false, roll>(tq, tk, tv, td, p, grid, st)
            : a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true, 0>(tq, tk, tv, td, p, grid, st)
-           : carry            ? launch_v<D, CAUSAL, OutT, false, 0, true>(tq, tk, tv, td, p, grid, st)
+           : carry            ? launch_v<D, CAUSAL, OutT, false, 0, true, D == 64>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(tq, tk, tv, td, p, grid, st)
            : !roll && p.nkb > kRolledBlocks ? launch_v<D, CAUSAL, OutT, false, 0, false, roll>(tq, tk, tv, td, p, grid, st)

@@ -53,6 +53,12 @@ def _varlen(lib, d, ws=WS, lse=None):
     return lib.sage3_fwd_varlen(C.byref(d), p(1 << 10), p(1 << 11), p(1 << 12), p(1 << 13), p(1 << 14), p(1 << 15), p(lse), p(ws), None)
 
 
+def _carried(lib, d):
+    p, carry = C.c_void_p, _cabi.Sage3Carry()
+    carry.o_out, carry.m_out, carry.l_out = (1 << 20,) * 3
+    return lib.sage3_attn_fwd_carry(C.byref(d), p(WS), C.byref(carry), None, None, None)
+
+
 def _log(lib):
     return [line.split(":") for line in lib.fake_log().decode().splitlines()]
 
@@ -102,11 +108,6 @@ def test_a_refused_launch_is_reported_and_ends_the_call(fake, call, kw, lse):
 def test_shared_memory_is_asked_for_once_per_kernel(fake):
     """Calls that between them launch every attention and every K kernel: in a second round no kernel's attributes are set again (that is a call into the
     runtime for every launch, paid by the shortest calls)."""
-    p, carry = C.c_void_p, _cabi.Sage3Carry()
-    carry.o_out, carry.m_out, carry.l_out = (1 << 20,) * 3
-
-    def carried(lib, d):
-        return lib.sage3_attn_fwd_carry(C.byref(d), p(WS), C.byref(carry), None, None, None)
     full = [dict(Nk=700), dict(Nk=3000), dict(Nq=128 * 33)]                                # whole tiles; many query blocks
     few = [dict(Nq=16, Hq=16), dict(Nq=1, Hq=8), dict(Nq=1, Hq=66, Hkv=1),                 # heads that share a tile, of 8, 4 and 66 query blocks
            dict(B=8, Nq=1, Hq=32, Hkv=8, Nk=20000), dict(B=8, Nq=1, Hq=8, Hkv=8, Nk=20000)]      # many key tiles
@@ -118,15 +119,17 @@ def test_shared_memory_is_asked_for_once_per_kernel(fake):
                 for causal in (0, 1):
                     kw = dict(dtype=dtype, D=D, is_causal=causal)
                     assert [_fwd(fake, _desc(**kw, **c)) for c in full + few] == [0] * (len(full) + len(few))
-                    assert [f(fake, _desc(**kw, Nk=n)) for f in (_varlen, carried) for n in (700, 3000, 9000)] == [0] * 6
+                    assert [f(fake, _desc(**kw, Nk=n)) for f in (_varlen, _carried) for n in (700, 3000, 9000)] == [0] * 6
         kernels |= {entry[1] for entry in _log(fake) if "attn_fwd" in entry[1] or "quant_k_delta" in entry[1]}
     assert len(kernels) >= 66 and fake.fake_attributes() == 0
 
 
 @pytest.mark.parametrize("call,Nk,causal,D,rolled", [(_fwd, 1024, 0, 64, 1), (_fwd, 1025, 0, 64, 0), (_fwd, 9000, 1, 64, 1), (_fwd, 9000, 0, 128, 1),
-                                                     (_varlen, 4096, 0, 64, 1), (_varlen, 4097, 0, 64, 0), (_varlen, 9000, 1, 64, 1), (_varlen, 9000, 0, 128, 1)])
+                                                     (_varlen, 4096, 0, 64, 1), (_varlen, 4097, 0, 64, 0), (_varlen, 9000, 1, 64, 1), (_varlen, 9000, 0, 128, 1),
+                                                     (_carried, 700, 0, 128, 0), (_carried, 9000, 1, 128, 0), (_carried, 700, 1, 64, 1), (_carried, 9000, 0, 64, 1)])
 def test_halves_are_unrolled_where_that_is_faster(fake, call, Nk, causal, D, rolled):
-    """The attention kernel's last template argument: its halves rolled, except at 64 channels without a mask over many key blocks."""
+    """The attention kernel's last template argument: its halves rolled, except at 64 channels without a mask over many key blocks, and with
+    carried state at 128 channels."""
     fake.fake_start(-1, 0)
     assert call(fake, _desc(Nk=Nk, Nq=Nk, is_causal=causal, D=D)) == 0
     name = [entry[1] for entry in _log(fake) if "attn_fwd" in entry[1]][0]
