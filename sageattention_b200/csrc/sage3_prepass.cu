@@ -466,17 +466,19 @@ __device__ __forceinline__ void quant_q_tile(
 // AROWS = 64: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
 // looks at), which makes room for a fourth block per SM:
 // 1 000 queries of 32 heads against 9 192 keys 143.9 -> 141.9 us per call, 4 250 tokens of 48 heads 359.0 -> 356.9 us.
-// AROWS = 32: up to eight query blocks and many tiles (token generation).  A block takes two (D = 64: three) tiles one after the other: its tensor
-// memory, mean and A tile are set up once, and the next tile's rows come in under this one's MMAs and read-out, which takes 80
-// registers at D = 128 (three blocks per SM; with four, spilled rows: 137.4 -> 147.1).  us per call, before / after: one token of 8 x 32 heads
-// against 8 192 keys of 8 kv heads 137.2 / 134.2 (D = 64 89.4 / 87.7), of 32 kv heads 464 / 432, four tokens of 16 x 64 heads against 16 000 472 / 451,
-// one against 12 000 at D = 64 212 / 195.
+// AROWS = 32: up to eight query blocks and many tiles: token generation, and calls with one Q mean per head (a "block" per query head then, however many
+// queries).  A block takes two (D = 64: three) tiles one after the other: its tensor memory, mean and A tile are set up once, and the next tile's rows
+// come in under this one's MMAs and read-out, which takes 80 registers at D = 128 (three blocks per SM; with four, spilled rows: 137.4 -> 147.1).
+// us per call, before / after: one token of 8 x 32 heads against 8 192 keys of 8 kv heads 137.4 / 134.9 (D = 64 89.6 / 87.4), of 32 kv heads 462 / 436
+// (271 / 249), four tokens of 16 x 64 heads against 16 000 472 / 456 (284 / 258).  Pre-pass alone, one Q mean per head: 2 x 32 heads x 16 384 tokens
+// 344 / 332 (212 / 200), 24 heads x 30 000 223 / 221 (129 / 124), 8 x 32 heads x 8 192, 8 kv heads 340 / 335 (190 / 187).
 // FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
-// Tiles that a block of the AROWS = 32 kernel takes, and the tiles of a call from which it is used: with fewer than some ten rounds of resident
-// blocks the coarser last round costs as much (148 SMs, 2 048 tiles 87.5 / 88.0 us at D = 128, 59.2 / 59.4 at D = 64; 3 008 109.7 / 109.7 and
-// 69.6 / 67.5).
+// Tiles that a block of the AROWS = 32 kernel takes, and the tiles per SM from which it is used: 4.5 rounds of resident blocks (3 x 2 tiles) at D = 128,
+// 1.7 (4 x 3 tiles) at D = 64.  With fewer the coarser last round costs what the rest gains.  One token of B x 32 heads, 8 kv heads, 148 SMs, pre-pass
+// alone, a tile per block / in turn: D = 128, 2 048 tiles 55.4 / 57.2, 2 560 69.4 / 68.5, 3 072 83.9 / 83.7, 3 584 98.3 / 98.2, 3 840 104.5 / 104.4, 4 480
+// 122.9 / 121.7, 5 120 139.7 / 136.6; D = 64, 2 048 34.7 / 34.9, 2 560 41.3 / 41.0, 3 072 47.2 / 45.1, 4 096 59.8 / 57.7, 5 120 77.9 / 71.7.
 __host__ __device__ constexpr int tiles_in_turn(int D) { return D == 128 ? 2 : 3; }
-constexpr int tiles_in_turn_from(int D) { return D == 128 ? 4000 : 3000; }
+constexpr int tiles_in_turn_per_sm(int D) { return D == 128 ? 27 : 20; }
 
 template <typename T, int D, int AROWS, bool FLAG>
 __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128) ? 3 : 4) quant_k_delta_kernel(
@@ -915,7 +917,10 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     // tensor maps for the K kernel: the Q means and delta_s of a kv head's query heads follow one another, so both are byte
     // tensors [B*Hkv][group * nqm][...] and one MMA takes the blocks of several heads
     const uint64_t rows = (uint64_t)(a.Hq / a.Hkv) * a.nqm;
-    const bool few = rows <= 64, in_turn = rows <= 8 && (int64_t)tiles_k * BHkv >= tiles_in_turn_from(D);
+    int dev = 0;
+    DeviceInfo info;
+    if ((e = current_device(&dev, &info)) != cudaSuccess) return e;
+    const bool few = rows <= 64, in_turn = rows <= 8 && (int64_t)tiles_k * BHkv >= (int64_t)tiles_in_turn_per_sm(D) * info.sms;
     const int a_rows = in_turn ? 32 : few ? 64 : 128;
     const size_t smem_k = (D / 64) * (128 + a_rows) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 || in_turn ? 1024 + a_rows * 256 : 0);
     alignas(64) CUtensorMap tm_qm, tm_delta;

@@ -136,6 +136,18 @@ def test_halves_are_unrolled_where_that_is_faster(fake, call, Nk, causal, D, rol
     assert f"ELb{rolled}EEEv" in name, name
 
 
+@pytest.mark.parametrize("D,tiles,heads,kw,rows", [
+    (128, 27 * 148, 1, {}, 32), (128, 27 * 148 - 1, 1, {}, 64), (64, 20 * 148, 8, {}, 32), (64, 20 * 148 - 1, 8, {}, 64), (64, 20 * 148, 9, {}, 64),
+    (128, 27 * 148, 8, dict(Nq=20000, per_block_mean=0), 32), (128, 27 * 148, 9, dict(Nq=20000, per_block_mean=0), 64), (128, 27 * 148, 1, dict(Nq=1025), 64)])
+def test_key_tiles_are_taken_in_turn_from_a_number_per_sm(fake, D, tiles, heads, kw, rows):
+    """The K kernel's rows of query blocks: 32, and several tiles per block, for up to eight blocks of all query heads of a kv head (one per head with
+    one Q mean) and a number of key tiles that counts in SMs (148 here)."""
+    fake.fake_start(-1, 0)
+    assert _fwd(fake, _desc(**{**dict(B=1, Hq=heads, Hkv=1, Nq=1, Nk=128 * tiles, D=D), **kw})) == 0
+    name = [entry[1] for entry in _log(fake) if "quant_k_delta" in entry[1]][0]
+    assert f"Li{D}ELi{rows}E" in name, name
+
+
 def test_a_launch_of_too_many_blocks_is_refused():
     """All pieces of the first pre-pass kernel are one grid: their number, not that of one kind, has to stay below 2^31."""
     d = _desc(B=60000, Hq=1, Hkv=1, Nq=128, Nk=6000000)       # 2.8e9 tiles of V

@@ -39,6 +39,24 @@ def test_split_tensors_equal_the_contiguous_call(cuda_device, B, Hq, Hkv, n, P, 
     assert torch.equal(got, ref)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_split_keys_in_turn_equal_the_contiguous_call(cuda_device, D):
+    """Few query blocks and many key tiles, the tokens of K and V in two buffers that meet inside a tile: a block of the K kernel takes several tiles in
+    turn, from both buffers."""
+    H, Nq, n = 40, 64, 6475
+    q, k, v = (t.to(cuda_device) for t in O.make_inputs(1, H, H, Nq, 2 * n, D, seed=65, k_offset_std=1.0))
+    ref = sageattn3(q, k, v)
+    cut = lambda x: [x[:, :, i * n:(i + 1) * n].contiguous() for i in range(2)]
+    ks, vs, out = cut(k), cut(v), torch.full_like(q, float("nan"))
+    prob = Sage3Problem.for_shape(1, H, H, Nq, 2 * n, D, q.dtype, cuda_device, q_stride=(H * Nq * D, Nq * D, D), k_stride=(H * n * D, n * D, D))
+    lib, st = _cabi.lib(), torch.cuda.current_stream(cuda_device).cuda_stream
+    qp, kp, vp, op = _parts([q], Nq), _parts(ks, n), _parts(vs, n), _parts([out], Nq)
+    assert lib.sage3_prepass_parts(C.byref(prob.desc), C.byref(qp), C.byref(kp), C.byref(vp), prob.ws.buf.data_ptr(), st) == 0
+    assert lib.sage3_attn_fwd_parts(C.byref(prob.desc), prob.ws.buf.data_ptr(), C.byref(op), None, st) == 0
+    assert prob.check_status() == 0
+    assert torch.equal(out, ref)
+
+
 def test_parts_argument_checks(cuda_device):
     prob = Sage3Problem.for_shape(1, 2, 2, 256, 256, 64, torch.bfloat16, cuda_device)
     lib = _cabi.lib()
