@@ -7,11 +7,11 @@
 //   warps 0, 1   Q K^T MMA issuers, for keys [0, 64) and [64, 128) of every item; warp 1 owns the tensor-memory allocation
 //   warp 2       P V MMA issuer
 //   warp 3       draws and publishes the units; TMA producer: Q tiles, then K (+ one delta_s row per tile) / V^T / scale atoms per block
-//                (Each on a scheduler of its own.  With the producer as warp 0 and the issuers as 1 and 3 nothing was faster and most
-//                calls 0.1 to 0.6 % slower: packed prompts 607.0 / 603.5 us, 3 001 tokens 90.6 / 90.3, 16 384 keys 5 788 / 5 780.)
+//                (Each on a scheduler of its own; which role on which makes little difference.  With the producer as warp 0 and the issuers as 1
+//                and 3, in turns on one machine: packed prompts 607.0 / 603.5 us, 3 001 tokens 90.6 / 90.3, 16 384 keys 5 788 / 5 780.)
 //   warps 4-19   four softmax groups of four warps; group g takes the items g, g + 4, ...  A thread owns one row of the block
 //                and walks its 128 keys in two halves of 64 (the scores of a half live in registers).
-//   warps 20-23  O rescale ("correction"), one warp per tensor-memory lane quarter, one wait per item: when a row of the quarter moved
+//   warps 20-23  O rescale ("correction"), one warp per tensor-memory lane quarter: when a row of the quarter moved
 //                its maximum, the warp multiplies the 32 O rows of its quarter by their factors before the block's
 //                P V MMA is issued; it also keeps the running row sums and writes O / l while the softmax groups are
 //                already at work on the next unit.
@@ -343,7 +343,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // Register budget: 768 threads start with 80 registers each, and that allocation (61 440) is all the CTA can
     // ever hold: 128 x kRoleRegs for warpgroup 0 (the copy and MMA roles) + 128 x kCorrRegs for the correction
     // warpgroup + 512 x kSoftRegs for the softmax warpgroups.  (An increase beyond the launch allocation would wait forever.)  With
-    // the halves of an item in one loop the softmax code needs 88, which leaves the others enough not to spill.
+    // the halves of an item in one loop the softmax code needs 88, which leaves the other warps 64: bytes spilled (stores / loads) 0 at D = 128 and at D = 64
+    // without a mask, 22 / 30 at D = 64 with one, 10 / 14 with carried state at D = 64, 4 / 4 with packed heads at D = 64.  Unrolled it needs 96 and the others have 48:
+    // 58 / 82 at D = 64, 82 / 114 for packed batches, 66 / 98 and (with a mask) 70 / 102 with carried state at D = 128; up to 32 rows 78 / 98.
     constexpr int kRoleRegs = PACK == 2 || !ROLL ? 48 : 64, kSoftRegs = PACK == 2 || !ROLL ? 96 : 88;
     constexpr int kCorrRegs = PACK == 2 || !ROLL ? 48 : 64;
     static_assert(128 * (kRoleRegs + kCorrRegs + C::kGroups * kSoftRegs) <= C::kThreads * 80, "registers");
