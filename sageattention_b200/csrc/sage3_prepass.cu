@@ -463,25 +463,11 @@ __device__ __forceinline__ void quant_q_tile(
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
 // ------------------------------------------------------------------------------------------------
-// AROWS = 64: up to 64 query blocks.  The A tile then has 64 rows (the MMA's other 64 read what lies behind it, for accumulator rows nobody
-// looks at), which makes room for a fourth block per SM:
-// 1 000 queries of 32 heads against 9 192 keys 143.9 -> 141.9 us per call, 4 250 tokens of 48 heads 359.0 -> 356.9 us.
-// AROWS = 32: up to eight query blocks and many tiles: token generation, and calls with one Q mean per head (a "block" per query head then, however many
-// queries).  A block takes two (D = 64: three) tiles one after the other: its tensor memory, mean and A tile are set up once, and the next tile's rows
-// come in under this one's MMAs and read-out, which takes 80 registers at D = 128 (three blocks per SM; with four, spilled rows: 137.4 -> 147.1).
-// us per call, before / after: one token of 8 x 32 heads against 8 192 keys of 8 kv heads 137.4 / 134.9 (D = 64 89.6 / 87.4), of 32 kv heads 462 / 436
-// (271 / 249), four tokens of 16 x 64 heads against 16 000 472 / 456 (284 / 258).  Pre-pass alone, one Q mean per head: 2 x 32 heads x 16 384 tokens
-// 344 / 332 (212 / 200), 24 heads x 30 000 223 / 221 (129 / 124), 8 x 32 heads x 8 192, 8 kv heads 340 / 335 (190 / 187).
+// AROWS = 64: D = 64 and 33 to 64 query blocks (the A tile then has 64 rows, the MMA's other 64 read what lies behind it, for accumulator rows nobody looks
+// at; four blocks per SM), where every tile finds a block at once, see launch_prepass_t.  Up to 64 query blocks are otherwise quant_k_delta_run_kernel's.
 // FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
-// Tiles that a block of the AROWS = 32 kernel takes, and the tiles per SM from which it is used: 4.5 rounds of resident blocks (3 x 2 tiles) at D = 128,
-// 1.7 (4 x 3 tiles) at D = 64.  With fewer the coarser last round costs what the rest gains.  One token of B x 32 heads, 8 kv heads, 148 SMs, pre-pass
-// alone, a tile per block / in turn: D = 128, 2 048 tiles 55.4 / 57.2, 2 560 69.4 / 68.5, 3 072 83.9 / 83.7, 3 584 98.3 / 98.2, 3 840 104.5 / 104.4, 4 480
-// 122.9 / 121.7, 5 120 139.7 / 136.6; D = 64, 2 048 34.7 / 34.9, 2 560 41.3 / 41.0, 3 072 47.2 / 45.1, 4 096 59.8 / 57.7, 5 120 77.9 / 71.7.
-__host__ __device__ constexpr int tiles_in_turn(int D) { return D == 128 ? 2 : 3; }
-constexpr int tiles_in_turn_per_sm(int D) { return D == 128 ? 27 : 20; }
-
 template <typename T, int D, int AROWS, bool FLAG>
-__global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128) ? 3 : 4) quant_k_delta_kernel(
+__global__ void __launch_bounds__(256, AROWS == 128 ? 3 : 4) quant_k_delta_kernel(
     const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
     T* __restrict__ km,                // [B*H][D]
     const float* __restrict__ part,    // partial column sums to form the mean from ([B*H][chunks][D]), or nullptr: `km` holds it
@@ -500,14 +486,13 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
     constexpr uint32_t kTmemCols = 128;
     constexpr bool kBf16 = sizeof(T) == 2 && Num<T>::kIsBf16;
 
-    constexpr int TILES = AROWS == 32 ? tiles_in_turn(D) : 1;
-    const int tile0 = blockIdx.x * TILES, bh = blockIdx.y;
+    const int tile = blockIdx.x, bh = blockIdx.y;
     int h;
     const int b = H.divmod(bh, h);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int c = t % CH, rl = t / CH;
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
-    int row0 = tile0 * kBlock;
+    const int row0 = tile * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
 
     extern __shared__ uint8_t smem_dyn[];
@@ -519,7 +504,7 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
     constexpr int kARows = AROWS, kASub = kARows * 128;
     constexpr int oA = 0, oB = SUB * kASub, oMean = oB + SUB * 16384, oSf = oMean + D * 4, oBar = oSf + SUB * 512;
     static_assert(oA + (SUB - 1) * kASub + 16384 <= oMean, "the MMA's 128 A rows stay inside the tiles");
-    constexpr int oStg = (D == 128 && TILES == 1) ? oA : ((oBar + 64 + 1023) / 1024) * 1024;
+    constexpr int oStg = D == 128 ? oA : ((oBar + 64 + 1023) / 1024) * 1024;
     T* s_mean = reinterpret_cast<T*>(sgen + oMean);
     uint8_t* s_sf = sgen + oSf;
     const uint32_t bar = sbase + oBar;
@@ -543,12 +528,9 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
         pdl_launch_dependents();
     }
     uint4 raw[ITEMS][2];
-    auto load_rows = [&]() {
-        x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
-            load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
-        });
-    };
-    load_rows();
+    x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
+        load16_packed<T>(p + c * 16, row0 + rl + RPP * i < N, raw[i][0], raw[i][1]);
+    });
     pdl_wait();                           // the K rows above are inputs; from here on results of the launches before are read
     // the first A tile (see below) comes in while K is quantized
     auto load_a = [&](int m0) {
@@ -561,7 +543,7 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
     if (t < D) {
         if (part != nullptr) {
             const T m = Num<T>::from_f(sum_chunks(part + (int64_t)bh * chunks * D + t, chunks, D) * (N > 0 ? 1.0f / (float)N : 0.f));
-            if (tile0 == 0) km[(int64_t)bh * D + t] = m;
+            if (tile == 0) km[(int64_t)bh * D + t] = m;
             s_mean[t] = m;
         } else {
             s_mean[t] = km[(int64_t)bh * D + t];
@@ -577,7 +559,6 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
     *reinterpret_cast<uint4*>(mu2 + 4) = reinterpret_cast<const uint4*>(s_mean)[2 * c + 1];
     uint32_t iter = 0;
     bool alive = true;
-    for (int it = 0; it < TILES; ++it) {
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const int rt = rl + RPP * i;          // row inside the tile
@@ -603,17 +584,10 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
     }
     __syncthreads();
     {
-        uint8_t* dst = sfs + ((int64_t)bh * (Np / kBlock) + tile0 + it) * (D / 64) * 512;
+        uint8_t* dst = sfs + ((int64_t)bh * (Np / kBlock) + tile) * (D / 64) * 512;
         if (t < (D / 64) * 32) reinterpret_cast<uint4*>(dst)[t] = reinterpret_cast<const uint4*>(s_sf)[t];
     }
 
-    const int tile_row0 = row0;
-    bool more = false;                    // the block's next tile: its rows come in under this one's MMAs
-    if constexpr (TILES > 1) {
-        row0 += kBlock;
-        more = it + 1 < TILES && row0 < N;
-        if (more) load_rows();
-    }
     // delta_s of all query heads of this kv head, 128 query blocks per MMA group
     constexpr uint32_t idesc = make_idesc_f16_kk(128, kBf16);
     const int quarter = warp & 3, chalf = warp >> 2;       // tensor-memory lane quarter, column half of the epilogue
@@ -626,7 +600,7 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
             __syncthreads();
             if (t == 0) load_a(m0);
         }
-        if (TILES == 1 || it == 0) alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);      // (several tiles: the A tile stays)
+        alive = mbar_wait(bar_a, iter & 1, abort_flag, status, kWaitDeltaA);
         tc_fence_before();
         alive = __syncthreads_and(alive ? 1 : 0) != 0;
         if (!alive) break;
@@ -652,19 +626,17 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
             const int stg_off = oStg + (chalf * (kARows / 32) + quarter) * 4096;
             uint8_t* stg = sgen + stg_off;
             uint32_t z = 0;               // FLAG: 0 while all values are finite
-            constexpr int kCols = TILES > 1 ? 16 : 32;      // (several tiles: the registers hold the next one's rows)
 #pragma unroll
-            for (int cc = 0; cc < 64 / kCols; ++cc) {
-                float v[kCols];
-                if constexpr (kCols == 32) tmem_ld32(acc + cc * 32, v);
-                else tmem_ld16(acc + cc * 16, v);
+            for (int cc = 0; cc < 2; ++cc) {
+                float v[32];
+                tmem_ld32(acc + cc * 32, v);
                 tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < kCols / 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     uint32_t p4[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) p4[e] = Num<T>::pack2(v[8 * i + 2 * e], v[8 * i + 2 * e + 1]);
-                    *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * (kCols / 8) + i) ^ (lane & 7)) << 4)) =
+                    *reinterpret_cast<uint4*>(stg + lane * 128 + (((cc * 4 + i) ^ (lane & 7)) << 4)) =
                         make_uint4(p4[0], p4[1], p4[2], p4[3]);
                     if constexpr (FLAG) {
 #pragma unroll
@@ -676,7 +648,7 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-                tma_store_3d(&tm_delta, sbase + stg_off, (tile_row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
+                tma_store_3d(&tm_delta, sbase + stg_off, (row0 + chalf * 64) * 2, m0 + quarter * 32, bh);
                 bulk_commit_group();
                 bulk_wait_group_read0();      // the engine has read the staging tile: it may be written again
             }
@@ -685,13 +657,300 @@ __global__ void __launch_bounds__(256, AROWS == 128 || (AROWS == 32 && D == 128)
         tc_fence_before();
         __syncthreads();      // the accumulator and the A tile are free again
     }
-    if (!more || !alive) break;
-    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// K for up to 64 query blocks per kv head (token generation, chunks of a prompt, calls with one Q mean per head, packed prompts): two blocks per SM
+// walk runs of tiles, all of one length, that go on from head to head.
+//   warps 0-7   hold the next tile's rows in registers (a row's load is issued as soon as the one before it in that place is used), smooth and quantize
+//               them, store k' as the operand of the MMA, and write delta_s of the tile before: nothing in their loop waits for a copy or an MMA
+//               that has just been started, and a barrier of all eight is met once per head
+//   warp 8      the MMAs, as delta_s^T: the 128 keys are the rows of the accumulator and the query blocks its columns, so that an MMA costs
+//               what the query blocks ask for and a warp's store covers 32 keys of a row
+// The kernel above spends a chain of load, quantization, copy, MMA and read-out per tile, with four block-wide barriers, and accumulator rows of 128 query
+// blocks where there are four.  What bounds this one: instructions (5 100 per tile, issue slots 63 % busy) and, at 5.0 TB/s, nearly HBM.  One token of 8 x 32
+// heads against 8 192 keys of 8 kv heads, this kernel's time 51.5 -> 34.3 us (D = 64 32.3 -> 23.0).  Pre-pass of 4 096 / 2 048 / 512 / 296 tiles, 8 kv
+// heads, us: 4 query blocks 108.1 / 55.6 / 19.6 / 16.6 -> 90.5 / 47.3 / 18.7 / 15.0, 64 blocks 158.3 / 83.0 / 24.3 / 20.7 -> 143.3 / 74.7 / 22.8 / 19.6, D = 64
+// 4 blocks 58.2 / 33.5 / 15.0 / 14.8 -> 50.1 / 29.0 / 14.6 / 14.5, 64 blocks 92.2 / 47.7 / 17.5 / 15.9 -> 84.4 / 45.1 / 18.5 / 14.6.  Variants of it, first figure
+// (51.5 before): rows copied to shared memory ahead by all warps 44.5, by a warp of its own 44.1 (shared memory then moves 160 KB per tile: the copy, the
+// read, k', and the MMA's operands), three blocks per SM 38.6 (two 36.0), one store per key and row 36.0 -> 35.5, row addresses ahead 34.3.
+// NR = 32 instead of 64 columns: up to eight query blocks from a number of tiles on.  (One token of 8 x 32 heads 90.5 / 91.8 us of pre-pass; with few
+// tiles neither shows.)
+// ------------------------------------------------------------------------------------------------
+// A place in the list of tiles: entry by entry, head by head, tile by tile.
+template <typename T>
+struct KCursor {
+    int bh, b, h, tile, nt, N;
+    int64_t off;
+    __device__ __forceinline__ void enter(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, int Nmax) {
+        N = Nmax;
+        off = x.base(b, h, sb, sh, sn, N);
+        nt = max(1, (N + kBlock - 1) / kBlock);
+    }
+    __device__ __forceinline__ bool next(int H) {             // true: another head, to be entered
+        if (++tile < nt) return false;
+        tile = 0;
+        ++bh;
+        if (++h == H) { h = 0; ++b; }
+        return true;
+    }
+};
+
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Tiles per SM from which calls of up to eight query blocks take the kernel for 32 of them.
+constexpr int kRun32TilesPerSm(int D) { return D == 128 ? 27 : 20; }
+
+template <int D, int NR>
+struct KRunCfg {
+    static constexpr int SUB = D / 64;                        // 64-element (128-byte) sub-tiles along K
+    static constexpr int kThreads = 256 + 32;
+    static constexpr int kBlocks = 2;                         // per SM
+    static constexpr int oK = 0, oQ = 2 * SUB * 16384, oMean = oQ + SUB * NR * 128, oBar = oMean + 2 * D * 2, kSmem = oBar + 64 + 1024;      // + slack for the alignment
+    static constexpr uint32_t kCols = 2 * NR < 32 ? 32 : 2 * NR;      // tensor memory: two accumulators
+};
+
+template <typename T, int D, int NR, bool FLAG>
+__global__ void __launch_bounds__(KRunCfg<D, NR>::kThreads, KRunCfg<D, NR>::kBlocks) quant_k_delta_run_kernel(
+    const __grid_constant__ Src<T> x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, FastDiv tiles, int B, int Nmax, int Np,
+    T* __restrict__ km, const float* __restrict__ part, int chunks, uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, T* __restrict__ delta, int rows,
+    int* __restrict__ status, int* __restrict__ nonfinite, const __grid_constant__ CUtensorMap tm_qm) {
+    using C = KRunCfg<D, NR>;
+    constexpr int CH = D / 16, RPP = 256 / CH, ITEMS = kBlock / RPP, SUB = C::SUB;
+    extern __shared__ uint8_t smem_dyn[];
+    const uint32_t sbase = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    uint8_t* sgen = smem_dyn + (sbase - smem_u32(smem_dyn));
+    const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31;
+    const uint32_t bar_ready = sbase + C::oBar, bar_mma = bar_ready + 16, bar_q = bar_mma + 16;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sgen + C::oBar + 48);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sgen + C::oBar + 52);
+    if (t == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_ready + 8 * i, 8);
+            mbar_init(bar_mma + 8 * i, 1);
+        }
+        mbar_init(bar_q, 1);
+        mbar_fence_init();
+    }
+    if (warp == 8) {
+        tmem_alloc(smem_u32(tmem_slot), C::kCols);
+        tmem_relinquish();
+        pdl_launch_dependents();          // (not before the tensor memory is this block's, see above)
+    }
+    // This block's run of tiles, the same number for every block.
+    KCursor<T> at;
+    int n;
+    {
+        int p0;
+        if (x.cu == nullptr) {
+            const int64_t total = (int64_t)B * H.d * tiles.d;
+            p0 = (int)(total * blockIdx.x / gridDim.x);
+            n = (int)(total * (blockIdx.x + 1) / gridDim.x) - p0;
+            at.bh = tiles.divmod(p0, at.tile);
+            at.b = H.divmod(at.bh, at.h);
+        } else {
+            auto tiles_of = [&](int b) { return b < B ? max(1, (min(max(x.cu[b + 1] - x.cu[b], 0), Nmax) + kBlock - 1) / kBlock) : 0; };
+            int all = 0;
+            for (int b0 = 0; b0 < B; b0 += 32) all += __reduce_add_sync(0xffffffffu, tiles_of(b0 + lane));
+            const int64_t total = (int64_t)all * H.d;
+            p0 = (int)(total * blockIdx.x / gridDim.x);
+            n = (int)(total * (blockIdx.x + 1) / gridDim.x) - p0;
+            at.b = at.h = at.tile = 0;
+            for (int b0 = 0; n > 0; b0 += 32) {
+                const int mine = tiles_of(b0 + lane);
+                const int here = __reduce_add_sync(0xffffffffu, mine) * (int)H.d;
+                if (p0 >= here) { p0 -= here; continue; }
+                for (int i = 0;; ++i) {
+                    const int nt = __shfl_sync(0xffffffffu, mine, i);
+                    if (p0 < nt * (int)H.d) {
+                        at.b = b0 + i;
+                        at.h = p0 / nt;
+                        at.tile = p0 - at.h * nt;
+                        break;
+                    }
+                    p0 -= nt * (int)H.d;
+                }
+                break;
+            }
+            at.bh = at.b * (int)H.d + at.h;
+        }
+        if (n > 0) at.enter(x, sb, sh, sn, Nmax);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    if (warp < 8) {
+        // ------------------------------------------------------------------ smoothing and quantization; delta_s of the tile before
+        // Microblock column and row of the thread: eight neighbouring lanes have four columns of two rows, whose chunks lie on different banks.
+        const int c = (lane & 3) | (D == 128 ? (lane >> 1) & 4 : 0);
+        const int rl = warp * (32 / CH) + (D == 128 ? ((lane >> 2) & 1) | ((lane >> 3) & 2) : lane >> 2);
+        const uint32_t place = (uint32_t)((c >> 2) * 16384 + rl * 128 + ((((2 * c) & 7) ^ (rl & 7)) << 4));      // of the microblock's first 16 bytes; the others: ^ 16
+        KCursor<T> ahead = at;
+        uint4 raw[ITEMS][2];
+        const T* src[ITEMS];              // this thread's rows of the tile `ahead`
+        int rows_ahead = 0;               // ... of which those are there whose number in the tile is less
+        auto locate = [&]() {
+            const int r = ahead.tile * kBlock + rl;
+            rows_ahead = ahead.N - r;
+            x.template rows_each<ITEMS>(ahead.off + c * 16, r, RPP, sn, [&](int i, const T* p) { src[i] = p; });
+        };
+        if (n > 0) {
+            locate();
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) load16_packed<T>(src[i], RPP * i < rows_ahead, raw[i][0], raw[i][1]);
+        }
+        pdl_wait();                       // the K rows are inputs; from here on results of the launches before are read
+        uint32_t mu2[8];                  // the 16 means of this thread's columns, packed
+        bool fresh = true;                // this head's mean is not in mu2 yet
+        int seg = 0;
+        // delta_s of a tile: a thread is a key (tensor-memory lane), the warps 0-3 and 4-7 have half of the query blocks each
+        auto write_delta = [&](int it, int bh, int tile) {
+            constexpr int HALF = NR / 2;
+            const int quarter = warp & 3, r0 = (warp >> 2) * HALF;
+            if (!mbar_try_wait(bar_mma + 8 * (it & 1), (it >> 1) & 1)) mbar_wait(bar_mma + 8 * (it & 1), (it >> 1) & 1, abort_flag, status, kWaitDeltaMma);
+            __syncwarp();
+            if (r0 < rows) {
+                tc_fence_after();
+                float v[HALF];
+                const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + (it & 1) * NR + r0;
+                if constexpr (HALF == 16) tmem_ld16(acc, v);
+                else tmem_ld32(acc, v);
+                tc_wait_ld();
+                tc_fence_before();
+                // Two neighbouring lanes swap one of two rows: each has two keys of one row then, and a store covers 64 bytes of both rows.
+                const int row = r0 + (lane & 1);
+                T* dst = delta + ((int64_t)bh * rows + row) * Np + tile * kBlock + quarter * 32 + (lane & ~1);
+                uint32_t z = 0;           // FLAG: 0 while all values are finite
+#pragma unroll
+                for (int r = 0; r < HALF; r += 2, dst += 2 * Np) {
+                    const uint32_t w = Num<T>::pack2(v[r], v[r + 1]), y = __shfl_xor_sync(0xffffffffu, w, 1);
+                    const uint32_t pair = __byte_perm(w, y, lane & 1 ? 0x3276 : 0x5410);
+                    if (row + r < rows) {
+                        *reinterpret_cast<uint32_t*>(dst) = pair;
+                        if (FLAG) z = Num<T>::zero_fma2(pair, z);
+                    }
+                }
+                if (FLAG && (z & 0x7fff7fffu) != 0) nonfinite[bh] = 1;
+            }
+        };
+        int bh_before = 0, tile_before = 0;
+        for (int it = 0; it < n; ++it) {
+            if (fresh) {
+                T* s_mean = reinterpret_cast<T*>(sgen + C::oMean) + (seg & 1) * D;
+                if (t < D) {
+                    T m;
+                    if (part != nullptr) {
+                        m = Num<T>::from_f(sum_chunks(part + (int64_t)at.bh * chunks * D + t, chunks, D) * (at.N > 0 ? 1.0f / (float)at.N : 0.f));
+                        if (at.tile == 0) km[(int64_t)at.bh * D + t] = m;
+                    } else {
+                        m = km[(int64_t)at.bh * D + t];
+                    }
+                    s_mean[t] = m;
+                }
+                bar_sync(1, 256);
+                *reinterpret_cast<uint4*>(mu2) = reinterpret_cast<const uint4*>(s_mean)[2 * c];
+                *reinterpret_cast<uint4*>(mu2 + 4) = reinterpret_cast<const uint4*>(s_mean)[2 * c + 1];
+                ++seg;
+            }
+            const bool more = it + 1 < n;
+            const int here = rows_ahead;
+            if (more) {
+                if (ahead.next((int)H.d)) ahead.enter(x, sb, sh, sn, Nmax);
+                locate();
+            }
+            const int row0 = at.tile * kBlock;
+            const bool edge = row0 + kBlock > at.N;
+            uint8_t *lo_half = sgen + C::oK + (it & 1) * SUB * 16384 + place, *hi_half = sgen + C::oK + (it & 1) * SUB * 16384 + (place ^ 16u);
+            uint32_t sf = 0;              // scale bytes of this thread's microblocks
+            uint8_t* code = codes + ((int64_t)at.bh * Np + row0 + rl) * (D / 2) + c * 8;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                const uint32_t x2[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
+                uint32_t w[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) w[j] = Num<T>::sub2(x2[j], mu2[j]);
+                if (edge) {                   // K is padded after smoothing: pad rows are 0
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) w[j] = RPP * i < here ? w[j] : 0u;
+                }
+                if (more) load16_packed<T>(src[i], RPP * i < rows_ahead, raw[i][0], raw[i][1]);
+                // k', the operand of the MMA: [row][16-byte chunk], 128-byte swizzle
+                *reinterpret_cast<uint4*>(lo_half + i * RPP * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4*>(hi_half + i * RPP * 128) = make_uint4(w[4], w[5], w[6], w[7]);
+                uint32_t lo, hi, sfb;
+                quant16_packed<T>(w, lo, hi, sfb);
+                *reinterpret_cast<uint2*>(code + i * RPP * (D / 2)) = make_uint2(lo, hi);
+                sf |= sfb << (8 * i);
+            }
+            fence_proxy_async_smem();
+            warp_arrive(bar_ready + 8 * (it & 1), lane);
+            // Scale bytes: four neighbouring lanes hold the four columns of a word of the atom, a byte of it per microblock
+            {
+                uint8_t* dst = sfs + ((int64_t)at.bh * (Np / kBlock) + at.tile) * SUB * 512 + (c >> 2) * 512;
+                const int l = lane & 3;
+                const uint32_t y = __shfl_xor_sync(0xffffffffu, sf, 1);
+                const uint32_t v = __byte_perm(sf, y, l & 1 ? 0x3715 : 0x6240);
+                const uint32_t z = __shfl_xor_sync(0xffffffffu, v, 2);
+                const uint32_t word = __byte_perm(v, z, l & 2 ? 0x3276 : 0x5410);      // of microblock l
+                if (ITEMS == 4 || l < 2) *reinterpret_cast<uint32_t*>(dst + sf_atom_offset(rl + RPP * l, 0)) = word;
+            }
+            if (it > 0) write_delta(it - 1, bh_before, tile_before);
+            bh_before = at.bh;
+            tile_before = at.tile;
+            fresh = at.next((int)H.d);
+            if (fresh && more) at.enter(x, sb, sh, sn, Nmax);
+        }
+        if (n > 0) write_delta(n - 1, bh_before, tile_before);
+    } else {
+        // ------------------------------------------------------------------ MMAs: delta_s^T [128 keys][query blocks] = k' qm^T
+        pdl_wait();
+        constexpr uint32_t idesc = make_idesc_f16_kk(NR, Num<T>::kIsBf16);
+        constexpr uint32_t hi_k = sdesc_hi(1024, kSwz128);
+        const uint32_t k_lo0 = __shfl_sync(0xffffffffu, sdesc_lo(sbase + C::oK, 16), 0), q_lo = __shfl_sync(0xffffffffu, sdesc_lo(sbase + C::oQ, 16), 0);
+        bool fresh = true;
+        uint32_t q_parity = 0;
+        for (int it = 0; it < n; ++it) {
+            const int st = it & 1;
+            if (fresh) {                  // this head's query-block means; the MMAs with the last ones' must be complete
+                if (it > 0) mbar_wait<true>(bar_mma + 8 * (st ^ 1), ((it - 1) >> 1) & 1, abort_flag, status, kWaitDeltaMma);
+                if (lane == 0) {
+                    mbar_expect_tx(bar_q, SUB * NR * 128);
+#pragma unroll
+                    for (int sub = 0; sub < SUB; ++sub) tma_load_3d(sbase + C::oQ + sub * NR * 128, &tm_qm, bar_q, sub * 128, 0, at.bh);
+                }
+                __syncwarp();
+                mbar_wait<true>(bar_q, q_parity, abort_flag, status, kWaitDeltaA);
+                q_parity ^= 1;
+            }
+            mbar_wait<true>(bar_ready + 8 * st, (it >> 1) & 1, abort_flag, status, kWaitDeltaA);
+            __syncwarp();
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t k_lo = k_lo0 + st * (SUB * 16384 / 16), acc = tmem + st * NR;
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    tc_mma_f16(acc, sdesc(k_lo + ((ks >> 2) * 16384 + (ks & 3) * 32) / 16, hi_k), sdesc(q_lo + ((ks >> 2) * NR * 128 + (ks & 3) * 32) / 16, hi_k),
+                               idesc, ks > 0);
+                tc_commit(bar_mma + 8 * st);
+            }
+            __syncwarp();
+            fresh = at.next((int)H.d);
+            if (fresh && it + 1 < n) at.enter(x, sb, sh, sn, Nmax);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        tc_fence_after();
+        tmem_dealloc(tmem, C::kCols);
     }
 }
 
@@ -920,27 +1179,45 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     int dev = 0;
     DeviceInfo info;
     if ((e = current_device(&dev, &info)) != cudaSuccess) return e;
-    const bool few = rows <= 64, in_turn = rows <= 8 && (int64_t)tiles_k * BHkv >= (int64_t)tiles_in_turn_per_sm(D) * info.sms;
-    const int a_rows = in_turn ? 32 : few ? 64 : 128;
-    const size_t smem_k = (D / 64) * (128 + a_rows) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 || in_turn ? 1024 + a_rows * 256 : 0);
-    alignas(64) CUtensorMap tm_qm, tm_delta;
-    if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, a_rows, 3) != 0 ||
-        encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
-        return cudaErrorInvalidValue;
-    auto k_kernel = [&](auto a_rows_, auto flag_) {
-        constexpr auto kern = quant_k_delta_kernel<T, D, decltype(a_rows_)::value, decltype(flag_)::value>;
-        const cudaError_t allowed = allow_smem<kern>((int)smem_k);
-        if (allowed != cudaSuccess) return allowed;
-        return launch(true, kern, dim3(in_turn ? (tiles_k + tiles_in_turn(D) - 1) / tiles_in_turn(D) : tiles_k, BHkv), dim3(256), smem_k, st, s.k, a.ks[0], a.ks[1], a.ks[2],
-                      s.Hkv, a.Nk, a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows,
-                      a.status, a.nonfinite, tm_qm, tm_delta);
+    const int64_t tiles = (int64_t)tiles_k * BHkv;
+    auto by_flag = [&](auto go) { return a.nonfinite != nullptr ? go(std::true_type()) : go(std::false_type()); };
+    auto run = [&](auto rows_) {
+        return by_flag([&](auto flag_) {
+            constexpr int NR = decltype(rows_)::value;
+            using C = KRunCfg<D, NR>;
+            constexpr auto kern = quant_k_delta_run_kernel<T, D, NR, decltype(flag_)::value>;
+            const cudaError_t allowed = allow_smem<kern>(C::kSmem);
+            if (allowed != cudaSuccess) return allowed;
+            alignas(64) CUtensorMap tm_qm;
+            if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, NR, 3) != 0) return cudaErrorInvalidValue;
+            const int64_t slots = (int64_t)C::kBlocks * info.sms;
+            return launch(true, kern, dim3((unsigned)(tiles < slots ? tiles : slots)), dim3(C::kThreads), (size_t)C::kSmem, st, s.k, a.ks[0], a.ks[1], a.ks[2],
+                          s.Hkv, s.tiles_k, a.B, a.Nk, a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf,
+                          delta, (int)rows, a.status, a.nonfinite, tm_qm);
+        });
     };
-    auto by_rows = [&](auto flag_) {
-        return in_turn ? k_kernel(std::integral_constant<int, 32>(), flag_)
-               : few   ? k_kernel(std::integral_constant<int, 64>(), flag_)
-                       : k_kernel(std::integral_constant<int, 128>(), flag_);
+    auto one_tile = [&](auto a_rows_) {
+        return by_flag([&](auto flag_) {
+            constexpr int AR = decltype(a_rows_)::value;
+            constexpr auto kern = quant_k_delta_kernel<T, D, AR, decltype(flag_)::value>;
+            constexpr size_t smem = (D / 64) * (128 + AR) * 128 + D * 4 + (D / 64) * 512 + 64 + 1024 + (D == 64 ? 1024 + AR * 256 : 0);
+            const cudaError_t allowed = allow_smem<kern>((int)smem);
+            if (allowed != cudaSuccess) return allowed;
+            alignas(64) CUtensorMap tm_qm, tm_delta;
+            if (encode_tiled_bytes(&tm_qm, qm, (uint64_t)D * 2, rows, (uint64_t)BHkv, 128, AR, 3) != 0 ||
+                encode_tiled_bytes(&tm_delta, delta, (uint64_t)a.Nk_p * 2, rows, (uint64_t)BHkv, 128, 32, 3) != 0)
+                return cudaErrorInvalidValue;
+            return launch(true, kern, dim3(tiles_k, BHkv), dim3(256), smem, st, s.k, a.ks[0], a.ks[1], a.ks[2],
+                          s.Hkv, a.Nk, a.Nk_p, km, km_inline ? (const float*)s.part_k : (const float*)nullptr, a.kchunks_k, a.k_codes, a.k_sf, (int)rows,
+                          a.status, a.nonfinite, tm_qm, tm_delta);
+        });
     };
-    return a.nonfinite != nullptr ? by_rows(std::true_type()) : by_rows(std::false_type());
+    if (rows > 64) return one_tile(std::integral_constant<int, 128>());
+    // D = 64, 33 to 64 query blocks, one tile per block against runs: 296 tiles 15.9 / 14.6, 400 16.5 / 17.7, 512 17.5 / 18.5, 1 024 26.8 / 26.6 us.  (148 SMs hold 592
+    // blocks of one and 296 of the other.  Up to 32 query blocks: 400 14.8 / 14.6, 512 16.4 / 16.0.)
+    if constexpr (D == 64)
+        if (rows > 32 && tiles > 2 * info.sms && tiles <= 4 * info.sms) return one_tile(std::integral_constant<int, 64>());
+    return rows <= 8 && tiles >= (int64_t)kRun32TilesPerSm(D) * info.sms ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 64>());
 }
 
 cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t st) {
