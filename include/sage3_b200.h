@@ -90,6 +90,8 @@ typedef struct Sage3Desc {
  *   qkm      fp32 [B][Hq][Nq_p]               q . km per query row (the part of q k^T that K smoothing removes;
  *                                             core.py:289-293 `lse_correction`), used by the LSE output (sage3_fwd and
  *                                             sage3_fwd_varlen write it only when `lse` is asked for)
+ *   (behind qkm, from 2 048 padded keys on and part of total_bytes: int32[160] flags, cleared by the pre-pass and by an attention call on
+ *   its own, and 160 accumulators of 128 rows, for query tiles whose keys two blocks of the attention kernel walk)
  */
 typedef struct Sage3Workspace {
     size_t status, kpart, km, qm, delta, q_codes, q_sf, k_codes, k_sf, v_codes, v_sf, qkm;

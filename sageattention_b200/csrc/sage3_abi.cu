@@ -92,12 +92,19 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     w->v_codes = off; off += align_up(B * Hkv * D * (nkp / 2));
     w->v_sf = off;    off += align_up(B * Hkv * (nkp / 128) * 1024);
     w->qkm = off;     off += align_up(B * Hq * nqp * sizeof(float));
+    if (nkp / 128 >= sage3::kSplitMinBlocks) off += align_up(sage3::kSplitSlots * sizeof(int32_t)) + align_up(sage3::kSplitSlots * sage3::split_state_floats(D) * sizeof(float));      // see split_region
     w->total_bytes = off;
     w->nq_pad = (int32_t)nqp;
     w->nk_pad = (int32_t)nkp;
     w->nqm = (int32_t)nqm;
     w->kchunks = (int32_t)kch_k;
     return SAGE3_OK;
+}
+
+// Flags and accumulators of query tiles whose keys two CTAs share, behind the last region of the layout; nullptr where the layout has none.
+int* split_region(const Sage3Desc* d, const Sage3Workspace& w, void* ws) {
+    if (w.nk_pad / 128 < sage3::kSplitMinBlocks) return nullptr;
+    return reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + w.qkm + align_up((size_t)d->B * d->Hq * w.nq_pad * sizeof(float)));
 }
 
 int check_arch() {
@@ -190,6 +197,9 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
     a.nonfinite = reinterpret_cast<const int*>(base + w.status) + kNonfiniteWord;
     a.cu_q = cu_q; a.cu_k = cu_k;
+    a.split_flags = split_region(desc, w, ws);
+    a.split_state = a.split_flags ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.split_flags) + align_up(sage3::kSplitSlots * sizeof(int32_t))) : nullptr;
+    if (!cleared && a.split_flags && sage3::checked(cudaMemsetAsync(a.split_flags, 0, sage3::kSplitSlots * sizeof(int32_t), st)) != cudaSuccess) return SAGE3_E_CUDA;
     int drv = 0;
     return sage3::launch_attn(a, st, &drv) == cudaSuccess ? SAGE3_OK : SAGE3_E_CUDA;
 }
@@ -346,6 +356,7 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     const bool shared = sage3::PackRule(desc->Nq, desc->Hq / desc->Hkv, cu_q == nullptr).heads > 1;
     a.nonfinite = shared ? a.status + kNonfiniteWord : nullptr;
     a.n_clear = kNonfiniteWord + (shared ? desc->B * desc->Hkv : 0);
+    a.split_flags = split_region(desc, w, ws);
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
         sage3::checked(cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)

@@ -84,6 +84,15 @@ struct AttnParams {
     const int* nonfinite;               // PACK: per (batch, kv head), delta_s holds values that are not finite
 };
 
+// Of the kernels whose last rounds are dealt out by key blocks: units from whole_units on are slots, see SplitPlan.
+struct SplitParams : AttnParams {
+    int slot_blocks, slot_rest;         // key blocks per slot; of slot 0
+    int rest0;                          // without a mask: first of the tiles dealt out by blocks, head by head; with one: of the first entries, one per pair
+    int* split_flags;
+    float* split_state;
+    uint32_t slot_first[kSplitSlots];   // first tile of a slot (12 bits) and first key block of it
+};
+
 constexpr int kUnitRing = 4;
 
 // PACK: few query rows and several query heads per kv head.  The rows of all these heads share one 128-row tile (row = head * Nq +
@@ -145,6 +154,7 @@ struct Cfg {
     static_assert(cSfP + 8 <= 512, "tensor memory");
     static constexpr uint64_t kSwzQK = (D == 128) ? kSwz64 : kSwz32;
     static constexpr uint32_t kSboQK = (D == 128) ? 512 : 256;
+    static constexpr size_t kState = split_state_floats(D);      // of a tile that two CTAs share
 };
 
 template <typename OutT> __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -262,10 +272,57 @@ __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
     return true;
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK, bool CARRY, bool ROLL>
+__device__ __forceinline__ float4 load_state(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+// Tile number j of those dealt out by key blocks.  Without a mask head by head; with one in the order of the pairs, of which the first ones of an odd number of
+// tiles per head have one tile.
+template <bool CAUSAL>
+__host__ __device__ __forceinline__ void rest_tile(int j, int nqt, int BHq, int whole, int rest0, int& bhq, int& mt) {
+    if (!CAUSAL) {
+        bhq = (rest0 + j) / nqt;
+        mt = rest0 + j - bhq * nqt;
+        return;
+    }
+    const int npair = (nqt + 1) >> 1, one = rest0;
+    const int pair = j < one ? whole + j : whole + one + ((j - one) >> 1);
+    bhq = pair % BHq;
+    mt = 2 * (npair - 1 - pair / BHq) + (j < one ? 0 : 1 - ((j - one) & 1));
+}
+
+// Key blocks of a query tile.
+template <bool CAUSAL>
+__host__ __device__ __forceinline__ int tile_blocks(int mt, int Nk, int shift) {
+    const int last = CAUSAL && mt * kBlock + kBlock - 1 + shift < Nk - 1 ? mt * kBlock + kBlock - 1 + shift : Nk - 1;
+    return last < 0 ? 0 : last / kBlock + 1;
+}
+
+// The part of tile j of the rest from key block lo on, `left` blocks of it at most, in slot m.
+template <bool CAUSAL>
+__device__ __forceinline__ void make_part(const SplitParams& p, int j, int lo, int left, int m, Unit& w) {
+    rest_tile<CAUSAL>(j, p.nqt, p.BHq, p.whole_units, p.rest0, w.bhq, w.mt0);
+    const int b = w.bhq / p.Hq, nb = tile_blocks<CAUSAL>(w.mt0, p.Nk, p.causal_shift), hi = min(nb, lo + left);
+    w.hq = w.bhq % p.Hq;
+    w.bhkv = b * p.Hkv + w.hq / (p.Hq / p.Hkv);
+    w.Nq = p.Nq;
+    w.Nk = p.Nk;
+    w.shift = p.causal_shift;
+    w.out_base = b * p.os0;
+    w.nv = 1;
+    w.two = w.d = 0;
+    w.nbmax = hi;
+    w.ns = w.nb[0] = hi - lo;
+    w.nb[1] = (hi < nb ? m : 0) | (lo > 0 ? m + 1 : 0) << 16;      // goes on from slot m - 1's part; leaves its own under m
+}
+
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK, int CARRY, bool ROLL>
 __global__ void __launch_bounds__(Cfg<D, PACK>::kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ AttnParams p) {
+                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_d,
+                const __grid_constant__ std::conditional_t<CARRY == 2, SplitParams, AttnParams> p) {
     using C = Cfg<D, PACK>;
     constexpr int S = C::kStages;
     extern __shared__ uint8_t smem_dyn[];
@@ -338,7 +395,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = uniform(*tmem_slot);
-    const bool carry_in = CARRY && p.carry_o_in != nullptr, carry_out = CARRY && p.carry_o_out != nullptr;
+    constexpr bool STATE = CARRY == 1, SPLIT = CARRY == 2;       // carried from call to call; from CTA to CTA
+    const bool carry_in = STATE && p.carry_o_in != nullptr, carry_out = STATE && p.carry_o_out != nullptr;
+    // SPLIT: slot whose accumulator this unit goes on from, and slot under which it leaves its own (-1: none).  A unit of one tile keeps them in nb[1].
+    auto part_in = [](const Unit& u) { return SPLIT && u.nv == 1 ? (u.nb[1] & 0xffff) - 1 : -1; };
+    auto part_out = [](const Unit& u) { return SPLIT && u.nv == 1 ? (u.nb[1] >> 16) - 1 : -1; };
 
     // Register budget: 768 threads start with 80 registers each, and that allocation (61 440) is all the CTA can
     // ever hold: 128 x kRoleRegs for warpgroup 0 (the copy and MMA roles) + 128 x kCorrRegs for the correction
@@ -353,7 +414,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // Carried state, us per three ranges attended (16 heads, 8 192 queries, ranges of 8 192 keys; D = 128 without / with a mask, D = 64 likewise): halves rolled, one
     // wait per item, row sums in registers 1 134, 676, 1 061, 603.  Sums in shared memory and, at D = 128, the halves unrolled 1 129, 660; at D = 64 rolled, the
     // factor waited for ahead of P and the output loop unrolled 1 048, 594.  Across: D = 128 rolled with the rest 1 130, 672, D = 64 unrolled 1 057, 610.
-    constexpr bool kFactorFirst = CARRY && ROLL;
+    constexpr bool kFactorFirst = STATE && ROLL;
     // A CTA runs unit after unit (the grid is one CTA per SM): the producer draws the next unit's number from a counter and
     // publishes the unit in shared memory, so the loads, scores and exponentials of the next unit fill in while the last one
     // drains, and uneven units (causal masks, packed batches) level out.
@@ -384,7 +445,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
           const Unit& w = *u;
           const int ns = w.ns, two = w.two, d = w.d;
-          for (int t = 0; t < w.nv; ++t) {
+          const int pin = part_in(w);
+          if constexpr (SPLIT) if (pin >= 0) {
+              // resume another CTA's tile
+              if (!warp_wait_word(p.split_flags + pin, 4, abort_flag, p.status, kWaitPart)) { ok = false; break; }
+              const float* state = p.split_state + (size_t)pin * C::kState;
+              l_s[0] = make_float2(load_written(state + 128 * D + 2 * row), load_written(state + 128 * D + 2 * row + 1));
+              const float4* from = reinterpret_cast<const float4*>(state) + row;
+#pragma unroll 1
+              for (uint32_t o_addr = tmem + lane_addr + C::cO, end = o_addr + D; o_addr != end; o_addr += 32, from += 8 * 128) {
+                  float o[32];
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) {
+                      const float4 v4 = load_state(from + q * 128);
+                      o[4 * q] = v4.x; o[4 * q + 1] = v4.y; o[4 * q + 2] = v4.z; o[4 * q + 3] = v4.w;
+                  }
+                  tmem_st16(o_addr, o);
+                  tmem_st16(o_addr + 16, o + 16);
+              }
+              tc_wait_st();
+          }
+          for (int t = 0; (!SPLIT || pin < 0) && t < w.nv; ++t) {
               l_s[t * 128] = make_float2(0.f, 0.f);
               m_s[t * 128] = -INFINITY;
               const int grow = (w.mt0 + t) * kBlock + row;
@@ -445,6 +526,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               m_s[0] = m;
           }
           float2 l0 = make_float2(0.f, 0.f), l1 = l0;              // running row sums of the two tiles (carried state: in l_s)
+          if (SPLIT && pin >= 0) l0 = l_s[0];
           for (int s = 0; PACK != 2 && s < ns; ++s) {
               const int sg = base + s, slot = sg & 7, ph = (sg >> 3) & 1;
               const int t = (s + d) & two;
@@ -458,7 +540,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const float2 ma = stat[slot * 128];
               const float alpha = ma.y;
               // the first block has nothing to rescale unless the accumulator was carried in
-              if ((!first || carry_in) && __any_sync(0xffffffffu, alpha != 1.0f)) {
+              if ((!first || carry_in || (SPLIT && part_in(w) >= 0)) && __any_sync(0xffffffffu, alpha != 1.0f)) {
                   // the P V MMA of the tile's previous block must have landed first
                   if (!first) {
                       const int sp = sg - 1 - two;
@@ -486,22 +568,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   rs = sum[slot * 128];
               }
               warp_arrive(bar(bOS + slot), lane);
-              float2 l = CARRY ? l_s[t * 128] : t ? l1 : l0;
+              float2 l = STATE ? l_s[t * 128] : t ? l1 : l0;
               l.x = fmaf(l.x, alpha, rs.x);
               l.y = fmaf(l.y, alpha, rs.y);
-              if (CARRY) l_s[t * 128] = l; else if (t) l1 = l; else l0 = l;
+              if (STATE) l_s[t * 128] = l; else if (t) l1 = l; else l0 = l;
               m_s[t * 128] = ma.x;
           }
-          if (PACK != 2 && !CARRY) {
+          if (PACK != 2 && !STATE) {
               l_s[0] = l0;
               l_s[128] = l1;
           }
+          const int pout = part_out(w);
           // ---------------------------------------------------------------- O / l of the unit's tiles
           // (The accumulators belong to the next unit once this warpgroup arrives for its first items.  PACK == 2: the warps without rows
           // stay away, the pipeline does not wait for them, and the barrier below may be two phases on by the time they look.)
           for (int t = 0; ok && broken == 0 && (PACK != 2 || quarter == 0) && t < w.nv; ++t) {
               const int grow = PACK ? prow_tok : (w.mt0 + t) * kBlock + row;
-              const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq;
+              const bool live = PACK ? prow_head < w.nb[1] : grow < w.Nq && (!SPLIT || pout < 0);
               const int bhq = w.bhq + prow_head, hq = w.hq + prow_head;
               const bool have = w.nb[t] > 0 || carry_in;
               const float2 l2 = l_s[t * 128];
@@ -548,6 +631,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
                       for (int q = 0; q < 16; ++q) o[q] = 0.f;
                   }
+                  if constexpr (SPLIT) if (pout >= 0) {
+                      float4* state = reinterpret_cast<float4*>(p.split_state + (size_t)pout * C::kState) + row;
+#pragma unroll
+                      for (int q = 0; q < 4; ++q) state[(c / 4 + q) * 128] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                  }
                   if (carry_out && live) {
 #pragma unroll
                       for (int q = 0; q < 4; ++q)
@@ -571,6 +659,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                   }
               }
           }
+          if constexpr (SPLIT) if (ok && pout >= 0) {
+              float* state = p.split_state + (size_t)pout * C::kState + 128 * D;
+              *reinterpret_cast<float2*>(state + 2 * row) = l_s[0];
+              state[256 + row] = m_s[0];
+              __threadfence();
+              __syncwarp();
+              if (lane == 0) atomicAdd(p.split_flags + pout, 1);
+          }
           unit_done(i);
           base += ns;
       }
@@ -586,7 +682,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
         int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
-        int next = 0, head = 0;                   // the unit after this one (lane 0); PACK: next head of a unit whose heads go one by one
+        int next = 0, head = 0;                   // the unit after this one (lane 0); PACK: next head of a unit whose heads go one by one; SPLIT: next part of a slot
+        int tile = 0, lo = 0, left = 0;           // SPLIT: of the slot, tile and first key block of its next part, key blocks left
         // V is loaded kLag blocks behind K.  A V stage is free four blocks after its K stage (scores, softmax and P lie between), and
         // with as few stages as D = 128 has room for, the K that the issuers want next would otherwise queue behind a V that
         // nobody is waiting for yet: they waited 740 cycles for every second item in an earlier kernel.  In this one the lag is worth little (us per call,
@@ -606,12 +703,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         };
         bool ok = true;
         while (ok) {
-            if (!PACK || head == 0) next = 0;     // (where heads never go one by one nothing is carried round the loop: 0.3 % at 8 192 keys)
+            if (!(PACK || SPLIT) || head == 0) next = 0;     // (where heads never go one by one nothing is carried round the loop: 0.3 % at 8 192 keys)
             if (lane == 0 && head == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
             Unit w;
             const bool more = u < p.units;
             if (!more) w.ns = -1;
-            else if (!make_unit<CAUSAL, VARLEN, PACK>(p, u, w)) { u = uniform(next); continue; }
+            else if (SPLIT && u >= p.whole_units) {
+                if constexpr (SPLIT) {
+                    const int m = u - p.whole_units;
+                    if (head == 0) {
+                        const uint32_t first = p.slot_first[m];
+                        tile = first & 0xfff;
+                        lo = first >> 12;
+                        left = m == 0 ? p.slot_rest : p.slot_blocks;
+                    }
+                    make_part<CAUSAL>(p, tile, lo, left, m, w);
+                }
+            } else if (!make_unit<CAUSAL, VARLEN, PACK>(p, u, w)) { u = uniform(next); continue; }
             // Heads that share a tile share the operand that adds delta_s (eight rows of it, the next heads' too), and 0 x NaN is NaN: where
             // one of the kv heads behind these rows has a delta_s that is not finite, the unit's heads are published one by one.
             bool last_head = true;
@@ -626,7 +734,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     }
                 }
             }
+            if (SPLIT && more && u >= p.whole_units) last_head = left == w.ns;
+            const int lowest = SPLIT && more && u >= p.whole_units ? lo : 0;
             auto advance = [&] {
+                if (SPLIT && u >= p.whole_units) {
+                    ++tile;
+                    lo = 0;
+                    left -= w.ns;
+                }
                 if (last_head) u = uniform(next);
                 head = last_head ? 0 : head + 1;
             };
@@ -679,7 +794,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                               C::kSfQkBytes, bar(bQF + qb));
                 }
             }
-            for (int n = w.nbmax - 1; n >= 0; --n) {
+            for (int n = w.nbmax - 1; n >= lowest; --n) {
                 if (!warp_wait<true>(bar(bKE + st), st_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
                 if (lane == 0) {
                     mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (box ? 8 : w.nv) * C::kDeltaBytes);
@@ -822,6 +937,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const Unit* u;
         for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
             const int ns = uniform(u->ns), two = uniform(u->two), d = uniform(u->d);
+            const bool resumed = carry_in || uniform(part_in(*u)) >= 0;
             unit_done(i);
             for (int s = 0; s < ns; ++s) {
                 const int slot = (base + s) & 7, t = (s + d) & two;
@@ -841,7 +957,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks)
                         tc_mma_nvfp4(o_col, sdesc(p_lo + 2 * ks, hi_pv), sdesc(v_lo + 2 * ks, hi_pv), idesc_pv, sfp_col + 4 * ks, sfv_col + 4 * ks,
-                                     s > two || (ks > 0) || carry_in);
+                                     s > two || (ks > 0) || resumed);
                     tc_commit(bar(bPV + slot));
                     if (closes) tc_commit(bar(bVE + st));
                 }
@@ -988,7 +1104,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 if (s > two) {
                     if (!warp_wait(bar(bM + slot_prev * 4 + quarter), ((sg - 1 - two) >> 3) & 1, abort_flag, p.status, kWaitPair)) return false;
                     m_old = stat[slot_prev * 128].x;
-                } else if (CARRY) {
+                } else if constexpr (SPLIT) {
+                    const int pin = uniform(part_in(*u));
+                    if (pin >= 0) {
+                        if (!warp_wait_word(p.split_flags + pin, 4, abort_flag, p.status, kWaitPart)) return false;
+                        m_old = load_written(p.split_state + (size_t)pin * C::kState + 128 * (D + 2) + r);
+                    }
+                } else if (STATE) {
                     if (carry_in && trow + r < u->Nq) m_old = p.carry_m_in[(size_t)u->bhq * p.Nq + trow + r];
                 }
                 return true;
@@ -1171,14 +1293,14 @@ int encode_tiled_bytes(void* map64, const void* base, uint64_t n0, uint64_t n1, 
     return (int)make_map(fn, static_cast<CUtensorMap*>(map64), base, n0, n1, n2, b0, b1, swz);
 }
 
-template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK, bool CARRY = false, bool ROLL = true>
+template <int D, bool CAUSAL, typename OutT, bool VARLEN, int PACK, int CARRY = 0, bool ROLL = true>
 static cudaError_t launch_v(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
-                            const AttnParams& p, int grid, cudaStream_t st) {
+                            const SplitParams& p, int grid, cudaStream_t st) {
     constexpr auto kern = attn_fwd_kernel<D, CAUSAL, OutT, VARLEN, PACK, CARRY, ROLL>;
     using C = Cfg<D, PACK>;
     cudaError_t e = allow_smem<kern>(C::kSmemBytes);
     if (e != cudaSuccess) return e;
-    return launch(true, kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, p);
+    return launch(true, kern, dim3(grid), dim3(C::kThreads), C::kSmemBytes, st, tq, tk, tv, td, static_cast<const std::conditional_t<CARRY == 2, SplitParams, AttnParams>&>(p));
 }
 
 // D = 64 without a mask, more key blocks than this: the halves of an item unrolled.  us per call, rolled / unrolled: 226 keys (2 x 48 heads,
@@ -1191,17 +1313,83 @@ constexpr int kRolledBlocks = 8, kRolledBlocksPacked = 32;
 
 template <int D, bool CAUSAL, typename OutT>
 static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& td,
-                            const AttnParams& p, int pack_mode, int grid, cudaStream_t st) {
+                            const SplitParams& p, int pack_mode, int grid, cudaStream_t st) {
     // packed variable-length batches and carried state run their own instantiations, so that the other kernels carry none of it
     const bool carry = a.carry_o_in != nullptr || a.carry_o_out != nullptr;
     constexpr bool roll = D == 128 || CAUSAL;        // at every length
-    return a.cu_q != nullptr && !roll && p.nkb > kRolledBlocksPacked ? launch_v<D, CAUSAL, OutT, true, 0, false, roll>(tq, tk, tv, td, p, grid, st)
+    return a.cu_q != nullptr && !roll && p.nkb > kRolledBlocksPacked ? launch_v<D, CAUSAL, OutT, true, 0, 0, roll>(tq, tk, tv, td, p, grid, st)
            : a.cu_q != nullptr ? launch_v<D, CAUSAL, OutT, true, 0>(tq, tk, tv, td, p, grid, st)
-           : carry            ? launch_v<D, CAUSAL, OutT, false, 0, true, D == 64>(tq, tk, tv, td, p, grid, st)
+           : carry            ? launch_v<D, CAUSAL, OutT, false, 0, 1, D == 64>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 2   ? launch_v<D, CAUSAL, OutT, false, 2>(tq, tk, tv, td, p, grid, st)
            : pack_mode == 1   ? launch_v<D, CAUSAL, OutT, false, 1>(tq, tk, tv, td, p, grid, st)
-           : !roll && p.nkb > kRolledBlocks ? launch_v<D, CAUSAL, OutT, false, 0, false, roll>(tq, tk, tv, td, p, grid, st)
+           : p.slot_blocks > 0 ? launch_v<D, CAUSAL, OutT, false, 0, 2>(tq, tk, tv, td, p, grid, st)
+           : !roll && p.nkb > kRolledBlocks ? launch_v<D, CAUSAL, OutT, false, 0, 0, roll>(tq, tk, tv, td, p, grid, st)
                               : launch_v<D, CAUSAL, OutT, false, 0>(tq, tk, tv, td, p, grid, st);
+}
+
+// The last rounds of units dealt out by key blocks.  Units are pairs of tiles, and 5.5 pairs per SM take as long as 6, 0.86 as long as 1: the tiles of the
+// round that is not full (where that is less than half full, of the one before too) are cut into slots of as many key blocks as come to one SM, in the
+// order tile after tile, blocks of a tile from its first key on (McNaughton 1959).  A CTA draws one slot and takes its parts in that order.  A tile lies in
+// one slot or two: the one behind has its last keys, at its own start, walks them, and leaves the accumulator, row sums and maxima in memory; the one
+// before has its first keys, at its end, and goes on from there.  So the same operations in the same order, and the same bits, as in one walk.  Slots are
+// drawn from the last to the first: the part that is waited for belongs to a slot drawn before, where it comes first and waits for nothing, so some CTA can
+// always go on, however many of them are resident.
+// us per call, without / with: 1 000 queries x 9 192 keys, 32 heads 139.3 / 127.9, 1 500 x 12 000, 28 heads 246.8 / 200.9, 600 x 5 000 84.5 / 61.3; 4 250 tokens
+// of 48 heads, D = 64 349.0 / 333.9; N tokens of H heads, D = 128 (64): 16 x 2 500 72.4 / 63.7 (63.8 / 55.4), 10 x 4 100 104.5 / 90.2 (94.3 / 80.4), 16 x 5 000 194.9
+// / 180.4 (174.3 / 162.3), 24 x 5 000 269.2 / 259.0 (239.7 / 233.2), 5 x 16 384 532 / 476 (498 / 454).
+// What it costs: some 8 blocks per slot (two more changes of units, 64 KB of accumulator in and out), and at D = 64 without a mask the rolled halves.  So: from 10 blocks
+// of gain, 1 / 80 of the call (less shows nothing: 16 384 x 24 heads, 1.15 %, 2 192 / 2 182, 8 192 x 32, 1.1 %, 792 / 794), there 1 / 25 (24 x 6 000, 3.2 %, 312 / 313, 40 x 5 000,
+// 1.6 %, 372 / 379).  With a mask only where it is that of a chunk of a longer sequence (tiles differ by a quarter of their blocks at most): pairs in order of their
+// length level out by themselves otherwise.
+struct SplitPlan { int whole = 0, slots = 0; };      // pairs ahead of the slots
+
+template <bool CAUSAL>
+static SplitPlan plan_split(const AttnArgs& a, int mode, int nqt, int pairs, int sms, SplitParams& p) {
+    p.slot_blocks = 0;
+    p.split_flags = a.split_flags;
+    p.split_state = a.split_state;
+    SplitPlan none, plan;
+    if (a.split_flags == nullptr || mode != 0 || a.cu_q != nullptr || a.carry_o_in != nullptr || a.carry_o_out != nullptr || sms > kSplitSlots) return none;
+    const int BHq = a.B * a.Hq, last = tile_blocks<CAUSAL>(nqt - 1, a.Nk, a.causal_shift);
+    if (last < kSplitMinBlocks || 4 * tile_blocks<CAUSAL>(0, a.Nk, a.causal_shift) < 3 * last) return none;
+    const int full = pairs / sms, over = pairs % sms;
+    const bool that_round = nqt > 1 && 2 * over > sms;      // the round that is not full is enough
+    if (over == 0 || (!that_round && full == 0)) return none;
+    plan.whole = pairs - over - (that_round ? 0 : sms);
+    // tiles of the rest
+    const int npair = (nqt + 1) / 2;
+    int tiles;
+    if (CAUSAL) {
+        p.rest0 = (nqt & 1) && plan.whole < BHq ? BHq - plan.whole : 0;
+        tiles = p.rest0 + 2 * (pairs - plan.whole - p.rest0);
+    } else {
+        p.rest0 = plan.whole / npair * nqt + 2 * (plan.whole % npair);
+        tiles = BHq * nqt - p.rest0;
+    }
+    auto blocks = [&](int j) {
+        int bhq, mt;
+        rest_tile<CAUSAL>(j, nqt, BHq, plan.whole, p.rest0, bhq, mt);
+        return tile_blocks<CAUSAL>(mt, a.Nk, a.causal_shift);
+    };
+    int sum = 0, most = 0;
+    for (int j = 0; j < tiles; ++j) {
+        const int n = blocks(j);
+        sum += n;
+        most = n > most ? n : most;
+    }
+    const int per = (sum + sms - 1) / sms > most ? (sum + sms - 1) / sms : most;
+    // blocks the rest takes without: its pairs in one round, or a round and one of single tiles (where a head has one tile, two of these)
+    const int before = that_round || nqt == 1 ? 2 * most : 3 * most, all = plan.whole / sms * (nqt == 1 ? 1 : 2) * most + before;
+    if (before - per < 10 || (before - per) * (a.D == 64 && !CAUSAL ? 25 : 80) < all) return none;
+    plan.slots = (sum + per - 1) / per;
+    p.slot_blocks = per;
+    p.slot_rest = sum - (plan.slots - 1) * per;
+    for (int j = 0, at = 0, i = 0; j < tiles && i < plan.slots; ++j) {      // slot plan.slots - 1 - i begins at block i * per of all tiles' blocks
+        const int n = blocks(j);
+        for (; i < plan.slots && i * per < at + n; ++i) p.slot_first[plan.slots - 1 - i] = (uint32_t)j | (uint32_t)(i * per - at) << 12;
+        at += n;
+    }
+    return plan;
 }
 
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
@@ -1235,7 +1423,7 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     const cudaError_t e = current_device(&dev, &info);
     if (e != cudaSuccess) return e;
     const int sms = info.sms;
-    AttnParams p;
+    SplitParams p;
     // Units of work: pairs of query tiles; when the last round of pairs fills at most half of the SMs it is dealt out as
     // single tiles (half the time for the round, twice the SMs).  With more than that single tiles need two rounds and lose the shared
     // K and V stages.  148 SMs, heads x 2 048 tokens, D = 128, never / this rule / always single: 68 pairs over 81.8 / 71.8 / 71.7 us,
@@ -1243,10 +1431,11 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), rest = pairs % sms;
     const bool split = nqt > 1 && 2 * rest <= sms;
     p.unit_counter = a.unit_counter;
-    p.whole_units = split ? pairs - rest : pairs;
+    const SplitPlan plan = a.is_causal ? plan_split<true>(a, mode, nqt, pairs, sms, p) : plan_split<false>(a, mode, nqt, pairs, sms, p);
+    p.whole_units = plan.slots > 0 ? plan.whole : split ? pairs - rest : pairs;
     p.pack_heads = pack;
     p.pack_tiles = (group + pack - 1) / pack;
-    p.units = mode ? a.B * a.Hkv * p.pack_tiles : split ? pairs + rest : pairs;
+    p.units = mode ? a.B * a.Hkv * p.pack_tiles : plan.slots > 0 ? plan.whole + plan.slots : split ? pairs + rest : pairs;
     const int grid = p.units < sms ? p.units : sms;
     p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;

@@ -16,7 +16,7 @@ constexpr int kMicro = 16;    // NVFP4 microblock
 enum : int {
     kWaitQFull = 101, kWaitKFull = 102, kWaitVFull = 103, kWaitKEmpty = 104, kWaitVEmpty = 105,
     kWaitSFull = 106, kWaitSEmpty = 107, kWaitPFull = 108, kWaitOReady = 109, kWaitPair = 110,
-    kWaitPEmpty = 113, kWaitAlpha = 114, kWaitOScaled = 112, kWaitDeltaMma = 116, kWaitDeltaA = 117, kWaitUnit = 118, kWaitSelfTest = 199
+    kWaitPEmpty = 113, kWaitAlpha = 114, kWaitOScaled = 112, kWaitDeltaMma = 116, kWaitDeltaA = 117, kWaitUnit = 118, kWaitPart = 119, kWaitSelfTest = 199
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -182,6 +182,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                 return false;
             }
         }
+    }
+}
+
+// Bounded wait of a whole warp until another CTA of the launch has raised the counter at `word` to `want`; what that CTA wrote before is then visible.
+__device__ __forceinline__ bool warp_wait_word(const int* word, int want, volatile int* abort_flag, int* status_word, int code) {
+    const uint32_t t0 = clock();
+    while (true) {
+        int v;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if (__all_sync(0xffffffffu, v >= want)) return true;
+        bool out = *abort_flag != 0;
+        if ((uint32_t)clock() - t0 > kWaitLimitCycles || *reinterpret_cast<volatile int*>(status_word) != 0) {
+            atomicCAS(status_word, 0, code);
+            *abort_flag = 1;
+            out = true;
+        }
+        if (__any_sync(0xffffffffu, out)) return false;
+        __nanosleep(100);
     }
 }
 

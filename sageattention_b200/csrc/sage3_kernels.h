@@ -35,6 +35,7 @@ struct PrepassArgs {
     int* clear;                    // words the first kernel zeroes: status words, the attention kernel's work counter, `nonfinite`
     int n_clear;
     int* nonfinite;                // per (batch, kv head): set when a delta_s value is not finite; nullptr: nobody asks (see PackRule)
+    int* split_flags;              // kSplitSlots words the first kernel zeroes too (nullptr: none)
     // packed variable-length sequences (both nullptr: every batch entry has Nq / Nk tokens): device int32 [B + 1], entry b
     // owns rows cu[b] .. cu[b + 1] of the packed tensor; Nq / Nk are then the maximum lengths, stride 0 is unused
     const int *cu_q, *cu_k;
@@ -60,7 +61,15 @@ struct AttnArgs {
     const int* prepass_status;      // the pre-pass's status word (non-zero: the workspace is incomplete, do nothing)
     const int* nonfinite;           // per (batch, kv head), from the pre-pass: delta_s holds values that are not finite
     const int *cu_q, *cu_k;         // packed variable-length sequences, as in PrepassArgs (nullptr: uniform lengths)
+    // Last round of units dealt out by key blocks (see SplitPlan); zeroed before the launch / scratch.  nullptr: not possible for these sizes.
+    int* split_flags;
+    float* split_state;
 };
+
+// The accumulator of a query tile whose keys two CTAs of the attention kernel share: fp32 O [D / 4][128 rows][4], row sums [128][2], maxima [128] per slot.
+constexpr int kSplitSlots = 160;      // CTAs (one per SM)
+constexpr int kSplitMinBlocks = 16;   // key blocks of a call, below which no tile is shared
+constexpr size_t split_state_floats(size_t D) { return 128 * D + 128 * 3; }
 
 // Few query rows and several heads per kv head (token generation): as many heads as fit share a 128-row tile, eight at most (the
 // operand that adds delta_s has eight rows); uniform lengths and no carried state only (`plain`).  Mode 2, where a warp takes a

@@ -1,0 +1,49 @@
+"""Last rounds of the attention kernel dealt out by key blocks: a query tile's keys may then be walked by two CTAs, the second going on from the accumulator
+the first leaves.  Numbers of pairs of tiles around one round and one and a half rounds of all SMs, one and two tiles per head, odd and even numbers of them, masks
+aligned at the bottom right, ragged ends: the bits of calls on one head alone, whose tiles are not shared, and the oracle's result."""
+import pytest
+import torch
+
+from oracle import sage3_oracle as O
+from sageattention_b200 import Sage3Problem, sageattn3
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H,group,Nq,Nk,causal", [
+    (75, 1, 200, 2048, False),        # 75 pairs on 148 SMs: just more than half a round
+    (74, 1, 200, 2048, False),        # half a round: single tiles, nothing shared
+    (136, 1, 256, 12000, False),      # 0.92 of a round
+    (160, 1, 100, 5000, False),       # one tile per head, a round and twelve
+    (230, 1, 90, 4000, False),        # ... and more than half a round
+    (149, 1, 130, 2100, False),       # a round and one pair: both rounds are dealt out
+    (100, 4, 384, 2500, False),       # odd: every other pair is one tile
+    (37, 1, 640, 3000, False),        # 111 pairs, five tiles per head
+    (300, 2, 129, 2048, False),       # two rounds and four
+    (32, 4, 1000, 9192, True),        # a chunk of a prompt: 128 pairs
+    (28, 7, 900, 5000, True),         # 112
+    (40, 5, 1153, 8000, True),        # ten tiles of a head in five pairs, 200 of them
+    (56, 7, 640, 4000, True),         # odd, 168 pairs, 56 of them one tile
+    (90, 1, 257, 2600, True),         # three tiles: the first pairs are one tile
+    (170, 2, 257, 2600, True),        # ... of which some are in the whole rounds
+    (40, 1, 1100, 6000, True),        # nine tiles: 200 pairs
+])
+def test_shared_tiles(cuda_device, D, H, group, Nq, Nk, causal):
+    g = torch.Generator(device=cuda_device).manual_seed(2100 + H)
+    q = torch.randn(1, H, Nq, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+    k, v = (torch.randn(1, H // group, Nk, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
+    p = Sage3Problem(q, k, v, is_causal=causal, return_lse=True)
+    for _ in range(2):                # (the second call finds the first one's flags and accumulators in the workspace)
+        p.run()
+    assert p.check_status() == 0
+    p.attention()                     # ... and the attention stage on its own
+    assert p.check_status() == 0
+    for h in range(0, H, max(1, H // 12)):
+        one, lse = sageattn3(q[:, h:h + 1], k[:, h // group:h // group + 1], v[:, h // group:h // group + 1], is_causal=causal, return_lse=True)
+        assert torch.equal(p.out[:, h:h + 1], one) and torch.equal(p.lse[:, h:h + 1], lse), h
+    # rows of a tile around the boundaries of slots: the whole head against 64-bit attention with the oracle's gate
+    h = H // 2
+    ref = O.sageattn3_oracle(q[:, h:h + 1, :].cpu(), k[:, h // group:h // group + 1].cpu(), v[:, h // group:h // group + 1].cpu(), is_causal=causal) if Nk <= 3000 else None
+    if ref is not None:
+        assert O.cosine(p.out[:, h:h + 1].cpu(), ref) >= 0.999 and O.rel_l1(p.out[:, h:h + 1].cpu(), ref) <= 0.01
