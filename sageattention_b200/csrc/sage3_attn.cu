@@ -87,7 +87,7 @@ struct AttnParams {
 // Of the kernels whose last rounds are dealt out by key blocks: units from whole_units on are slots, see SplitPlan.
 struct SplitParams : AttnParams {
     int slot_blocks, slot_rest;         // key blocks per slot; of slot 0
-    int rest0;                          // without a mask: first of the tiles dealt out by blocks, head by head; with one: of the first entries, one per pair
+    int rest0;                          // see rest_tile
     int* split_flags;
     float* split_state;
     uint32_t slot_first[kSplitSlots];   // first tile of a slot (12 bits) and first key block of it
@@ -201,7 +201,7 @@ struct __align__(16) Unit {
 // Unit number u of the launch; false when it is empty (beyond a short sequence of a packed batch).
 // Order: without a mask pairs of tiles of one head are neighbours (its K and V are shared in L2); under a causal mask the
 // pairs with the most keys of all heads come first, so that the short ones level out the end of the launch.
-template <bool CAUSAL, bool VARLEN, int PACK>
+template <bool CAUSAL, bool VARLEN, int PACK, bool SPLIT>
 __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
     if constexpr (PACK) {
         w.bhkv = u / p.pack_tiles;
@@ -220,7 +220,7 @@ __device__ __forceinline__ bool make_unit(const AttnParams& p, int u, Unit& w) {
         w.two = w.d = 0;
         return true;
     }
-    const int npair = (p.nqt + 1) >> 1;
+    const int npair = (p.nqt + (SPLIT && !CAUSAL ? 0 : 1)) >> 1;      // (SPLIT, see rest_tile)
     int pair = u, half = -1;
     if (u >= p.whole_units) {                      // the last units are single tiles
         pair = p.whole_units + ((u - p.whole_units) >> 1);
@@ -278,13 +278,19 @@ __device__ __forceinline__ float4 load_state(const float4* p) {
     return v;
 }
 
-// Tile number j of those dealt out by key blocks.  Without a mask head by head; with one in the order of the pairs, of which the first ones of an odd number of
-// tiles per head have one tile.
+// Tile number j of those dealt out by key blocks.  Without a mask the last ones of an odd number of tiles per head (whole units are pairs then, so that the rounds
+// ahead are even), and the tiles from pair number rest0 / 2 on; with one in the order of the pairs, of which the first rest0 have one tile.
 template <bool CAUSAL>
 __host__ __device__ __forceinline__ void rest_tile(int j, int nqt, int BHq, int whole, int rest0, int& bhq, int& mt) {
     if (!CAUSAL) {
-        bhq = (rest0 + j) / nqt;
-        mt = rest0 + j - bhq * nqt;
+        const int odd = nqt & 1 ? BHq : 0;
+        if (j < odd) {
+            bhq = j;
+            mt = nqt - 1;
+        } else {
+            bhq = (rest0 + j - odd) / (nqt & ~1);
+            mt = rest0 + j - odd - bhq * (nqt & ~1);
+        }
         return;
     }
     const int npair = (nqt + 1) >> 1, one = rest0;
@@ -719,7 +725,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     }
                     make_part<CAUSAL>(p, tile, lo, left, m, w);
                 }
-            } else if (!make_unit<CAUSAL, VARLEN, PACK>(p, u, w)) { u = uniform(next); continue; }
+            } else if (!make_unit<CAUSAL, VARLEN, PACK, SPLIT>(p, u, w)) { u = uniform(next); continue; }
             // Heads that share a tile share the operand that adds delta_s (eight rows of it, the next heads' too), and 0 x NaN is NaN: where
             // one of the kv heads behind these rows has a delta_s that is not finite, the unit's heads are published one by one.
             bool last_head = true;
@@ -1328,7 +1334,7 @@ static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUte
 }
 
 // The last rounds of units dealt out by key blocks.  Units are pairs of tiles, and 5.5 pairs per SM take as long as 6, 0.86 as long as 1: the tiles of the
-// round that is not full (where that is less than half full, of the one before too) are cut into slots of as many key blocks as come to one SM, in the
+// round that is not full (of the one before too, where that leaves less than a tile per SM) are cut into slots of as many key blocks as come to one SM, in the
 // order tile after tile, blocks of a tile from its first key on (McNaughton 1959).  A CTA draws one slot and takes its parts in that order.  A tile lies in
 // one slot or two: the one behind has its last keys, at its own start, walks them, and leaves the accumulator, row sums and maxima in memory; the one
 // before has its first keys, at its end, and goes on from there.  So the same operations in the same order, and the same bits, as in one walk.  Slots are
@@ -1340,7 +1346,8 @@ static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUte
 // What it costs: some 8 blocks per slot (two more changes of units, 64 KB of accumulator in and out), and at D = 64 without a mask the rolled halves.  So: from 10 blocks
 // of gain, 1 / 80 of the call (less shows nothing: 16 384 x 24 heads, 1.15 %, 2 192 / 2 182, 8 192 x 32, 1.1 %, 792 / 794), there 1 / 25 (24 x 6 000, 3.2 %, 312 / 313, 40 x 5 000,
 // 1.6 %, 372 / 379).  With a mask only where it is that of a chunk of a longer sequence (tiles differ by a quarter of their blocks at most): pairs in order of their
-// length level out by themselves otherwise.
+// length level out by themselves otherwise.  The rounds ahead have to be even, since a CTA's slot is as long as any other's: 2 x 32 heads x 10 590 tokens, 83 tiles per head of which
+// one was a unit of its own in them, 2 526 / 2 555.
 struct SplitPlan { int whole = 0, slots = 0; };      // pairs ahead of the slots
 
 template <bool CAUSAL>
@@ -1352,42 +1359,55 @@ static SplitPlan plan_split(const AttnArgs& a, int mode, int nqt, int pairs, int
     if (a.split_flags == nullptr || mode != 0 || a.cu_q != nullptr || a.carry_o_in != nullptr || a.carry_o_out != nullptr || sms > kSplitSlots) return none;
     const int BHq = a.B * a.Hq, last = tile_blocks<CAUSAL>(nqt - 1, a.Nk, a.causal_shift);
     if (last < kSplitMinBlocks || 4 * tile_blocks<CAUSAL>(0, a.Nk, a.causal_shift) < 3 * last) return none;
-    const int full = pairs / sms, over = pairs % sms;
-    const bool that_round = nqt > 1 && 2 * over > sms;      // the round that is not full is enough
-    if (over == 0 || (!that_round && full == 0)) return none;
-    plan.whole = pairs - over - (that_round ? 0 : sms);
-    // tiles of the rest
-    const int npair = (nqt + 1) / 2;
-    int tiles;
+    const bool odd = (nqt & 1) != 0;
+    int tiles;                        // dealt out by blocks
+    double before;                    // blocks per SM without slots
     if (CAUSAL) {
-        p.rest0 = (nqt & 1) && plan.whole < BHq ? BHq - plan.whole : 0;
+        const int full = pairs / sms, over = pairs % sms;
+        const bool that_round = 2 * over > sms;      // the round that is not full is enough
+        if (over == 0 || (!that_round && full == 0)) return none;
+        plan.whole = pairs - over - (that_round ? 0 : sms);
+        if (odd && plan.whole > 0) return none;      // (the rounds ahead of the slots are not even)
+        p.rest0 = odd ? BHq : 0;
         tiles = p.rest0 + 2 * (pairs - plan.whole - p.rest0);
+        before = nqt == 1 ? (full + 1) * (double)last : (2 * full + (that_round ? 2 : 1) - (odd ? 0.5 : 0)) * last;      // (odd: units of one tile among them level out)
     } else {
-        p.rest0 = plan.whole / npair * nqt + 2 * (plan.whole % npair);
-        tiles = BHq * nqt - p.rest0;
+        // rounds of whole pairs ahead such that one to three tiles per SM are left
+        const int64_t all = (int64_t)BHq * nqt;
+        const int whole_pairs = BHq * (nqt / 2);
+        int64_t rounds = all / (2 * sms);
+        if (rounds > 0 && all - rounds * 2 * sms < sms) --rounds;
+        if (rounds * sms > whole_pairs || all - rounds * 2 * sms > 4 * sms || all <= sms) return none;
+        plan.whole = (int)rounds * sms;
+        p.rest0 = 2 * plan.whole;
+        tiles = (int)(all - p.rest0);
+        const int full = pairs / sms, over = pairs % sms;
+        // (an odd number of tiles per head: one unit of a head is a single tile, which levels out half of a tile)
+        before = nqt == 1 ? (double)((all + sms - 1) / sms) * last
+               : odd      ? ((double)all / sms + 0.5) * last
+                          : (2 * full + (over == 0 ? 0 : 2 * over > sms ? 2 : 1)) * (double)last;
     }
     auto blocks = [&](int j) {
         int bhq, mt;
         rest_tile<CAUSAL>(j, nqt, BHq, plan.whole, p.rest0, bhq, mt);
         return tile_blocks<CAUSAL>(mt, a.Nk, a.causal_shift);
     };
-    int sum = 0, most = 0;
-    for (int j = 0; j < tiles; ++j) {
-        const int n = blocks(j);
-        sum += n;
-        most = n > most ? n : most;
-    }
+    int sum = CAUSAL ? 0 : tiles * last, most = last;
+    for (int j = 0; CAUSAL && j < tiles; ++j) sum += blocks(j);
     const int per = (sum + sms - 1) / sms > most ? (sum + sms - 1) / sms : most;
-    // blocks the rest takes without: its pairs in one round, or a round and one of single tiles (where a head has one tile, two of these)
-    const int before = that_round || nqt == 1 ? 2 * most : 3 * most, all = plan.whole / sms * (nqt == 1 ? 1 : 2) * most + before;
-    if (before - per < 10 || (before - per) * (a.D == 64 && !CAUSAL ? 25 : 80) < all) return none;
+    const double gain = before - per - plan.whole / sms * 2.0 * last;
+    if (gain < 10 || gain * (a.D == 64 && !CAUSAL ? 25 : 80) < before) return none;
     plan.slots = (sum + per - 1) / per;
     p.slot_blocks = per;
     p.slot_rest = sum - (plan.slots - 1) * per;
-    for (int j = 0, at = 0, i = 0; j < tiles && i < plan.slots; ++j) {      // slot plan.slots - 1 - i begins at block i * per of all tiles' blocks
-        const int n = blocks(j);
-        for (; i < plan.slots && i * per < at + n; ++i) p.slot_first[plan.slots - 1 - i] = (uint32_t)j | (uint32_t)(i * per - at) << 12;
-        at += n;
+    for (int i = 0, j = 0, at = 0; i < plan.slots; ++i) {      // slot plan.slots - 1 - i begins at block i * per of all tiles' blocks; tile j's first one is number `at`
+        if (!CAUSAL) {
+            j = i * per / last;
+            at = j * last;
+        } else {
+            for (int n; at + (n = blocks(j)) <= i * per; ++j) at += n;
+        }
+        p.slot_first[plan.slots - 1 - i] = (uint32_t)j | (uint32_t)(i * per - at) << 12;
     }
     return plan;
 }
