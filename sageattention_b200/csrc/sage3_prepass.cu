@@ -463,7 +463,7 @@ __device__ __forceinline__ void quant_q_tile(
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
 // ------------------------------------------------------------------------------------------------
-// AROWS = 64: up to 64 query blocks and up to one tile per SM, or, at D = 64, two to four (the A tile then has 64 rows, the MMA's other 64 read what lies behind it,
+// AROWS = 64: up to 64 query blocks and up to one tile per SM, or, at D = 64, up to four (the A tile then has 64 rows, the MMA's other 64 read what lies behind it,
 // for accumulator rows nobody looks at; four blocks per SM), see launch_prepass_t.  Up to 64 query blocks are otherwise quant_k_delta_run_kernel's.
 // FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
 template <typename T, int D, int AROWS, bool FLAG>
@@ -1223,9 +1223,10 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     if (tiles <= info.sms) return one_tile(std::integral_constant<int, 64>());
     // D = 64, a block per tile against runs of tiles, where four blocks of the one fit an SM at once and two of the other take a second turn.  64 query blocks, pre-pass:
     // 296 tiles 15.9 / 14.6, 400 16.5 / 17.7, 512 17.5 / 18.5, 1 024 26.8 / 26.6 us; whole calls: 512 tokens 4 x 32 heads, 2 048 queries 74.0 / 75.0, 1 280 tokens of 40 heads
-    // 42.5 / 43.0, 1 024 of 48 36.9 / 38.0, 1 700 of 32 63.5 / 63.6.
+    // 42.5 / 43.0, 1 024 of 48 36.9 / 38.0, 1 700 of 32 63.5 / 63.6.  Up to two
+    // tiles per SM it is a turn each; 500 queries of 16 heads, 2 715 keys of 8 (176 tiles of 8 query blocks) 32.8 / 33.6.
     if constexpr (D == 64)
-        if (tiles > 2 * info.sms && tiles <= 4 * info.sms) return one_tile(std::integral_constant<int, 64>());
+        if ((rows <= 32 || tiles > 2 * info.sms) && tiles <= 4 * info.sms) return one_tile(std::integral_constant<int, 64>());
     return rows <= 8 && tiles >= (int64_t)kRun32TilesPerSm(D) * info.sms ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 64>());
 }
 
