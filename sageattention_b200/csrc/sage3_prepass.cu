@@ -294,6 +294,26 @@ struct MeanParts {
     bool wait;                         // the sums come from the launch before this one (programmatic dependent launch)
 };
 
+// Microblock column and (first) row of a thread in a tile of 128 rows: eight neighbouring lanes have four columns of two rows.  With the 16-byte chunks of odd
+// rows in swapped pairs (or in the swizzle of an MMA operand) these eight lie on different banks.
+template <int D> __device__ __forceinline__ int micro_col(int lane) { return (lane & 3) | (D == 128 ? (lane >> 1) & 4 : 0); }
+template <int D> __device__ __forceinline__ int micro_row(int warp, int lane) {
+    return D == 128 ? warp * 4 + (((lane >> 2) & 1) | ((lane >> 3) & 2)) : warp * 8 + (lane >> 2);
+}
+
+// Scale bytes of a tile, from threads that hold those of rows rl, rl + RPP, ... in bytes 0, 1, ...: four neighbouring lanes have the four columns of a word of the
+// atom, and store the word of one microblock each.
+template <int D>
+__device__ __forceinline__ void store_scales(uint8_t* tile, uint32_t sf, int c, int rl, int lane) {
+    constexpr int CH = D / 16, RPP = 256 / CH, ITEMS = kBlock / RPP;
+    const int l = lane & 3;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, sf, 1);
+    const uint32_t v = __byte_perm(sf, y, l & 1 ? 0x3715 : 0x6240);
+    const uint32_t z = __shfl_xor_sync(0xffffffffu, v, 2);
+    const uint32_t word = __byte_perm(v, z, l & 2 ? 0x3276 : 0x5410);
+    if (ITEMS == 4 || l < 2) *reinterpret_cast<uint32_t*>(tile + (c >> 2) * 512 + sf_atom_offset(rl + RPP * l, 0)) = word;
+}
+
 template <typename T, int D, int MODE>
 __device__ __forceinline__ void quant_q_tile(
     const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
@@ -312,15 +332,14 @@ __device__ __forceinline__ void quant_q_tile(
 
     int h;
     const int b = H.divmod(bh, h);
-    const int t = threadIdx.x;
-    const int c = t % CH, rl = t / CH;
+    const int t = threadIdx.x, lane = t & 31;
+    const int c = micro_col<D>(lane), rl = micro_row<D>(t >> 5, lane);
     const int64_t bh_off = x.base(b, h, sb, sh, sn, N);
     const int row0 = tile * kBlock;
     if (row0 >= N && row0 > 0) return;    // a tile beyond this entry's padded length (variable-length batches only)
 
     T* s_mean = reinterpret_cast<T*>(smem_raw);                                // [D]
-    uint8_t* s_sf = smem_raw + D * 4;                                          // [(D/64) * 512]
-    uint8_t* s_more = s_sf + (D / 64) * 512;                                   // block mean only: staged tile, chain sums
+    uint8_t* s_more = smem_raw + D * 4;                                        // block mean only: staged tile, chain sums
 
     uint4 raw[ITEMS][2];
     x.template rows_each<ITEMS>(bh_off, row0 + rl, RPP, sn, [&](int i, const T* p) {
@@ -354,7 +373,7 @@ __device__ __forceinline__ void quant_q_tile(
 #pragma unroll
             for (int j = 0; j < 16; ++j) dot = fmaf(f[j], kf[j], dot);
 #pragma unroll
-            for (int off = 1; off < CH; off <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
+            for (int off = 1; off < CH; off <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off == 4 ? 8 : off);      // (see micro_col)
             if (c == 0) qkm[(int64_t)bh * Np + row0 + rl + RPP * i] = dot;
         }
     }
@@ -374,17 +393,19 @@ __device__ __forceinline__ void quant_q_tile(
         T* s_part = s_tile + kBlock * D;                                       // [R][PITCH]
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
-            uint4* dst = reinterpret_cast<uint4*>(s_tile + (rl + RPP * i) * D + c * 16);
-            dst[0] = raw[i][0];
-            dst[1] = raw[i][1];
+            uint8_t* dst = reinterpret_cast<uint8_t*>(s_tile + (rl + RPP * i) * D);
+            *reinterpret_cast<uint4*>(dst + ((2 * c ^ (rl & 1)) << 4)) = raw[i][0];
+            *reinterpret_cast<uint4*>(dst + (((2 * c ^ (rl & 1)) ^ 1) << 4)) = raw[i][1];
         }
         __syncthreads();
         {
             const int chain = t / (D / 4), c4 = (t % (D / 4)) * 4;
-            uint2 acc = *reinterpret_cast<const uint2*>(s_tile + chain * D + c4);
+            static_assert(R % 2 == 0, "the rows of a chain are all odd or all even");
+            const T* place = s_tile + chain * D + (((c4 >> 3) ^ (chain & 1)) << 3) + (c4 & 4);
+            uint2 acc = *reinterpret_cast<const uint2*>(place);
 #pragma unroll
             for (int rep = 1; rep < REPS; ++rep) {
-                const uint2 w1 = *reinterpret_cast<const uint2*>(s_tile + (rep * R + chain) * D + c4);
+                const uint2 w1 = *reinterpret_cast<const uint2*>(place + rep * R * D);
                 acc.x = Num<T>::add2(acc.x, w1.x);
                 acc.y = Num<T>::add2(acc.y, w1.y);
             }
@@ -431,10 +452,10 @@ __device__ __forceinline__ void quant_q_tile(
     *reinterpret_cast<uint4*>(mu2) = reinterpret_cast<const uint4*>(s_mean)[2 * c];
     *reinterpret_cast<uint4*>(mu2 + 4) = reinterpret_cast<const uint4*>(s_mean)[2 * c + 1];
 
+    uint8_t* code = codes + ((int64_t)bh * Np + row0 + rl) * (D / 2) + c * 8;
+    uint32_t sf = 0;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
-        const int rt = rl + RPP * i;          // row inside the tile
-        const int r = row0 + rt;
         // rows beyond N hold 0 - mean (Q is padded before smoothing); they are never read back
         const uint32_t x2[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
         uint32_t d2[8];
@@ -442,15 +463,10 @@ __device__ __forceinline__ void quant_q_tile(
         for (int j = 0; j < 8; ++j) d2[j] = Num<T>::sub2(x2[j], mu2[j]);
         uint32_t lo, hi, sfb;
         quant16_packed<T>(d2, lo, hi, sfb);
-        *reinterpret_cast<uint2*>(codes + ((int64_t)bh * Np + r) * (D / 2) + c * 8) = make_uint2(lo, hi);
-        s_sf[sf_atom_offset(rt, c)] = static_cast<uint8_t>(sfb);
+        *reinterpret_cast<uint2*>(code + i * RPP * (D / 2)) = make_uint2(lo, hi);
+        sf |= sfb << (8 * i);
     }
-    __syncthreads();
-    // scale factors of the tile: (D/64) atoms of 512 bytes, contiguous
-    {
-        uint8_t* dst = sfs + ((int64_t)bh * (Np / kBlock) + tile) * (D / 64) * 512;
-        if (t < (D / 64) * 32) reinterpret_cast<uint4*>(dst)[t] = reinterpret_cast<const uint4*>(s_sf)[t];
-    }
+    store_scales<D>(sfs + ((int64_t)bh * (Np / kBlock) + tile) * (D / 64) * 512, sf, c, rl, lane);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -789,9 +805,7 @@ __global__ void __launch_bounds__(KRunCfg<D, NR>::kThreads, KRunCfg<D, NR>::kBlo
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     if (warp < 8) {
         // ------------------------------------------------------------------ smoothing and quantization; delta_s of the tile before
-        // Microblock column and row of the thread: eight neighbouring lanes have four columns of two rows, whose chunks lie on different banks.
-        const int c = (lane & 3) | (D == 128 ? (lane >> 1) & 4 : 0);
-        const int rl = warp * (32 / CH) + (D == 128 ? ((lane >> 2) & 1) | ((lane >> 3) & 2) : lane >> 2);
+        const int c = micro_col<D>(lane), rl = micro_row<D>(warp, lane);
         const uint32_t place = (uint32_t)((c >> 2) * 16384 + rl * 128 + ((((2 * c) & 7) ^ (rl & 7)) << 4));      // of the microblock's first 16 bytes; the others: ^ 16
         KCursor<T> ahead = at;
         uint4 raw[ITEMS][2];
@@ -892,16 +906,7 @@ __global__ void __launch_bounds__(KRunCfg<D, NR>::kThreads, KRunCfg<D, NR>::kBlo
             }
             fence_proxy_async_smem();
             warp_arrive(bar_ready + 8 * (it & 1), lane);
-            // Scale bytes: four neighbouring lanes hold the four columns of a word of the atom, a byte of it per microblock
-            {
-                uint8_t* dst = sfs + ((int64_t)at.bh * (Np / kBlock) + at.tile) * SUB * 512 + (c >> 2) * 512;
-                const int l = lane & 3;
-                const uint32_t y = __shfl_xor_sync(0xffffffffu, sf, 1);
-                const uint32_t v = __byte_perm(sf, y, l & 1 ? 0x3715 : 0x6240);
-                const uint32_t z = __shfl_xor_sync(0xffffffffu, v, 2);
-                const uint32_t word = __byte_perm(v, z, l & 2 ? 0x3276 : 0x5410);      // of microblock l
-                if (ITEMS == 4 || l < 2) *reinterpret_cast<uint32_t*>(dst + sf_atom_offset(rl + RPP * l, 0)) = word;
-            }
+            store_scales<D>(sfs + ((int64_t)at.bh * (Np / kBlock) + at.tile) * SUB * 512, sf, c, rl, lane);
             if (it > 0) write_delta(it - 1, bh_before, tile_before);
             bh_before = at.bh;
             tile_before = at.tile;
@@ -960,7 +965,7 @@ __global__ void __launch_bounds__(KRunCfg<D, NR>::kThreads, KRunCfg<D, NR>::kBlo
 template <typename T, int D>
 __device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64_t sh, int64_t sn, FastDiv H, int N, int Np,
                                               uint8_t* __restrict__ codes, uint8_t* __restrict__ sfs, int tile, int bh, uint8_t* smem_raw) {
-    constexpr int PITCH = D + 2;          // elements; word pitch odd -> column reads are conflict-free
+    constexpr int PITCH = D;              // elements (rows are stored in 16-byte pieces, and read a word per lane along a row)
     int h;
     const int b = H.divmod(bh, h);
     const int t = threadIdx.x;
@@ -986,8 +991,7 @@ __device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64
         });
 #pragma unroll
         for (int i = 0; i < kBlock / RPP; ++i) {
-            uint32_t* dst = reinterpret_cast<uint32_t*>(s_v + (rl + i * RPP) * PITCH + c8 * 8);   // 4-byte aligned (PITCH even)
-            dst[0] = val[i].x; dst[1] = val[i].y; dst[2] = val[i].z; dst[3] = val[i].w;
+            *reinterpret_cast<uint4*>(s_v + (rl + i * RPP) * PITCH + c8 * 8) = val[i];
         }
     }
     __syncthreads();
@@ -1007,14 +1011,15 @@ __device__ __forceinline__ void quant_vt_tile(const Src<T>& x, int64_t sb, int64
         for (int ch = 0; ch < 2; ++ch) {
             uint32_t sfb;
             const float inv = micro_scale(ch == 0 ? amax2.x : amax2.y, sfb);
+            const uint64_t inv2 = pack2f(inv, inv);
             uint32_t code[2];
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
                 float y[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 v2 = Num<T>::to_f2(w[8 * g + i]);
-                    y[i] = __fmul_rn(ch == 0 ? v2.x : v2.y, inv);
+                for (int i = 0; i < 8; i += 2) {
+                    const float2 v2 = Num<T>::to_f2(w[8 * g + i]), v3 = Num<T>::to_f2(w[8 * g + i + 1]);
+                    unpack2f(mul2(ch == 0 ? pack2f(v2.x, v3.x) : pack2f(v2.y, v3.y), inv2), y[i], y[i + 1]);
                 }
                 code[g] = cvt_e2m1x8(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]);
             }
@@ -1063,12 +1068,15 @@ struct StageArgs {
 
 template <typename T, int D>
 struct StageCfg {
-    static constexpr int kQ = D * 4 + (D / 64) * 512 + (kBlock * D + 4 * (32 / (D / 8)) * (D + 8)) * (int)sizeof(T);   // staged tile and chain sums
-    static constexpr int kV = ((kBlock * (D + 2) * (int)sizeof(T) + 15) / 16) * 16 + D * 72 + 1024;
+    static constexpr int kQ = D * 4 + (kBlock * D + 4 * (32 / (D / 8)) * (D + 8)) * (int)sizeof(T);   // staged tile and chain sums
+    static constexpr int kV = kBlock * D * (int)sizeof(T) + D * 72 + 1024;
     static constexpr int kCol = (2048 / D) * (D + 1) * 4;
     static constexpr int kSmem = kQ > kV ? (kQ > kCol ? kQ : kCol) : (kV > kCol ? kV : kCol);
 };
 
+// Next to HBM the shared-memory pipe bounds it (62 to 65 % busy, issue slots 52 %), so the tiles stand there without bank conflicts: Q's rows in pairs of swapped chunks, V's in
+// 16-byte pieces (as words of padded rows every store took four turns), the scale bytes put together by shuffles instead of in a staged atom behind one more barrier.  Stage
+// kernel, us: 17 550 queries of 96 heads, D = 64 67.4 -> 62.3, D = 128 115.0 -> 109.5; K sums and V of 8 x 8 x 8 192 keys 55.4 -> 52.4 (5.8 TB/s), D = 64 27.6 -> 26.4.
 // Six resident blocks at D = 64 (40 registers, column sums four rows deep): 17 550 queries of 96 heads 71 -> 58 us against four.  At
 // D = 128 four: five spill (131 -> 149 us for 8 x 8 x 8 192 keys with their K kernel).
 template <typename T, int D>
