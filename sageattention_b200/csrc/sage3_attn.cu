@@ -105,7 +105,8 @@ constexpr int kUnitRing = 4;
 // w takes keys 32 w .. 32 w + 31 of the block for all of them: a quarter of the exponentials per warp.  The four exchange their
 // maxima through shared memory; P, its scales and the accumulator are those of rows 0..31.  Same operations per score, and the row
 // sums are added in the same order, so the same bits.  D = 128, 8 sequences x 32 heads x 1 token against 8 192 keys of 8 kv heads:
-// 166.4 -> 143.1 us per call, pre-pass included (D = 64: 116.8 -> 92.2 us).  The copy warp's and the MMA issuer's instructions bound it.
+// 166.4 -> 143.1 us per call, pre-pass included (D = 64: 116.8 -> 92.2 us).  The copy warps' and the MMA issuer's instructions bound it: K, V and delta_s have
+// a copy warp each.
 template <int D, int PACK>
 struct Cfg {
     // K and V^T stages, each shared by the two query tiles (as many as fit: PACK, see oP)
@@ -352,6 +353,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         uint32_t count = 1;                                      // copies landed, MMAs complete, one warp's statistics
         if (i >= bQE && i < bKF) count = PACK == 2 ? 1 : 2;      // Q buffer free: the Q K^T issuers are done with it
         if (i >= bKE && i < bKE + S) count = PACK == 2 ? 1 : 2;  // K stage free: likewise
+        if (i >= bKF && i < bKE) count = PACK == 2 ? 2 : 1;      // K and its scales; delta_s by a warp of its own
         if (i >= bSE && i < bM) count = 4;                       // S buffer free: the four warps of its group hold the scores
         if (i >= bPF && i < bPV) count = 4;                      // P, its scales and the row sums written
         if (i >= bOS && i < bX) count = PACK == 2 ? 1 : 4;       // the correction warps are done with O (and have seen P written)
@@ -446,6 +448,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // The pre-pass gave up (the workspace is then incomplete): the units are walked, but nothing is written.  (Read here, needed at
       // the first epilogue: off the path to the first scores.)
       const int broken = *reinterpret_cast<const volatile int*>(p.prepass_status);
+      int dst = 0, dst_parity = 1;              // PACK == 2: stage of delta_s
       const Unit* u;
       bool ok = true;
       for (int i = 0; ok && (u = next_unit(i)) != nullptr; ++i) {
@@ -496,6 +499,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               }
           }
           if constexpr (PACK == 2) {
+              if (quarter == 1) {
+                  // delta_s of the unit's blocks: a copy less for the warp that has K.  One token of 8 x 32 heads, 8 192 keys of 8 kv heads 117.2 -> 116.8 us per call
+                  // (D = 64 77.5 -> 76.2), of one sequence, 16 000 keys 76.8 -> 76.2 (63.6 -> 62.1).
+                  const bool box = w.nb[1] > 1;
+                  const uint16_t* src = p.delta + (size_t)w.bhq * p.nqm * ((size_t)p.nkb * kBlock);
+                  for (int n = w.nbmax - 1; n >= 0; --n) {
+                      if (!warp_wait<true>(bar(bKE + dst), dst_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
+                      if (lane == 0) {
+                          mbar_expect_tx(bar(bKF + dst), (box ? 8 : 1) * C::kDeltaBytes);
+                          if (box) tma_load_3d(sbase + C::oDelta + dst * C::kDeltaStage, &tm_d, bar(bKF + dst), 0, w.bhq, n * (kBlock / 8));
+                          else bulk_load(sbase + C::oDelta + dst * C::kDeltaStage, src + (size_t)n * kBlock, C::kDeltaBytes, bar(bKF + dst));
+                      }
+                      __syncwarp();
+                      if (++dst == S) { dst = 0; dst_parity ^= 1; }
+                  }
+              }
               // One warp holds all rows: it waits for P alone (the factor was written before), reads all it needs, and keeps the sums in
               // registers.  (Waiting for the factor and for P with the sums in shared memory took it 1 000 cycles per block.)
               float2 l = make_float2(0.f, 0.f);
@@ -803,14 +822,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int n = w.nbmax - 1; n >= lowest; --n) {
                 if (!warp_wait<true>(bar(bKE + st), st_parity, abort_flag, p.status, kWaitKEmpty)) { ok = false; break; }
                 if (lane == 0) {
-                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (box ? 8 : w.nv) * C::kDeltaBytes);
+                    mbar_expect_tx(bar(bKF + st), C::kKBytes + C::kSfQkBytes + (PACK == 2 ? 0 : box ? 8 : w.nv) * C::kDeltaBytes);
                     tma_load_3d(sbase + C::oK + st * C::kKBytes, &tm_k, bar(bKF + st), 0, n * kBlock, w.bhkv);
                     bulk_load(sbase + C::oSfK + st * 1024, p.k_sf + ((size_t)w.bhkv * p.nkb + n) * C::kSfQkBytes,
                               C::kSfQkBytes, bar(bKF + st));
                     // box: [16 chunks of 8 keys][8 heads], the canonical core matrices of an MN-major operand (heads beyond the packed ones
                     // bring finite data that meets zeros).  One tensor copy: 64 copies of 16 bytes took 2.9 us per key block.
-                    if (box) tma_load_3d(sbase + C::oDelta + st * C::kDeltaStage, &tm_d, bar(bKF + st), 0, w.bhq, n * (kBlock / 8));
-                    for (int t = 0; !box && t < w.nv; ++t)
+                    if (PACK != 2 && box) tma_load_3d(sbase + C::oDelta + st * C::kDeltaStage, &tm_d, bar(bKF + st), 0, w.bhq, n * (kBlock / 8));
+                    for (int t = 0; PACK != 2 && !box && t < w.nv; ++t)
                         bulk_load(sbase + C::oDelta + (PACK ? st * C::kDeltaStage : (st * 2 + t) * C::kDeltaPitch), dptr0 + t * dstep + (size_t)n * kBlock,
                                   C::kDeltaBytes, bar(bKF + st));
                 }
