@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(256, AROWS == 128 ? 3 : 4) quant_k_delta_kerne
 }
 
 // ------------------------------------------------------------------------------------------------
-// K for up to 64 query blocks per kv head (token generation, chunks of a prompt, calls with one Q mean per head, packed prompts): two blocks per SM
+// K for up to 64 query blocks per kv head, D = 64 up to 128 (token generation, chunks of a prompt, calls with one Q mean per head, packed prompts): two blocks per SM
 // walk runs of tiles, all of one length, that go on from head to head.
 //   warps 0-7   hold the next tile's rows in registers (a row's load is issued as soon as the one before it in that place is used), smooth and quantize
 //               them, store k' as the operand of the MMA, and write delta_s of the tile before: nothing in their loop waits for a copy or an MMA
@@ -833,25 +833,30 @@ __global__ void __launch_bounds__(KRunCfg<D, NR>::kThreads, KRunCfg<D, NR>::kBlo
             __syncwarp();
             if (r0 < rows) {
                 tc_fence_after();
-                float v[HALF];
-                const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + (it & 1) * NR + r0;
-                if constexpr (HALF == 16) tmem_ld16(acc, v);
-                else tmem_ld32(acc, v);
-                tc_wait_ld();
-                tc_fence_before();
                 // Two neighbouring lanes swap one of two rows: each has two keys of one row then, and a store covers 64 bytes of both rows.
                 const int row = r0 + (lane & 1);
                 T* dst = delta + ((int64_t)bh * rows + row) * Np + tile * kBlock + quarter * 32 + (lane & ~1);
                 uint32_t z = 0;           // FLAG: 0 while all values are finite
+                constexpr int STEP = HALF < 32 ? HALF : 32;
 #pragma unroll
-                for (int r = 0; r < HALF; r += 2, dst += 2 * Np) {
-                    const uint32_t w = Num<T>::pack2(v[r], v[r + 1]), y = __shfl_xor_sync(0xffffffffu, w, 1);
-                    const uint32_t pair = __byte_perm(w, y, lane & 1 ? 0x3276 : 0x5410);
-                    if (row + r < rows) {
-                        *reinterpret_cast<uint32_t*>(dst) = pair;
-                        if (FLAG) z = Num<T>::zero_fma2(pair, z);
+                for (int c0 = 0; c0 < HALF; c0 += STEP) {
+                    if (c0 > 0 && r0 + c0 >= rows) break;
+                    float v[STEP];
+                    const uint32_t acc = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + (it & 1) * NR + r0 + c0;
+                    if constexpr (STEP == 16) tmem_ld16(acc, v);
+                    else tmem_ld32(acc, v);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int r = 0; r < STEP; r += 2, dst += 2 * Np) {
+                        const uint32_t w = Num<T>::pack2(v[r], v[r + 1]), y = __shfl_xor_sync(0xffffffffu, w, 1);
+                        const uint32_t pair = __byte_perm(w, y, lane & 1 ? 0x3276 : 0x5410);
+                        if (row + c0 + r < rows) {
+                            *reinterpret_cast<uint32_t*>(dst) = pair;
+                            if (FLAG) z = Num<T>::zero_fma2(pair, z);
+                        }
                     }
                 }
+                tc_fence_before();
                 if (FLAG && (z & 0x7fff7fffu) != 0) nonfinite[bh] = 1;
             }
         };
@@ -1225,6 +1230,11 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
                           a.status, a.nonfinite, tm_qm, tm_delta);
         });
     };
+    // 65 to 128 query blocks, D = 64 (at D = 128 the wider accumulator spills: 3 000 tokens of 4 x 32 heads, 96 blocks 57.5 / 59.0 us of pre-pass): runs, where all blocks of one
+    // tile, three per SM, would not be resident at once, or two per SM are enough.  Pre-pass, one tile per block / runs: 16 000 tokens of 2 x 32 heads 211.7 / 192.3, 9 000 of 40 71.5 / 64.5,
+    // 4 000 of 8 x 32 (8 kv heads) 84.3 / 81.7, of 2 x 32 (512 tiles) 26.7 / 24.8, 4 096 of 32 (256) 18.4 / 16.8; not: 2 600 of 2 x 32 (336) 18.6 / 20.5, 3 400 (432) 22.5 / 22.6.
+    if constexpr (D == 64)
+        if (rows > 64 && rows <= 128 && ((tiles > info.sms && tiles <= 2 * info.sms) || tiles > 3 * info.sms)) return run(std::integral_constant<int, 128>());
     if (rows > 64) return one_tile(std::integral_constant<int, 128>());
     // Up to one tile per SM nothing goes on in a run, and the block of one tile is quicker to its end: 1 829 tokens of 4 x 2 heads 30.8 / 30.9 us per call, D = 64 26.7 / 28.7, 1 024 of
     // two heads 22.6 / 22.7 (19.9 / 20.4), 700 of 2 x 8 heads, causal, 22.6 / 22.6 (19.2 / 20.5).

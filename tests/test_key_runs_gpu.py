@@ -1,4 +1,4 @@
-"""The K kernel for up to 64 query blocks per kv head: its blocks walk runs of key tiles, two blocks per SM, a run going on into the next head.  Numbers of
+"""The K kernel for up to 64 query blocks per kv head (D = 64: 128): its blocks walk runs of key tiles, two blocks per SM, a run going on into the next head.  Numbers of
 tiles around the blocks that are resident, query blocks around the 32 and 64 columns of an accumulator and the halves of them that a warp writes, ragged
 last tiles, tokens split over buffers: codes, scales, means and delta_s as the oracle forms them and as a call on one head alone gives them."""
 import pytest
@@ -35,6 +35,8 @@ def _workspace(p, B, Hkv):
     (7, 128 * 9, 45, 9),         # 63
     (4, 128 * 16, 61, 10),       # 64
     (4, 128 * 16, 33, 15),       # 64, 495 tiles: D = 64 has a block per tile
+    (5, 128 * 13, 40, 10),       # 65: D = 64 has an accumulator of 128 columns
+    (8, 128 * 16, 40, 10),       # 128
     (8, 1, 100, 40),             # 4 000 tiles and up to eight query blocks: the accumulator of 32 columns
 ])
 def test_runs_of_key_tiles(cuda_device, D, group, Nq, tiles, heads):
