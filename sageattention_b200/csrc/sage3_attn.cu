@@ -62,7 +62,7 @@ struct AttnParams {
     int BHq, Hq, Hkv, Nq, Nk, nqt, nkb, nqm;   // nqt = query tiles per head, nkb = KV blocks per head
     int units, whole_units;             // units of work; those from whole_units on are single query tiles instead of pairs
     int pack_heads, pack_tiles;         // PACK kernels: query heads per tile, tiles per kv head
-    int* unit_counter;                  // zero at launch: next unit after the first gridDim.x
+    int* unit_counter;                  // zero at launch: next unit after the first gridDim.x (CARRY == 2 and no whole units: all are drawn)
     float sm_scale_log2;
     const float* sm_scale_per_head;
     const uint8_t *q_sf, *k_sf, *v_sf;
@@ -707,6 +707,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // ------------------------------------------------------------------ TMA producer
         int st = 0, st_parity = 1;                // K / V stage; parity of its "free" phase (a fresh barrier passes parity 1)
         int u = blockIdx.x, k = 0, kq = 0;        // unit number; units published, units with items
+        // SPLIT: a slot is always drawn, the first unit too where that is one, so that the slots before it are in the hands of CTAs that run, in whatever order CTAs
+        // are started.  (Its CTA draws on at its end: ahead of that it would take the slot of one that has just been started.)
+        const int drawn = SPLIT && p.whole_units == 0 ? 0 : gridDim.x;
+        if (drawn == 0) u = uniform(lane == 0 ? atomicAdd(p.unit_counter, 1) : 0);
         int next = 0, head = 0;                   // the unit after this one (lane 0); PACK: next head of a unit whose heads go one by one; SPLIT: next part of a slot
         int tile = 0, lo = 0, left = 0;           // SPLIT: of the slot, tile and first key block of its next part, key blocks left
         // V is loaded kLag blocks behind K.  A V stage is free four blocks after its K stage (scores, softmax and P lie between), and
@@ -729,7 +733,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         bool ok = true;
         while (ok) {
             if (!(PACK || SPLIT) || head == 0) next = 0;     // (where heads never go one by one nothing is carried round the loop: 0.3 % at 8 192 keys)
-            if (lane == 0 && head == 0) next = gridDim.x + atomicAdd(p.unit_counter, 1);
+            if (lane == 0 && head == 0 && (!SPLIT || u < p.whole_units)) next = drawn + atomicAdd(p.unit_counter, 1);
             Unit w;
             const bool more = u < p.units;
             if (!more) w.ns = -1;
@@ -766,6 +770,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     ++tile;
                     lo = 0;
                     left -= w.ns;
+                    if (last_head && lane == 0) next = drawn + atomicAdd(p.unit_counter, 1);
                 }
                 if (last_head) u = uniform(next);
                 head = last_head ? 0 : head + 1;

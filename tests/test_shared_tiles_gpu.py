@@ -47,3 +47,37 @@ def test_shared_tiles(cuda_device, D, H, group, Nq, Nk, causal):
     ref = O.sageattn3_oracle(q[:, h:h + 1, :].cpu(), k[:, h // group:h // group + 1].cpu(), v[:, h // group:h // group + 1].cpu(), is_causal=causal) if Nk <= 3000 else None
     if ref is not None:
         assert O.cosine(p.out[:, h:h + 1].cpu(), ref) >= 0.999 and O.rel_l1(p.out[:, h:h + 1].cpu(), ref) <= 0.01
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_shared_tiles_on_two_streams_and_in_a_graph(cuda_device, D):
+    """Two streams whose kernels take SMs from one another, and a captured call replayed: the results of calls one after the other."""
+    g = torch.Generator(device=cuda_device).manual_seed(2200 + D)
+    problems = []
+    for H, Nq, Nk, causal in ((32, 1000, 6000, True), (100, 384, 2500, False)):
+        q = torch.randn(1, H, Nq, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+        k, v = (torch.randn(1, H // 4, Nk, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
+        p = Sage3Problem(q, k, v, is_causal=causal)
+        problems.append((p, p.run().clone()))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in problems]
+    for p, _ in problems:
+        p.out.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for (p, _), st in zip(problems, streams):
+            with torch.cuda.stream(st):
+                p.run()
+    torch.cuda.synchronize()
+    for p, want in problems:
+        assert p.check_status() == 0 and torch.equal(p.out, want)
+    p, want = problems[0]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        p.run()
+        p.attention()
+    p.out.zero_()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert p.check_status() == 0 and torch.equal(p.out, want)
