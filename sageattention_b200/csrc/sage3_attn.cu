@@ -688,9 +688,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               float* state = p.split_state + (size_t)pout * C::kState + 128 * D;
               *reinterpret_cast<float2*>(state + 2 * row) = l_s[0];
               state[256 + row] = m_s[0];
-              __threadfence();
-              __syncwarp();
-              if (lane == 0) atomicAdd(p.split_flags + pout, 1);
+              warp_raise_word(p.split_flags + pout, lane);
           }
           unit_done(i);
           base += ns;

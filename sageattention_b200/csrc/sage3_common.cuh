@@ -185,7 +185,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// Bounded wait of a whole warp until another CTA of the launch has raised the counter at `word` to `want`; what that CTA wrote before is then visible.
+// Raises the counter at `word` by one for a converged warp.  The release stands behind the __syncwarp, so it covers what the other lanes have written too
+// (a fence of each lane ahead of it would leave their writes unordered with lane 0's addition).
+__device__ __forceinline__ void warp_raise_word(int* word, int lane) {
+    __syncwarp();
+    if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(word) : "memory");
+}
+
+// Bounded wait of a whole warp until warps of another CTA of the launch have raised the counter at `word` to `want`; what these wrote before is then visible.
 __device__ __forceinline__ bool warp_wait_word(const int* word, int want, volatile int* abort_flag, int* status_word, int code) {
     const uint32_t t0 = clock();
     while (true) {
