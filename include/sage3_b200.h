@@ -75,8 +75,9 @@ typedef struct Sage3Desc {
  *   status   int32[64]                        device-written status words (0 = fine): [0, 32) pre-pass, [32, 64) attention;
  *                                             the pre-pass clears all, attention on its own its half only, so that
  *                                             sage3_check_status after sage3_fwd sees what either stage reported
- *                                             (behind them, word 64: the attention kernel's work counter; words 65 ...: per
- *                                             (batch, kv head), delta_s holds a value that is not finite)
+ *                                             (behind them, word 64: the attention kernel's work counter; from 2 048 padded keys on int32[160]
+ *                                             flags of query tiles whose keys two blocks of the attention kernel walk; then per (batch,
+ *                                             kv head): delta_s holds a value that is not finite)
  *   kpart    fp32 [B*Hkv][chunks][D]          scratch: partial column sums of K (followed by those of Q when per_block_mean = 0)
  *   km       dtype[B][Hkv][D]                 mean of K over its Nk tokens
  *   qm       dtype[B][Hq][nqm][D]             Q means; nqm = Nq_p/128, or 1 when per_block_mean = 0
@@ -90,8 +91,7 @@ typedef struct Sage3Desc {
  *   qkm      fp32 [B][Hq][Nq_p]               q . km per query row (the part of q k^T that K smoothing removes;
  *                                             core.py:289-293 `lse_correction`), used by the LSE output (sage3_fwd and
  *                                             sage3_fwd_varlen write it only when `lse` is asked for)
- *   (behind qkm, from 2 048 padded keys on and part of total_bytes: int32[160] flags, cleared by the pre-pass and by an attention call on
- *   its own, and 160 accumulators of 128 rows, for query tiles whose keys two blocks of the attention kernel walk)
+ *   (behind qkm, from 2 048 padded keys on and part of total_bytes: 160 accumulators of 128 rows, for those query tiles)
  */
 typedef struct Sage3Workspace {
     size_t status, kpart, km, qm, delta, q_codes, q_sf, k_codes, k_sf, v_codes, v_sf, qkm;

@@ -42,8 +42,12 @@ constexpr size_t kWsAlign = 256;    // required alignment of the workspace base 
 inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 // Words of the status region: [0, 32) what the pre-pass reports, [32, 64) what the attention kernel reports, then its work counter, then
-// one word per (batch, kv head) that the pre-pass sets when a value of its delta_s is not finite.  The first pre-pass kernel clears all.
-constexpr int kAttnStatusWord = 32, kUnitCounterWord = 64, kNonfiniteWord = 65;
+// the flags of shared query tiles (where the layout has room for their accumulators), then one word per (batch, kv head) that the pre-pass
+// sets when a value of its delta_s is not finite.  The first pre-pass kernel clears all; what is the attention kernel's lies in one piece, since
+// an attention call on its own clears it with one memset (a second one takes 1.0 to 1.6 us: one token of 32 heads, 3 072 keys 18.5 -> 19.9).
+constexpr int kAttnStatusWord = 32, kUnitCounterWord = 64, kSplitFlagsWord = 65;
+inline bool shares_tiles(const Sage3Workspace& w) { return w.nk_pad / 128 >= sage3::kSplitMinBlocks; }
+inline int nonfinite_word(const Sage3Workspace& w) { return kSplitFlagsWord + (shares_tiles(w) ? sage3::kSplitSlots : 0); }
 
 int validate(const Sage3Desc* d) {
     if (!d) return SAGE3_E_NULL;
@@ -79,8 +83,9 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     const size_t kch_k = ((size_t)d->Nk + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t kch_q = ((size_t)d->Nq + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t part = B * Hkv * kch_k + (d->per_block_mean ? 0 : B * Hq * kch_q);
+    w->nk_pad = (int32_t)nkp;
     size_t off = 0;
-    w->status = off;  off += align_up((kNonfiniteWord + B * Hkv) * sizeof(int32_t));
+    w->status = off;  off += align_up((nonfinite_word(*w) + B * Hkv) * sizeof(int32_t));
     w->kpart = off;   off += align_up(part * D * sizeof(float));
     w->km = off;      off += align_up(B * Hkv * D * 2);
     w->qm = off;      off += align_up(B * Hq * nqm * D * 2);
@@ -92,19 +97,18 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     w->v_codes = off; off += align_up(B * Hkv * D * (nkp / 2));
     w->v_sf = off;    off += align_up(B * Hkv * (nkp / 128) * 1024);
     w->qkm = off;     off += align_up(B * Hq * nqp * sizeof(float));
-    if (nkp / 128 >= sage3::kSplitMinBlocks) off += align_up(sage3::kSplitSlots * sizeof(int32_t)) + align_up(sage3::kSplitSlots * sage3::split_state_floats(D) * sizeof(float));      // see split_region
+    if (shares_tiles(*w)) off += align_up(sage3::kSplitSlots * sage3::split_state_floats(D) * sizeof(float));      // see split_state
     w->total_bytes = off;
     w->nq_pad = (int32_t)nqp;
-    w->nk_pad = (int32_t)nkp;
     w->nqm = (int32_t)nqm;
     w->kchunks = (int32_t)kch_k;
     return SAGE3_OK;
 }
 
-// Flags and accumulators of query tiles whose keys two CTAs share, behind the last region of the layout; nullptr where the layout has none.
-int* split_region(const Sage3Desc* d, const Sage3Workspace& w, void* ws) {
-    if (w.nk_pad / 128 < sage3::kSplitMinBlocks) return nullptr;
-    return reinterpret_cast<int*>(static_cast<uint8_t*>(ws) + w.qkm + align_up((size_t)d->B * d->Hq * w.nq_pad * sizeof(float)));
+// Accumulators of query tiles whose keys two CTAs share, behind the last region of the layout; nullptr where the layout has none.
+float* split_state(const Sage3Desc* d, const Sage3Workspace& w, void* ws) {
+    if (!shares_tiles(w)) return nullptr;
+    return reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + w.qkm + align_up((size_t)d->B * d->Hq * w.nq_pad * sizeof(float)));
 }
 
 int check_arch() {
@@ -148,7 +152,7 @@ sage3::PartsPtr one_part(const void* p) {
     return r;
 }
 
-// `cleared`: the pre-pass of the same call has already zeroed the attention half of the status words and the work counter.  An attention
+// `cleared`: the pre-pass of the same call has already zeroed the attention half of the status words, the work counter and the flags.  An attention
 // call on its own zeroes these and leaves the pre-pass half alone, so that a wait the pre-pass gave up on stays on record (the kernel
 // then walks its units without writing anything).
 int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float* lse, void* stream, bool cleared = false,
@@ -172,7 +176,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* base = static_cast<uint8_t*>(ws);
     if (!cleared && sage3::checked(cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0,
-                                                   (kUnitCounterWord + 1 - kAttnStatusWord) * sizeof(int32_t), st)) != cudaSuccess)
+                                                   (nonfinite_word(w) - kAttnStatusWord) * sizeof(int32_t), st)) != cudaSuccess)
         return SAGE3_E_CUDA;
     sage3::AttnArgs a;
     a.B = desc->B; a.Hq = desc->Hq; a.Hkv = desc->Hkv; a.Nq = desc->Nq; a.Nk = desc->Nk; a.D = desc->D;
@@ -195,11 +199,10 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.status = reinterpret_cast<int*>(base + w.status) + kAttnStatusWord;
     a.unit_counter = reinterpret_cast<int*>(base + w.status) + kUnitCounterWord;
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
-    a.nonfinite = reinterpret_cast<const int*>(base + w.status) + kNonfiniteWord;
+    a.nonfinite = reinterpret_cast<const int*>(base + w.status) + nonfinite_word(w);
     a.cu_q = cu_q; a.cu_k = cu_k;
-    a.split_flags = split_region(desc, w, ws);
-    a.split_state = a.split_flags ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.split_flags) + align_up(sage3::kSplitSlots * sizeof(int32_t))) : nullptr;
-    if (!cleared && a.split_flags && sage3::checked(cudaMemsetAsync(a.split_flags, 0, sage3::kSplitSlots * sizeof(int32_t), st)) != cudaSuccess) return SAGE3_E_CUDA;
+    a.split_state = split_state(desc, w, ws);
+    a.split_flags = a.split_state ? reinterpret_cast<int*>(base + w.status) + kSplitFlagsWord : nullptr;
     int drv = 0;
     return sage3::launch_attn(a, st, &drv) == cudaSuccess ? SAGE3_OK : SAGE3_E_CUDA;
 }
@@ -354,9 +357,8 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     a.clear = a.status;
     // (without carried state, which only the attention call knows about: a word more or less per head costs nothing)
     const bool shared = sage3::PackRule(desc->Nq, desc->Hq / desc->Hkv, cu_q == nullptr).heads > 1;
-    a.nonfinite = shared ? a.status + kNonfiniteWord : nullptr;
-    a.n_clear = kNonfiniteWord + (shared ? desc->B * desc->Hkv : 0);
-    a.split_flags = split_region(desc, w, ws);
+    a.nonfinite = shared ? a.status + nonfinite_word(w) : nullptr;
+    a.n_clear = nonfinite_word(w) + (shared ? desc->B * desc->Hkv : 0);
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
         sage3::checked(cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)

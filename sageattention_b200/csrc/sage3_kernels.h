@@ -32,10 +32,9 @@ struct PrepassArgs {
     float* qkm;                    // fp32 [B][Hq][Nq_p]: q . km per query row
     int* status;                   // device status words (bounded waits report here)
     int want_qkm;                  // q . km per query row is wanted (the LSE output needs it)
-    int* clear;                    // words the first kernel zeroes: status words, the attention kernel's work counter, `nonfinite`
+    int* clear;                    // words the first kernel zeroes: status words, the attention kernel's work counter and flags, `nonfinite`
     int n_clear;
     int* nonfinite;                // per (batch, kv head): set when a delta_s value is not finite; nullptr: nobody asks (see PackRule)
-    int* split_flags;              // kSplitSlots words the first kernel zeroes too (nullptr: none)
     // packed variable-length sequences (both nullptr: every batch entry has Nq / Nk tokens): device int32 [B + 1], entry b
     // owns rows cu[b] .. cu[b + 1] of the packed tensor; Nq / Nk are then the maximum lengths, stride 0 is unused
     const int *cu_q, *cu_k;
@@ -61,7 +60,7 @@ struct AttnArgs {
     const int* prepass_status;      // the pre-pass's status word (non-zero: the workspace is incomplete, do nothing)
     const int* nonfinite;           // per (batch, kv head), from the pre-pass: delta_s holds values that are not finite
     const int *cu_q, *cu_k;         // packed variable-length sequences, as in PrepassArgs (nullptr: uniform lengths)
-    // Last round of units dealt out by key blocks (see SplitPlan); zeroed before the launch / scratch.  nullptr: not possible for these sizes.
+    // Last rounds of units dealt out by key blocks (see SplitPlan): flags, zeroed before the launch, and scratch.  nullptr: not possible for these sizes.
     int* split_flags;
     float* split_state;
 };

@@ -1066,10 +1066,11 @@ struct StageArgs {
     uint8_t *q_codes, *q_sf, *v_codes, *v_sf;
     float* qkm;                        // nullptr: not wanted
     MeanParts means;
-    int* clear;                        // words to zero: status, work counter, `nonfinite` (nullptr: not in this launch)
+    int* clear;                        // words to zero: status, work counter, flags, `nonfinite` (nullptr: not in this launch)
     int n_clear;
-    int* clear2;                       // kSplitSlots more (nullptr: none)
 };
+
+constexpr int kMostCleared = 512;      // words
 
 template <typename T, int D>
 struct StageCfg {
@@ -1089,9 +1090,10 @@ __global__ void __launch_bounds__(256, D == 64 ? 6 : 4) prepass_stage_kernel(con
     extern __shared__ __align__(16) uint8_t smem_raw[];
     pdl_launch_dependents();
     int i = blockIdx.x;
-    if (i == 0) {
-        if (a.clear != nullptr && threadIdx.x < a.n_clear) a.clear[threadIdx.x] = 0;
-        if (a.clear2 != nullptr && threadIdx.x < kSplitSlots) a.clear2[threadIdx.x] = 0;
+    if (i == 0 && a.clear != nullptr) {
+#pragma unroll
+        for (int j = 0; j < kMostCleared; j += 256)
+            if (threadIdx.x + j < a.n_clear) a.clear[threadIdx.x + j] = 0;
     }
     int tile, bh;
     if (i < a.n_colk) {
@@ -1157,9 +1159,8 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
     s.part_k = a.kpart; s.part_q = a.kpart + (size_t)BHkv * a.kchunks_k * D;
     s.km = km; s.qm = qm;
     s.q_codes = a.q_codes; s.q_sf = a.q_sf; s.v_codes = a.v_codes; s.v_sf = a.v_sf;
-    s.clear = a.clear; s.n_clear = a.n_clear < 256 ? a.n_clear : 256;      // by the threads of one block
-    s.clear2 = a.split_flags;
-    if (a.n_clear > 256 && (e = checked(cudaMemsetAsync(a.clear + 256, 0, (a.n_clear - 256) * sizeof(int), st))) != cudaSuccess) return e;
+    s.clear = a.clear; s.n_clear = a.n_clear < kMostCleared ? a.n_clear : kMostCleared;
+    if (a.n_clear > kMostCleared && (e = checked(cudaMemsetAsync(a.clear + kMostCleared, 0, (a.n_clear - kMostCleared) * sizeof(int), st))) != cudaSuccess) return e;
     // Q waits for the means when it is smoothed by one mean per head (api.py:88-90) or when q . km is wanted
     const bool q_late = !a.per_block_mean || a.want_qkm;
     const bool km_here = !a.km_given;
@@ -1181,7 +1182,7 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
         s.n_colk = s.n_colq = s.n_v = 0;
         s.n_q = tiles_q * BHq;
         s.qkm = a.want_qkm ? a.qkm : nullptr;
-        s.clear = s.clear2 = nullptr;
+        s.clear = nullptr;
         s.means.k = km_inline ? s.part_k : nullptr;
         s.means.q = qm_inline ? s.part_q : nullptr;
         s.means.chunks_k = a.kchunks_k;

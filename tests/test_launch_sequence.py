@@ -105,6 +105,29 @@ def test_a_refused_launch_is_reported_and_ends_the_call(fake, call, kw, lse):
         assert fake.fake_last_error() == 0, i
 
 
+def _attn(lib, d):
+    p = C.c_void_p
+    return lib.sage3_attn_fwd(C.byref(d), p(WS), p(1 << 15), None, None)
+
+
+def _attn_parts(lib, d):
+    p, parts = C.c_void_p, _cabi.Sage3Parts()
+    parts.parts, parts.rows_per_part = 2, (d.Nq + 1) // 2
+    parts.base[0] = parts.base[1] = 1 << 15
+    return lib.sage3_attn_fwd_parts(C.byref(d), p(WS), C.byref(parts), None, None)
+
+
+@pytest.mark.parametrize("call,kw", [
+    (_attn, {}), (_attn, dict(Nk=9000)), (_attn, dict(Nq=1000, Nk=9192, Hq=32, is_causal=1, D=128)),      # ... tiles shared
+    (_attn, dict(Nq=1, Hq=32, Nk=9000)), (_carried, dict(Nk=9000)), (_attn_parts, dict(Nq=1000, Nk=9192, Hq=32, D=128)), (_attn_parts, dict(Nk=9000))])
+def test_attention_on_its_own_is_one_memset_and_one_kernel(fake, call, kw):
+    """What the kernel wants cleared lies in one piece: each further stream operation takes longer than a microsecond."""
+    fake.fake_start(-1, 0)
+    assert call(fake, _desc(**kw)) == 0
+    names = [entry[1] for entry in _log(fake)]
+    assert len(names) == 2 and names[0] == "memset" and "attn_fwd" in names[1], names
+
+
 def test_shared_memory_is_asked_for_once_per_kernel(fake):
     """Calls that between them launch every attention and every K kernel: in a second round no kernel's attributes are set again (that is a call into the
     runtime for every launch, paid by the shortest calls)."""
