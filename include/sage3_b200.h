@@ -47,6 +47,13 @@ enum {
 enum { SAGE3_FP16 = 0, SAGE3_BF16 = 1 };
 
 /*
+ * Sage3Desc.reserved: leaves the flags and accumulators of shared query tiles out of the workspace (some 11 MB at D = 128, 5.6 MB at D = 64, of a problem
+ * of more than 32 queries and 2 048 padded keys or more).  The same results; a call whose last rounds of work do not fill the GPU takes longer.  For a
+ * workspace of fixed size, and for packed batches and carried state, which share no tiles in any case.
+ */
+#define SAGE3_NO_SHARED_TILES 0x6e6f7374
+
+/*
  * Problem description.  Tensors are addressed as x[b][h][n][d] with the element strides given here and
  * d contiguous, so "HND" ([B,H,N,D]) and "NHD" ([B,N,H,D]) callers use the same code path
  * (the keyword surface of sageattention/core.py:79-157 `tensor_layout`).
@@ -60,7 +67,7 @@ typedef struct Sage3Desc {
     int32_t dtype;            /* SAGE3_FP16 | SAGE3_BF16: element type of q, k, v and out */
     int32_t is_causal;
     int32_t per_block_mean;   /* 1: Q smoothed per 128-row block (api.py:86-87); 0: one mean per head (api.py:88-90) */
-    int32_t reserved;
+    int32_t reserved;         /* SAGE3_NO_SHARED_TILES: a workspace without room for shared query tiles (any other value: with) */
     int64_t q_stride[3];      /* element strides of q for (b, h, n) */
     int64_t k_stride[3];
     int64_t v_stride[3];
@@ -75,7 +82,7 @@ typedef struct Sage3Desc {
  *   status   int32[64]                        device-written status words (0 = fine): [0, 32) pre-pass, [32, 64) attention;
  *                                             the pre-pass clears all, attention on its own its half only, so that
  *                                             sage3_check_status after sage3_fwd sees what either stage reported
- *                                             (behind them, word 64: the attention kernel's work counter; from 2 048 padded keys on int32[160]
+ *                                             (behind them, word 64: the attention kernel's work counter; where tiles may be shared int32[160]
  *                                             flags of query tiles whose keys two blocks of the attention kernel walk; then per (batch,
  *                                             kv head): delta_s holds a value that is not finite)
  *   kpart    fp32 [B*Hkv][chunks][D]          scratch: partial column sums of K (followed by those of Q when per_block_mean = 0)
@@ -91,7 +98,8 @@ typedef struct Sage3Desc {
  *   qkm      fp32 [B][Hq][Nq_p]               q . km per query row (the part of q k^T that K smoothing removes;
  *                                             core.py:289-293 `lse_correction`), used by the LSE output (sage3_fwd and
  *                                             sage3_fwd_varlen write it only when `lse` is asked for)
- *   (behind qkm, from 2 048 padded keys on and part of total_bytes: 160 accumulators of 128 rows, for those query tiles)
+ *   (behind qkm, for more than 32 queries and 2 048 padded keys or more, unless desc->reserved is SAGE3_NO_SHARED_TILES, and part of
+ *   total_bytes: 160 accumulators of 128 rows, for those query tiles)
  */
 typedef struct Sage3Workspace {
     size_t status, kpart, km, qm, delta, q_codes, q_sf, k_codes, k_sf, v_codes, v_sf, qkm;

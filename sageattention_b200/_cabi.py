@@ -14,6 +14,7 @@ LIB_PATH = _PKG / "libsage3_b200.so"
 SAGE3_FP16, SAGE3_BF16 = 0, 1
 ABI_VERSION = 4          # SAGE3_ABI_VERSION of include/sage3_b200.h this module's structs were written for
 SAGE3_OK = 0
+NO_SHARED_TILES = 0x6e6f7374     # SAGE3_NO_SHARED_TILES: Sage3Desc.reserved
 SAGE3_E_DEVICE_WAIT = -9
 
 

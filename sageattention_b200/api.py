@@ -49,14 +49,23 @@ class Workspace:
         return self.buf[off: off + nbytes] if nbytes is not None else self.buf[off:]
 
 
+def _layout(desc: _cabi.Sage3Desc) -> _cabi.Sage3Workspace:
+    lay = _cabi.Sage3Workspace()
+    _cabi.check(_cabi.lib().sage3_workspace_layout(C.byref(desc), C.byref(lay)), "sage3_workspace_layout")
+    return lay
+
+
 CACHED_WORKSPACE = object()      # `workspace=` value: take the per-(device, stream) buffer the functional entry points share
 
 
 class Sage3Problem:
-    """Shapes, strides and workspace of one call; reusable while shapes, strides and dtype stay the same."""
+    """Shapes, strides and workspace of one call; reusable while shapes, strides and dtype stay the same.
+
+    `shared_tiles=False` leaves the accumulators of query tiles that two blocks of the attention kernel share out of the workspace (problems that carry state from
+    call to call have no use for them); so does a `workspace` that has room for all but these.  The result is the same."""
 
     def __init__(self, q, k, v, tensor_layout="HND", is_causal=False, sm_scale=None, per_block_mean=True,
-                 out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, return_lse: bool = False):
+                 out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, return_lse: bool = False, shared_tiles: bool = True):
         if tensor_layout not in ("HND", "NHD"):
             raise ValueError(f"tensor_layout must be 'HND' or 'NHD', got {tensor_layout!r}")
         for name, t in (("q", q), ("k", k), ("v", v)):
@@ -115,14 +124,19 @@ class Sage3Problem:
                 raise ValueError("sm_scale must be positive")
         self.desc = d
 
-        lay = _cabi.Sage3Workspace()
-        _cabi.check(_cabi.lib().sage3_workspace_layout(C.byref(d), C.byref(lay)), "sage3_workspace_layout")
+        if not shared_tiles:
+            d.reserved = _cabi.NO_SHARED_TILES
+        lay = _layout(d)
         if workspace is CACHED_WORKSPACE:
             workspace = _shared_buffer(q.device, lay.total_bytes + 256)
         elif workspace is None:
             workspace = torch.empty(lay.total_bytes + 256, dtype=torch.uint8, device=q.device)
-        elif workspace.numel() < lay.total_bytes + 256 or workspace.dtype != torch.uint8 or workspace.device != q.device:
-            raise ValueError(f"workspace must be a uint8 CUDA tensor of at least {lay.total_bytes + 256} bytes")
+        else:
+            if workspace.numel() < lay.total_bytes + 256:
+                d.reserved = _cabi.NO_SHARED_TILES
+                lay = _layout(d)
+            if workspace.numel() < lay.total_bytes + 256 or workspace.dtype != torch.uint8 or workspace.device != q.device:
+                raise ValueError(f"workspace must be a uint8 CUDA tensor of at least {lay.total_bytes + 256} bytes")
         shift = (-workspace.data_ptr()) % 256
         self.ws = Workspace(workspace[shift: shift + lay.total_bytes], lay)
 
@@ -150,8 +164,7 @@ class Sage3Problem:
         d.o_stride = (C.c_int64 * 3)(*(o_stride or q_stride or (Hq * Nq * D, Nq * D, D)))
         d.sm_scale = 0.0 if sm_scale is None else float(sm_scale)
         self.desc = d
-        lay = _cabi.Sage3Workspace()
-        _cabi.check(_cabi.lib().sage3_workspace_layout(C.byref(d), C.byref(lay)), "sage3_workspace_layout")
+        lay = _layout(d)
         workspace = torch.empty(lay.total_bytes + 256, dtype=torch.uint8, device=device)
         shift = (-workspace.data_ptr()) % 256
         self.ws = Workspace(workspace[shift: shift + lay.total_bytes], lay)
@@ -398,6 +411,7 @@ def _varlen_impl(q, k, v, cq, ck, max_seqlen_q, max_seqlen_k, is_causal, sm_scal
     if q.shape[0] == 0:
         return (out, lse) if return_lse else out
     d = _cabi.Sage3Desc()
+    d.reserved = _cabi.NO_SHARED_TILES            # (a packed batch shares none)
     d.B, d.Hq, d.Hkv, d.Nq, d.Nk, d.D = nseq, Hq, Hkv, max_seqlen_q, max_seqlen_k, D
     d.dtype = _DTYPES[q.dtype]
     d.is_causal = int(bool(is_causal))

@@ -46,8 +46,12 @@ inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 // sets when a value of its delta_s is not finite.  The first pre-pass kernel clears all; what is the attention kernel's lies in one piece, since
 // an attention call on its own clears it with one memset (a second one takes 1.0 to 1.6 us: one token of 32 heads, 3 072 keys 18.5 -> 19.9).
 constexpr int kAttnStatusWord = 32, kUnitCounterWord = 64, kSplitFlagsWord = 65;
-inline bool shares_tiles(const Sage3Workspace& w) { return w.nk_pad / 128 >= sage3::kSplitMinBlocks; }
-inline int nonfinite_word(const Sage3Workspace& w) { return kSplitFlagsWord + (shares_tiles(w) ? sage3::kSplitSlots : 0); }
+// Whether the layout has room for shared tiles.  (Up to 32 query rows are PackRule's mode 2 whatever the heads, and are not dealt out.  The number of heads has no part
+// in it, so that a workspace large enough for one problem is large enough for any that is smaller in every size.)
+inline bool shares_tiles(const Sage3Desc* d) {
+    return ((int64_t)d->Nk + 127) / 128 >= sage3::kSplitMinBlocks && d->Nq > 32 && d->reserved != SAGE3_NO_SHARED_TILES;
+}
+inline int nonfinite_word(const Sage3Desc* d) { return kSplitFlagsWord + (shares_tiles(d) ? sage3::kSplitSlots : 0); }
 
 int validate(const Sage3Desc* d) {
     if (!d) return SAGE3_E_NULL;
@@ -83,9 +87,8 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     const size_t kch_k = ((size_t)d->Nk + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t kch_q = ((size_t)d->Nq + sage3::kRowsPerChunk - 1) / sage3::kRowsPerChunk;
     const size_t part = B * Hkv * kch_k + (d->per_block_mean ? 0 : B * Hq * kch_q);
-    w->nk_pad = (int32_t)nkp;
     size_t off = 0;
-    w->status = off;  off += align_up((nonfinite_word(*w) + B * Hkv) * sizeof(int32_t));
+    w->status = off;  off += align_up((nonfinite_word(d) + B * Hkv) * sizeof(int32_t));
     w->kpart = off;   off += align_up(part * D * sizeof(float));
     w->km = off;      off += align_up(B * Hkv * D * 2);
     w->qm = off;      off += align_up(B * Hq * nqm * D * 2);
@@ -97,9 +100,10 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
     w->v_codes = off; off += align_up(B * Hkv * D * (nkp / 2));
     w->v_sf = off;    off += align_up(B * Hkv * (nkp / 128) * 1024);
     w->qkm = off;     off += align_up(B * Hq * nqp * sizeof(float));
-    if (shares_tiles(*w)) off += align_up(sage3::kSplitSlots * sage3::split_state_floats(D) * sizeof(float));      // see split_state
+    if (shares_tiles(d)) off += align_up(sage3::kSplitSlots * sage3::split_state_floats(D) * sizeof(float));      // see split_state
     w->total_bytes = off;
     w->nq_pad = (int32_t)nqp;
+    w->nk_pad = (int32_t)nkp;
     w->nqm = (int32_t)nqm;
     w->kchunks = (int32_t)kch_k;
     return SAGE3_OK;
@@ -107,7 +111,7 @@ int layout(const Sage3Desc* d, Sage3Workspace* w) {
 
 // Accumulators of query tiles whose keys two CTAs share, behind the last region of the layout; nullptr where the layout has none.
 float* split_state(const Sage3Desc* d, const Sage3Workspace& w, void* ws) {
-    if (!shares_tiles(w)) return nullptr;
+    if (!shares_tiles(d)) return nullptr;
     return reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + w.qkm + align_up((size_t)d->B * d->Hq * w.nq_pad * sizeof(float)));
 }
 
@@ -176,7 +180,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* base = static_cast<uint8_t*>(ws);
     if (!cleared && sage3::checked(cudaMemsetAsync(base + w.status + kAttnStatusWord * sizeof(int32_t), 0,
-                                                   (nonfinite_word(w) - kAttnStatusWord) * sizeof(int32_t), st)) != cudaSuccess)
+                                                   (nonfinite_word(desc) - kAttnStatusWord) * sizeof(int32_t), st)) != cudaSuccess)
         return SAGE3_E_CUDA;
     sage3::AttnArgs a;
     a.B = desc->B; a.Hq = desc->Hq; a.Hkv = desc->Hkv; a.Nq = desc->Nq; a.Nk = desc->Nk; a.D = desc->D;
@@ -199,7 +203,7 @@ int attn_impl(const Sage3Desc* desc, void* ws, const sage3::PartsPtr& out, float
     a.status = reinterpret_cast<int*>(base + w.status) + kAttnStatusWord;
     a.unit_counter = reinterpret_cast<int*>(base + w.status) + kUnitCounterWord;
     a.prepass_status = reinterpret_cast<const int*>(base + w.status);
-    a.nonfinite = reinterpret_cast<const int*>(base + w.status) + nonfinite_word(w);
+    a.nonfinite = reinterpret_cast<const int*>(base + w.status) + nonfinite_word(desc);
     a.cu_q = cu_q; a.cu_k = cu_k;
     a.split_state = split_state(desc, w, ws);
     a.split_flags = a.split_state ? reinterpret_cast<int*>(base + w.status) + kSplitFlagsWord : nullptr;
@@ -357,8 +361,8 @@ static int prepass_impl(const Sage3Desc* desc, const sage3::PartsPtr& q, const s
     a.clear = a.status;
     // (without carried state, which only the attention call knows about: a word more or less per head costs nothing)
     const bool shared = sage3::PackRule(desc->Nq, desc->Hq / desc->Hkv, cu_q == nullptr).heads > 1;
-    a.nonfinite = shared ? a.status + nonfinite_word(w) : nullptr;
-    a.n_clear = nonfinite_word(w) + (shared ? desc->B * desc->Hkv : 0);
+    a.nonfinite = shared ? a.status + nonfinite_word(desc) : nullptr;
+    a.n_clear = nonfinite_word(desc) + (shared ? desc->B * desc->Hkv : 0);
     a.km_given = km_in != nullptr;
     if (km_in != nullptr &&
         sage3::checked(cudaMemcpyAsync(a.km, km_in, (size_t)desc->B * desc->Hkv * desc->D * 2, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)

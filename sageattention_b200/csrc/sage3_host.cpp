@@ -155,6 +155,7 @@ PyObject* fwd_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
         q.size(0) == 0 || k.size(0) == 0 || max_q < 1 || max_k < 1 || max_q > most || max_k > most || !usable(q) || !usable(k) || !usable(v))
         Py_RETURN_NONE;
     Sage3Desc d = {};
+    d.reserved = SAGE3_NO_SHARED_TILES;                // (a packed batch shares none)
     d.B = (int32_t)nseq; d.Hq = (int32_t)Hq; d.Hkv = (int32_t)Hkv; d.Nq = (int32_t)max_q; d.Nk = (int32_t)max_k; d.D = (int32_t)D;
     d.dtype = q.scalar_type() == at::kBFloat16 ? SAGE3_BF16 : SAGE3_FP16;
     d.is_causal = causal;

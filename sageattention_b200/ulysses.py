@@ -294,7 +294,7 @@ def context_parallel_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     stream = torch.cuda.current_stream(dev).cuda_stream
     out = torch.empty_like(qh)
     lse = torch.empty(B, Hq, n, dtype=torch.float32, device=dev) if return_lse else None
-    prob = Sage3Problem(qh, kh, vh, "HND", is_causal, sm_scale, per_block_mean, out=out)
+    prob = Sage3Problem(qh, kh, vh, "HND", is_causal, sm_scale, per_block_mean, out=out, shared_tiles=False)
 
     # K mean of the whole sequence, in the single call's order: per-rank partial column sums (512-row chunks, written by
     # the pre-pass into its workspace), gathered, added chunk by chunk in fp32, scaled by 1 / N, rounded once

@@ -61,6 +61,28 @@ def test_ragged_and_global_mean_layout():
     assert (w.nq_pad, w.nk_pad, w.nqm, w.kchunks) == (17792, 17792, 1, 35)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_room_for_shared_tiles(D):
+    """Flags and accumulators of shared query tiles: for 2 048 padded keys and more than 32 queries on, unless they are left out; the workspace is then
+    what it is without them.  A problem that is smaller in every size fits the workspace of a larger one."""
+    lib = _cabi.lib()
+
+    def sizes(**kw):
+        d, w = _desc(D=D, **kw), _cabi.Sage3Workspace()
+        assert lib.sage3_workspace_layout(C.byref(d), C.byref(w)) == 0
+        without = w.qkm + (d.B * d.Hq * w.nq_pad * 4 + 1023) // 1024 * 1024 - (w.kpart - (65 + d.B * d.Hkv + 255) // 256 * 1024)
+        return w.total_bytes, without
+    for kw, room in ((dict(Nq=1024, Nk=1920), False), (dict(Nq=1024, Nk=1921), True), (dict(Nq=32, Nk=9000), False), (dict(Nq=33, Nk=9000), True),
+                     (dict(B=9, Hq=32, Hkv=32, Nq=300, Nk=9000), True)):
+        total, without = sizes(**kw)
+        assert (160 * (128 * D + 384) * 4 <= total - without <= 160 * (128 * D + 384) * 4 + 2048) if room else total == without, kw
+        assert sizes(**kw, reserved=_cabi.NO_SHARED_TILES) == (without, without)
+        assert sizes(**kw, reserved=1) == (total, without)
+    for B, H, Nq, Nk in ((1, 1, 64, 2048), (2, 8, 300, 2048), (4, 32, 64, 9000)):
+        most = sizes(B=B, Hq=H, Hkv=1, Nq=Nq, Nk=Nk)[0]
+        assert all(sizes(B=b, Hq=h, Hkv=1, Nq=nq, Nk=nk)[0] <= most for b in (1, B) for h in (1, H) for nq in (1, 32, 33, Nq) for nk in (1, 2047, 2048, Nk))
+
+
 @pytest.mark.parametrize("kw,code", [
     (dict(D=96), -2), (dict(D=256), -2), (dict(Hq=3, Hkv=2), -2), (dict(Nq=0), -2), (dict(B=-1), -2),
     (dict(dtype=7), -3), (dict(Nk=1 << 25), -8),

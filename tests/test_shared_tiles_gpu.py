@@ -81,3 +81,23 @@ def test_shared_tiles_on_two_streams_and_in_a_graph(cuda_device, D):
         graph.replay()
     torch.cuda.synchronize()
     assert p.check_status() == 0 and torch.equal(p.out, want)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_workspace_without_room_for_shared_tiles(cuda_device, D):
+    """A workspace that has room for all but the flags and accumulators is accepted, and the result is the same; one that is smaller is refused."""
+    g = torch.Generator(device=cuda_device).manual_seed(2300 + D)
+    q = torch.randn(2, 32, 1000, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+    k, v = (torch.randn(2, 32, 6000, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
+    want = Sage3Problem(q, k, v, is_causal=True)
+    want.run()
+    assert want.desc.reserved == 0
+    need = Sage3Problem(q, k, v, is_causal=True, shared_tiles=False).ws.layout.total_bytes + 256
+    assert need < want.ws.layout.total_bytes
+    p = Sage3Problem(q, k, v, is_causal=True, workspace=torch.full((need,), 255, dtype=torch.uint8, device=cuda_device))
+    for _ in range(2):
+        assert torch.equal(p.run(), want.out)
+    assert p.check_status() == 0
+    assert torch.equal(sageattn3(q, k, v, is_causal=True, workspace=torch.empty(need, dtype=torch.uint8, device=cuda_device)), want.out)
+    with pytest.raises(ValueError, match=str(need)):
+        Sage3Problem(q, k, v, is_causal=True, workspace=torch.empty(need - 1, dtype=torch.uint8, device=cuda_device))
