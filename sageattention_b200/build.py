@@ -18,7 +18,7 @@ LIB = PKG / "libsage3_b200.so"
 HOST_LIB = PKG / "_host.so"
 HOST_SOURCE = "sage3_host.cpp"
 SOURCES = ["sage3_abi.cu", "sage3_prepass.cu", "sage3_attn.cu"]
-HEADERS = ["sage3_common.cuh", "sage3_kernels.h"]
+HEADERS = ["sage3_common.cuh", "sage3_kernels.h", "sage3_split.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 

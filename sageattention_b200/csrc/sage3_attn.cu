@@ -51,6 +51,7 @@
 
 #include "sage3_common.cuh"
 #include "sage3_kernels.h"
+#include "sage3_split.h"
 
 namespace sage3 {
 
@@ -90,7 +91,7 @@ struct SplitParams : AttnParams {
     int rest0;                          // see rest_tile
     int* split_flags;
     float* split_state;
-    uint32_t slot_first[kSplitSlots];   // first tile of a slot (12 bits) and first key block of it
+    uint32_t slot_first[kSplitSlots];
 };
 
 constexpr int kUnitRing = 4;
@@ -277,34 +278,6 @@ __device__ __forceinline__ float4 load_state(const float4* p) {
     float4 v;
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
     return v;
-}
-
-// Tile number j of those dealt out by key blocks.  Without a mask the last ones of an odd number of tiles per head (whole units are pairs then, so that the rounds
-// ahead are even), and the tiles from pair number rest0 / 2 on; with one in the order of the pairs, of which the first rest0 have one tile.
-template <bool CAUSAL>
-__host__ __device__ __forceinline__ void rest_tile(int j, int nqt, int BHq, int whole, int rest0, int& bhq, int& mt) {
-    if (!CAUSAL) {
-        const int odd = nqt & 1 ? BHq : 0;
-        if (j < odd) {
-            bhq = j;
-            mt = nqt - 1;
-        } else {
-            bhq = (rest0 + j - odd) / (nqt & ~1);
-            mt = rest0 + j - odd - bhq * (nqt & ~1);
-        }
-        return;
-    }
-    const int npair = (nqt + 1) >> 1, one = rest0;
-    const int pair = j < one ? whole + j : whole + one + ((j - one) >> 1);
-    bhq = pair % BHq;
-    mt = 2 * (npair - 1 - pair / BHq) + (j < one ? 0 : 1 - ((j - one) & 1));
-}
-
-// Key blocks of a query tile.
-template <bool CAUSAL>
-__host__ __device__ __forceinline__ int tile_blocks(int mt, int Nk, int shift) {
-    const int last = CAUSAL && mt * kBlock + kBlock - 1 + shift < Nk - 1 ? mt * kBlock + kBlock - 1 + shift : Nk - 1;
-    return last < 0 ? 0 : last / kBlock + 1;
 }
 
 // The part of tile j of the rest from key block lo on, `left` blocks of it at most, in slot m.
@@ -1355,85 +1328,6 @@ static cudaError_t launch_t(const AttnArgs& a, const CUtensorMap& tq, const CUte
                               : launch_v<D, CAUSAL, OutT, false, 0>(tq, tk, tv, td, p, grid, st);
 }
 
-// The last rounds of units dealt out by key blocks.  Units are pairs of tiles, and 5.5 pairs per SM take as long as 6, 0.86 as long as 1: the tiles of the
-// round that is not full (of the one before too, where that leaves less than a tile per SM) are cut into slots of as many key blocks as come to one SM, in the
-// order tile after tile, blocks of a tile from its first key on (McNaughton 1959).  A CTA draws one slot and takes its parts in that order.  A tile lies in
-// one slot or two: the one behind has its last keys, at its own start, walks them, and leaves the accumulator, row sums and maxima in memory; the one
-// before has its first keys, at its end, and goes on from there.  So the same operations in the same order, and the same bits, as in one walk.  Slots are
-// drawn from the last to the first: the part that is waited for belongs to a slot drawn before, where it comes first and waits for nothing, so some CTA can
-// always go on, however many of them are resident.
-// us per call, without / with: 1 000 queries x 9 192 keys, 32 heads 139.3 / 127.9, 1 500 x 12 000, 28 heads 246.8 / 200.9, 600 x 5 000 84.5 / 61.3; 4 250 tokens
-// of 48 heads, D = 64 349.0 / 333.9; N tokens of H heads, D = 128 (64): 16 x 2 500 72.4 / 63.7 (63.8 / 55.4), 10 x 4 100 104.5 / 90.2 (94.3 / 80.4), 16 x 5 000 194.9
-// / 180.4 (174.3 / 162.3), 24 x 5 000 269.2 / 259.0 (239.7 / 233.2), 5 x 16 384 532 / 476 (498 / 454).
-// What it costs: some 8 blocks per slot (two more changes of units, 64 KB of accumulator in and out), and at D = 64 without a mask the rolled halves.  So: from 10 blocks
-// of gain, 1 / 80 of the call (less shows nothing: 16 384 x 24 heads, 1.15 %, 2 192 / 2 182, 8 192 x 32, 1.1 %, 792 / 794), there 1 / 25 (24 x 6 000, 3.2 %, 312 / 313, 40 x 5 000,
-// 1.6 %, 372 / 379).  With a mask only where it is that of a chunk of a longer sequence (tiles differ by a quarter of their blocks at most): pairs in order of their
-// length level out by themselves otherwise.  The rounds ahead have to be even, since a CTA's slot is as long as any other's: 2 x 32 heads x 10 590 tokens, 83 tiles per head of which
-// one was a unit of its own in them, 2 526 / 2 555.
-struct SplitPlan { int whole = 0, slots = 0; };      // pairs ahead of the slots
-
-template <bool CAUSAL>
-static SplitPlan plan_split(const AttnArgs& a, int mode, int nqt, int pairs, int sms, SplitParams& p) {
-    p.slot_blocks = 0;
-    p.split_flags = a.split_flags;
-    p.split_state = a.split_state;
-    SplitPlan none, plan;
-    if (a.split_flags == nullptr || mode != 0 || a.cu_q != nullptr || a.carry_o_in != nullptr || a.carry_o_out != nullptr || sms > kSplitSlots) return none;
-    const int BHq = a.B * a.Hq, last = tile_blocks<CAUSAL>(nqt - 1, a.Nk, a.causal_shift);
-    if (last < kSplitMinBlocks || 4 * tile_blocks<CAUSAL>(0, a.Nk, a.causal_shift) < 3 * last) return none;
-    const bool odd = (nqt & 1) != 0;
-    int tiles;                        // dealt out by blocks
-    double before;                    // blocks per SM without slots
-    if (CAUSAL) {
-        const int full = pairs / sms, over = pairs % sms;
-        const bool that_round = 2 * over > sms;      // the round that is not full is enough
-        if (over == 0 || (!that_round && full == 0)) return none;
-        plan.whole = pairs - over - (that_round ? 0 : sms);
-        if (odd && plan.whole > 0) return none;      // (the rounds ahead of the slots are not even)
-        p.rest0 = odd ? BHq : 0;
-        tiles = p.rest0 + 2 * (pairs - plan.whole - p.rest0);
-        before = nqt == 1 ? (full + 1) * (double)last : (2 * full + (that_round ? 2 : 1) - (odd ? 0.5 : 0)) * last;      // (odd: units of one tile among them level out)
-    } else {
-        // rounds of whole pairs ahead such that one to three tiles per SM are left
-        const int64_t all = (int64_t)BHq * nqt;
-        const int whole_pairs = BHq * (nqt / 2);
-        int64_t rounds = all / (2 * sms);
-        if (rounds > 0 && all - rounds * 2 * sms < sms) --rounds;
-        if (rounds * sms > whole_pairs || all - rounds * 2 * sms > 4 * sms || all <= sms) return none;
-        plan.whole = (int)rounds * sms;
-        p.rest0 = 2 * plan.whole;
-        tiles = (int)(all - p.rest0);
-        const int full = pairs / sms, over = pairs % sms;
-        // (an odd number of tiles per head: one unit of a head is a single tile, which levels out half of a tile)
-        before = nqt == 1 ? (double)((all + sms - 1) / sms) * last
-               : odd      ? ((double)all / sms + 0.5) * last
-                          : (2 * full + (over == 0 ? 0 : 2 * over > sms ? 2 : 1)) * (double)last;
-    }
-    auto blocks = [&](int j) {
-        int bhq, mt;
-        rest_tile<CAUSAL>(j, nqt, BHq, plan.whole, p.rest0, bhq, mt);
-        return tile_blocks<CAUSAL>(mt, a.Nk, a.causal_shift);
-    };
-    int sum = CAUSAL ? 0 : tiles * last, most = last;
-    for (int j = 0; CAUSAL && j < tiles; ++j) sum += blocks(j);
-    const int per = (sum + sms - 1) / sms > most ? (sum + sms - 1) / sms : most;
-    const double gain = before - per - plan.whole / sms * 2.0 * last;
-    if (gain < 10 || gain * (a.D == 64 && !CAUSAL ? 25 : 80) < before) return none;
-    plan.slots = (sum + per - 1) / per;
-    p.slot_blocks = per;
-    p.slot_rest = sum - (plan.slots - 1) * per;
-    for (int i = 0, j = 0, at = 0; i < plan.slots; ++i) {      // slot plan.slots - 1 - i begins at block i * per of all tiles' blocks; tile j's first one is number `at`
-        if (!CAUSAL) {
-            j = i * per / last;
-            at = j * last;
-        } else {
-            for (int n; at + (n = blocks(j)) <= i * per; ++j) at += n;
-        }
-        p.slot_first[plan.slots - 1 - i] = (uint32_t)j | (uint32_t)(i * per - at) << 12;
-    }
-    return plan;
-}
-
 cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     *driver_rc = 0;
     EncodeTiledFn fn = get_encode_fn();
@@ -1473,7 +1367,12 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), rest = pairs % sms;
     const bool split = nqt > 1 && 2 * rest <= sms;
     p.unit_counter = a.unit_counter;
-    const SplitPlan plan = a.is_causal ? plan_split<true>(a, mode, nqt, pairs, sms, p) : plan_split<false>(a, mode, nqt, pairs, sms, p);
+    SplitPlan plan;
+    if (a.split_flags != nullptr && mode == 0 && a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr)
+        plan = a.is_causal ? plan_split<true>(a.B * a.Hq, nqt, a.Nk, a.causal_shift, a.D, sms) : plan_split<false>(a.B * a.Hq, nqt, a.Nk, a.causal_shift, a.D, sms);
+    p.slot_blocks = plan.blocks; p.slot_rest = plan.rest; p.rest0 = plan.rest0;
+    p.split_flags = a.split_flags; p.split_state = a.split_state;
+    for (int i = 0; i < plan.slots; ++i) p.slot_first[i] = plan.first[i];
     p.whole_units = plan.slots > 0 ? plan.whole : split ? pairs - rest : pairs;
     p.pack_heads = pack;
     p.pack_tiles = (group + pack - 1) / pack;

@@ -9,7 +9,6 @@
 
 namespace sage3 {
 
-constexpr int kBlock = 128;   // query-tile rows and keys per KV block
 constexpr int kMicro = 16;    // NVFP4 microblock
 
 // status-word codes written by device code when a bounded wait gives up

@@ -8,6 +8,7 @@
 
 namespace sage3 {
 
+constexpr int kBlock = 128;          // query-tile rows and keys per KV block
 constexpr int kRowsPerChunk = 512;   // rows per partial column sum (fixes the summation order)
 constexpr int kMaxParts = 8;         // a tensor's tokens may be split over this many buffers (one per GPU of a node)
 
