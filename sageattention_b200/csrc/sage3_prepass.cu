@@ -479,8 +479,8 @@ __device__ __forceinline__ void quant_q_tile(
 // map over delta), so the threads' load / store instructions carry only the K rows, the codes and the staging of
 // the converted accumulator.
 // ------------------------------------------------------------------------------------------------
-// AROWS = 64: up to 64 query blocks and up to one tile per SM, or, at D = 64, up to four (the A tile then has 64 rows, the MMA's other 64 read what lies behind it,
-// for accumulator rows nobody looks at; four blocks per SM), see launch_prepass_t.  Up to 64 query blocks are otherwise quant_k_delta_run_kernel's.
+// AROWS = 64: up to 64 query blocks (the A tile then has 64 rows, the MMA's other 64 read what lies behind it, for accumulator rows nobody looks at; four blocks
+// per SM) where few tiles come to an SM, see launch_prepass_t.  Up to 64 query blocks are otherwise quant_k_delta_run_kernel's.
 // FLAG: notes whether a value of delta_s is not finite, for calls whose heads share a tile in the attention kernel.
 template <typename T, int D, int AROWS, bool FLAG>
 __global__ void __launch_bounds__(256, AROWS == 128 ? 3 : 4) quant_k_delta_kernel(
@@ -696,8 +696,9 @@ __global__ void __launch_bounds__(256, AROWS == 128 ? 3 : 4) quant_k_delta_kerne
 // 4 blocks 58.2 / 33.5 / 15.0 / 14.8 -> 50.1 / 29.0 / 14.6 / 14.5, 64 blocks 92.2 / 47.7 / 17.5 / 15.9 -> 84.4 / 45.1 / 18.5 / 14.6.  Variants of it, first figure
 // (51.5 before): rows copied to shared memory ahead by all warps 44.5, by a warp of its own 44.1 (shared memory then moves 160 KB per tile: the copy, the
 // read, k', and the MMA's operands), three blocks per SM 38.6 (two 36.0), one store per key and row 36.0 -> 35.5, row addresses ahead 34.3.
-// NR = 32 instead of 64 columns: up to eight query blocks from a number of tiles on.  (One token of 8 x 32 heads 90.5 / 91.8 us of pre-pass; with few
-// tiles neither shows.)
+// NR = 32 instead of 64 columns: up to 32 query blocks (half of the read-out and of its registers).  Pre-pass with 64 / 32 columns, us: one token of 4 x 32 heads, 8 kv heads, 4 096
+// keys 28.7 / 27.6 (D = 64 20.5 / 19.3), 8 192 47.1 / 46.0 (30.5 / 28.1), of 8 x 32 heads 92.2 / 90.3 (53.3 / 49.2), of 8 x 28 heads, 4 kv heads, 9 000 keys 53.7 / 53.2 (34.8 / 31.9); 24
+// query blocks, 2 x 8 x 16 000 keys 50.9 / 50.7 (32.6 / 31.2).
 // ------------------------------------------------------------------------------------------------
 // A place in the list of tiles: entry by entry, head by head, tile by tile.
 template <typename T>
@@ -719,9 +720,6 @@ struct KCursor {
 };
 
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-
-// Tiles per SM from which calls of up to eight query blocks take the kernel for 32 of them.
-constexpr int kRun32TilesPerSm(int D) { return D == 128 ? 27 : 20; }
 
 template <int D, int NR>
 struct KRunCfg {
@@ -1231,22 +1229,22 @@ static cudaError_t launch_prepass_t(const PrepassArgs& a, cudaStream_t st) {
                           a.status, a.nonfinite, tm_qm, tm_delta);
         });
     };
-    // 65 to 128 query blocks, D = 64 (at D = 128 the wider accumulator spills: 3 000 tokens of 4 x 32 heads, 96 blocks 57.5 / 59.0 us of pre-pass): runs, where all blocks of one
-    // tile, three per SM, would not be resident at once, or two per SM are enough.  Pre-pass, one tile per block / runs: 16 000 tokens of 2 x 32 heads 211.7 / 192.3, 9 000 of 40 71.5 / 64.5,
-    // 4 000 of 8 x 32 (8 kv heads) 84.3 / 81.7, of 2 x 32 (512 tiles) 26.7 / 24.8, 4 096 of 32 (256) 18.4 / 16.8; not: 2 600 of 2 x 32 (336) 18.6 / 20.5, 3 400 (432) 22.5 / 22.6.
+    // Which kernel, us per call with a block per tile / runs.
+    // Up to one tile per SM nothing goes on in a run: the pre-pass alone is shorter with runs (1 024 tokens of 16 heads 15.2 / 12.8), but the attention kernel starts later behind
+    // them: D = 128, 1 024 of 16 25.1 / 26.1, 500 queries of 32 heads, 1 000 keys of 8 24.6 / 26.4, 1 500 of 12 29.8 / 30.6, 256 of 8 16.4 / 16.7, 2 048 of 8 32.7 / 32.8; D = 64, 1 829 of
+    // 4 x 2 26.7 / 28.7, 700 of 2 x 8, causal, 19.2 / 20.5.
+    // At D = 64 four blocks of one tile fit an SM at once, two of the other kernel: a block per tile between two and three tiles per SM, too.  Up to 64 query blocks, 2.2 tiles per SM 70.2
+    // / 71.3, 73.8 / 74.6, 2.6 21.4 / 21.9, 2.7 42.0 / 42.7, 37.5 / 37.9, 2.8 89.3 / 89.7; 3.1 35.4 / 35.0, 96.3 / 96.3, 3.4 69.5 / 67.8, 78.5 / 78.1, 3.7 73.8 / 72.0, 161.1 / 160.9, 3.8 54.4 /
+    // 53.3, 3.9 23.8 / 22.6, 59.1 / 57.4, 204.7 / 203.9.  Up to 32 also between one and two, where it is by turns the faster and the slower: 1.1 20.5 / 21.7, 47.2 / 48.0, 1.4 51.1 / 51.1, 34.9 /
+    // 35.8, 1.6 40.9 / 41.0, 18.4 / 18.0, 1.8 44.3 / 43.5, 43.0 / 43.1, 2.0 28.5 / 27.1, 67.6 / 67.6.
+    // 65 to 128 query blocks at D = 64 alike (at D = 128 the wider accumulator spills: 3 000 tokens of 4 x 32 heads, 96 blocks 57.5 / 59.0 us of pre-pass).  Pre-pass: 16 000 tokens of
+    // 2 x 32 heads 211.7 / 192.3, 9 000 of 40 71.5 / 64.5, 4 000 of 8 x 32 (8 kv heads) 84.3 / 81.7, of 2 x 32 (512 tiles) 26.7 / 24.8, 4 096 of 32 (256) 18.4 / 16.8; between two and three 2 600
+    // of 2 x 32 (336) 18.6 / 20.5, 3 400 (432) 22.5 / 22.6.
+    const bool runs = D == 64 ? rows <= 128 && (tiles > 3 * info.sms || (rows > 32 && tiles > info.sms && tiles <= 2 * info.sms)) : rows <= 64 && tiles > info.sms;
+    if (!runs) return rows > 64 ? one_tile(std::integral_constant<int, 128>()) : one_tile(std::integral_constant<int, 64>());
     if constexpr (D == 64)
-        if (rows > 64 && rows <= 128 && ((tiles > info.sms && tiles <= 2 * info.sms) || tiles > 3 * info.sms)) return run(std::integral_constant<int, 128>());
-    if (rows > 64) return one_tile(std::integral_constant<int, 128>());
-    // Up to one tile per SM nothing goes on in a run, and the block of one tile is quicker to its end: 1 829 tokens of 4 x 2 heads 30.8 / 30.9 us per call, D = 64 26.7 / 28.7, 1 024 of
-    // two heads 22.6 / 22.7 (19.9 / 20.4), 700 of 2 x 8 heads, causal, 22.6 / 22.6 (19.2 / 20.5).
-    if (tiles <= info.sms) return one_tile(std::integral_constant<int, 64>());
-    // D = 64, a block per tile against runs of tiles, where four blocks of the one fit an SM at once and two of the other take a second turn.  64 query blocks, pre-pass:
-    // 296 tiles 15.9 / 14.6, 400 16.5 / 17.7, 512 17.5 / 18.5, 1 024 26.8 / 26.6 us; whole calls: 512 tokens 4 x 32 heads, 2 048 queries 74.0 / 75.0, 1 280 tokens of 40 heads
-    // 42.5 / 43.0, 1 024 of 48 36.9 / 38.0, 1 700 of 32 63.5 / 63.6.  Up to two
-    // tiles per SM it is a turn each; 500 queries of 16 heads, 2 715 keys of 8 (176 tiles of 8 query blocks) 32.8 / 33.6.
-    if constexpr (D == 64)
-        if ((rows <= 32 || tiles > 2 * info.sms) && tiles <= 4 * info.sms) return one_tile(std::integral_constant<int, 64>());
-    return rows <= 8 && tiles >= (int64_t)kRun32TilesPerSm(D) * info.sms ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 64>());
+        if (rows > 64) return run(std::integral_constant<int, 128>());
+    return rows > 32 ? run(std::integral_constant<int, 64>()) : run(std::integral_constant<int, 32>());
 }
 
 cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t st) {

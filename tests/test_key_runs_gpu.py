@@ -30,14 +30,17 @@ def _workspace(p, B, Hkv):
     (1, 1, 37, 8),               # 296 tiles: one per block on 148 SMs
     (8, 1, 99, 3),               # 297: one block has two
     (3, 128 * 5 + 1, 98, 3),     # 18 query blocks, 294 tiles
-    (1, 128 * 32, 50, 12),       # 32 query blocks: one half of the accumulator's columns
-    (1, 128 * 33, 50, 12),       # 33
+    (2, 128 * 8, 37, 13),        # 16, 481 tiles: one half of an accumulator of 32 columns
+    (1, 128 * 17, 37, 13),       # 17
+    (1, 128 * 32, 50, 12),       # 32: all columns of it
+    (1, 128 * 33, 50, 12),       # 33: an accumulator of 64 columns
     (7, 128 * 9, 45, 9),         # 63
     (4, 128 * 16, 61, 10),       # 64
-    (4, 128 * 16, 33, 15),       # 64, 495 tiles: D = 64 has a block per tile
+    (4, 128 * 16, 33, 12),       # 64, 396 tiles: D = 64 has a block per tile
+    (4, 128 * 16, 33, 15),       # 64, 495 tiles
     (5, 128 * 13, 40, 10),       # 65: D = 64 has an accumulator of 128 columns
     (8, 128 * 16, 40, 10),       # 128
-    (8, 1, 100, 40),             # 4 000 tiles and up to eight query blocks: the accumulator of 32 columns
+    (8, 1, 100, 40),             # 4 000 tiles
 ])
 def test_runs_of_key_tiles(cuda_device, D, group, Nq, tiles, heads):
     g = torch.Generator(device=cuda_device).manual_seed(2000 + tiles + Nq)

@@ -159,16 +159,20 @@ def test_halves_are_unrolled_where_that_is_faster(fake, call, Nk, causal, D, rol
     assert f"ELb{rolled}EEEv" in name, name
 
 
-@pytest.mark.parametrize("D,tiles,heads,kw,rows", [
-    (128, 27 * 148, 1, {}, 32), (128, 27 * 148 - 1, 1, {}, 64), (64, 20 * 148, 8, {}, 32), (64, 20 * 148 - 1, 8, {}, 64), (64, 20 * 148, 9, {}, 64),
-    (128, 27 * 148, 8, dict(Nq=20000, per_block_mean=0), 32), (128, 27 * 148, 9, dict(Nq=20000, per_block_mean=0), 64), (128, 27 * 148, 1, dict(Nq=1025), 64)])
-def test_key_tiles_are_taken_in_turn_from_a_number_per_sm(fake, D, tiles, heads, kw, rows):
-    """The K kernel's rows of query blocks: 32, and several tiles per block, for up to eight blocks of all query heads of a kv head (one per head with
-    one Q mean) and a number of key tiles that counts in SMs (148 here)."""
-    fake.fake_start(-1, 0)
-    assert _fwd(fake, _desc(**{**dict(B=1, Hq=heads, Hkv=1, Nq=1, Nk=128 * tiles, D=D), **kw})) == 0
-    name = [entry[1] for entry in _log(fake) if "quant_k_delta" in entry[1]][0]
-    assert f"Li{D}ELi{rows}E" in name, name
+@pytest.mark.parametrize("D,tiles,blocks,kernel,rows", [
+    (128, 148, 1, "", 64), (128, 148, 64, "", 64), (128, 148, 65, "", 128), (128, 149, 32, "_run", 32), (128, 149, 33, "_run", 64), (128, 149, 64, "_run", 64),
+    (128, 149, 65, "", 128), (128, 4000, 8, "_run", 32), (128, 4000, 65, "", 128),
+    (64, 148, 32, "", 64), (64, 148, 128, "", 128), (64, 149, 32, "", 64), (64, 149, 33, "_run", 64), (64, 296, 64, "_run", 64), (64, 296, 65, "_run", 128), (64, 297, 33, "", 64),
+    (64, 297, 128, "", 128), (64, 444, 32, "", 64), (64, 444, 64, "", 64), (64, 444, 65, "", 128), (64, 445, 1, "_run", 32), (64, 445, 32, "_run", 32), (64, 445, 64, "_run", 64),
+    (64, 445, 128, "_run", 128), (64, 445, 129, "", 128), (64, 4000, 8, "_run", 32)])
+def test_which_kernel_takes_k(fake, D, tiles, blocks, kernel, rows):
+    """A block of the K kernel has one tile or walks a run of them, by the number of key tiles per SM (148 here) and of query blocks of all query heads of a kv head (one per
+    head with one Q mean); the rows or columns that it has for these."""
+    name = f"quant_k_delta{kernel}_kernelI13__nv_bfloat16Li{D}ELi{rows}E"
+    for kw in (dict(Nq=1, Hq=blocks), dict(Nq=128 * blocks - 5, Hq=1), dict(Nq=300, Hq=blocks, per_block_mean=0)):
+        fake.fake_start(-1, 0)
+        assert _fwd(fake, _desc(**dict(dict(B=1, Hkv=1, Nk=128 * tiles, D=D), **kw))) == 0
+        assert [entry[1] for entry in _log(fake) if "quant_k_delta" in entry[1]][0].find(name) >= 0, kw
 
 
 def test_a_launch_of_too_many_blocks_is_refused():
