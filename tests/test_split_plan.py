@@ -8,6 +8,8 @@ import subprocess
 
 import pytest
 
+from tests import test_shared_tiles_gpu
+
 SLOTS = 160
 
 
@@ -96,3 +98,27 @@ def test_the_largest_plans_fit_their_fields(lib, causal):
             check(lib, causal, heads, nqt, 1 << 24, (1 << 24) - 128 * nqt, 128, sms)
     assert check(lib, causal, 200, 1, 1 << 24, (1 << 24) - 128, 128, 148)
     assert not check(lib, causal, 200, 1, 1 << 24, (1 << 24) - 128, 128, SLOTS + 1)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("H,group,Nq,Nk,causal,rounds", test_shared_tiles_gpu.CASES)
+def test_the_cases_run_on_the_gpu_are_what_they_claim(lib, D, H, group, Nq, Nk, causal, rounds):
+    whole, *_, first = plan(lib, causal, H, (Nq + 127) // 128, Nk, Nk - Nq, D)
+    assert (whole // 148 if first else None) == rounds
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_calls_alone_share_nothing_and_both_streams_do(lib, D):
+    """What the GPU tests compare with, and the problems that they run at the same time."""
+    for H, group, Nq, Nk, causal, rounds in test_shared_tiles_gpu.CASES:
+        assert not plan(lib, causal, 1, (Nq + 127) // 128, Nk, Nk - Nq, D)[-1]
+    assert plan(lib, True, 32, 8, 6000, 5000, D)[-1] and plan(lib, False, 100, 3, 3200, 2816, D)[-1]
+    assert plan(lib, True, 64, 8, 6000, 5000, D)[-1]          # two batch entries, in a workspace without room for it
+    # a part of one block behind a border, some of whose rows see none of its keys
+    *_, rest0, first = plan(lib, True, 48, 7, 4166, 3381, D)
+    tile = (C.c_int * 2)()
+    alone = 0
+    for j, lo in first:
+        lib.split_tile(1, j, 7, 48, 0, rest0, tile)
+        alone += 0 < lo == lib.split_blocks(1, tile[1], 4166, 3381) - 1
+    assert alone >= 3 and 3381 % 128 > 32
