@@ -51,6 +51,12 @@ void fake_start(int refuse, int pause_us) {
     g_attributes = 0;
 }
 const char* fake_log() { return g_log.c_str(); }
+const char* fake_kernels() {                      // every kernel of the library, one per line
+    static std::string names;
+    names.clear();
+    if (g_names) for (const auto& k : *g_names) names += k.second + "\n";
+    return names.c_str();
+}
 int fake_last_error() { return t_last; }
 int fake_attributes() { return g_attributes; }
 

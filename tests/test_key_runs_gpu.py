@@ -1,11 +1,15 @@
-"""The K kernel for up to 64 query blocks per kv head (D = 64: 128): its blocks walk runs of key tiles, two blocks per SM, a run going on into the next head.  Numbers of
-tiles around the blocks that are resident, query blocks around the 32 and 64 columns of an accumulator and the halves of them that a warp writes, ragged
-last tiles, tokens split over buffers: codes, scales, means and delta_s as the oracle forms them and as a call on one head alone gives them."""
+"""The K kernel whose blocks walk runs of key tiles, two blocks per SM, a run going on into the next head (up to 64 query blocks per kv head; D = 64: 128).  Numbers of
+tiles around the blocks that are resident, query blocks around the 32, 64 and 128 columns of an accumulator and the halves of them that a warp writes, ragged
+last tiles, tokens split over buffers: codes, scales, means and delta_s as a call on one head alone gives them, whose tiles have a block each, and as the oracle
+and 64-bit sums do."""
+import ctypes as C
+
 import pytest
 import torch
 
 from oracle import sage3_oracle as O
-from sageattention_b200 import Sage3Problem
+from sageattention_b200 import Sage3Problem, _cabi
+from tests._util import canon, deatomize_sf
 
 pytestmark = pytest.mark.gpu
 
@@ -25,6 +29,7 @@ def _workspace(p, B, Hkv):
     return km, codes, sf, delta
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("group,Nq,tiles,heads", [
     (1, 1, 37, 8),               # 296 tiles: one per block on 148 SMs
@@ -42,12 +47,12 @@ def _workspace(p, B, Hkv):
     (8, 128 * 16, 40, 10),       # 128
     (8, 1, 100, 40),             # 4 000 tiles
 ])
-def test_runs_of_key_tiles(cuda_device, D, group, Nq, tiles, heads):
+def test_runs_of_key_tiles(cuda_device, D, group, Nq, tiles, heads, dtype):
     g = torch.Generator(device=cuda_device).manual_seed(2000 + tiles + Nq)
     Nk = tiles * 128 - 37
-    k, v = (torch.randn(1, heads, Nk, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
-    q = torch.randn(1, heads * group, Nq, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
-    k += 2 * torch.randn(heads, 1, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
+    k, v = (torch.randn(1, heads, Nk, D, device=cuda_device, dtype=dtype, generator=g) for _ in range(2))
+    q = torch.randn(1, heads * group, Nq, D, device=cuda_device, dtype=dtype, generator=g)
+    k += 2 * torch.randn(heads, 1, D, device=cuda_device, dtype=dtype, generator=g)
     whole = Sage3Problem(q, k, v)
     whole.prepass()
     got = _workspace(whole, 1, heads)
@@ -56,14 +61,39 @@ def test_runs_of_key_tiles(cuda_device, D, group, Nq, tiles, heads):
         one.prepass()
         for name, a, b in zip(("mean", "codes", "scales", "delta_s"), got, _workspace(one, 1, 1)):
             assert torch.equal(a[h], b[0]), (name, h)
-    # delta_s against 64 bits: one rounding to bf16, and sums of D products in 32 bits that differ in order
+    # the tokens of K and V in two buffers that meet inside a tile
+    n, strides = (Nk + 1) // 2, (C.c_int64 * 3)
+    parts = []
+    cut = [[x[:, :, i * n:(i + 1) * n].contiguous() for i in range(2)] for x in (k, v)]
+    cut = [[torch.nn.functional.pad(x, (0, 0, 0, n - x.shape[2])) for x in pieces] for pieces in cut]
+    for pieces, rows in (([q], Nq), (cut[0], n), (cut[1], n)):
+        p = _cabi.Sage3Parts()
+        p.parts, p.rows_per_part = len(pieces), rows
+        for i, x in enumerate(pieces):
+            p.base[i] = x.data_ptr()
+        parts.append(p)
+    split = Sage3Problem(q, k, v)
+    split.ws.buf.fill_(255)
+    split.desc.k_stride = split.desc.v_stride = strides(heads * n * D, n * D, D)
+    assert _cabi.lib().sage3_prepass_parts(C.byref(split.desc), *map(C.byref, parts), split.ws.buf.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert split.check_status() == 0
+    for name, a, b in zip(("mean", "codes", "scales", "delta_s"), got, _workspace(split, 1, heads)):
+        assert torch.equal(a, b), name
+    # the mean within one rounding of the exact one; codes and scales of what it leaves are the oracle's
     h, nk_p = heads - 1, (Nk + 127) // 128 * 128
-    km = got[0][h].view(torch.bfloat16)
-    kp = (k[0, h].float() - km.float()).to(torch.bfloat16).double()
-    nqm = whole.ws.layout.nqm
-    qm = whole.ws.buf[whole.ws.layout.qm: whole.ws.layout.qm + heads * group * nqm * D * 2].view(torch.bfloat16).view(heads, group * nqm, D)[h].double()
+    km = got[0][h].view(dtype)
+    eps = torch.finfo(dtype).eps
+    mean = k[0, h].double().mean(0)
+    assert ((km.double() - mean).abs() <= eps * mean.abs() + 1e-6).all()
+    kp = (k[0, h].float() - km.float()).to(dtype)
+    codes, scales, _ = O.quant_microblocks(O.pad_rows(kp.cpu()))
+    assert torch.equal(canon(O.unpack_nibbles(got[1][h].cpu().view(nk_p, D // 2))), canon(codes))
+    assert torch.equal(deatomize_sf(got[2][h].cpu(), 1, nk_p // 128, D // 64)[0], scales)
+    # delta_s against 64 bits: one rounding to 16, and sums of D products in 32 bits that differ in order
+    kp, nqm = kp.double(), whole.ws.layout.nqm
+    qm = whole.ws.buf[whole.ws.layout.qm: whole.ws.layout.qm + heads * group * nqm * D * 2].view(dtype).view(heads, group * nqm, D)[h].double()
     exact = qm @ kp.T
-    mine = got[3][h].view(torch.bfloat16).view(group * nqm, nk_p)
+    mine = got[3][h].view(dtype).view(group * nqm, nk_p)
     assert (mine[:, Nk:] == 0).all()
-    bound = exact.abs() * 2.0 ** -8 + (qm.abs() @ kp.abs().T) * D * 2.0 ** -24
+    bound = exact.abs() * eps + (qm.abs() @ kp.abs().T) * D * 2.0 ** -24
     assert ((mine[:, :Nk].double() - exact).abs() <= bound).all()

@@ -27,7 +27,7 @@ def fake(tmp_path_factory):
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", f"-isystem{cuda / 'include'}",
                            str(pathlib.Path(__file__).with_name("fake_cudart.cpp")), *map(str, objs), "-o", str(so), "-lpthread"])
     lib = C.CDLL(str(so))
-    lib.fake_log.restype = C.c_char_p
+    lib.fake_log.restype = lib.fake_kernels.restype = C.c_char_p
     return lib
 
 
@@ -129,11 +129,14 @@ def test_attention_on_its_own_is_one_memset_and_one_kernel(fake, call, kw):
 
 
 def test_shared_memory_is_asked_for_once_per_kernel(fake):
-    """Calls that between them launch every attention and every K kernel: in a second round no kernel's attributes are set again (that is a call into the
+    """Calls that between them launch every attention and every K kernel of the library: in a second round no kernel's attributes are set again (that is a call into the
     runtime for every launch, paid by the shortest calls)."""
-    full = [dict(Nk=700), dict(Nk=3000), dict(Nq=128 * 33)]                                # whole tiles; many query blocks
+    full = [dict(Nk=700), dict(Nk=3000), dict(Nq=128 * 33),                                # whole tiles; many query blocks
+            dict(Hq=32, Nq=1000, Nk=9192),                                                 # tiles shared
+            dict(Hq=2, Hkv=1, Nq=128 * 17, Nk=60000), dict(Hq=4, Hkv=1, Nq=128 * 17, Nk=60000)]      # 34 and 68 query blocks over many key tiles
     few = [dict(Nq=16, Hq=16), dict(Nq=1, Hq=8), dict(Nq=1, Hq=66, Hkv=1),                 # heads that share a tile, of 8, 4 and 66 query blocks
-           dict(B=8, Nq=1, Hq=32, Hkv=8, Nk=20000), dict(B=8, Nq=1, Hq=8, Hkv=8, Nk=20000)]      # many key tiles
+           dict(B=8, Nq=1, Hq=32, Hkv=8, Nk=20000), dict(B=8, Nq=1, Hq=8, Hkv=8, Nk=20000),      # many key tiles
+           dict(Nq=1, Hq=33, Hkv=1, Nk=60000), dict(Nq=1, Hq=66, Hkv=1, Nk=60000)]
     kernels = set()
     for _ in range(2):
         fake.fake_start(-1, 0)
@@ -144,7 +147,8 @@ def test_shared_memory_is_asked_for_once_per_kernel(fake):
                     assert [_fwd(fake, _desc(**kw, **c)) for c in full + few] == [0] * (len(full) + len(few))
                     assert [f(fake, _desc(**kw, Nk=n)) for f in (_varlen, _carried) for n in (700, 3000, 9000)] == [0] * 6
         kernels |= {entry[1] for entry in _log(fake) if "attn_fwd" in entry[1] or "quant_k_delta" in entry[1]}
-    assert len(kernels) >= 66 and fake.fake_attributes() == 0
+    assert kernels == {k for k in fake.fake_kernels().decode().split() if "attn_fwd" in k or "quant_k_delta" in k} and len(kernels) == 88
+    assert fake.fake_attributes() == 0
 
 
 @pytest.mark.parametrize("call,Nk,causal,D,rolled", [(_fwd, 1024, 0, 64, 1), (_fwd, 1025, 0, 64, 0), (_fwd, 9000, 1, 64, 1), (_fwd, 9000, 0, 128, 1),

@@ -40,9 +40,9 @@ def test_split_tensors_equal_the_contiguous_call(cuda_device, B, Hq, Hkv, n, P, 
 
 
 @pytest.mark.parametrize("D", [64, 128])
-def test_split_keys_in_turn_equal_the_contiguous_call(cuda_device, D):
-    """Few query blocks and many key tiles, the tokens of K and V in two buffers that meet inside a tile: a block of the K kernel takes several tiles in
-    turn, from both buffers."""
+def test_split_keys_in_runs_equal_the_contiguous_call(cuda_device, D):
+    """Few query blocks and many key tiles, the tokens of K and V in two buffers that meet inside a tile: a block of the K kernel walks a run of tiles
+    from both buffers, on into the next head."""
     H, Nq, n = 40, 64, 6475
     q, k, v = (t.to(cuda_device) for t in O.make_inputs(1, H, H, Nq, 2 * n, D, seed=65, k_offset_std=1.0))
     ref = sageattn3(q, k, v)

@@ -117,10 +117,9 @@ def test_packed_batch_around_the_length_that_unrolls(cuda_device, longest):
 
 
 @pytest.mark.parametrize("D,tiles,kv_heads", [(128, 101, 40), (128, 100, 40), (64, 76, 40), (64, 77, 40), (64, 78, 40)])
-def test_key_tiles_in_turn(cuda_device, D, tiles, kv_heads):
-    """Few query blocks and many key tiles: a block of the K kernel takes two (D = 64: three) tiles one after the other.  Numbers of tiles that it
-    divides and does not, a ragged last tile: the same bits as with two kv heads, where every tile has a block of its own.  One head
-    has a key that is not finite in a block's second tile: it stays there."""
+def test_key_tiles_in_runs(cuda_device, D, tiles, kv_heads):
+    """Few query blocks and many key tiles: a block of the K kernel walks a run of tiles that ends and begins inside heads, with a ragged last tile: the same
+    bits as with one kv head, where every tile has a block of its own.  One head has a key that is not finite in its second tile: it stays there."""
     g = torch.Generator(device=cuda_device).manual_seed(1500 + tiles)
     Nk, group = tiles * 128 - 5, 4
     k, v = (torch.randn(1, kv_heads, Nk, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
@@ -129,16 +128,16 @@ def test_key_tiles_in_turn(cuda_device, D, tiles, kv_heads):
         if bad:
             k[0, 5, 130] = float("nan")
         out = sageattn3(q, k, v, is_causal=True)
-        for h in (0, 5, kv_heads - 2):
-            few = sageattn3(q[:, h * group:(h + 2) * group], k[:, h:h + 2], v[:, h:h + 2], is_causal=True)
-            assert torch.equal(out[:, h * group:(h + 2) * group].nan_to_num(7.0), few.nan_to_num(7.0)), (h, bad)
+        for h in (0, 1, 5, 6, kv_heads - 2, kv_heads - 1):
+            few = sageattn3(q[:, h * group:(h + 1) * group], k[:, h:h + 1], v[:, h:h + 1], is_causal=True)
+            assert torch.equal(out[:, h * group:(h + 1) * group].nan_to_num(7.0), few.nan_to_num(7.0)), (h, bad)
         assert torch.isfinite(out[:, 6 * group:]).all() and torch.isfinite(out[:, :5 * group]).all()
 
 
 @pytest.mark.parametrize("D,N,causal", [(128, 5120, False), (64, 3790, True)])
-def test_key_tiles_in_turn_with_one_mean_per_head(cuda_device, D, N, causal):
-    """One Q mean per head: the K kernel sees one query block per head, however many queries, and takes tiles in turn here too.  The same bits as with
-    two kv heads, where every tile has a block of its own."""
+def test_key_tiles_in_runs_with_one_mean_per_head(cuda_device, D, N, causal):
+    """One Q mean per head: the K kernel sees one query block per head, however many queries, and walks runs of tiles here too.  The same bits as with
+    two kv heads, where every tile (80 or 60 of them) has a block of its own."""
     Hkv, group = 100, 2
     g = torch.Generator(device=cuda_device).manual_seed(1600 + N)
     k, v = (torch.randn(1, Hkv, N, D, device=cuda_device, dtype=torch.float16, generator=g) for _ in range(2))
@@ -151,9 +150,9 @@ def test_key_tiles_in_turn_with_one_mean_per_head(cuda_device, D, N, causal):
 
 @pytest.mark.parametrize("pbm", [True, False])
 @pytest.mark.parametrize("D", [64, 128])
-def test_key_tiles_in_turn_in_a_packed_batch(cuda_device, D, pbm):
-    """A packed batch whose sequences end in a block's first tile, in one of its later tiles or between blocks, or have no keys: every sequence as it is
-    alone, where every tile has a block of its own."""
+def test_key_tiles_in_runs_in_a_packed_batch(cuda_device, D, pbm):
+    """A packed batch whose sequences end in a run's first tile, in one of its later tiles or between runs, or have no keys: every sequence as it is
+    alone, and a head of it, where every tile has a block of its own."""
     Hkv, group, longest = 8, 2, 51 * 128
     lens = [longest, 1, 127, 128, 129, 0, 255, 256, 257, 384, 385, 640, 6000 + 13]
     n_q = [1, 3, 1, 1, 2, 1, 1, 5, 1, 1, 1, 1, 60]
@@ -162,7 +161,7 @@ def test_key_tiles_in_turn_in_a_packed_batch(cuda_device, D, pbm):
     q = torch.randn(sum(n_q), Hkv * group, D, device=cuda_device, dtype=torch.bfloat16, generator=g)
     k, v = (torch.randn(sum(lens), Hkv, D, device=cuda_device, dtype=torch.bfloat16, generator=g) for _ in range(2))
     cu_q, cu_k = (torch.tensor([0] + n).cumsum(0).to(device=cuda_device, dtype=torch.int32) for n in (n_q, lens))
-    assert B * Hkv * (longest // 128) >= 27 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    assert B * Hkv * (longest // 128) >= 3 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
     out = sageattn_varlen(q, k, v, cu_q, cu_k, max(n_q), longest, per_block_mean=pbm)
     q0 = k0 = 0
     for i, (m, n) in enumerate(zip(n_q, lens)):
@@ -171,4 +170,7 @@ def test_key_tiles_in_turn_in_a_packed_batch(cuda_device, D, pbm):
             assert (mine == 0).all(), i
         else:
             assert torch.equal(mine, sageattn3(q[None, q0:q0 + m], k[None, k0:k0 + n], v[None, k0:k0 + n], tensor_layout="NHD", per_block_mean=pbm)[0]), i
+            for h in (0, Hkv - 1):
+                one = (q[None, q0:q0 + m, h * group:(h + 1) * group], k[None, k0:k0 + n, h:h + 1], v[None, k0:k0 + n, h:h + 1])
+                assert torch.equal(mine[:, h * group:(h + 1) * group], sageattn3(*one, tensor_layout="NHD", per_block_mean=pbm)[0]), (i, h)
         q0, k0 = q0 + m, k0 + n
