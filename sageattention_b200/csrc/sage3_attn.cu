@@ -1360,12 +1360,8 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     if (e != cudaSuccess) return e;
     const int sms = info.sms;
     SplitParams p;
-    // Units of work: pairs of query tiles; when the last round of pairs fills at most half of the SMs it is dealt out as
-    // single tiles (half the time for the round, twice the SMs).  With more than that single tiles need two rounds and lose the shared
-    // K and V stages.  148 SMs, heads x 2 048 tokens, D = 128, never / this rule / always single: 68 pairs over 81.8 / 71.8 / 71.7 us,
-    // 76 over 82.8 / 82.8 / 85.9 us, 140 over 87.5 / 87.4 / 92.9 us.
-    const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), rest = pairs % sms;
-    const bool split = nqt > 1 && 2 * rest <= sms;
+    // Units of work: pairs of query tiles; in the last rounds single tiles or slots of key blocks.
+    const int nqt = a.Nq_p / kBlock, pairs = a.B * a.Hq * ((nqt + 1) / 2), whole = whole_pairs(nqt, pairs, sms);
     p.unit_counter = a.unit_counter;
     SplitPlan plan;
     if (a.split_flags != nullptr && mode == 0 && a.cu_q == nullptr && a.carry_o_in == nullptr && a.carry_o_out == nullptr)
@@ -1373,10 +1369,10 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.slot_blocks = plan.blocks; p.slot_rest = plan.rest; p.rest0 = plan.rest0;
     p.split_flags = a.split_flags; p.split_state = a.split_state;
     for (int i = 0; i < plan.slots; ++i) p.slot_first[i] = plan.first[i];
-    p.whole_units = plan.slots > 0 ? plan.whole : split ? pairs - rest : pairs;
+    p.whole_units = plan.slots > 0 ? plan.whole : whole;
     p.pack_heads = pack;
     p.pack_tiles = (group + pack - 1) / pack;
-    p.units = mode ? a.B * a.Hkv * p.pack_tiles : plan.slots > 0 ? plan.whole + plan.slots : split ? pairs + rest : pairs;
+    p.units = mode ? a.B * a.Hkv * p.pack_tiles : plan.slots > 0 ? plan.whole + plan.slots : 2 * pairs - whole;
     const int grid = p.units < sms ? p.units : sms;
     p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;

@@ -13,6 +13,7 @@ void split_tile(int causal, int j, int nqt, int BHq, int whole, int rest0, int* 
     if (causal) sage3::rest_tile<true>(j, nqt, BHq, whole, rest0, out[0], out[1]);
     else sage3::rest_tile<false>(j, nqt, BHq, whole, rest0, out[0], out[1]);
 }
+int split_walk(int causal, int BHq, int nqt, int sms) { return causal ? sage3::longest_walk<true>(BHq, nqt, sms) : sage3::longest_walk<false>(BHq, nqt, sms); }
 int split_blocks(int causal, int mt, int Nk, int shift) {
     return causal ? sage3::tile_blocks<true>(mt, Nk, shift) : sage3::tile_blocks<false>(mt, Nk, shift);
 }

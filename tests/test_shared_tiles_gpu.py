@@ -21,8 +21,9 @@ CASES = [
     (160, 1, 100, 5000, False, 0),        # one tile per head, a round and twelve
     (230, 1, 90, 4000, False, 0),         # ... and more than half a round
     (149, 1, 130, 2100, False, 0),        # a round and one pair: both rounds are dealt out
-    (100, 4, 384, 2500, False, None),     # odd: every other pair is one tile; gains less than ten blocks
-    (100, 4, 384, 3200, False, 0),        # ... more
+    (100, 4, 384, 2500, False, 0),        # odd: every other pair is one tile
+    (100, 4, 384, 3200, False, 0),
+    (49, 1, 330, 2100, False, 0),         # fewer tiles than SMs, in more pairs than half of these: a slot per tile
     (37, 1, 640, 3000, False, 0),         # 111 pairs, five tiles per head
     (300, 2, 129, 2048, False, 1),        # two rounds and four
     (60, 1, 1152, 4000, False, 1),        # odd, a whole round ahead: the last tiles of all heads come first

@@ -100,6 +100,42 @@ def test_the_largest_plans_fit_their_fields(lib, causal):
     assert not check(lib, causal, 200, 1, 1 << 24, (1 << 24) - 128, 128, SLOTS + 1)
 
 
+def walk(causal, heads, nqt, sms):
+    """SM by SM: what the one that ends last walks, in tiles, where each draws its next unit when it begins one, those with two tiles first."""
+    npair = (nqt + 1) // 2
+    pairs = [2 if nqt % 2 == 0 or (p >= heads if causal else p % npair != npair - 1) else 1 for p in range(heads * npair)]
+    rest = len(pairs) % sms
+    whole = len(pairs) - rest if nqt > 1 and 2 * rest <= sms else len(pairs)
+    units = pairs[:whole] + [1] * sum(pairs[whole:])
+    queue = iter(units[sms:])
+    ends = {}                                                   # time -> units drawn by the SMs that end one then
+    for u in sorted(units[:sms], reverse=True):
+        ends.setdefault(u, []).append(next(queue, 0))
+    t = last = 0
+    while ends:
+        t += 1
+        for u in sorted(ends.pop(t, []), reverse=True):
+            last = t
+            if u:
+                ends.setdefault(t + u, []).append(next(queue, 0))
+    return last
+
+
+def test_the_walk_without_slots(lib):
+    r = random.Random(9)
+    for _ in range(3000):
+        sms, nqt = r.choice((148, 148, 132, 1, 2, 7, 31)), int(1.6 ** r.uniform(0, 9))
+        heads, causal = max(1, int(r.uniform(0.3, 12) * sms / nqt)), r.random() < 0.5
+        assert lib.split_walk(int(causal), heads, nqt, sms) == walk(causal, heads, nqt, sms), (causal, heads, nqt, sms)
+
+
+@pytest.mark.parametrize("heads,N,D,shared", [(12, 2830, 64, False), (28, 3143, 64, False), (24, 3604, 128, True), (28, 3926, 128, False), (28, 3143, 128, False),      # odd numbers of tiles
+                                              (5, 7547, 128, True), (6, 6245, 128, True), (3, 6272, 128, True), (6, 8997, 64, False), (5, 16384, 128, True), (24, 16384, 128, False),
+                                              (64, 6979, 128, True), (24, 119056, 128, True), (32, 8192, 128, False)])
+def test_slots_where_they_save_more_than_they_cost(lib, heads, N, D, shared):
+    assert bool(plan(lib, False, heads, (N + 127) // 128, N, 0, D)[-1]) == shared
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("H,group,Nq,Nk,causal,rounds", test_shared_tiles_gpu.CASES)
 def test_the_cases_run_on_the_gpu_are_what_they_claim(lib, D, H, group, Nq, Nk, causal, rounds):
