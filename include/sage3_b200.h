@@ -47,7 +47,7 @@ enum {
 enum { SAGE3_FP16 = 0, SAGE3_BF16 = 1 };
 
 /*
- * Sage3Desc.reserved: leaves the flags and accumulators of shared query tiles out of the workspace (some 11 MB at D = 128, 5.6 MB at D = 64, of a problem
+ * Sage3Desc.reserved: leaves the flags and accumulators of shared query tiles out of the workspace (some 11 MB at D = 128, 5.5 MB at D = 64, of a problem
  * of more than 32 queries and 2 048 padded keys or more).  The same results; a call whose last rounds of work do not fill the GPU takes longer.  For a
  * workspace of fixed size, and for packed batches and carried state, which share no tiles in any case.
  */

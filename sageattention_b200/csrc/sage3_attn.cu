@@ -1372,7 +1372,7 @@ cudaError_t launch_attn(const AttnArgs& a, cudaStream_t st, int* driver_rc) {
     p.whole_units = plan.slots > 0 ? plan.whole : whole;
     p.pack_heads = pack;
     p.pack_tiles = (group + pack - 1) / pack;
-    p.units = mode ? a.B * a.Hkv * p.pack_tiles : plan.slots > 0 ? plan.whole + plan.slots : 2 * pairs - whole;
+    p.units = mode ? a.B * a.Hkv * p.pack_tiles : plan.slots > 0 ? plan.whole + plan.slots : whole + 2 * (pairs - whole);
     const int grid = p.units < sms ? p.units : sms;
     p.BHq = a.B * a.Hq;
     p.Hq = a.Hq; p.Hkv = a.Hkv; p.Nq = a.Nq; p.Nk = a.Nk;

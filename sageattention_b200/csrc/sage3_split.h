@@ -88,7 +88,7 @@ template <bool CAUSAL>
 inline int longest_walk(int BHq, int nqt, int sms) {
     const int npair = (nqt + 1) / 2, pairs = BHq * npair, whole = whole_pairs(nqt, pairs, sms);
     auto singles = [&](int n) { return nqt % 2 == 0 ? 0 : !CAUSAL ? n / npair : n < BHq ? n : BHq; };      // among the first n pairs
-    const int units = 2 * pairs - whole - singles(pairs) + singles(whole);
+    const int units = whole + 2 * (pairs - whole) - (singles(pairs) - singles(whole));
     int next = 0;
     struct Count { int none, one, two; };
     auto draw = [&](int n) {

@@ -179,12 +179,12 @@ def test_scale_of_every_microblock_maximum(cuda_device, dtype):
 
 @pytest.mark.parametrize("what", ["k_nan", "q_inf", "delta_overflow"])
 @pytest.mark.parametrize("Nq,Hq,Hkv,D", [(1, 32, 8, 128), (1, 4, 4, 64), (9, 14, 2, 128), (40, 6, 2, 64), (4, 18, 2, 128), (2, 32, 4, 64),
-                                              (1, 400, 200, 64)])
+                                              (1, 400, 200, 64), (1, 1000, 500, 64)])
 def test_non_finite_values_stay_with_their_head(cuda_device, Nq, Hq, Hkv, D, what):
     """Heads that share a tile share the operand that adds delta_s, where 0 x NaN and 0 x Inf are NaN.  One query head, or one kv
     head, of sequence 1 is not finite (a NaN key, an Inf query, an fp16 delta_s that overflows): sequence 0 and the other heads
     get the bits of a call without it, and the head itself what the packed variable-length path, one head per tile, gives it.
-    (400 kv heads: more notes than one block clears.)"""
+    (400 kv heads: more notes than a block has threads; 1 000: more than one block clears.)"""
     dtype = torch.float16 if what == "delta_overflow" else torch.bfloat16
     Nk, B, g = 400, 2, Hq // Hkv
     q, k, v = _inputs(cuda_device, B, Hq, Hkv, Nq, Nk, D, seed=1300 + Nq + Hq, dtype=dtype)
